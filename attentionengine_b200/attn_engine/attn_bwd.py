@@ -17,6 +17,7 @@ shape, 4 % at head dim 128 and 16 % at head dim 64).
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 from dataclasses import dataclass
 
@@ -176,10 +177,14 @@ def batch_ranges(B: int, ctas_per_batch_row: int, sms: int, want: int, min_round
     return 1
 
 
+@functools.lru_cache(maxsize=None)
+def sm_count(dev) -> int:
+    return torch.cuda.get_device_properties(dev).multi_processor_count
+
+
 def _batch_parts(B, Hq, Sq, dev):
     want = int(os.environ.get("AE_B200_BWD_PARTS", BWD_PARTS))
-    sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    return batch_ranges(B, Hq * ((Sq + 127) // 128), sms, want, min_rounds=8)
+    return batch_ranges(B, Hq * ((Sq + 127) // 128), sm_count(dev), want, min_rounds=8)
 
 
 def _side_streams(eng, dev, n):

@@ -21,8 +21,6 @@ positions.
 """
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
 
 from .. import runtime as rt
@@ -79,7 +77,8 @@ class AttnDecode:
                 self.combine = rt.compile_module(self.combine_src, "ae_mla_combine", cfg2)
         self.num_split = None  # None = choose per call
         self.last_num_split = None
-        self._status = None
+        self._plan = None  # the native side, made at the first call
+        self._splits = {}  # (batch rows, kv tiles) -> split count
 
     def pick_splits(self, B: int, Skv: int) -> int:
         """Split count that minimises waves x (kv tiles per split + 3): a CTA occupies an SM alone, so the CTAs run in
@@ -88,8 +87,10 @@ class AttnDecode:
         state but no combine of its own."""
         if self.combine is None:
             return 1
-        units = B * (self.Hkv if self.Hq > self.Hkv else self.Hq)
         n_tiles = -(-Skv // 128)
+        if (B, n_tiles) in self._splits:
+            return self._splits[B, n_tiles]
+        units = B * (self.Hkv if self.Hq > self.Hkv else self.Hq)
         best, best_cost = 1, None
         for n in range(1, min(32, n_tiles) + 1):
             tps = -(-n_tiles // n)
@@ -98,6 +99,9 @@ class AttnDecode:
             cost = -(-units * n // N_SM) * (tps + 3)
             if best_cost is None or cost < best_cost:
                 best, best_cost = n, cost
+        if len(self._splits) >= 4096:  # a serving loop over many batch sizes and lengths must not grow without bound
+            self._splits.clear()
+        self._splits[B, n_tiles] = best
         return best
 
     # ------------------------------------------------------------------------------------------------------
@@ -146,7 +150,33 @@ class AttnDecode:
     def __call__(self, q, k, v, *custom):
         return self._run(q, k, v, custom, None, None)
 
+    def _native_plan(self):
+        if self._plan is None:
+            from .attn_engine import custom_slots
+            self._plan = rt.host().DecodePlan(self.kernel.handle.value, self.combine.handle.value if self.combine else 0,
+                                              self.dtype == torch.bfloat16, self.Hq, self.Hkv, self.Sq, self.D, self.DV,
+                                              len(self.low.final_names), custom_slots(self.low.custom))
+        return self._plan
+
+    @property
+    def status(self):
+        return self._plan.status if self._plan is not None else None
+
     def _run(self, q, k, v, custom, meta, block_table):
+        if meta is None:
+            n_split = self.num_split or self.pick_splits(q.shape[0], k.shape[1])
+            m = None
+        else:
+            n_split = 1
+            m = (meta["work"], meta["n_items"], meta["seqlens"], meta["part_off"], meta["n_slots"], meta["max_seqlen"], meta["B"])
+        o = rt.host().decode(self._plan or self._native_plan(), q, k, v, custom, n_split, m, block_table)
+        if o is None:
+            self._refuse(q, k, v, custom, meta, block_table, n_split)
+        self.last_num_split = n_split if meta is None else meta["n_slots"] / q.shape[0]
+        return o
+
+    def _refuse(self, q, k, v, custom, meta, block_table, n_split):
+        """The native path did not take these tensors: raise what is wrong with them."""
         for name, t in (("q", q), ("k", k), ("v", v)):
             if not t.is_cuda:
                 raise rt.AeError(f"{name} must be a CUDA tensor: this back end has no CPU path")
@@ -173,47 +203,11 @@ class AttnDecode:
         specs = self.low.custom
         if len(custom) != len(specs):
             raise TypeError(f"expected {len(specs)} custom input(s) {[s.name for s in specs]}, got {len(custom)}")
-        dev = q.device
-        n_split = 1 if meta is not None else (self.num_split or self.pick_splits(B, Skv))
         if n_split > 1 and self.combine is None:
             raise ValueError("more than one split needs OnlineFunc.combine")
-        o = torch.empty(B, Sq, Hq, self.DV, dtype=self.dtype, device=dev)
-        p = rt.DecodeParams()
-        p.q, p.k, p.v, p.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr()
-        for name, t in (("q_stride", q), ("k_stride", k), ("v_stride", v)):
-            setattr(p, name, (C.c_int64 * 3)(t.stride(0), t.stride(1), t.stride(2)))
-        keep = []
         for sp, t in zip(specs, custom):
             if sp.is_16bit:
                 raise NotImplementedError("tile-shaped custom inputs are not wired into the decode kernel")
-            t = t.to(torch.float32)
-            keep.append(t)
-            p.custom[sp.slot] = t.data_ptr()
-            for d, slot in enumerate(sp.dim_slots):
-                if slot >= 0 and t.shape[d] > 1:
-                    p.custom_stride[sp.slot][slot] = t.stride(d)
-        n_slots = meta["n_slots"] if meta is not None else (B * n_split if n_split > 1 else 0)
-        if n_slots:
-            part = torch.empty(n_slots, Sq * Hq, self.DV, dtype=torch.float32, device=dev)
-            p.o_partial = part.data_ptr()
-            keep.append(part)
-            for i in range(len(self.low.final_names)):
-                f = torch.empty(n_slots, Sq * Hq, dtype=torch.float32, device=dev)
-                p.rowscale_partial[i] = f.data_ptr()
-                keep.append(f)
-        p.B, p.Hq, p.Hkv, p.Sq, p.Skv, p.n_split = B, Hq, Hkv, Sq, Skv, n_split
-        if meta is not None:
-            p.work, p.n_items = meta["work"].data_ptr(), meta["n_items"]
-            p.seqlens, p.part_off = meta["seqlens"].data_ptr(), meta["part_off"].data_ptr()
-            p.Skv = meta["max_seqlen"]
-            if block_table is not None:
-                p.block_table, p.max_pages, p.num_pages = block_table.data_ptr(), block_table.shape[1], k.shape[0]
-        if self._status is None or self._status.device != dev:
-            self._status = torch.zeros(1, dtype=torch.int32, device=dev)
-        p.status = self._status.data_ptr()
-        stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-        rt.check(rt.lib().ae_launch_attn_decode(self.kernel.handle, C.byref(p), stream), "ae_launch_attn_decode")
-        if n_split > 1 or (meta is not None and meta["n_slots"] > B):
-            rt.check(rt.lib().ae_launch_decode_combine(self.combine.handle, C.byref(p), stream), "ae_launch_decode_combine")
-        self.last_num_split = n_split if meta is None else meta["n_slots"] / B
-        return o
+            if not t.is_cuda:
+                raise rt.AeError("custom inputs must be CUDA tensors: this back end has no CPU path")
+        raise ValueError("tensors do not fit this engine")

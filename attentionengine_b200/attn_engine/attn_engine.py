@@ -18,6 +18,7 @@ import torch
 from .. import runtime as rt
 from ..core.transform.core import (CustomIO, SymbolicArray, SymbolScalar, Var, block_mask_counts)
 from ..lower.cuda_lower import LoweredAttention, lower_attention
+from . import attn_bwd
 
 
 class OnlineFunc:
@@ -68,11 +69,6 @@ _DYN_PROBE = 1024  # sequence length on which a dynamic-shape engine classifies 
 MAX_LIST_KV_TILES = 2048  # kv tiles a block list may cover (AE_MAX_KT of attn_fwd.cuh): 262,144 keys
 
 _TORCH_DTYPES = {torch.float16: rt.DTYPE_F16, torch.bfloat16: rt.DTYPE_BF16}
-
-
-def _strides3(t: torch.Tensor):
-    # [B, S, H, D] -> (batch, seq, head) element strides
-    return (C.c_int64 * 3)(t.stride(0), t.stride(1), t.stride(2))
 
 
 def _block_lists(cnt: torch.Tensor, q_blk: int, kv_blk: int, Sq: int, Skv: int, B: int, H: int, device):
@@ -163,29 +159,9 @@ class _AttnKernels:
         return self._bwd_fused
 
 
-class _AttentionFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, eng, q, k, v, *custom):
-        eng._check_qkv(q, k, v)
-        with torch.cuda.device(q.device):  # the C ABI launches on the current device's context
-            o, finals, lists = eng._launch_fwd(q, k, v, custom, block_mask=eng._call_block_mask, return_lists=True)
-        ctx.eng = eng
-        ctx.lists = lists  # the tile lists this forward walked: its backward walks the same ones
-        ctx.n_custom = len(custom)
-        ctx.save_for_backward(q, k, v, o, *finals, *custom)
-        ctx.n_final = len(finals)
-        return o
-
-    @staticmethod
-    def backward(ctx, d_o):
-        eng = ctx.eng
-        saved = ctx.saved_tensors
-        q, k, v, o = saved[:4]
-        finals = saved[4:4 + ctx.n_final]
-        custom = saved[4 + ctx.n_final:]
-        with torch.cuda.device(q.device):
-            dq, dk, dv = eng._launch_bwd(q, k, v, o, d_o, finals, custom, ctx.lists)
-        return (None, dq, dk, dv) + (None,) * ctx.n_custom
+def custom_slots(specs) -> list:
+    """What the native host path needs of the custom inputs: (slot, 16-bit tile?, index slot of every dim)."""
+    return [(sp.slot, bool(sp.is_16bit), [int(d) for d in sp.dim_slots]) for sp in specs]
 
 
 class AttentionEngine:
@@ -210,9 +186,8 @@ class AttentionEngine:
         self.extern_block_mask = extern_block_mask
         self.bwd_mode = None  # "fused" | "split"; None = the package default (attn_bwd.DEFAULT_MODE)
         self.block_mask = None
-        self._call_block_mask = None
         self._lists = None
-        self._status = None
+        self._plan = None  # the native side of this engine, made at its first call
         dynamic = any(isinstance(x, str) for x in (B, Hq, Sq, Skv))
         self._dynamic = dynamic
         self._lists_by_shape = {}
@@ -302,6 +277,36 @@ class AttentionEngine:
         self.tl_code = self.kernels.fwd_src  # name kept from the reference (attn_engine.py:365): generated source
 
     # ------------------------------------------------------------------------------------------
+    def _native_plan(self):
+        if self._plan is None:
+            k, low = self.kernels, self.lowered
+            self._plan = rt.host().AttnPlan(k.fwd.handle.value, self.dtype == torch.bfloat16, self.D, self.DV,
+                                            len(low.final_names), bool(low.uses_doosum), custom_slots(low.custom))
+        return self._plan
+
+    def _native_bwd(self, B, Hq, Sq, device_index):
+        """Called by the autograd node: True when the backward is the one-pass form as one launch, which the node issues
+        itself; False: it goes through ``_launch_bwd``."""
+        if (self.bwd_mode or attn_bwd.DEFAULT_MODE) != "fused" or attn_bwd._batch_parts(B, Hq, Sq, device_index) > 1:
+            return False
+        plan = self._plan
+        if not plan.fused:
+            k = self.kernels.bwd_fused
+            plan.prep, plan.cast, plan.fused = k.prep.handle.value, k.cast.handle.value, k.fused.handle.value
+        return True
+
+    @property
+    def _status(self):
+        part = self._mla or self._decode
+        if part is not None:
+            return part.status
+        return self._plan.status if self._plan is not None else None
+
+    @_status.setter
+    def _status(self, t):
+        if self._mla is None and self._decode is None:
+            self._native_plan().status = t
+
     def _get_status(self, device):
         if self._status is None or self._status.device != device:
             self._status = torch.zeros(1, dtype=torch.int32, device=device)
@@ -309,14 +314,11 @@ class AttentionEngine:
 
     def check_status(self):
         """Raise if a kernel of this engine recorded a bounded-wait timeout."""
-        if self._mla is not None:
-            self._status = self._mla._status
-        if self._decode is not None:
-            self._status = self._decode._status
-        if self._status is not None:
-            code = int(self._status.item())
+        status = self._status
+        if status is not None:
+            code = int(status.item())
             if code:
-                self._status.zero_()
+                status.zero_()
                 raise rt.AeError(f"kernel reported status 0x{code:x} (a bounded wait gave up)")
 
     def _ensure_lists(self, device, block_mask: Optional[torch.Tensor], B, Hq, Sq, Skv):
@@ -393,27 +395,32 @@ class AttentionEngine:
             raise ValueError("inconsistent q/k/v shapes")
         return B, Sq, Hq, Skv, Hkv
 
-    def _launch_fwd(self, q, k, v, custom, block_mask=None, return_lists=False):
-        B, Sq, Hq, Skv, Hkv = self._check_qkv(q, k, v)
-        dev = q.device
-        o = torch.empty(B, Sq, Hq, self.DV, dtype=self.dtype, device=dev)
-        finals = [torch.empty(B, Hq, Sq, dtype=torch.float32, device=dev) for _ in self.lowered.final_names]
-        p = rt.AttnParams()
-        p.q, p.k, p.v, p.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr()
-        p.q_stride, p.k_stride, p.v_stride, p.o_stride = _strides3(q), _strides3(k), _strides3(v), _strides3(o)
-        for i, f in enumerate(finals):
-            p.final_rowscales[i] = f.data_ptr()
-        p.custom, p.custom_stride, keep = self._custom_args(custom, Sq, Skv)
-        lists = self._ensure_lists(dev, block_mask if block_mask is not None else (
+    def _tile_lists(self, q, k, v, block_mask):
+        if self.mask_mode != 2:
+            return None
+        B, Sq, Hq, Skv, _ = self._check_qkv(q, k, v)
+        return self._ensure_lists(q.device, block_mask if block_mask is not None else (
             self.block_mask if self.extern_block_mask else None), B, Hq, Sq, Skv)
-        if lists is not None:
-            p.block_count, p.block_index = lists[0].data_ptr(), lists[1].data_ptr()
-        p.B, p.Hq, p.Hkv, p.Sq, p.Skv = B, Hq, Hkv, Sq, Skv
-        p.status = self._get_status(dev).data_ptr()
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        rt.check(rt.lib().ae_launch_attn_fwd(self.kernels.fwd.handle, C.byref(p), C.c_void_p(stream)),
-                 "ae_launch_attn_fwd")
-        return (o, finals, lists) if return_lists else (o, finals)
+
+    def _refuse(self, q, k, v, custom):
+        """The native path did not take these tensors: raise what is wrong with them."""
+        _, Sq, _, Skv, _ = self._check_qkv(q, k, v)
+        for t in custom:
+            if not t.is_cuda:
+                raise rt.AeError("custom inputs must be CUDA tensors: this back end has no CPU path")
+        self._custom_args(custom, Sq, Skv)
+        raise ValueError("tensors do not fit this engine")
+
+    def _launch_fwd(self, q, k, v, custom, block_mask=None):
+        """Forward without autograd: (o, [final row scales])."""
+        lists = self._tile_lists(q, k, v, block_mask)
+        res = rt.host().attn(self._native_plan(), self, q, k, v, custom, lists, True)
+        return res if res is not None else self._refuse(q, k, v, custom)
+
+    def _apply(self, q, k, v, custom, block_mask):
+        lists = self._tile_lists(q, k, v, block_mask) if self.mask_mode == 2 else None
+        o = rt.host().attn(self._plan or self._native_plan(), self, q, k, v, custom, lists, False)
+        return o if o is not None else self._refuse(q, k, v, custom)
 
     def decode_paged(self, q, kcache, block_table, cache_seqlens, num_split=None):
         """kv_shared engines: decode over a paged KV pool with one length per batch row, returns (out, lse)."""
@@ -458,15 +465,11 @@ class AttentionEngine:
             self.block_mask = block_mask  # kept as the reference keeps it; the call below uses its own copy
             self.extern_block_mask = True
         q, k, v, *custom = args
-        self._call_block_mask = block_mask if block_mask is not None else (
-            self.block_mask if self.extern_block_mask else None)
-        try:
-            if getattr(self, "DV_total", self.DV) != self.DV:
-                if v.shape[-1] != self.DV_total:
-                    raise ValueError(f"v has head dim {v.shape[-1]}, engine was built for {self.DV_total}")
-                outs = [_AttentionFn.apply(self, q, k, v[..., i:i + self.DV], *custom)
-                        for i in range(0, self.DV_total, self.DV)]
-                return torch.cat(outs, dim=-1)
-            return _AttentionFn.apply(self, q, k, v, *custom)
-        finally:
-            self._call_block_mask = None
+        if block_mask is None and self.extern_block_mask:
+            block_mask = self.block_mask
+        if self.DV_total != self.DV:
+            if v.shape[-1] != self.DV_total:
+                raise ValueError(f"v has head dim {v.shape[-1]}, engine was built for {self.DV_total}")
+            return torch.cat([self._apply(q, k, v[..., i:i + self.DV], custom, block_mask)
+                              for i in range(0, self.DV_total, self.DV)], dim=-1)
+        return self._apply(q, k, v, custom, block_mask)

@@ -49,29 +49,6 @@ def _align(t: torch.Tensor, names: tuple, ndim: int) -> torch.Tensor:
     return t.reshape(shape)
 
 
-class _Scan(torch.autograd.Function):
-    """The scan on the mod-ed tensors; gradients flow on into the eager mods through torch autograd
-    (the reference chains the traced mod derivatives by hand, linear_tl.py:1203-1214)."""
-
-    @staticmethod
-    def forward(ctx, eng, q, k, v, a):
-        q, k, v, a = q.contiguous(), k.contiguous(), v.contiguous(), a.float().contiguous()
-        ctx.eng = eng
-        # with a backward to come (value blocks of 64), the forward also writes the chunk start-states it has at hand
-        hs = eng._new_states(v) if (any(ctx.needs_input_grad) and v.shape[3] == 64) else None
-        o = eng._launch(q, k, v, a, h_out=hs)
-        ctx.has_states = hs is not None
-        ctx.save_for_backward(q, k, v, a, *([hs] if hs is not None else []))
-        return o
-
-    @staticmethod
-    def backward(ctx, d_o):
-        q, k, v, a = ctx.saved_tensors[:4]
-        hs = ctx.saved_tensors[4] if ctx.has_states else None
-        dq, dk, dv, da = ctx.eng._launch_bwd(q, k, v, a, d_o.contiguous(), hs=hs)
-        return None, dq, dk, dv, da
-
-
 class _RowScale(torch.autograd.Function):
     """y = x * s[..., None] for x [B, H, T, D] 16-bit and s [B, H, T]: the `v * dt` shape of mod, as one streaming
     kernel each way (csrc/kernels/rowscale.cuh) instead of PyTorch's broadcast multiply and 64-wide reduction."""
@@ -117,54 +94,6 @@ class _Skip(torch.autograd.Function):
         return None, g, gx, gd
 
 
-class _ScaleScanSkip(torch.autograd.Function):
-    """y = scan(q, k, x * s[..., None], a) + x * d[head] as one node.  Forward: one launch of the scan kernel built
-    with the two mods inside.  Backward: the two gradients that meet at x (through the scaled rows and through the
-    skip) and the row sums for s and d come out of one pass over x (ae_vskip_bwd) instead of two kernels and an add."""
-
-    @staticmethod
-    def forward(ctx, eng, q, k, x, a, s, d, asc=None):
-        q, k, x, a, s = q.contiguous(), k.contiguous(), x.contiguous(), a.float().contiguous(), s.contiguous()
-        df = d.detach().float().reshape(-1).contiguous()
-        # a decay mod of the form decay * custom[heads]: a is the decay as passed, the kernels scale it
-        af = None if asc is None else asc.detach().float().reshape(-1).contiguous()
-        ctx.asc_meta = None if asc is None else (asc.shape, asc.dtype)
-        # one kernel: the scan scales its V rows by s, adds x * d[head] to its output rows and writes the scaled v
-        # for the backward (only when a gradient is wanted)
-        need_v = any(ctx.needs_input_grad)
-        v = torch.empty_like(x) if need_v else None
-        hs = eng._new_states(x) if need_v else None  # the chunk start-states, for the reverse pass
-        y = eng._launch(q, k, x, a, vscale=s, dskip=df, v_out=v, h_out=hs, ascale=af)
-        ctx.eng, ctx.d_shape, ctx.d_dtype = eng, d.shape, d.dtype
-        if not need_v:
-            return y
-        ctx.save_for_backward(q, k, v, a, x, s, df, hs, af)
-        return y
-
-    @staticmethod
-    def backward(ctx, g):
-        q, k, v, a, x, s, df, hs, af = ctx.saved_tensors
-        g = g.contiguous()
-        gasc = None
-        if int(os.environ.get("AE_B200_LIN_BWD_MODS", LIN_BWD_MODS)):
-            # the reverse pass built with the two mods inside: no pass over x of its own
-            res = ctx.eng._launch_bwd(q, k, v, a, g, hs=hs, mods=(x, s, df), ascale=af)
-            dq, dk, gx, da, gs, rows = res[:6]
-            if af is not None:
-                gasc = res[6].sum(dim=0).reshape(ctx.asc_meta[0]).to(ctx.asc_meta[1])
-            return None, dq, dk, gx, da, gs, rows.sum(dim=0).reshape(ctx.d_shape).to(ctx.d_dtype), gasc
-        res = ctx.eng._launch_bwd(q, k, v, a, g, hs=hs, ascale=af)
-        dq, dk, dv, da = res[:4]
-        if af is not None:
-            gasc = res[4].sum(dim=0).reshape(ctx.asc_meta[0]).to(ctx.asc_meta[1])
-        gx, gs = torch.empty_like(x), torch.empty_like(s)
-        rows = torch.empty(x.shape[:3], dtype=torch.float32, device=x.device)
-        ctx.eng._rowscale("vskip_bwd", x, s, g=g, g2=dv, d=df, gx=gx, gs=gs, gs2=rows, rows_per_head=x.shape[2],
-                          n_heads=x.shape[1])
-        gd = rows.sum(dim=(0, 2)).reshape(ctx.d_shape).to(ctx.d_dtype)
-        return None, dq, dk, gx, da, gs, gd, gasc
-
-
 class LinearAttentionEngine:
     def __init__(self, qkv_meta, q_mod=None, k_mod=None, v_mod=None, decay_mod=None, custom_io=None, tune=False,
                  tune_filename="tune_result", tune_bwd=False, o_mod=None):
@@ -192,7 +121,7 @@ class LinearAttentionEngine:
             self._o_leaves = (SymbolScalar("o", Var("o"), shape_idx=dims), SymbolScalar("v", Var("v"), shape_idx=dims))
             self._o_traced = o_mod(*self._o_leaves, self.custom_io)
         self._bf16 = self.dtype == torch.bfloat16
-        self._status = None
+        self._plan = None  # the native side, made at the first call
         self._bwd = None
         self._bwd_mods = None
         self._streams = {}
@@ -202,6 +131,61 @@ class LinearAttentionEngine:
         # of the reference use D = 256, DV = 512) are sums over key blocks of independent value blocks, see _scan().
         self._dv_block = self.DV if self.DV in (64, 128) else (128 if self.DV % 128 == 0 else 64)
         self.fwd, self.tl_code = self._fwd_kernel(self._dv_block)
+        self._block = self._block_operands()
+        self._decay_factor = None
+        if "decay" in self._traced:
+            self._decay_factor = self._factor(self._traced["decay"][1], self._traced["decay"][0], ("heads",))
+
+    def _native_plan(self):
+        if self._plan is None:
+            self._plan = rt.host().ScanPlan(self._bf16)
+        return self._plan
+
+    @property
+    def _status(self):
+        return self._plan.status if self._plan is not None else None
+
+    @_status.setter
+    def _status(self, t):
+        self._native_plan().status = t
+
+    def _load_block_kernel(self):
+        self._native_plan().fwd_mods = self._fwd_kernel(64, mods=True)[0].handle.value
+
+    def _native_bwd(self, B, H, sums, mods, device_index):
+        """Called by the autograd node: 1 when the backward is one launch of the reverse pass (and its head sums), which
+        the node issues itself; 0: it goes through ``_bwd_from_saved``."""
+        if mods and not int(os.environ.get("AE_B200_LIN_BWD_MODS", LIN_BWD_MODS)):
+            return 0
+        if sums and self._bwd_batch_parts(B, H, device_index) > 1:
+            return 0
+        plan = self._plan
+        if not (plan.bwd_mods if mods else plan.bwd):
+            states, bwd = self._bwd_kernels(mods)
+            plan.states = states.handle.value
+            if mods:
+                plan.bwd_mods = bwd.handle.value
+            else:
+                plan.bwd = bwd.handle.value
+            plan.head_sum = self._head_sum_kernel(128).handle.value
+        return 1
+
+    def _bwd_from_saved(self, q, k, v, a, g, hs, x, s, d, asc):
+        """Gradients from what a forward saved: (dq, dk, dv, da), or with the block's mods (x, s, d given) (dq, dk, gx, da,
+        gs, gd [B, H], gasc [B, H] or None)."""
+        if x is None:
+            return self._launch_bwd(q, k, v, a, g, hs=hs)
+        if int(os.environ.get("AE_B200_LIN_BWD_MODS", LIN_BWD_MODS)):
+            # the reverse pass built with the two mods inside: no pass over x of its own
+            res = self._launch_bwd(q, k, v, a, g, hs=hs, mods=(x, s, d), ascale=asc)
+            return res if asc is not None else res + (None,)
+        res = self._launch_bwd(q, k, v, a, g, hs=hs, ascale=asc)
+        dq, dk, dv, da = res[:4]
+        gx, gs = torch.empty_like(x), torch.empty_like(s)
+        rows = torch.empty(x.shape[:3], dtype=torch.float32, device=x.device)
+        self._rowscale("vskip_bwd", x, s, g=g, g2=dv, d=d, gx=gx, gs=gs, gs2=rows, rows_per_head=x.shape[2],
+                       n_heads=x.shape[1])
+        return dq, dk, gx, da, gs, rows.sum(dim=2), res[4] if asc is not None else None
 
     def _fwd_kernel(self, dv: int, mods: bool = False):
         """The forward kernel for value blocks of ``dv``; ``mods``: the build with the row scale of v and the skip
@@ -337,9 +321,9 @@ class LinearAttentionEngine:
     def _bwd_batch_parts(self, B, H, dev):
         """Into how many batch ranges the reverse pass is split (see _launch_bwd): 4 or 2 when the batch divides and a
         range still has one CTA per SM, else 1."""
-        from .attn_bwd import batch_ranges
+        from .attn_bwd import batch_ranges, sm_count
         want = int(os.environ.get("AE_B200_LIN_BWD_PARTS", LIN_BWD_PARTS))
-        return batch_ranges(B, H, torch.cuda.get_device_properties(dev).multi_processor_count, want)
+        return batch_ranges(B, H, sm_count(dev), want)
 
     def _side_streams(self, dev, n):
         """n side streams of this engine on ``dev`` with an event to start them after the caller's stream and one each
@@ -354,17 +338,20 @@ class LinearAttentionEngine:
         """[B, H, T, D] -> [B, n_out, T, D]: sum over the H / n_out heads of each group, fp32 accumulation, one pass."""
         B, H, T, D = x.shape
         y = out if out is not None else torch.empty(B, n_out, T, D, dtype=x.dtype, device=x.device)
+        p = rt.RowScaleParams()
+        p.x, p.y, p.n_rows, p.rows_per_head, p.n_heads = x.data_ptr(), y.data_ptr(), B * n_out * T, T, H // n_out
+        stream = C.c_void_p((stream if stream is not None else torch.cuda.current_stream(x.device)).cuda_stream)
+        rt.check(rt.lib().ae_launch_rowscale(self._head_sum_kernel(D).handle, C.byref(p), stream), "ae_launch_rowscale")
+        return y
+
+    def _head_sum_kernel(self, D):
         key = ("head_sum", D, False)
         if key not in self._rowscale_mods:
             pre = f"#define AE_BF16 {int(self._bf16)}\n#define AE_RS_D {D}\n#define AE_RS_S16 0\n"
             cfg = rt.KernelConfig(kind=rt.KIND_ROWSCALE, dtype=rt.DTYPE_BF16 if self._bf16 else rt.DTYPE_F16, head_dim=D,
                                   head_dim_v=D, threads=256, smem_bytes=0, stages=1, mask_mode=0)
             self._rowscale_mods[key] = rt.compile_module(rt.kernel_source("rowscale.cuh", prelude=pre), "ae_head_sum", cfg)
-        p = rt.RowScaleParams()
-        p.x, p.y, p.n_rows, p.rows_per_head, p.n_heads = x.data_ptr(), y.data_ptr(), B * n_out * T, T, H // n_out
-        stream = C.c_void_p((stream if stream is not None else torch.cuda.current_stream(x.device)).cuda_stream)
-        rt.check(rt.lib().ae_launch_rowscale(self._rowscale_mods[key].handle, C.byref(p), stream), "ae_launch_rowscale")
-        return y
+        return self._rowscale_mods[key]
 
     def _rowscale(self, which, x, s, rows_per_head=0, n_heads=0, **out):
         """Launch one of the streaming kernels of rowscale.cuh: "fwd" / "bwd" (one scale per row) or "skip_fwd" /
@@ -418,23 +405,41 @@ class LinearAttentionEngine:
         y = evaluate(out, env)
         return y if name == "decay" else y.to(x.dtype)
 
-    def _decay_scale_operand(self, decay, custom):
-        """The custom tensor c when the traced decay_mod is exactly ``decay * c`` with c indexed by heads only (fp32,
-        [1, H] or [H]); None otherwise (the mod then runs as eager PyTorch)."""
-        if "decay" not in self._traced or decay.dtype != torch.float32:
-            return None
-        leaf, out = self._traced["decay"]
+    def _factor(self, out, leaf, names):
+        """Position among the custom inputs of c when the traced value is exactly ``leaf * c`` with c indexed by ``names``
+        (dims of size one aside), else None."""
         if out.code.type != "Mul" or len(out.prev) != 2:
             return None
         other = out.prev[1] if out.prev[0] is leaf else out.prev[0] if out.prev[1] is leaf else None
-        if other is None:
-            return None
-        for (cname, sym), t in zip(self.custom_io.input_tensors.items(), custom):
-            if sym is other:
-                names = tuple(str(n) for n in sym.shape_idx if str(n) != "1")
-                if names == ("heads",) and t.numel() == self.H and t.dtype == torch.float32:
-                    return t
+        for i, sym in enumerate(self.custom_io.input_tensors.values()):
+            if sym is other and tuple(str(n) for n in sym.shape_idx if str(n) != "1") == names:
+                return i
         return None
+
+    def _decay_scale_operand(self, decay, custom):
+        """The custom tensor c when the traced decay_mod is exactly ``decay * c`` with c indexed by heads only (fp32,
+        [1, H] or [H]); None otherwise (the mod then runs as eager PyTorch)."""
+        i = self._decay_factor
+        if i is None or decay.dtype != torch.float32 or custom[i].dtype != torch.float32 or custom[i].numel() != self.H:
+            return None
+        return custom[i]
+
+    def _block_operands(self):
+        """The Mamba2 block, recognised in the traces: ``v * s[b, h, t]`` into the scan and ``o + v * d[h]`` after it, for the
+        head sizes its kernels take: (position of s, position of d) among the custom inputs."""
+        if self.o_mod is None or "v" not in self._traced or self.DK != 128 or self.DV != 64:
+            return None
+        leaf, out = self._traced["v"]
+        s = self._factor(out, leaf, ("batch", "heads", "seq_len"))
+        o_leaf, v_leaf = self._o_leaves
+        out = self._o_traced
+        if s is None or out.code.type != "Add" or len(out.prev) != 2:
+            return None
+        mul = out.prev[1] if out.prev[0] is o_leaf else out.prev[0] if out.prev[1] is o_leaf else None
+        d = None if mul is None else self._factor(mul, v_leaf, ("heads",))
+        if d is None:
+            return None
+        return s, d
 
     def _skip_operand(self, custom):
         """The custom tensor d when the traced o_mod is exactly ``o + v * d`` with d indexed by heads only (fp32,
@@ -494,6 +499,11 @@ class LinearAttentionEngine:
                  "ae_launch_linear_fwd")
         return o
 
+    def _native_scan(self, q, k, v, a):
+        """The scan on the mod-ed tensors as one autograd node; gradients flow on into the eager mods through torch autograd
+        (the reference chains the traced mod derivatives by hand, linear_tl.py:1203-1214)."""
+        return rt.host().scan(self._native_plan(), self._fwd_kernel(v.shape[3])[0].handle.value, self, q, k, v, a)
+
     def _scan(self, q, k, v, a):
         """The scan on heads of any supported size, from kernels that take 128 key dims and 64 / 128 value dims.
         Value blocks are independent problems sharing q, k and the decay (o[:, block] depends on v[:, block] only): they
@@ -504,14 +514,14 @@ class LinearAttentionEngine:
         want_grad = torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v, a))
         dvb = 64 if (want_grad or DV % 128) else 128
         if DK == 128 and DV == dvb:
-            return _Scan.apply(self, q, k, v, a)
+            return self._native_scan(q, k, v, a)
         n_dv = DV // dvb
         if n_dv > 1:
             v = v.view(B, H, T, n_dv, dvb).permute(0, 1, 3, 2, 4).reshape(B, H * n_dv, T, dvb)
             a = a.repeat_interleave(n_dv, dim=1)
         o = None
         for j in range(DK // 128):
-            oj = _Scan.apply(self, q[..., j * 128:(j + 1) * 128], k[..., j * 128:(j + 1) * 128], v, a)
+            oj = self._native_scan(q[..., j * 128:(j + 1) * 128], k[..., j * 128:(j + 1) * 128], v, a)
             o = oj.float() if o is None else o + oj.float()
         o = o.to(self.dtype)
         if n_dv > 1:
@@ -529,6 +539,8 @@ class LinearAttentionEngine:
         for name, t in (("q", q), ("k", k), ("v", v), ("decay", decay)):
             if not t.is_cuda:
                 raise rt.AeError(f"{name} must be a CUDA tensor: this back end has no CPU path")
+        if q.device.index == torch.cuda.current_device():
+            return self._call(q, k, v, decay, *custom)
         with torch.cuda.device(q.device):  # the C ABI launches on the current device's context
             return self._call(q, k, v, decay, *custom)
 
@@ -541,15 +553,14 @@ class LinearAttentionEngine:
             raise ValueError("inconsistent q/k/v shapes")
         qm = self._apply_mod("q", q, custom)
         km = self._apply_mod("k", k, custom)
-        if self.o_mod is not None and "v" in self._traced and self.DK == 128 and self.DV == 64 and v.dtype == self.dtype:
-            # `v * s[b, h, t]` into the scan and `o + v * d[h]` after it (the Mamba2 block): one autograd node, which
-            # also takes a decay mod of the form `decay * c[h]` into the kernels
-            s, d = self._rowscale_operand("v", v, custom), self._skip_operand(custom)
-            if s is not None and d is not None:
-                c = self._decay_scale_operand(decay, custom) if LIN_DECAY_SCALE else None
-                if c is not None:
-                    return _ScaleScanSkip.apply(self, qm, km, v, decay, s, d, c)
-                return _ScaleScanSkip.apply(self, qm, km, v, self._apply_mod("decay", decay, custom), s, d, None)
+        if self._block is not None:
+            # the block as one node; a decay mod of another form than `decay * c[h]` is applied first
+            i_s, i_d = self._block
+            c = self._decay_scale_operand(decay, custom) if LIN_DECAY_SCALE else None
+            a = decay if c is not None else self._apply_mod("decay", decay, custom).float()
+            y = rt.host().scan_block(self._native_plan(), self, qm, km, v, a, custom[i_s], custom[i_d], c)
+            if y is not None:
+                return y
         a = self._apply_mod("decay", decay, custom)
         vm = self._apply_mod("v", v, custom)
         o = self._scan(qm, km, vm, a)

@@ -8,8 +8,6 @@ user's ``score * softmax_scale`` decides the scale.  Forward only, as in the ref
 """
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
 
 from .. import runtime as rt
@@ -45,7 +43,17 @@ class MlaDecode:
         self.combine_src = head + defs + comb
         self.combine = rt.compile_module(self.combine_src, "ae_mla_combine", cfg2)
         self.num_split = None  # None = choose per call
-        self._status = None
+        self._plan = None  # the native side, made at the first call
+
+    def _native_plan(self):
+        if self._plan is None:
+            self._plan = rt.host().MlaPlan(self.decode.handle.value, self.combine.handle.value, self.dtype == torch.bfloat16,
+                                           len(self.low.final_names))
+        return self._plan
+
+    @property
+    def status(self):
+        return self._plan.status if self._plan is not None else None
 
     @staticmethod
     def pick_splits(B: int, S: int) -> int:
@@ -59,38 +67,15 @@ class MlaDecode:
         return n
 
     def __call__(self, q, q_pe, kv, k_pe):
-        for name, t in (("q", q), ("q_pe", q_pe), ("kv", kv), ("k_pe", k_pe)):
-            if not t.is_cuda:
-                raise rt.AeError(f"{name} must be a CUDA tensor: this back end has no CPU path")
-            if t.dtype != self.dtype:
-                raise TypeError(f"{name} has dtype {t.dtype}, engine was built for {self.dtype}")
-        B, one, H, DV = q.shape
-        S = kv.shape[1]
-        if one != 1 or DV != 512 or q_pe.shape != (B, 1, H, 64) or kv.shape != (B, S, 1, 512) or k_pe.shape != (B, S, 1, 64):
+        n_split = self.num_split or self.pick_splits(q.shape[0], kv.shape[1])
+        o = rt.host().mla(self._plan or self._native_plan(), q, q_pe, kv, k_pe, n_split)
+        if o is None:  # not launched: say what does not fit
+            for name, t in (("q", q), ("q_pe", q_pe), ("kv", kv), ("k_pe", k_pe)):
+                if not t.is_cuda:
+                    raise rt.AeError(f"{name} must be a CUDA tensor: this back end has no CPU path")
+                if t.dtype != self.dtype:
+                    raise TypeError(f"{name} has dtype {t.dtype}, engine was built for {self.dtype}")
             raise ValueError("expected q [B,1,H,512], q_pe [B,1,H,64], kv [B,S,1,512], k_pe [B,S,1,64]")
-        q, q_pe, kv, k_pe = (t.contiguous() for t in (q, q_pe, kv, k_pe))
-        dev = q.device
-        n_split = self.num_split or self.pick_splits(B, S)
-        o = torch.empty(B, 1, H, 512, dtype=self.dtype, device=dev)
-        p = rt.MlaParams()
-        p.q, p.q_pe, p.kv, p.k_pe, p.o = q.data_ptr(), q_pe.data_ptr(), kv.data_ptr(), k_pe.data_ptr(), o.data_ptr()
-        keep = []
-        if n_split > 1:
-            part = torch.empty(B, n_split, H, 512, dtype=torch.float32, device=dev)
-            p.o_partial = part.data_ptr()
-            keep.append(part)
-            for i in range(len(self.low.final_names)):
-                f = torch.empty(B, n_split, H, dtype=torch.float32, device=dev)
-                p.rowscale_partial[i] = f.data_ptr()
-                keep.append(f)
-        p.B, p.H, p.S, p.n_split = B, H, S, n_split
-        if self._status is None or self._status.device != dev:
-            self._status = torch.zeros(1, dtype=torch.int32, device=dev)
-        p.status = self._status.data_ptr()
-        stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-        rt.check(rt.lib().ae_launch_mla_decode(self.decode.handle, C.byref(p), stream), "ae_launch_mla_decode")
-        if n_split > 1:
-            rt.check(rt.lib().ae_launch_mla_combine(self.combine.handle, C.byref(p), stream), "ae_launch_mla_combine")
         self.last_num_split = n_split
         return o
 
@@ -100,9 +85,20 @@ class MlaDecode:
         The call of the reference's CuTe kv-shared path (core/template/cute_template_kvshared/flash_mla_interface.py:73-113,
         attn_script/mla_decode_cute.py:295-303): q [B, 1, H, 576] (latent 512 + rope 64), kcache [num_pages, 64, 1, 576]
         or [num_pages, 64, 576], block_table [B, max_pages] int32 (page of each 64-key tile), cache_seqlens [B] int32.
-        Every row gets the same split count over the longest row's tiles."""
+        Every row is cut into the same number of shares of its own tiles, so the launch needs no length on the host; the
+        lengths are read back behind the launches only to raise on one outside the table."""
         if list(self.low.final_names) != ["lse"]:
             raise NotImplementedError("the paged call returns the log-sum-exp: the online function must have the final row scale 'lse'")
+        n_split = num_split or self.num_split or self.pick_splits(q.shape[0], block_table.shape[1] * 64)
+        res = rt.host().mla_paged(self._plan or self._native_plan(), q, kcache, block_table, cache_seqlens, n_split)
+        if res is None:
+            self._refuse_paged(q, kcache, block_table, cache_seqlens)
+        if not res:
+            raise ValueError("cache_seqlens must lie in [1, max_pages * 64]")
+        self.last_num_split = n_split
+        return res
+
+    def _refuse_paged(self, q, kcache, block_table, cache_seqlens):
         for name, t in (("q", q), ("kcache", kcache)):
             if not t.is_cuda:
                 raise rt.AeError(f"{name} must be a CUDA tensor: this back end has no CPU path")
@@ -117,39 +113,6 @@ class MlaDecode:
             kcache = kcache[:, :, 0]
         if kcache.shape[1:] != (64, 576) or not kcache.is_contiguous():
             raise ValueError("expected a contiguous kcache of 64-key pages, [num_pages, 64, (1,) 576]")
-        dev = q.device
-        block_table = block_table.to(device=dev, dtype=torch.int32).contiguous()
-        cache_seqlens = cache_seqlens.to(device=dev, dtype=torch.int32).contiguous()
-        if block_table.shape[0] != B or cache_seqlens.shape != (B,):
+        if block_table.shape[0] != q.shape[0] or cache_seqlens.shape != (q.shape[0],):
             raise ValueError("block_table is [B, max_pages], cache_seqlens is [B]")
-        max_pages = block_table.shape[1]
-        max_seqlen = int(cache_seqlens.max().item())  # host read: the grid and the split ranges depend on it
-        if max_seqlen < 1 or int(cache_seqlens.min().item()) < 1 or max_seqlen > max_pages * 64:
-            raise ValueError("cache_seqlens must lie in [1, max_pages * 64]")
-        q_nope = q[:, 0, :, :512].contiguous()
-        q_pe = q[:, 0, :, 512:].contiguous()
-        n_split = num_split or self.num_split or self.pick_splits(B, max_seqlen)
-        o = torch.empty(B, 1, H, 512, dtype=self.dtype, device=dev)
-        fr = torch.empty(B, n_split, H, dtype=torch.float32, device=dev)
-        p = rt.MlaPagedParams()
-        p.q, p.q_pe, p.kcache, p.o = q_nope.data_ptr(), q_pe.data_ptr(), kcache.data_ptr(), o.data_ptr()
-        p.block_table, p.cache_seqlens = block_table.data_ptr(), cache_seqlens.data_ptr()
-        p.rowscale_partial[0] = fr.data_ptr()
-        part = None
-        if n_split > 1:
-            part = torch.empty(B, n_split, H, 512, dtype=torch.float32, device=dev)
-            p.o_partial = part.data_ptr()
-        p.B, p.H, p.num_pages, p.max_pages, p.max_seqlen, p.n_split = B, H, kcache.shape[0], max_pages, max_seqlen, n_split
-        if self._status is None or self._status.device != dev:
-            self._status = torch.zeros(1, dtype=torch.int32, device=dev)
-        p.status = self._status.data_ptr()
-        stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-        rt.check(rt.lib().ae_launch_mla_decode_paged(self.decode.handle, C.byref(p), stream), "ae_launch_mla_decode_paged")
-        if n_split > 1:
-            pc = rt.MlaParams()
-            pc.o, pc.o_partial = o.data_ptr(), part.data_ptr()
-            pc.rowscale_partial[0] = fr.data_ptr()
-            pc.B, pc.H, pc.S, pc.n_split = B, H, max_seqlen, n_split
-            rt.check(rt.lib().ae_launch_mla_combine(self.combine.handle, C.byref(pc), stream), "ae_launch_mla_combine")
-        self.last_num_split = n_split
-        return o, torch.logsumexp(fr, dim=1)
+        raise ValueError("tensors do not fit this engine")

@@ -713,12 +713,6 @@ int ae_launch_mla_decode_paged(void* module, const AeMlaPagedParams* p, void* st
     set_error("paged MLA decode: need 1 <= H <= 128, 1 <= max_seqlen <= max_pages * 64, 1 <= n_split <= 32");
     return AE_ERR_INVALID;
   }
-  const int n_tiles = (p->max_seqlen + 63) / 64;
-  const int tps = (n_tiles + p->n_split - 1) / p->n_split;
-  if ((int64_t)(p->n_split - 1) * tps >= n_tiles) {
-    set_error("MLA decode: n_split leaves an empty split");
-    return AE_ERR_INVALID;
-  }
   if (p->n_split > 1 && !p->o_partial) {
     set_error("MLA decode: o_partial scratch required when n_split > 1");
     return AE_ERR_INVALID;
@@ -728,15 +722,15 @@ int ae_launch_mla_decode_paged(void* module, const AeMlaPagedParams* p, void* st
   AeMlaArgs a;
   memset(&a, 0, sizeof a);
   const int64_t pool_rows = (int64_t)p->num_pages * 64;
-  if ((rc = make_3d_map(&a.tm_q, p->q, m->cfg.dtype, 512, p->H, p->B, 128))) return rc;
-  if ((rc = make_3d_map(&a.tm_qpe, p->q_pe, m->cfg.dtype, 64, p->H, p->B, 128))) return rc;
+  if ((rc = make_3d_map(&a.tm_q, p->q, m->cfg.dtype, 512, p->H, p->B, 128, p->q_row_stride))) return rc;
+  if ((rc = make_3d_map(&a.tm_qpe, p->q_pe, m->cfg.dtype, 64, p->H, p->B, 128, p->q_row_stride))) return rc;
   // the pool as one batch of num_pages * 64 rows of 576 elements: latent part and rope part are column slices
   if ((rc = make_3d_map(&a.tm_kv, p->kcache, m->cfg.dtype, 512, pool_rows, 1, 64, 576))) return rc;
   if ((rc = make_3d_map(&a.tm_kpe, (const char*)p->kcache + 512 * 2, m->cfg.dtype, 64, pool_rows, 1, 64, 576))) return rc;
   a.o = p->o;
   a.o_part = p->o_partial;
   for (int i = 0; i < AE_MAX_FINAL; ++i) a.fr_part[i] = p->rowscale_partial[i];
-  a.B = p->B; a.H = p->H; a.S = p->max_seqlen; a.n_split = p->n_split; a.tiles_per_split = tps;
+  a.B = p->B; a.H = p->H; a.S = p->max_seqlen; a.n_split = p->n_split;
   a.status = p->status;
   a.block_table = p->block_table;
   a.seqlens = p->cache_seqlens;
@@ -760,6 +754,7 @@ int ae_launch_mla_combine(void* module, const AeMlaParams* p, void* stream) {
   a.o_part = p->o_partial;
   for (int i = 0; i < AE_MAX_FINAL; ++i) a.fr_part[i] = p->rowscale_partial[i];
   a.B = p->B; a.H = p->H; a.DV = 512; a.n_split = p->n_split;
+  a.lse_out = p->lse_out;
   return launch(m, (unsigned)((p->H + 3) / 4), (unsigned)p->B, 1, &a, stream);
 }
 

@@ -115,8 +115,8 @@ struct AeMlaArgs {
   int B, H, S, n_split, tiles_per_split;
   u32* status;
   // paged KV (null = the dense layout above): tm_kv / tm_kpe then cover the page pool as rows (page * 64 + r) of one
-  // batch, tile i of batch row b is page block_table[b * max_pages + i], and row b holds seqlens[b] keys
-  // (S = the longest row; a split that starts past a row's last tile writes zero partials with -inf row scales).
+  // batch, tile i of batch row b is page block_table[b * max_pages + i], and row b holds seqlens[b] keys, clamped to
+  // [0, S], that its n_split shares divide (a share past the row's last tile writes zero partials with -inf row scales).
   const int* block_table;
   const int* seqlens;
   int max_pages;
@@ -128,6 +128,7 @@ struct AeMlaCombineArgs {
   int B, H, DV, n_split;
   const int* part_off;  // [B + 1] or null: row b owns the partial slots part_off[b] .. part_off[b + 1] - 1 (at most 32);
                         // null = n_split slots per row.  A row with a single slot was written directly and is skipped.
+  float* lse_out;       // [B, H] or null: log-sum-exp over the splits of fr_part[0]
 };
 
 // ---- chunked linear attention / SSD scan forward (kernel ae_linear_fwd) -------------------

@@ -31,6 +31,13 @@ extern "C" __global__ void __launch_bounds__(128) ae_mla_combine(const AeMlaComb
 #pragma unroll
   for (int i = 0; i < AE_NFINAL; ++i)
     fr[i] = lane < n_split ? args.fr_part[i][(slot0 + lane) * args.H + h] : -__int_as_float(0x7f800000);
+#if AE_NFINAL > 0
+  if (args.lse_out) {
+    const float m = ae_warp_max(fr[0]);
+    const float sum = ae_warp_sum(lane < n_split ? expf(fr[0] - m) : 0.f);
+    if (lane == 0) args.lse_out[(i64)b * args.H + h] = m + logf(sum);
+  }
+#endif
   float w = ae_combine(fr);
   if (lane >= n_split) w = 0.f;
   u16* orow = (u16*)args.o + ((i64)b * args.H + h) * args.DV;

@@ -73,10 +73,16 @@ extern "C" __global__ void __launch_bounds__(192, 1) ae_mla_decode(const __grid_
 #ifdef AE_TRACE
   const bool trace_on = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (threadIdx.x & 31) == 0;
 #endif
-  const int S_b = args.seqlens ? args.seqlens[b] : args.S;  // keys of this batch row
+  // keys of this batch row; rows of different lengths are cut into n_split shares each by its own tiles
+  int S_b = args.S, tps = args.tiles_per_split;
+  if (args.seqlens) {
+    const int len = args.seqlens[b];
+    S_b = len < 0 ? 0 : (len < args.S ? len : args.S);
+    tps = ((S_b + AE_MLA_BN - 1) / AE_MLA_BN + args.n_split - 1) / args.n_split;
+  }
   const int n_tiles = (S_b + AE_MLA_BN - 1) / AE_MLA_BN;
-  const int t_begin = split * args.tiles_per_split;
-  int t_end = t_begin + args.tiles_per_split;
+  const int t_begin = split * tps;
+  int t_end = t_begin + tps;
   if (t_end > n_tiles) t_end = n_tiles;
   const int n_steps = t_end > t_begin ? t_end - t_begin : 0;
 

@@ -76,7 +76,8 @@ class AttnBwdParams(C.Structure):
 class MlaParams(C.Structure):
     _fields_ = [("q", C.c_void_p), ("q_pe", C.c_void_p), ("kv", C.c_void_p), ("k_pe", C.c_void_p), ("o", C.c_void_p),
                 ("o_partial", C.c_void_p), ("rowscale_partial", C.c_void_p * AE_MAX_FINAL),
-                ("B", C.c_int32), ("H", C.c_int32), ("S", C.c_int32), ("n_split", C.c_int32), ("status", C.c_void_p)]
+                ("B", C.c_int32), ("H", C.c_int32), ("S", C.c_int32), ("n_split", C.c_int32), ("status", C.c_void_p),
+                ("lse_out", C.c_void_p)]
 
 
 class DecodeParams(C.Structure):
@@ -101,7 +102,7 @@ class MlaPagedParams(C.Structure):
                 ("cache_seqlens", C.c_void_p), ("o", C.c_void_p), ("o_partial", C.c_void_p),
                 ("rowscale_partial", C.c_void_p * AE_MAX_FINAL),
                 ("B", C.c_int32), ("H", C.c_int32), ("num_pages", C.c_int32), ("max_pages", C.c_int32),
-                ("max_seqlen", C.c_int32), ("n_split", C.c_int32), ("status", C.c_void_p)]
+                ("max_seqlen", C.c_int32), ("n_split", C.c_int32), ("status", C.c_void_p), ("q_row_stride", C.c_int64)]
 
 
 class LinearParams(C.Structure):
@@ -165,6 +166,23 @@ def lib() -> C.CDLL:
                                           C.c_void_p, C.c_void_p]
             _lib = L
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/ae_host.cpp).  No fallback: a missing extension raises."""
+    global _host
+    if _host is None:
+        lib()  # libae_b200.so first: its absence has a message of its own
+        try:
+            from . import _ae_host
+        except ImportError as e:
+            raise AeError(f"attentionengine_b200/_ae_host.so cannot be loaded ({e}): run `python -c 'import __graft_entry__ as g; "
+                          "g.build()'` (there is no fallback path)") from e
+        _host = _ae_host
+    return _host
 
 
 def check(rc: int, what: str = ""):

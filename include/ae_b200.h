@@ -218,6 +218,7 @@ typedef struct AeMlaParams {
   float* rowscale_partial[AE_MAX_FINAL_ROWSCALES]; /* each [B, n_split, H] fp32 scratch */
   int32_t B, H, S, n_split;
   uint32_t* status;
+  float* lse_out; /* ae_launch_mla_combine only, optional: [B, H] log-sum-exp over the splits of rowscale_partial[0] */
 } AeMlaParams;
 
 int ae_launch_mla_decode(void* module, const AeMlaParams* p, void* stream);
@@ -226,8 +227,9 @@ int ae_launch_mla_combine(void* module, const AeMlaParams* p, void* stream);
 /* The same decode over a paged KV pool with one length per batch row: the call of the reference's CuTe kv-shared
  * path, `flash_mla_with_kvcache(q, k_cache, block_table, cache_seqlens, ...)`
  * (core/template/cute_template_kvshared/flash_mla_interface.py:73-113; script attn_script/mla_decode_cute.py:295-303),
- * whose scheduler metadata (`get_mla_metadata`) has no counterpart here: every batch row gets the same n_split over
- * the longest row's tiles, and a split that starts past a shorter row's end contributes nothing.  Pages hold 64 keys.
+ * whose scheduler metadata (`get_mla_metadata`) has no counterpart here: every batch row is cut into n_split shares of
+ * its own tiles, and a share that starts past a short row's end contributes nothing.  The kernel reads the lengths and
+ * clamps them to [0, max_seqlen]: no access leaves the block table, whatever they hold.  Pages hold 64 keys.
  * The merge is `ae_launch_mla_combine` with q / kv unused (fill o, o_partial, rowscale_partial, B, H, n_split). */
 typedef struct AeMlaPagedParams {
   const void* q;                /* [B, H, 512] contiguous: the latent part of the query */
@@ -238,8 +240,9 @@ typedef struct AeMlaPagedParams {
   void* o;                      /* [B, H, 512] */
   float* o_partial;             /* [B, n_split, H, 512] fp32 (n_split > 1) */
   float* rowscale_partial[AE_MAX_FINAL_ROWSCALES]; /* each [B, n_split, H]; with n_split == 1 the final row scales */
-  int32_t B, H, num_pages, max_pages, max_seqlen, n_split;
+  int32_t B, H, num_pages, max_pages, max_seqlen, n_split; /* max_seqlen <= max_pages * 64: bound of the lengths */
   uint32_t* status;
+  int64_t q_row_stride; /* elements between the heads of q and of q_pe (576: one [B, H, 576] tensor); 0 = contiguous */
 } AeMlaPagedParams;
 
 int ae_launch_mla_decode_paged(void* module, const AeMlaPagedParams* p, void* stream);

@@ -1031,3 +1031,19 @@ def test_value_head_dim_above_128_runs_as_value_blocks():
     o, (dq, dk, dv) = orc.fwd_bwd(lambda a, b, c: orc.softmax_attention(a, b, c, True), (q, k, v), d_o)
     for name, g, r in zip(("o", "dq", "dk", "dv"), got, (o, dq, dk, dv)):
         _check(name, g, r, dtype)
+
+
+@pytest.mark.parametrize("lens", [[0, 100], [100, 257], [-1, 100]])
+def test_mla_paged_lengths_outside_the_table_raise(lens):
+    """The lengths are checked behind the launches: the kernels clamp them to the block table, the call raises."""
+    B, H, dtype = 2, 16, torch.float16
+    eng = helpers.mla_engine(B, H, 256, dtype, 1 / math.sqrt(192))
+    q = torch.zeros(B, 1, H, 576, dtype=dtype, device="cuda")
+    kcache = torch.zeros(B * 4, 64, 1, 576, dtype=dtype, device="cuda")
+    table = torch.arange(B * 4, dtype=torch.int32, device="cuda").view(B, 4)
+    with pytest.raises(ValueError, match="cache_seqlens"):
+        eng.decode_paged(q, kcache, table, torch.tensor(lens, dtype=torch.int32, device="cuda"))
+    o, lse = eng.decode_paged(q, kcache, table, torch.tensor([1, 256], dtype=torch.int32, device="cuda"))
+    torch.cuda.synchronize()
+    eng.check_status()
+    assert not o.any() and torch.allclose(lse.cpu(), torch.tensor([1.0, 256.0]).log().view(2, 1).expand(2, H), atol=1e-5)
