@@ -456,9 +456,9 @@ ae_attn_bwd_dkv(const __grid_constant__ AeAttnBwdArgs args) {
         for (int j = 0; j < AE_NCS; ++j) fr[j] = e == 0 ? cv[j].x : (e == 1 ? cv[j].y : (e == 2 ? cv[j].z : cv[j].w));
       };
       auto keep_of = [&](int q_idx) -> bool {
-        bool keep = row_valid && q_idx < args.Sq;
+        bool keep = row_valid & (q_idx < args.Sq);  // bitwise and selects: short-circuit forms became one branch per element
 #if AE_MASK_MODE != 0
-        if (st.partial) keep = keep && ae_mask(b, st.hq, q_idx, kv_idx);
+        keep = keep & (!st.partial | ae_mask(b, st.hq, q_idx, kv_idx));
 #endif
         return keep;
       };
@@ -489,7 +489,7 @@ ae_attn_bwd_dkv(const __grid_constant__ AeAttnBwdArgs args) {
               float fr[AE_NCS];
               col_scales(c, i, e, fr, cv);
               float p = ae_bwd_p(sv[i + e], fr, b, st.hq, q_idx, kv_idx, cu, i + e);
-              if (kMasked && !keep_of(q_idx)) p = 0.f;
+              if (kMasked) p = keep_of(q_idx) ? p : 0.f;
               p4[e] = p;
               pkeep[ci][i + e] = p;
 #if AE_DS_USES_S
@@ -545,7 +545,7 @@ ae_attn_bwd_dkv(const __grid_constant__ AeAttnBwdArgs args) {
               if (kMasked) keep = keep_of(q_idx);
               float dsv = ae_bwd_ds(sraw, keep ? dp[i + e] : 0.f, pkeep[ci][i + e], fr, fr[AE_NFINAL], b, st.hq, q_idx,
                                     kv_idx, cu);
-              if (kMasked && !keep) dsv = 0.f;
+              if (kMasked) dsv = keep ? dsv : 0.f;
               ds4[e] = dsv;
             }
             dk[(i >> 1) + 0] = pack2<AE_BF16>(ds4[0], ds4[1]);

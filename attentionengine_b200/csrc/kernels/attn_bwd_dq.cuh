@@ -355,9 +355,9 @@ ae_attn_bwd_dq(const __grid_constant__ AeAttnBwdArgs args) {
       float skeep[NCH][32];
 #endif
       auto keep_of = [&](int kv_idx) -> bool {
-        bool keep = kv_idx < args.Skv;
+        bool keep = kv_idx < args.Skv;  // bitwise and selects: short-circuit forms became one branch per element
 #if AE_MASK_MODE != 0
-        if (partial) keep = keep && ae_mask(b, hq, q_idx, kv_idx);
+        keep = keep & (!partial | ae_mask(b, hq, q_idx, kv_idx));
 #endif
         return keep;
       };
@@ -388,7 +388,7 @@ ae_attn_bwd_dq(const __grid_constant__ AeAttnBwdArgs args) {
           for (int i = 0; i < 32; ++i) {
             const int kv_idx = kv0 + c * 32 + i;
             float p = ae_bwd_p(sv[ci][i], fr, b, hq, q_idx, kv_idx, cu, i);
-            if (kMasked && !keep_of(kv_idx)) p = 0.f;
+            if (kMasked) p = keep_of(kv_idx) ? p : 0.f;
             pkeep[ci][i] = p;
 #if AE_DS_USES_S
             skeep[ci][i] = sv[ci][i];
@@ -424,7 +424,7 @@ ae_attn_bwd_dq(const __grid_constant__ AeAttnBwdArgs args) {
               bool keep = true;
               if (kMasked) keep = keep_of(kv_idx);
               float dsv = ae_bwd_ds(sraw, keep ? dp[i + e] : 0.f, pkeep[ci][i + e], fr, delta, b, hq, q_idx, kv_idx, cu);
-              if (kMasked && !keep) dsv = 0.f;
+              if (kMasked) dsv = keep ? dsv : 0.f;
               ds2[e] = dsv;
             }
             pk[i >> 1] = pack2<AE_BF16>(ds2[0], ds2[1]);

@@ -526,11 +526,11 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
               col_scales(e, fr, cv);
               float p = ae_bwd_p(sv[i + e], fr, b, st.hq, q_idx, kv_idx, cu, i + e);
               if (kMasked) {
-                bool keep = row_valid && q_idx < args.Sq;
+                bool keep = row_valid & (q_idx < args.Sq);  // bitwise and selects: short-circuit forms became one branch per element
 #if AE_MASK_MODE != 0
-                if (st.partial) keep = keep && ae_mask(b, st.hq, q_idx, kv_idx);
+                keep = keep & (!st.partial | ae_mask(b, st.hq, q_idx, kv_idx));
 #endif
-                if (!keep) p = 0.f;
+                p = keep ? p : 0.f;
               }
               p4[e] = p;
               pkeep[ci][i + e] = p;
@@ -585,14 +585,14 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
 #endif
               bool keep = true;
               if (kMasked) {
-                keep = row_valid && q_idx < args.Sq;
+                keep = row_valid & (q_idx < args.Sq);
 #if AE_MASK_MODE != 0
-                if (st.partial) keep = keep && ae_mask(b, st.hq, q_idx, kv_idx);
+                keep = keep & (!st.partial | ae_mask(b, st.hq, q_idx, kv_idx));
 #endif
               }
               float dsv = ae_bwd_ds(sraw, keep ? dp[i + e] : 0.f, pkeep[ci][i + e], fr, fr[AE_NFINAL], b, st.hq, q_idx,
                                     kv_idx, cu);
-              if (kMasked && !keep) dsv = 0.f;
+              if (kMasked) dsv = keep ? dsv : 0.f;
               ds4[e] = dsv;
             }
             dk[(i >> 1) + 0] = pack2<AE_BF16>(ds4[0], ds4[1]);

@@ -292,12 +292,12 @@ ae_attn_fwd_pair(const __grid_constant__ AeAttnFwdArgs args) {
             const int kv_idx = kv0 + c;
             bool keep = kv_idx < args.Skv;
 #if AE_MASK_MODE != 0
-            if (partial) keep = keep && ae_mask(b, h_row, q_idx, kv_idx);
+            keep = keep & (!partial | ae_mask(b, h_row, q_idx, kv_idx));
 #endif
 #if AE_MASK_NEG_INF
-            if (!keep) s[c] = -__int_as_float(0x7f800000);
+            s[c] = keep ? s[c] : -__int_as_float(0x7f800000);
 #else
-            if (kv_idx >= args.Skv) s[c] = 0.f;  // additive mask value 0: scores stay as they are
+            s[c] = kv_idx < args.Skv ? s[c] : 0.f;  // additive mask value 0: scores stay as they are
             (void)keep;
 #endif
           }

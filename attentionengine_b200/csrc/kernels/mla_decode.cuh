@@ -268,7 +268,7 @@ extern "C" __global__ void __launch_bounds__(192, 1) ae_mla_decode(const __grid_
       if (kv0 + AE_MLA_BN > S_b) {
 #pragma unroll
         for (int c = 0; c < AE_MLA_BN; ++c)
-          if (kv0 + c >= S_b) sc[c] = -__int_as_float(0x7f800000);
+          sc[c] = kv0 + c < S_b ? sc[c] : -__int_as_float(0x7f800000);
       }
       const float o_scale = ae_online_fwd<AE_MLA_BN>(sc, st, b, h, 0, kv0, cu);
       {
