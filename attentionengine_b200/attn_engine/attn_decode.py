@@ -51,7 +51,7 @@ class AttnDecode:
         # at most 128 rows: one q tile in shared memory, its space goes to a third K / V stage
         nq, stages = (1, 3) if self.rows <= 128 else (2, 2)
         smem = nq * 128 * D * 2 + stages * 128 * (D + DV) * 2 + 512 + 1024
-        cfg = rt.KernelConfig(kind=rt.KIND_ATTN_DECODE, dtype=tag, head_dim=D, head_dim_v=DV, threads=320,
+        cfg = rt.KernelConfig(kind=rt.KIND_ATTN_DECODE, dtype=tag, head_dim=D, head_dim_v=DV, threads=192 if nq == 1 else 384,
                               smem_bytes=smem, stages=stages, mask_mode=mask_mode)
         cfg.reserved[1] = len(self.low.final_names)
         prelude = self.low.prelude_fwd.replace("#define AE_STAGES 2\n", f"#define AE_STAGES {stages}\n")

@@ -98,7 +98,6 @@ def _block_lists(cnt: torch.Tensor, q_blk: int, kv_blk: int, Sq: int, Skv: int, 
 
 
 FWD_PAIR = 0  # 1: the forward over CTA pairs where it applies
-FWD_FORM = (1, 0)  # (threads per score row, turn-taking) of the forward kernel when no tuned entry says otherwise
 
 
 class _AttnKernels:
@@ -109,15 +108,7 @@ class _AttnKernels:
         self.low = low
         self.D, self.DV, self.dtype_tag, self.mask_mode, self.stages = D, DV, dtype_tag, mask_mode, stages
         self.tuned = tuned or {}  # tile choices of the backward kernels (attentionengine_b200/tune.py)
-        # forward form: threads per score row (1 or 2) and whether the two q tiles take turns; from the tuned table,
-        # AE_B200_FWD_RSPLIT / AE_B200_FWD_TURNS override (experiments)
-        rsplit, turns = self.tuned.get("fwd_form", FWD_FORM)
-        rsplit = int(os.environ.get("AE_B200_FWD_RSPLIT", rsplit))
-        turns = int(os.environ.get("AE_B200_FWD_TURNS", turns))
-        self.fwd_form = (rsplit, turns)
         smem = 2 * 128 * D * 2 + stages * 128 * (D + DV) * 2 + 512 + 1024
-        if rsplit > 1:
-            smem += 2 * 2 * rsplit * 128 * 4  # partial row reductions exchanged between the threads of a row
         if mask_mode == 2:
             smem += 4 * MAX_LIST_KV_TILES  # the CTA's merged tile walk
         # forward over CTA pairs (tcgen05 cta_group::2): for the shapes it is written for, when the tuned entry or
@@ -135,9 +126,8 @@ class _AttnKernels:
             self.fwd = rt.compile_module(self.fwd_src, "ae_attn_fwd_pair", cfg)
         else:
             cfg = rt.KernelConfig(kind=rt.KIND_ATTN_FWD, dtype=dtype_tag, head_dim=D, head_dim_v=DV,
-                                  threads=rsplit * 256 + 64, smem_bytes=smem, stages=stages, mask_mode=mask_mode)
-            self.fwd_src = rt.kernel_source("attn_fwd.cuh", prelude=low.prelude_fwd,
-                                            defines={"AE_RSPLIT": rsplit, "AE_TURNS": turns})
+                                  threads=384, smem_bytes=smem, stages=stages, mask_mode=mask_mode)
+            self.fwd_src = rt.kernel_source("attn_fwd.cuh", prelude=low.prelude_fwd)
             self.fwd = rt.compile_module(self.fwd_src, "ae_attn_fwd", cfg)
         self._bwd = None
         self._bwd_fused = None

@@ -460,8 +460,25 @@ int ae_launch_attn_fwd(void* module, const AeAttnParams* p, void* stream) {
   args.n_kt = (p->Skv + 127) / 128;
   args.status = p->status;
   // single-CTA kernel: two q tiles per CTA; pair kernel: one per CTA, two per cluster (of two CTAs along x)
-  const unsigned gx = pair ? 2u * (unsigned)((args.n_qt + 1) / 2) : (unsigned)((args.n_qt + 1) / 2);
-  return launch(m, gx, (unsigned)p->Hq, (unsigned)p->B, &args, stream);
+  const unsigned n_pair = (unsigned)((args.n_qt + 1) / 2);
+  if (pair) return launch(m, 2u * n_pair, (unsigned)p->Hq, (unsigned)p->B, &args, stream);
+  // Under a causal mask the CTAs of a head differ by the length of their walk: the longest of ALL heads go first, so that the
+  // last CTAs to start are the shortest.  That many heads' K and V are in use at a time, so the grid runs in sections of
+  // heads whose K and V fit L2 (half of it).  Without a causal mask all walks are alike: one head after the other.
+  int64_t sec = 1;
+  if (m->cfg.mask_mode == 1) {
+    const int64_t g = p->Hq / p->Hkv, kv_bytes = (int64_t)p->Skv * (D + DV) * 2;
+    sec = g * ((int64_t)63 * 1024 * 1024 / kv_bytes);
+    if (sec < g) sec = g;
+    if (sec > (int64_t)p->B * p->Hq) sec = (int64_t)p->B * p->Hq;
+  }
+  args.sec = (int)sec;
+  const int64_t ctas = (int64_t)n_pair * p->Hq * p->B;
+  if (ctas > 0x7fffffff) {
+    set_error("attention forward: too many q tiles for one launch");
+    return AE_ERR_INVALID;
+  }
+  return launch(m, (unsigned)ctas, 1, 1, &args, stream);
 }
 
 static int fill_bwd_args(Module* m, const AeAttnBwdParams* p, AeAttnBwdArgs* a, int q_rows, int kv_rows) {

@@ -46,6 +46,7 @@ struct AeAttnFwdArgs {
   const int* blk_idx;  // [B, Hq, n_qt, n_kt] kv tile index | (partial << 30)  (mask mode 2)
   int B, Hq, Hkv, Sq, Skv;
   int n_qt, n_kt;  // number of 128-row q tiles / 128-column kv tiles
+  int sec;         // (batch, q-head) units per section of the grid (not the decode build)
   u32* status;
   // Split-KV decode (the same kernel built with AE_DECODE): one CTA per (split, head unit, batch) owns ALL query rows
   // of its unit (at most 256) and the kv tiles [split * tiles_per_split, ...).  gq > 1: the unit is a kv head and the

@@ -150,6 +150,14 @@ AE_DEVICE bool mbar_wait(u64* bar, u32 parity, AeCtaCtl* ctl, u32* g_status, u32
   }
 }
 
+// The same wait by every lane of a row warp.  The lanes leave the polling loop one by one; the vote brings them together
+// again before the warp-collective tcgen05.ld / st that follow (left to the compiler, a wait that really had to poll in
+// the middle of the recurrence once ran them with a diverged warp: wrong results and hung waits).
+AE_DEVICE bool mbar_wait_row(bool ok, u64* bar, u32 parity, AeCtaCtl* ctl, u32* g_status, u32 site) {
+  if (ok) ok = mbar_wait(bar, parity, ctl, g_status, site);
+  return __all_sync(0xffffffffu, ok);
+}
+
 // The same wait run by every lane of a warp; the result is made warp-uniform by a vote.
 AE_DEVICE bool mbar_wait_w(u64* bar, u32 parity, AeCtaCtl* ctl, u32* g_status, u32 site) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, ctl, g_status, site));

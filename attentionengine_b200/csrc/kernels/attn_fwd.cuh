@@ -8,10 +8,9 @@
 //                     row i: it reads its 128 scores from TMEM, applies mask,
 //                     score_mod and the online recurrence in registers (no shuffles),
 //                     writes P back to TMEM as 16-bit pairs, rescales O when needed
-//                     and runs the epilogue.  (AE_RSPLIT = 2: four row warpgroups, two
-//                     threads per row with 64 columns each; the roles below move up.)
+//                     and runs the epilogue.
 //   warp 8          : TMA producer (Q once, K/V ring of AE_STAGES stages).
-//   warp 9          : tcgen05.mma issuer; owns the TMEM allocation.
+//   warp 9          : tcgen05.mma issuer; owns the TMEM allocation.  (Warps 10, 11 only give up registers.)
 // TMEM columns: S0 | S1 | O0 | O1 (P_t aliases the first half of S_t).
 // While one group runs its recurrence the tensor pipe runs the other tile's MMAs.
 //
@@ -37,30 +36,17 @@
 // runs two tiles ahead of P V, so the row threads find the next tile's scores ready when they finish a tile
 // (S MMA -> row pass -> P V MMA is no longer one chain per tile).
 #define AE_PINGPONG (AE_DECODE && AE_NQ == 1)
-// AE_TURNS = 1: the two row warpgroups take turns (named barriers 1 and 2 as a token), so that one group's row pass
-// runs while the tensor pipe works on the other tile.  Off by default: measured slower with all exponentials on the
-// special-function unit (a group's row pass is then longer than the other tile's two MMAs); a sweep candidate together
-// with AE_EXP_POLY_PERIOD.
-#ifndef AE_TURNS
-#define AE_TURNS 0
+// P of a tile is handed to the MMA warp in AE_P_PIECES column blocks, each on a barrier of its own: P V of the first block
+// runs under the exponentials of the next.
+#ifndef AE_P_PIECES
+#define AE_P_PIECES (AE_PINGPONG ? 1 : 2)
 #endif
-#if AE_TURNS && AE_DECODE
-#error "turn-taking is for the two-tile forward"
-#endif
-// AE_RSPLIT = 2: two threads per score row (warpgroups 2t and 2t + 1 work on q tile t, 64 kv columns each).  A row
-// pass is then half as long, which is what lets the two tiles alternate (AE_TURNS) with the tensor pipe busy on one
-// while the other's rows run.  Row reductions are completed between the two threads of a row by the generated
-// ae_row_xchg (shared memory slot + named barrier 3 + t).  The second half keeps its P in the second half of its own
-// score columns (16-bit pairs at column 96 ...), so that no thread writes TMEM columns another thread still reads.
-#ifndef AE_RSPLIT
-#define AE_RSPLIT 1
-#endif
-#if AE_RSPLIT != 1 && (AE_RSPLIT != 2 || AE_DECODE)
-#error "rows are split over two threads in the two-tile forward only"
-#endif
-#define AE_ROW_WARPS (8 * AE_RSPLIT)
-#define AE_NTHREADS (AE_ROW_WARPS * 32 + 64)
-#define AE_NC (AE_BN / AE_RSPLIT)  // score columns per row thread
+#define AE_ROW_WARPS (4 * AE_NQ)
+// One thread per row holds a tile's 128 scores, the P it makes of them and the packed block on its way to TMEM: the row
+// warpgroups take registers from the TMA / MMA warpgroup (launched with 168 per thread; 208 + 208 + 88 = 3 x 168; with 72
+// the MMA warp spills).
+#define AE_REG_SPLIT (!AE_PINGPONG)
+#define AE_NTHREADS (AE_ROW_WARPS * 32 + (AE_REG_SPLIT ? 128 : 64))
 #if AE_PINGPONG && AE_STAGES < 3
 #error "the two-ahead S GEMM needs three K / V stages"
 #endif
@@ -79,18 +65,22 @@
 #define AE_SMEM_K (AE_NQ * AE_Q_BYTES)
 #define AE_SMEM_V (AE_SMEM_K + AE_STAGES * AE_K_BYTES)
 #define AE_SMEM_BAR (AE_SMEM_V + AE_STAGES * AE_V_BYTES)
-#define AE_SMEM_XCH (AE_SMEM_BAR + 512)  // AE_RSPLIT = 2 only: [q tile][phase][half][row] partial row reductions
-#define AE_SMEM_STEPS (AE_SMEM_XCH + (AE_RSPLIT > 1 ? 2 * 2 * AE_RSPLIT * 128 * 4 : 0))  // mask mode 2 only: one word per kv tile
+#define AE_SMEM_STEPS (AE_SMEM_BAR + 512)  // mask mode 2 only: one word per kv tile
 #define AE_MAX_KT 2048                    // kv tiles a block list may cover (4 * AE_MAX_KT bytes of shared memory)
 
 struct AeFwdBars {
   u64 q_full[2];
+#if AE_PINGPONG
   u64 k_full[AE_STAGES];
   u64 k_empty[AE_STAGES];
   u64 v_full[AE_STAGES];
   u64 v_empty[AE_STAGES];
-  u64 s_full[2];
   u64 p_full[2];
+#else
+  u64 kv_full[AE_STAGES];  // fill n of the ring: V of step n - 1 and K of step n, on one barrier
+  u64 kv_empty[AE_STAGES];
+#endif
+  u64 s_full[2];
   u64 o_done[2];
   AeCtaCtl ctl;
   int n_steps;  // mask mode 2: length of the merged walk
@@ -152,12 +142,17 @@ ae_attn_fwd(const __grid_constant__ AeAttnFwdArgs args) {
 #define AE_SKV skv
 #else
 #define AE_SKV args.Skv
-  // heaviest (latest) q tiles first: better tail under a causal mask
-  const int qpair = (int)gridDim.x - 1 - (int)blockIdx.x;
-  const int hq = blockIdx.y;
-  const int b = blockIdx.z;
+  // One-dimensional grid: sections of args.sec (batch, q-head) units; inside a section all units' last q pair first, then
+  // all their last but one, ... (see ae_launch_attn_fwd for the choice of the section).
+  const int n_pair = (args.n_qt + 1) / 2;
+  const int per_sec = args.sec * n_pair;
+  const int sec0 = (int)blockIdx.x / per_sec * args.sec, in_sec = (int)blockIdx.x % per_sec;
+  const int n_unit = args.B * args.Hq - sec0 < args.sec ? args.B * args.Hq - sec0 : args.sec;
+  const int unit = sec0 + in_sec % n_unit;
+  const int hq = unit % args.Hq;
+  const int b = unit / args.Hq;
   const int hk = hq / (args.Hq / args.Hkv);
-  const int qt0 = qpair * 2;
+  const int qt0 = (n_pair - 1 - in_sec / n_unit) * 2;
   const int kt_off = 0;
 #endif
 
@@ -220,14 +215,21 @@ ae_attn_fwd(const __grid_constant__ AeAttnFwdArgs args) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars->q_full[i], 1);
       mbar_init(&bars->s_full[i], 1);
-      mbar_init(&bars->p_full[i], 4 * AE_RSPLIT);
+#if AE_PINGPONG
+      mbar_init(&bars->p_full[i], 4);
+#endif
       mbar_init(&bars->o_done[i], 1);
     }
     for (int i = 0; i < AE_STAGES; ++i) {
+#if AE_PINGPONG
       mbar_init(&bars->k_full[i], 1);
       mbar_init(&bars->k_empty[i], 1);
       mbar_init(&bars->v_full[i], 1);
       mbar_init(&bars->v_empty[i], 1);
+#else
+      mbar_init(&bars->kv_full[i], 1);
+      mbar_init(&bars->kv_empty[i], 1);
+#endif
     }
     mbar_fence_init();
   }
@@ -299,6 +301,10 @@ ae_attn_fwd(const __grid_constant__ AeAttnFwdArgs args) {
 #endif
   const u32 TM_S0 = 0, TM_S1 = 128, TM_O0 = 256, TM_O1 = 256 + AE_DV;
 
+  if (warp >= AE_ROW_WARPS) {
+#if AE_REG_SPLIT
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+#endif
   if (warp == AE_ROW_WARPS) {
     // =============================== TMA producer ===============================
     if (lane == 0) {
@@ -318,62 +324,62 @@ ae_attn_fwd(const __grid_constant__ AeAttnFwdArgs args) {
                       hq, (qt0 + t) * AE_BM, b);
       }
       AeKvStep st;
-      int it = 0;
-      while (next_step(st)) {
+#if AE_DECODE
+      // paged K / V (args.block_table): the pool is one batch of num_pages * 128 rows, tile kt of row b is a page
+      auto kv_row = [&](int kt) { return args.block_table ? args.block_table[(i64)b * args.max_pages + kt] * AE_BN : kt * AE_BN; };
+      const int kv_b = args.block_table ? 0 : b;
+#else
+      auto kv_row = [&](int kt) { return kt * AE_BN; };
+      const int kv_b = b;
+#endif
+      auto load_k = [&](int stage, int row0, u64* bar) {
+        for (int dh = 0; dh < AE_D / 64; ++dh)
+          tma_load_bshd(smem + AE_SMEM_K + stage * AE_K_BYTES + dh * (AE_BN * 128), &args.tm_k, bar, dh * 64, hk, row0, kv_b);
+      };
+      auto load_v = [&](int stage, int row0, u64* bar) {
+        for (int dh = 0; dh < AE_DV / 64; ++dh)
+          tma_load_bshd(smem + AE_SMEM_V + stage * AE_V_BYTES + dh * (AE_BN * 128), &args.tm_v, bar, dh * 64, hk, row0, kv_b);
+      };
+#if AE_PINGPONG
+      for (int it = 0; next_step(st); ++it) {
         const int stage = it % AE_STAGES;
         const u32 par = ((it / AE_STAGES) & 1) ^ 1;
-#if AE_DECODE
-        // paged K / V (args.block_table): the pool is one batch of num_pages * 128 rows, tile kt of row b is a page
-        const int kv_row0 = args.block_table ? args.block_table[(i64)b * args.max_pages + st.kt] * AE_BN : st.kt * AE_BN;
-        const int kv_b = args.block_table ? 0 : b;
-#else
-        const int kv_row0 = st.kt * AE_BN;
-        const int kv_b = b;
-#endif
+        const int row0 = kv_row(st.kt);
         if (!mbar_wait(&bars->k_empty[stage], par, ctl, args.status, 1)) break;
         mbar_arrive_expect_tx(&bars->k_full[stage], AE_K_BYTES);
-        for (int dh = 0; dh < AE_D / 64; ++dh)
-          tma_load_bshd(smem + AE_SMEM_K + stage * AE_K_BYTES + dh * (AE_BN * 128), &args.tm_k, &bars->k_full[stage],
-                      dh * 64, hk, kv_row0, kv_b);
+        load_k(stage, row0, &bars->k_full[stage]);
         if (!mbar_wait(&bars->v_empty[stage], par, ctl, args.status, 2)) break;
         mbar_arrive_expect_tx(&bars->v_full[stage], AE_V_BYTES);
-        for (int dh = 0; dh < AE_DV / 64; ++dh)
-          tma_load_bshd(smem + AE_SMEM_V + stage * AE_V_BYTES + dh * (AE_BN * 128), &args.tm_v, &bars->v_full[stage],
-                      dh * 64, hk, kv_row0, kv_b);
-        ++it;
+        load_v(stage, row0, &bars->v_full[stage]);
       }
+#else
+      // fill n: V of step n - 1 (not for n = 0) and K of step n (not past the last step)
+      int v_row = 0;
+      bool have = next_step(st);
+      for (int n = 0; have || n > 0; ++n) {
+        const int stage = n % AE_STAGES;
+        if (!mbar_wait(&bars->kv_empty[stage], ((n / AE_STAGES) & 1) ^ 1, ctl, args.status, 1)) break;
+        mbar_arrive_expect_tx(&bars->kv_full[stage], (have ? AE_K_BYTES : 0) + (n > 0 ? AE_V_BYTES : 0));
+        const int row0 = have ? kv_row(st.kt) : 0;
+        if (n > 0) load_v(stage, v_row, &bars->kv_full[stage]);
+        if (!have) break;
+        load_k(stage, row0, &bars->kv_full[stage]);
+        v_row = row0;
+        have = next_step(st);
+      }
+#endif
     }
   } else if (warp == AE_ROW_WARPS + 1) {
     // =============================== MMA issuer =================================
-    if (lane == 0) {
-      const u32 idesc_s = umma_idesc_f16(AE_BM, AE_BN, AE_BF16, 0, 0);
-      const u32 idesc_o = umma_idesc_f16(AE_BM, AE_DV, AE_BF16, 0, 1);
-      const u32 q_addr = smem_u32(smem + AE_SMEM_Q);
-      const u32 k_addr = smem_u32(smem + AE_SMEM_K);
-      const u32 v_addr = smem_u32(smem + AE_SMEM_V);
-      const u64 dk0 = umma_base_k(k_addr);
-      const u64 dv0 = umma_base_mn(v_addr, AE_BN);
-      // q tile index as a compile-time constant: every per-tile quantity stays in a named register
-      auto issue_s = [&](auto T, int stage) {
-        constexpr int t = decltype(T)::value;
-        const u64 da = umma_base_k(q_addr + t * AE_Q_BYTES);
-        const u64 db = dk0 + (u64)((stage * AE_K_BYTES) >> 4);
-        const u32 d = tmem + (t ? TM_S1 : TM_S0);
-#pragma unroll
-        for (int kk = 0; kk < AE_D / 16; ++kk)
-          umma_ss(d, umma_step_k(da, kk, AE_BM), umma_step_k(db, kk, AE_BN), idesc_s, kk > 0);
-      };
-      auto issue_pv = [&](auto T, int stage, u32 acc) {
-        constexpr int t = decltype(T)::value;
-        const u64 db = dv0 + (u64)((stage * AE_V_BYTES) >> 4);
-        const u32 d = tmem + (t ? TM_O1 : TM_O0);
-        const u32 a = tmem + (t ? TM_S1 : TM_S0);
-#pragma unroll
-        for (int kk = 0; kk < AE_BN / 16; ++kk)
-          umma_ts(d, a + kk * 8 + ((AE_RSPLIT > 1 && kk >= AE_BN / 32) ? 64 : 0), umma_step_mn(db, kk), idesc_o, acc | (kk > 0));
-      };
-
+    const u32 idesc_s = umma_idesc_f16(AE_BM, AE_BN, AE_BF16, 0, 0);
+    const u32 idesc_o = umma_idesc_f16(AE_BM, AE_DV, AE_BF16, 0, 1);
+    const u32 q_addr = smem_u32(smem + AE_SMEM_Q);
+    const u32 k_addr = smem_u32(smem + AE_SMEM_K);
+    const u32 v_addr = smem_u32(smem + AE_SMEM_V);
+    const u64 dk0 = umma_base_k(k_addr);
+    const u64 dv0 = umma_base_mn(v_addr, AE_BN);
 #if AE_PINGPONG
+    if (lane == 0) {
       // kv tiles kt_off .. kt_off + n_steps - 1 in order (no mask in a decode build); tile n uses K / V stage n % AE_STAGES,
       // S region n & 1 and phase n >> 1 of that region's s_full / p_full; O (region 0) takes every P V.
       auto s_into = [&](int n) {
@@ -425,95 +431,102 @@ ae_attn_fwd(const __grid_constant__ AeAttnFwdArgs args) {
         ok = mbar_wait(&bars->v_empty[l % AE_STAGES], (l / AE_STAGES) & 1, ctl, args.status, 12) &&
              mbar_wait(&bars->k_empty[l % AE_STAGES], (l / AE_STAGES) & 1, ctl, args.status, 13);
       }
+    }
 #else
-      // The walk is consumed one step ahead for the S GEMMs.
-      AeKvStep cur, nxt;
-      bool ok = true;
-      bool have = next_step(cur);
-      int it = 0;
-      u32 np0 = 0, np1 = 0;  // P tiles consumed per q tile
-      u32 q_ready = 0;       // bit t: Q tile t has landed
+    // All 32 lanes run the control flow, one elected lane issues.  What bounds the kernel is this warp: with six barrier
+    // waits (160 - 200 clk each next to the MMAs' shared-memory reads) and six commits per step it needed 3900 clk for the
+    // 2048 clk of MMAs of a step, whatever the row threads did.  Now a step has one mbarrier wait (K of the next step and V
+    // of this one arrive together), named barriers for the P hand-off (about 20 clk), and three commits.
+    auto issue_s = [&](auto T, int stage) {
+      constexpr int t = decltype(T)::value;
+      const u64 da = umma_base_k(q_addr + t * AE_Q_BYTES);
+      const u64 db = dk0 + (u64)((stage * AE_K_BYTES) >> 4);
+      const u32 d = tmem + (t ? TM_S1 : TM_S0);
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < AE_D / 16; ++kk)
+          umma_ss(d, umma_step_k(da, kk, AE_BM), umma_step_k(db, kk, AE_BN), idesc_s, kk > 0);
+        umma_commit(&bars->s_full[t]);
+      }
+    };
+    // q tile and column block of P as compile-time constants: every per-tile quantity stays in a named register
+    auto issue_pv = [&](auto T, auto PC, int stage, u32 acc) {
+      constexpr int t = decltype(T)::value;
+      constexpr int k0 = decltype(PC)::value * (AE_BN / 16 / AE_P_PIECES);
+      const u64 db = dv0 + (u64)((stage * AE_V_BYTES) >> 4);
+      const u32 d = tmem + (t ? TM_O1 : TM_O0);
+      const u32 a = tmem + (t ? TM_S1 : TM_S0);
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = k0; kk < k0 + AE_BN / 16 / AE_P_PIECES; ++kk)
+          umma_ts(d, a + kk * 8, umma_step_mn(db, kk), idesc_o, acc | (kk > 0));
+      }
+    };
+    AeKvStep cur, nxt;
+    bool have = next_step(cur);
+    bool ok = true;
+    u32 np0 = 0, np1 = 0;  // P tiles consumed per q tile
+    if (have) {
+      ok = mbar_wait_w(&bars->kv_full[0], 0, ctl, args.status, 3);
       auto first_s = [&](auto T) {
         constexpr int t = decltype(T)::value;
         if (!ok || !(cur.flags & (1u << t))) return;
-        ok = mbar_wait(&bars->q_full[t], 0, ctl, args.status, 4);
-        q_ready |= 1u << t;
-        tc_fence_after_sync();
-        issue_s(T, 0);
-        umma_commit(&bars->s_full[t]);
+        ok = mbar_wait_w(&bars->q_full[t], 0, ctl, args.status, 4);
+        if (ok) issue_s(T, 0);
       };
-      if (have) {
-        ok = mbar_wait(&bars->k_full[0], 0, ctl, args.status, 3);
-        tc_fence_after_sync();
-        first_s(AeInt<0>{});
-        first_s(AeInt<1>{});
-        umma_commit(&bars->k_empty[0]);
-      }
-      while (have && ok) {
-        const int stage = it % AE_STAGES;
-        const u32 par = (it / AE_STAGES) & 1;
-        const bool have_n = next_step(nxt);
-        const int nstage = (it + 1) % AE_STAGES;
-        const u32 npar = ((it + 1) / AE_STAGES) & 1;
-        bool v_ready = false, k_ready = false;
-        auto tile_step = [&](auto T, u32& np) {
-          constexpr int t = decltype(T)::value;
-          if (!ok) return;
-          AE_TRW(true, 0, it * 8 + t * 4 + 0);
-          if (cur.flags & (1u << t)) {
-            ok = mbar_wait(&bars->p_full[t], np & 1, ctl, args.status, 5);
-            if (!ok) return;
-            AE_TRW(true, 0, it * 8 + t * 4 + 1);
-            if (!v_ready) {
-              ok = mbar_wait(&bars->v_full[stage], par, ctl, args.status, 6);
-              if (!ok) return;
-              v_ready = true;
-            }
-            tc_fence_after_sync();
-            issue_pv(T, stage, np > 0);
-            umma_commit(&bars->o_done[t]);
-            np++;
-            AE_TRW(true, 0, it * 8 + t * 4 + 2);
-          }
-          if (have_n && (nxt.flags & (1u << t))) {
-            if (!k_ready) {
-              ok = mbar_wait(&bars->k_full[nstage], npar, ctl, args.status, 7);
-              if (!ok) return;
-              k_ready = true;
-            }
-            if (!(q_ready & (1u << t))) {  // Q of this tile is awaited once
-              ok = mbar_wait(&bars->q_full[t], 0, ctl, args.status, 8);
-              if (!ok) return;
-              q_ready |= 1u << t;
-            }
-            // (no tcgen05 fence: the waits above are for shared-memory operands; the S region's last TMEM accesses by
-            // other threads were fenced with the p_full wait of the step that made them)
-            issue_s(T, nstage);
-            umma_commit(&bars->s_full[t]);
-            AE_TRW(true, 0, it * 8 + t * 4 + 3);
-          }
-        };
-        tile_step(AeInt<0>{}, np0);
-        tile_step(AeInt<1>{}, np1);
-        if (!ok) break;
-        umma_commit(&bars->v_empty[stage]);
-        if (have_n) umma_commit(&bars->k_empty[nstage]);
-        cur = nxt;
-        have = have_n;
-        ++it;
-      }
-      // every commit of this thread has arrived before the CTA may retire (the last slot releases have no other waiter)
-      if (ok && it > 0) {
-        const int l = it - 1;
-        ok = mbar_wait(&bars->v_empty[l % AE_STAGES], (l / AE_STAGES) & 1, ctl, args.status, 12) &&
-             mbar_wait(&bars->k_empty[l % AE_STAGES], (l / AE_STAGES) & 1, ctl, args.status, 13);
-      }
-#endif  // AE_PINGPONG
+      first_s(AeInt<0>{});
+      if constexpr (AE_NQ > 1) first_s(AeInt<1>{});
+      umma_commit_w(&bars->kv_empty[0]);
     }
+    int n = 0;  // fill of the ring that holds V of this step and K of the next
+    while (have && ok) {
+      ++n;
+      const int stage = n % AE_STAGES;
+      const bool have_n = next_step(nxt);
+      if (!have_n) nxt.flags = 0;
+      // A row group that gave up on a wait arrives for that step and leaves; the abort word then ends this loop before it
+      // would wait for the group's next arrival.
+      ok = mbar_wait_w(&bars->kv_full[stage], (n / AE_STAGES) & 1, ctl, args.status, 6) && !ctl->abort;
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      auto tile_step = [&](auto T, u32& np) {
+        constexpr int t = decltype(T)::value;
+        if (!(cur.flags & (1u << t))) return;
+        AE_TRW(lane == 0, 0, (n - 1) * 8 + t * 4 + 0);
+        auto block = [&](auto PC) {
+          constexpr int k = decltype(PC)::value;
+          named_bar_sync(1 + t * AE_P_PIECES + k, 128 + 32);  // block k of P is in TMEM
+          tc_fence_after_sync();
+          AE_TRW(lane == 0 && k == 0, 0, (n - 1) * 8 + t * 4 + 1);
+          issue_pv(T, PC, stage, k > 0 ? 1u : (u32)(np > 0));
+        };
+        block(AeInt<0>{});
+        if constexpr (AE_P_PIECES > 1) block(AeInt<1>{});
+        np++;
+        AE_TRW(lane == 0, 0, (n - 1) * 8 + t * 4 + 2);
+        // S of the next step over P of this one (MMAs run in issue order); s_full also says that P V has completed
+        if (nxt.flags & (1u << t))
+          issue_s(T, stage);
+        else
+          umma_commit_w(&bars->o_done[t]);  // the tile's last P V
+        AE_TRW(lane == 0, 0, (n - 1) * 8 + t * 4 + 3);
+      };
+      tile_step(AeInt<0>{}, np0);
+      if constexpr (AE_NQ > 1) tile_step(AeInt<1>{}, np1);
+      umma_commit_w(&bars->kv_empty[stage]);
+      cur = nxt;
+      have = have_n;
+    }
+    // every commit of this warp has arrived before the CTA may retire (the last slot release has no other waiter)
+    if (ok && n > 0) ok = mbar_wait_w(&bars->kv_empty[n % AE_STAGES], (n / AE_STAGES) & 1, ctl, args.status, 12);
+#endif  // AE_PINGPONG
+  }
   } else {
+#if AE_REG_SPLIT
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+#endif
     // =============================== row warpgroups =============================
-    const int t = warp / (4 * AE_RSPLIT);    // q tile of this group
-    const u32 half = (warp >> 2) & (AE_RSPLIT - 1);  // which columns of the row this thread takes
+    const int t = warp / 4;                  // q tile of this group
     const u32 row = threadIdx.x & 127;       // row inside the tile == TMEM lane
     const u32 lane_base = ((warp & 3) * 32) << 16;
     const u32 tm_s = tmem + (t ? TM_S1 : TM_S0) + lane_base;
@@ -542,51 +555,27 @@ ae_attn_fwd(const __grid_constant__ AeAttnFwdArgs args) {
 
     AeRow st;
     st.init();
-#if AE_RSPLIT > 1
-    st.xch = (volatile float*)(smem + AE_SMEM_XCH) + t * (2 * AE_RSPLIT * 128);
-    st.xme = half * 128 + row;
-    st.xother = (half ^ 1u) * 128 + row;
-    st.xbar = 3 + t;
-    st.xn = AE_RSPLIT * 128;
-    st.xphase = 0;
-#endif
     u32 n_done = 0;
     bool ok = true;
     AeKvStep step;
-#if AE_TURNS
-    // group 0 goes first: group 1 hands it the token once before the walk.  Every group passes the token at every
-    // step of the walk, also at steps its tile sits out, so the two sides stay in step whatever the masks are.
-    if (t == 1) named_bar_arrive(1, AE_RSPLIT * 256);
-#endif
     while (next_step(step)) {
-#if AE_TURNS
-      if (!(step.flags & (1u << t))) {
-        named_bar_sync(1 + t, AE_RSPLIT * 256);
-        named_bar_arrive(2 - t, AE_RSPLIT * 256);
-        continue;
-      }
-#else
       if (!(step.flags & (1u << t))) continue;
-#endif
 #if AE_PINGPONG
       // scores of this group's n-th tile: region n & 1, phase n >> 1 of that region's barriers
       const u32 rgn = n_done & 1u;
       const u32 tm_s_n = tmem + (rgn ? TM_S1 : TM_S0) + lane_base;
       u64* const s_bar = &bars->s_full[rgn];
-      u64* const p_bar = &bars->p_full[rgn];
+      auto p_ready = [&](auto) { mbar_arrive_warp(&bars->p_full[rgn]); };
       const u32 s_par = (n_done >> 1) & 1u;
 #else
       const u32 tm_s_n = tm_s;
       u64* const s_bar = &bars->s_full[t];
-      u64* const p_bar = &bars->p_full[t];
+      auto p_ready = [&](auto K) { named_bar_arrive(1 + t * AE_P_PIECES + decltype(K)::value, 128 + 32); };
       const u32 s_par = n_done & 1u;
 #endif
-      AE_TRW((warp & 3) == 0 && half == 0 && lane == 0, 1 + t, n_done * 8 + 0);
-      ok = ok && mbar_wait(s_bar, s_par, ctl, args.status, 9);
-      AE_TRW((warp & 3) == 0 && half == 0 && lane == 0, 1 + t, n_done * 8 + 1);
-#if AE_TURNS
-      named_bar_sync(1 + t, AE_RSPLIT * 256);  // this group's turn
-#endif
+      AE_TRW((warp & 3) == 0 && lane == 0, 1 + t, n_done * 8 + 0);
+      ok = mbar_wait_row(ok, s_bar, s_par, ctl, args.status, 9);
+      AE_TRW((warp & 3) == 0 && lane == 0, 1 + t, n_done * 8 + 1);
       tc_fence_after_sync();
 #if AE_MASK_MODE == 2
       if ((step.flags >> (4 + t)) & 1u) {
@@ -595,92 +584,95 @@ ae_attn_fwd(const __grid_constant__ AeAttnFwdArgs args) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) z[i] = 0u;
 #pragma unroll
-        for (int hh = (int)half; hh < AE_BN / 64; hh += AE_RSPLIT) tmem_st32(tm_s_n + hh * 32 + (AE_RSPLIT > 1 ? hh * 64 : 0), z);
+        for (int hh = 0; hh < AE_BN / 64; ++hh) tmem_st32(tm_s_n + hh * 32, z);
         tc_wait_st();
         tc_fence_before_sync();
-        mbar_arrive_warp(p_bar);
-#if AE_TURNS
-        named_bar_arrive(2 - t, AE_RSPLIT * 256);
-#endif
+        p_ready(AeInt<0>{});
+        if constexpr (AE_P_PIECES > 1) p_ready(AeInt<1>{});
         ++n_done;
+        if (!ok) break;
         continue;
       }
 #endif
-      float s[AE_NC];
-#if AE_RSPLIT > 1
-      tmem_ld_f32x64(tm_s_n + half * AE_NC, s);
-#else
+      float s[AE_BN];
       tmem_ld_f32x128(tm_s_n, s);
-#endif
-      AE_TRW((warp & 3) == 0 && half == 0 && lane == 0, 1 + t, n_done * 8 + 2);
-      const int kv0 = step.kt * AE_BN + (int)half * AE_NC;  // first kv column of this thread
+      AE_TRW((warp & 3) == 0 && lane == 0, 1 + t, n_done * 8 + 2);
+      const int kv0 = step.kt * AE_BN;
       const bool tail = (step.kt * AE_BN + AE_BN > AE_SKV);
       const bool partial = (step.flags >> (2 + t)) & 1u;
-      if (partial || tail) {
+      // Compile-time columns and selects: with `partial`, `tail` and the mask in one short-circuit condition every element
+      // became a branch (10,700 clk for a masked tile, not 1,900).
+      if (tail) {
+        const int lim = AE_SKV - kv0;
 #pragma unroll
-        for (int c = 0; c < AE_NC; ++c) {
-          const int kv_idx = kv0 + c;
-          bool keep = kv_idx < AE_SKV;
-#if AE_MASK_MODE != 0
-          if (partial) keep = keep && ae_mask(b, h_row, q_idx, kv_idx);
-#endif
-#if AE_MASK_NEG_INF
-          if (!keep) s[c] = -__int_as_float(0x7f800000);
-#else
-          if (kv_idx >= AE_SKV) s[c] = 0.f;  // additive mask value 0: scores stay as they are
-          (void)keep;
-#endif
-        }
+        for (int c = 0; c < AE_BN; ++c) s[c] = c < lim ? s[c] : (AE_MASK_NEG_INF ? -__int_as_float(0x7f800000) : 0.f);
       }
-      const float o_scale = ae_online_fwd<AE_NC>(s, st, b, h_row, q_idx, kv0, cu);
-#if AE_TURNS
-      named_bar_arrive(2 - t, AE_RSPLIT * 256);  // the exponentials are done: the other group's turn
-#endif
-
-      AE_TRW((warp & 3) == 0 && half == 0 && lane == 0, 1 + t, n_done * 8 + 3);
-      // P -> TMEM (16-bit pairs, column c/2 holds kv columns c, c+1)
-      {
-        u32 pk[32];
+#if AE_MASK_MODE != 0 && AE_MASK_NEG_INF  // (additive mask value 0: scores stay as they are)
+      if (partial) {
 #pragma unroll
-        for (int hh = 0; hh < AE_NC / 64; ++hh) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) pk[i] = pack2<AE_BF16>(s[hh * 64 + 2 * i], s[hh * 64 + 2 * i + 1]);
-          tmem_st32(tm_s_n + hh * 32 + (AE_RSPLIT > 1 ? half * 96 : 0), pk);
-        }
+        for (int c = 0; c < AE_BN; ++c) s[c] = ae_mask(b, h_row, q_idx, kv0 + c) ? s[c] : -__int_as_float(0x7f800000);
       }
+#endif
+      ae_online_tile<AE_P_PIECES>(s, st, b, h_row, q_idx, kv0, cu, [&](auto K, float o_scale, float (&p)[AE_BN]) {
+        constexpr int k = decltype(K)::value;
+        constexpr int W = AE_BN / AE_P_PIECES;  // columns of a block
+        if constexpr (k == -1) {
 #if !AE_O_SCALE_ONE
-      // O is rescaled only when some row of the warp needs it; only then must the previous step's P V have
-      // completed.  (A skipped wait cannot alias: o_done runs at most one phase ahead of this warp's arrivals.)
-      if (n_done > 0 && __any_sync(0xffffffffu, o_scale != 1.0f)) {
-        ok = ok && mbar_wait(&bars->o_done[t], (n_done - 1) & 1, ctl, args.status, 10);
-        tc_fence_after_sync();
-#pragma unroll
-        for (int c = (int)half; c < AE_DV / 32; c += AE_RSPLIT) {  // the threads of a row share its O columns
-          float f[32];
-          u32 r[32];
-          tmem_ld_f32x32(tm_o + c * 32, f);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(f[i] * o_scale);
-          tmem_st32(tm_o + c * 32, r);
-        }
-      }
+          // O is rescaled only when some row of the warp needs it.
+#if AE_PINGPONG
+          // Only then must the previous step's P V have completed.  (A skipped wait cannot alias: o_done runs at most one
+          // phase ahead of this warp's arrivals.)
+          if (n_done > 0 && __any_sync(0xffffffffu, o_scale != 1.0f)) {
+            ok = mbar_wait_row(ok, &bars->o_done[t], (n_done - 1) & 1, ctl, args.status, 10);
+            tc_fence_after_sync();
+#else
+          // The previous step's P V has completed: it was issued before these scores' S GEMM.
+          if (n_done > 0 && __any_sync(0xffffffffu, o_scale != 1.0f)) {
 #endif
-      tc_wait_st();
-      AE_TRW((warp & 3) == 0 && half == 0 && lane == 0, 1 + t, n_done * 8 + 4);
-      tc_fence_before_sync();
-      mbar_arrive_warp(p_bar);
-      AE_TRW((warp & 3) == 0 && half == 0 && lane == 0, 1 + t, n_done * 8 + 5);
+#pragma unroll
+            for (int c = 0; c < AE_DV / 32; ++c) {
+              float f[32];
+              u32 r[32];
+              tmem_ld_f32x32(tm_o + c * 32, f);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(f[i] * o_scale);
+              tmem_st32(tm_o + c * 32, r);
+            }
+          }
+#endif
+        } else {
+          AE_TRW((warp & 3) == 0 && lane == 0 && k == AE_P_PIECES - 1, 1 + t, n_done * 8 + 3);
+          // P -> TMEM (16-bit pairs, column c/2 holds kv columns c, c+1)
+          {
+            u32 pk[32];
+#pragma unroll
+            for (int hh = 0; hh < W / 64; ++hh) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) pk[i] = pack2<AE_BF16>(p[k * W + hh * 64 + 2 * i], p[k * W + hh * 64 + 2 * i + 1]);
+              tmem_st32(tm_s_n + k * (W / 2) + hh * 32, pk);
+            }
+          }
+          tc_wait_st();
+          AE_TRW((warp & 3) == 0 && lane == 0 && k == AE_P_PIECES - 1, 1 + t, n_done * 8 + 4);
+          tc_fence_before_sync();
+          p_ready(K);
+        }
+      });
+      AE_TRW((warp & 3) == 0 && lane == 0, 1 + t, n_done * 8 + 5);
       ++n_done;
+#if !AE_PINGPONG
+      if (!ok) break;
+#endif
     }
 
     // ---- epilogue ------------------------------------------------------------------
 #if AE_PINGPONG
     // The S GEMM of the last tile was issued before the P V of the tile before it, so o_done may still be two phases
     // short here: a parity wait can only tell neighbouring phases apart, hence one wait per missing phase.
-    if (n_done > 1) ok = ok && mbar_wait(&bars->o_done[t], (n_done - 2) & 1, ctl, args.status, 14);
+    if (n_done > 1) ok = mbar_wait_row(ok, &bars->o_done[t], (n_done - 2) & 1, ctl, args.status, 14);
 #endif
     if (n_done > 0) {
-      ok = ok && mbar_wait(&bars->o_done[t], (n_done - 1) & 1, ctl, args.status, 11);
+      ok = mbar_wait_row(ok, &bars->o_done[t], AE_PINGPONG ? (n_done - 1) & 1 : 0, ctl, args.status, 11);
       tc_fence_after_sync();
     }
     // tcgen05.ld is warp-collective: every lane of the warp runs it; only the stores are per-row.
@@ -693,7 +685,7 @@ ae_attn_fwd(const __grid_constant__ AeAttnFwdArgs args) {
       float* prow = args.o_part + part_row * AE_DV;
 #endif
 #pragma unroll
-      for (int c = (int)half; c < AE_DV / 32; c += AE_RSPLIT) {
+      for (int c = 0; c < AE_DV / 32; ++c) {
         float r[32];
         if (n_done > 0) {
           tmem_ld_f32x32(tm_o + c * 32, r);
@@ -724,7 +716,7 @@ ae_attn_fwd(const __grid_constant__ AeAttnFwdArgs args) {
         }
       }
 #if AE_NFINAL > 0
-      if (store && half == 0) {
+      if (store) {
         float fr[AE_NFINAL];
         ae_final_rowscales(st, fr);
 #pragma unroll

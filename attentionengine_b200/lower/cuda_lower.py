@@ -83,6 +83,7 @@ class Emitter:
         self.n = n_cols
         self.tile_mode = tile_mode  # "array": tiles are float[N]; "scalar": inside a per-element function
         self.lines: list[str] = []
+        self.tile_exprs: dict[str, str] = {}          # tile array -> its element expression (of column c)
         self.names: dict[int, tuple[str, str]] = {}   # id(value) -> (expr, kind), materialised
         self.aff: dict[int, tuple] = {}               # id(value) -> (base (expr, kind), a Scal|None, b Scal|None)
         self.used_leaves: set[str] = set()
@@ -184,8 +185,8 @@ class Emitter:
     def _new_tile(self, expr_of_c: str) -> tuple[str, str]:
         name = self._tmp()
         if self.tile_mode == "array":
-            self.lines.append(f"float {name}[{self.n}];")
-            self.lines.append(f"#pragma unroll\nfor (int c = 0; c < {self.n}; ++c) {name}[c] = {expr_of_c};")
+            self.tile_exprs[name] = expr_of_c
+            self.lines.append(f"float {name}[{self.n}];\n  #pragma unroll\n  for (int c = 0; c < {self.n}; ++c) {name}[c] = {expr_of_c};")
             return name + "[{c}]", "tile"
         self.lines.append(f"const float {name} = {expr_of_c};")
         return name, "tile"
@@ -612,6 +613,36 @@ def _lazy_max_is_invariant(online_func, raw, t_scores, rs_in, new_scores, new_rs
         return False
 
 
+def _split_recurrence(em: Emitter, p_expr: str, o_expr: str):
+    """The emitted statements of online_fwd in three parts: what the row scalars behind P and o_scale need (``pre``), the
+    element-wise statements that make P from them (``tiles``: (array name, element expression)), which may run column block by
+    column block, and what only the new row states need (``post``).  Temporaries are numbered in the order of their
+    definition, so a statement defines the highest number it names."""
+    def tokens(text):
+        return {int(n) for n in re.findall(r"\bt(\d+)", text)}
+
+    groups: dict[int, list[str]] = {}
+    for line in em.lines:
+        groups.setdefault(max(tokens(line)), []).append(line)
+    deps = {n: set().union(*(tokens(l) for l in ls)) - {n} for n, ls in groups.items()}
+    tile = {n for n in groups if f"t{n}" in em.tile_exprs}
+
+    def closure(ns):
+        todo, seen = list(ns), set()
+        while todo:
+            n = todo.pop()
+            if n not in seen:
+                seen.add(n)
+                todo += deps[n]
+        return seen
+
+    need = closure(tokens(p_expr))
+    pre = closure({n for n in need if n not in tile} | tokens(o_expr))
+    part = {n: "pre" if n in pre else "tiles" if n in need else "post" for n in groups}
+    text = {k: "".join("  " + l + "\n" for n in sorted(groups) if part[n] == k for l in groups[n]) for k in ("pre", "post")}
+    return text["pre"], [(f"t{n}", em.tile_exprs[f"t{n}"]) for n in sorted(groups) if part[n] == "tiles"], text["post"]
+
+
 def lower_attention(score_mod, mask_mod, online_func, custom_fwd_inputs: CustomIO, *, D: int, DV: int, bf16: bool,
                     mask_mode: int, stages: int = 2, mask_value: str = "-inf") -> LoweredAttention:
     """Trace the user callables and produce the kernel preludes.
@@ -702,16 +733,31 @@ def lower_attention(score_mod, mask_mod, online_func, custom_fwd_inputs: CustomI
     o_scale_one = (o_kind == "const" and float(o_expr.rstrip("f")) == 1.0)
     new_exprs = {k: em.ref(v) for k, v in new_rs.items()}
     p_expr = em.ref(new_scores, "c")
-    body = em.body()
-    body += "".join(f"  const float n_{k} = {e};\n" for k, e in new_exprs.items())
-    body += f"  const float o_scale_ = {o_expr};\n"
-    if p_expr != "s[c]":
-        body += f"  #pragma unroll\nfor (int c = 0; c < N; ++c) s[c] = {p_expr};\n"
-    body += "".join(f"  st.st_{k} = n_{k};\n" for k in new_exprs)
-    src.append("// s[] holds the raw (masked) scores q.k on entry and P on exit: score_mod and online_fwd in one pass\n"
+    pre, tiles, post = _split_recurrence(em, p_expr, o_expr)
+    element = "".join(f"      {n}[c] = {e};\n" for n, e in tiles) + f"      p_[c] = {p_expr};\n"
+    src.append("// One score tile of a row, score_mod and online_fwd in one pass.  s[] holds the raw (masked) scores q.k.  `sink` is\n"
+               "// called with AeInt<-1> once o_scale is known, then with AeInt<k> as soon as the k-th of PIECES column blocks of P is\n"
+               "// made; what only the row states need (the row sum of a softmax) follows the last block.\n"
+               "template <int PIECES, int N, class Sink>\nAE_DEVICE void ae_online_tile(float (&s)[N], AeRow& st, int b, int h, int q_idx, "
+               "int kv0, const AeCustom& cu, Sink&& sink) {\n"
+               "  static_assert(N % (8 * PIECES) == 0, \"tile loops take eight columns at a time\");\n"
+               + pre + f"  const float o_scale_ = {o_expr};\n  float p_[N];\n"
+               + "".join(f"  float {n}[N];\n" for n, _ in tiles)
+               + "  sink(AeInt<-1>{}, o_scale_, p_);\n"
+               "  auto block = [&](auto K) {\n    constexpr int c0 = decltype(K)::value * (N / PIECES);\n"
+               "    #pragma unroll\n    for (int c = c0; c < c0 + N / PIECES; ++c) {\n" + element + "    }\n    sink(K, o_scale_, p_);\n  };\n"
+               "  block(AeInt<0>{});\n"
+               "  if constexpr (PIECES > 1) block(AeInt<1>{});\n"
+               "  if constexpr (PIECES > 2) { block(AeInt<2>{}); block(AeInt<3>{}); }\n"
+               + post + "".join(f"  const float n_{k} = {e};\n" for k, e in new_exprs.items())
+               + "".join(f"  st.st_{k} = n_{k};\n" for k in new_exprs) + "}\n"
+               "// The same with P left in s[]; returns o_scale.\n"
                "template <int N>\nAE_DEVICE float ae_online_fwd(float (&s)[N], AeRow& st, int b, int h, int q_idx, "
-               "int kv0, const AeCustom& cu) {\n  static_assert(N % 8 == 0, \"tile loops take eight columns at a time\");\n"
-               + body + "  return o_scale_;\n}\n")
+               "int kv0, const AeCustom& cu) {\n  float osc = 1.f, p[N];\n"
+               "  ae_online_tile<1>(s, st, b, h, q_idx, kv0, cu, [&](auto K, float o_scale, float (&x)[N]) {\n"
+               "    if constexpr (decltype(K)::value == -1) {\n      osc = o_scale;\n    } else {\n"
+               "      #pragma unroll\n      for (int c = 0; c < N; ++c) p[c] = x[c];\n    }\n  });\n"
+               "  #pragma unroll\n  for (int c = 0; c < N; ++c) s[c] = p[c];\n  return osc;\n}\n")
 
     # ---- epilogue --------------------------------------------------------------------------------------
     o_sym = SymbolicArray("o", Var("o"), shape_idx=["block_M", "dimv"])
