@@ -70,7 +70,7 @@ class AttnDecode:
                 comb = (rt.KERNEL_DIR / "mla_combine.cuh").read_text().replace("//%%AE_COMBINE_FUNCTOR%%", functor)
                 head = (rt.KERNEL_DIR / "ae_sm100.cuh").read_text().replace("#pragma once\n", "") + \
                     (rt.KERNEL_DIR / "ae_args.h").read_text()
-                defs = f"#define AE_BF16 {int(bf16)}\n#define AE_NFINAL {len(self.low.final_names)}\n"
+                defs = f"#define AE_BF16 {int(bf16)}\n#define AE_NFINAL {len(self.low.final_names)}\n#define AE_DV {DV}\n"
                 self.combine_src = head + defs + comb
                 cfg2 = rt.KernelConfig(kind=rt.KIND_MLA_COMBINE, dtype=tag, head_dim=D, head_dim_v=DV, threads=128,
                                        smem_bytes=0)

@@ -13,7 +13,6 @@ import torch
 from .. import runtime as rt
 from ..lower.cuda_lower import lower_attention, lower_combine
 
-MLA_BN = 64  # kv rows per tile: five of the nine query blocks (80 KB) and two 72 KB KV stages fill shared memory
 N_SM = 148
 
 
@@ -29,54 +28,46 @@ class MlaDecode:
         bf16 = dtype == torch.bfloat16
         self.low = lower_attention(score_mod, None, online_func, custom_fwd_inputs, D=D, DV=DV, bf16=bf16, mask_mode=0)
         tag = rt.DTYPE_BF16 if bf16 else rt.DTYPE_F16
-        prelude = self.low.prelude_fwd + f"#define AE_MLA_BN {MLA_BN}\n"
-        smem = 5 * 128 * 128 + 2 * 9 * MLA_BN * 128 + 256 + 1024  # 230,656 B of the 232,448 a CTA can have
+        # Q and K (9 blocks of 64 x 128 B each), V (4 blocks of 128 x 128 B), P, barriers, exchanged row reductions, alignment
+        smem = 18 * 64 * 128 + 4 * 128 * 128 + 2 * 64 * 128 + 512 + 1024 + 1024
         cfg = rt.KernelConfig(kind=rt.KIND_MLA_DECODE, dtype=tag, head_dim=D, head_dim_v=DV, threads=192,
                               smem_bytes=smem, stages=1, mask_mode=0)
-        cfg.reserved[0] = MLA_BN
-        self.src = rt.kernel_source("mla_decode.cuh", prelude=prelude)
+        self.src = rt.kernel_source("mla_decode.cuh", prelude=self.low.prelude_fwd, defines={"AE_RSPLIT": 2, "AE_XCH_ROWS": 64})
         self.decode = rt.compile_module(self.src, "ae_mla_decode", cfg)
         comb = (rt.KERNEL_DIR / "mla_combine.cuh").read_text().replace("//%%AE_COMBINE_FUNCTOR%%", lower_combine(online_func))
         cfg2 = rt.KernelConfig(kind=rt.KIND_MLA_COMBINE, dtype=tag, head_dim=D, head_dim_v=DV, threads=128, smem_bytes=0)
         head = (rt.KERNEL_DIR / "ae_sm100.cuh").read_text().replace("#pragma once\n", "") + (rt.KERNEL_DIR / "ae_args.h").read_text()
-        defs = f"#define AE_BF16 {int(bf16)}\n#define AE_NFINAL {len(self.low.final_names)}\n"
+        defs = f"#define AE_BF16 {int(bf16)}\n#define AE_NFINAL {len(self.low.final_names)}\n#define AE_DV {DV}\n"
         self.combine_src = head + defs + comb
         self.combine = rt.compile_module(self.combine_src, "ae_mla_combine", cfg2)
-        self.num_split = None  # None = choose per call
+        # None = the kernel cuts the tiles of all rows into equal intervals, one per CTA pair (its split 0); n = n shares per row
+        self.num_split = None
+        from .attn_engine import OnlineFunc
+        overridden = getattr(type(online_func), "combine", None) is not OnlineFunc.combine
+        self._auto_split = 0 if overridden or not self.low.final_names else 1  # row state without a combine: rows stay whole
+        self.last_num_split = None
         self._plan = None  # the native side, made at the first call
 
     def _native_plan(self):
         if self._plan is None:
             self._plan = rt.host().MlaPlan(self.decode.handle.value, self.combine.handle.value, self.dtype == torch.bfloat16,
-                                           len(self.low.final_names))
+                                           len(self.low.final_names), N_SM // 2)
         return self._plan
 
     @property
     def status(self):
         return self._plan.status if self._plan is not None else None
 
-    @staticmethod
-    def pick_splits(B: int, S: int) -> int:
-        """Enough CTAs (2 per batch row and split) to cover the 148 SMs once, never an empty split: a second split
-        re-reads nothing but adds the combine pass, which measured slower as soon as one wave was full."""
-        n_tiles = -(-S // MLA_BN)
-        want = max(1, -(-N_SM // (2 * B)))
-        n = min(want, 32, n_tiles)
-        while n > 1 and (n - 1) * (-(-n_tiles // n)) >= n_tiles:
-            n -= 1
-        return n
-
     def __call__(self, q, q_pe, kv, k_pe):
-        n_split = self.num_split or self.pick_splits(q.shape[0], kv.shape[1])
-        o = rt.host().mla(self._plan or self._native_plan(), q, q_pe, kv, k_pe, n_split)
-        if o is None:  # not launched: say what does not fit
+        res = rt.host().mla(self._plan or self._native_plan(), q, q_pe, kv, k_pe, self.num_split or self._auto_split)
+        if res is None:  # not launched: say what does not fit
             for name, t in (("q", q), ("q_pe", q_pe), ("kv", kv), ("k_pe", k_pe)):
                 if not t.is_cuda:
                     raise rt.AeError(f"{name} must be a CUDA tensor: this back end has no CPU path")
                 if t.dtype != self.dtype:
                     raise TypeError(f"{name} has dtype {t.dtype}, engine was built for {self.dtype}")
             raise ValueError("expected q [B,1,H,512], q_pe [B,1,H,64], kv [B,S,1,512], k_pe [B,S,1,64]")
-        self.last_num_split = n_split
+        o, self.last_num_split = res
         return o
 
     def paged(self, q, kcache, block_table, cache_seqlens, num_split=None):
@@ -85,18 +76,18 @@ class MlaDecode:
         The call of the reference's CuTe kv-shared path (core/template/cute_template_kvshared/flash_mla_interface.py:73-113,
         attn_script/mla_decode_cute.py:295-303): q [B, 1, H, 576] (latent 512 + rope 64), kcache [num_pages, 64, 1, 576]
         or [num_pages, 64, 576], block_table [B, max_pages] int32 (page of each 64-key tile), cache_seqlens [B] int32.
-        Every row is cut into the same number of shares of its own tiles, so the launch needs no length on the host; the
-        lengths are read back behind the launches only to raise on one outside the table."""
+        The kernel cuts the work by the lengths itself, so the launch needs none on the host; they are read back behind the
+        launches only to raise on one outside the table."""
         if list(self.low.final_names) != ["lse"]:
             raise NotImplementedError("the paged call returns the log-sum-exp: the online function must have the final row scale 'lse'")
-        n_split = num_split or self.num_split or self.pick_splits(q.shape[0], block_table.shape[1] * 64)
-        res = rt.host().mla_paged(self._plan or self._native_plan(), q, kcache, block_table, cache_seqlens, n_split)
+        res = rt.host().mla_paged(self._plan or self._native_plan(), q, kcache, block_table, cache_seqlens,
+                                  num_split or self.num_split or self._auto_split)
         if res is None:
             self._refuse_paged(q, kcache, block_table, cache_seqlens)
         if not res:
             raise ValueError("cache_seqlens must lie in [1, max_pages * 64]")
-        self.last_num_split = n_split
-        return res
+        o, lse, self.last_num_split = res
+        return o, lse
 
     def _refuse_paged(self, q, kcache, block_table, cache_seqlens):
         for name, t in (("q", q), ("kcache", kcache)):

@@ -19,6 +19,7 @@
 #include <torch/csrc/utils/pybind.h>
 #include <ATen/ATen.h>
 
+#include <algorithm>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -380,7 +381,23 @@ py::object decode(const std::shared_ptr<DecodePlan>& plan, const Tensor& q, cons
 // ---------------------------------------------------------------------------------------------------- MLA decode
 struct MlaPlan : Plan {
   void *kernel = nullptr, *combine = nullptr;
-  int n_final = 0;
+  int n_final = 0, pairs = 1;  // CTA pairs the device holds at a time
+  // intervals the rows' tiles are cut into: one per pair, two 128-key tiles at least
+  int clusters(int64_t tiles) const { return (int)std::max<int64_t>(1, std::min<int64_t>(pairs, (tiles + 1) / 2)); }
+};
+
+// Partials, their row scales and the row table of a split call, in one allocation.
+struct MlaScratch {
+  Tensor buf;
+  float *part = nullptr, *scales = nullptr;
+  int32_t* rows = nullptr;
+  MlaScratch(int64_t slots, int64_t H, int n_final, int64_t B, const Tensor& like) {
+    const int64_t n = slots * H;
+    buf = at::empty({n * (512 + n_final) + 2 * B}, like.options().dtype(at::kFloat));
+    part = (float*)buf.data_ptr();
+    scales = part + n * 512;
+    rows = (int32_t*)(scales + n * n_final);
+  }
 };
 
 bool same(const Tensor& t, std::initializer_list<int64_t> shape) { return t.sizes() == at::IntArrayRef(shape.begin(), shape.size()); }
@@ -398,23 +415,31 @@ py::object mla(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, const Tens
   c10::cuda::CUDAGuard guard(q.device());
   at::AutoGradMode no_grad(false);
   const Tensor Q = q.contiguous(), QP = q_pe.contiguous(), KV = kv.contiguous(), KP = k_pe.contiguous();
-  Tensor o = at::empty({B, 1, H, 512}, q.options()), part;
+  Tensor o = at::empty({B, 1, H, 512}, q.options());
   AeMlaParams p;
   memset(&p, 0, sizeof p);
   p.q = Q.data_ptr(); p.q_pe = QP.data_ptr(); p.kv = KV.data_ptr(); p.k_pe = KP.data_ptr(); p.o = o.data_ptr();
-  if (n_split > 1) {
-    const int64_t rows = B * n_split * H;
-    part = at::empty({rows * (512 + P.n_final)}, q.options().dtype(at::kFloat));
-    p.o_partial = (float*)part.data_ptr();
-    for (int i = 0; i < P.n_final; ++i) p.rowscale_partial[i] = p.o_partial + rows * 512 + rows * i;
-  }
   p.B = (int)B; p.H = (int)H; p.S = (int)S; p.n_split = n_split;
+  std::optional<MlaScratch> scratch;
+  bool merge = n_split > 1;
+  if (n_split != 1) {
+    const int64_t n_t = (S + 127) / 128;
+    p.n_clusters = P.clusters(B * n_t);
+    scratch.emplace(n_split ? B * n_split : 2 * (int64_t)p.n_clusters, H, P.n_final, B, q);
+    p.o_partial = scratch->part;
+    for (int i = 0; i < P.n_final; ++i) p.rowscale_partial[i] = scratch->scales + (scratch->scales - scratch->part) / 512 * i;
+    p.row_info = scratch->rows;
+    if (n_split == 0) {
+      const int64_t share = (B * n_t + p.n_clusters - 1) / p.n_clusters;
+      merge = share % n_t != 0;  // intervals of whole rows leave nothing to merge
+    }
+  }
   p.status = word(plan->status_for(q));
   void* st = stream_of(q);
   check(ae_launch_mla_decode(P.kernel, &p, st), "ae_launch_mla_decode");
-  if (n_split > 1) check(ae_launch_mla_combine(P.combine, &p, st), "ae_launch_mla_combine");
+  if (merge) check(ae_launch_mla_combine(P.combine, &p, st), "ae_launch_mla_combine");
   py::gil_scoped_acquire gil;
-  return py::cast(o);
+  return py::make_tuple(o, n_split ? (double)n_split : std::max(merge ? 1.0 + 1.0 / B : 1.0, (double)p.n_clusters / B));
 }
 
 // Pinned landing place of the row lengths and the event behind their copy, one per thread and device.
@@ -429,9 +454,9 @@ struct Lengths {
   }
 };
 
-// (o, lse) over a paged cache.  The row lengths are checked on the host, as before, but behind the launches: their copy is
+// (o, lse, shares per row) over a paged cache; n_split 0: equal intervals of all rows' tiles.  The row lengths are checked on the host, as before, but behind the launches: their copy is
 // queued in front of the kernels, which clamp every length to the block table themselves, so the stream never drains for
-// the check.  Returns (o, lse), None when the tensors do not fit, or an empty tuple for lengths outside their range.
+// the check.  Returns None when the tensors do not fit, or an empty tuple for lengths outside their range.
 py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, const Tensor& pool, const Tensor& table_in,
                      const Tensor& lens_in, int n_split) {
   const MlaPlan& P = *plan;
@@ -465,7 +490,7 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
   const Tensor Q = q.contiguous();
   Tensor o = at::empty({B, 1, H, 512}, q.options());
   const auto f32 = q.options().dtype(at::kFloat);
-  Tensor lse = at::empty({B, H}, f32), part;
+  Tensor lse = at::empty({B, H}, f32);
   AeMlaPagedParams p;
   memset(&p, 0, sizeof p);
   p.q = Q.data_ptr();
@@ -474,24 +499,25 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
   p.kcache = pool.data_ptr(); p.o = o.data_ptr();
   p.block_table = (const int32_t*)table.data_ptr();
   p.cache_seqlens = (const int32_t*)lens.data_ptr();
-  if (n_split > 1) {
-    const int64_t rows = B * n_split * H;
-    part = at::empty({rows * 513}, f32);
-    p.o_partial = (float*)part.data_ptr();
-    p.rowscale_partial[0] = p.o_partial + rows * 512;
-  } else {
-    p.rowscale_partial[0] = (float*)lse.data_ptr();
-  }
+  p.lse_out = (float*)lse.data_ptr();
   p.B = (int)B; p.H = (int)H; p.num_pages = (int)pool.size(0); p.max_pages = (int)max_pages;
   p.max_seqlen = (int)(max_pages * 64); p.n_split = n_split;
+  std::optional<MlaScratch> scratch;
+  if (n_split != 1) {
+    p.n_clusters = P.clusters(B * ((max_pages + 1) / 2));
+    scratch.emplace(n_split ? B * n_split : 2 * (int64_t)p.n_clusters, H, 1, B, q);
+    p.o_partial = scratch->part;
+    p.rowscale_partial[0] = scratch->scales;
+    p.row_info = scratch->rows;
+  }
   p.status = word(plan->status_for(q));
   check(ae_launch_mla_decode_paged(P.kernel, &p, st), "ae_launch_mla_decode_paged");
-  if (n_split > 1) {
+  if (n_split != 1) {
     AeMlaParams m;
     memset(&m, 0, sizeof m);
     m.o = p.o; m.o_partial = p.o_partial; m.rowscale_partial[0] = p.rowscale_partial[0];
-    m.B = p.B; m.H = p.H; m.S = p.max_seqlen; m.n_split = n_split;
-    m.lse_out = (float*)lse.data_ptr();
+    m.B = p.B; m.H = p.H; m.S = p.max_seqlen; m.n_split = n_split; m.row_info = p.row_info;
+    m.lse_out = p.lse_out;
     check(ae_launch_mla_combine(P.combine, &m, st), "ae_launch_mla_combine");
   }
   C10_CUDA_CHECK(cudaEventSynchronize(land.copied));
@@ -499,7 +525,7 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
   for (int64_t b = 0; b < B; ++b) in_range = in_range && land.host[b] >= 1 && land.host[b] <= max_pages * 64;
   py::gil_scoped_acquire gil;
   if (!in_range) return py::tuple();
-  return py::make_tuple(o, lse);
+  return py::make_tuple(o, lse, n_split ? (double)n_split : (double)p.n_clusters / B);
 }
 
 // ---------------------------------------------------------------------------------------------------- scan
@@ -744,11 +770,12 @@ PYBIND11_MODULE(_ae_host, m) {
         return p;
       })) AE_STATUS(DecodePlan);
   py::class_<MlaPlan, std::shared_ptr<MlaPlan>>(m, "MlaPlan")
-      .def(py::init([](uint64_t kernel, uint64_t combine, bool bf16, int n_final) {
+      .def(py::init([](uint64_t kernel, uint64_t combine, bool bf16, int n_final, int pairs) {
         auto p = std::make_shared<MlaPlan>();
         p->kernel = handle(kernel); p->combine = handle(combine);
         p->dtype = bf16 ? at::kBFloat16 : at::kHalf;
         p->n_final = n_final;
+        p->pairs = pairs;
         return p;
       })) AE_STATUS(MlaPlan);
   py::class_<ScanPlan, std::shared_ptr<ScanPlan>>(m, "ScanPlan")

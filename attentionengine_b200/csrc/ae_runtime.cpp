@@ -675,84 +675,96 @@ static int make_3d_map(AeTmaDesc* out, const void* base, int dtype, int64_t cols
   return AE_OK;
 }
 
-int ae_launch_mla_decode(void* module, const AeMlaParams* p, void* stream) {
-  if (!module || !p || !p->q || !p->q_pe || !p->kv || !p->k_pe || !p->o) return AE_ERR_INVALID;
-  Module* m = (Module*)module;
+// What the dense and the paged call share: shape checks, the split or interval arguments, the grid.
+static int mla_common(Module* m, AeMlaArgs& a, int B, int H, int n_split, int n_clusters, float* o_partial,
+                      float* const rowscale_partial[], int* row_info, float* lse_out) {
   if (m->cfg.kind != AE_KIND_MLA_DECODE) {
     set_error("module kind does not match the entry point");
     return AE_ERR_UNSUPPORTED;
   }
-  const int bn = m->cfg.reserved[0];
-  if (p->B <= 0 || p->S <= 0 || p->H <= 0 || p->H > 128 || p->n_split < 1 || p->n_split > 32 || (bn != 64 && bn != 128)) {
-    set_error("MLA decode: need 1 <= H <= 128, S > 0, 1 <= n_split <= 32");
+  if (B <= 0 || H <= 0 || H > 128 || n_split < 0 || n_split > 32 || (n_split == 0 && (n_clusters < 1 || n_clusters > 4096))) {
+    set_error("MLA decode: need 1 <= H <= 128, 0 <= n_split <= 32 and, with n_split == 0, n_clusters >= 1");
     return AE_ERR_INVALID;
   }
-  const int n_tiles = (p->S + bn - 1) / bn;
-  const int tps = (n_tiles + p->n_split - 1) / p->n_split;
-  if ((int64_t)(p->n_split - 1) * tps >= n_tiles) {
-    set_error("MLA decode: n_split leaves an empty split");
+  if (n_split != 1 && !o_partial) {
+    set_error("MLA decode: o_partial scratch required when n_split != 1");
     return AE_ERR_INVALID;
   }
-  if (p->n_split > 1 && !p->o_partial) {
-    set_error("MLA decode: o_partial scratch required when n_split > 1");
+  if (n_split == 0 && !row_info) {
+    set_error("MLA decode: row_info scratch required when n_split == 0");
     return AE_ERR_INVALID;
   }
-  int rc = ensure_loaded(m);
-  if (rc) return rc;
+  a.o_part = o_partial;
+  for (int i = 0; i < AE_MAX_FINAL; ++i) a.fr_part[i] = rowscale_partial[i];
+  a.B = B; a.H = H; a.n_split = n_split; a.n_clusters = n_clusters;
+  a.row_info = row_info;
+  a.lse_out = lse_out;
+  return AE_OK;
+}
+
+int ae_launch_mla_decode(void* module, const AeMlaParams* p, void* stream) {
+  if (!module || !p || !p->q || !p->q_pe || !p->kv || !p->k_pe || !p->o) return AE_ERR_INVALID;
+  Module* m = (Module*)module;
   AeMlaArgs a;
   memset(&a, 0, sizeof a);
-  if ((rc = make_3d_map(&a.tm_q, p->q, m->cfg.dtype, 512, p->H, p->B, 128))) return rc;
-  if ((rc = make_3d_map(&a.tm_qpe, p->q_pe, m->cfg.dtype, 64, p->H, p->B, 128))) return rc;
-  if ((rc = make_3d_map(&a.tm_kv, p->kv, m->cfg.dtype, 512, p->S, p->B, bn))) return rc;
-  if ((rc = make_3d_map(&a.tm_kpe, p->k_pe, m->cfg.dtype, 64, p->S, p->B, bn))) return rc;
+  int rc = mla_common(m, a, p->B, p->H, p->n_split, p->n_clusters, p->o_partial, p->rowscale_partial, p->row_info, p->lse_out);
+  if (rc) return rc;
+  if (p->S <= 0) {
+    set_error("MLA decode: S > 0");
+    return AE_ERR_INVALID;
+  }
+  if (p->n_split > 1) {
+    const int n = (p->S + 63) / 64, tps = (n + p->n_split - 1) / p->n_split;
+    if ((int64_t)(p->n_split - 1) * tps >= n) {
+      set_error("MLA decode: n_split leaves an empty split");
+      return AE_ERR_INVALID;
+    }
+  }
+  rc = ensure_loaded(m);
+  if (rc) return rc;
+  if ((rc = make_3d_map(&a.tm_q, p->q, m->cfg.dtype, 512, p->H, p->B, 64))) return rc;
+  if ((rc = make_3d_map(&a.tm_qpe, p->q_pe, m->cfg.dtype, 64, p->H, p->B, 64))) return rc;
+  if ((rc = make_3d_map(&a.tm_kv, p->kv, m->cfg.dtype, 512, p->S, p->B, 64))) return rc;
+  if ((rc = make_3d_map(&a.tm_kpe, p->k_pe, m->cfg.dtype, 64, p->S, p->B, 64))) return rc;
   a.o = p->o;
-  a.o_part = p->o_partial;
-  for (int i = 0; i < AE_MAX_FINAL; ++i) a.fr_part[i] = p->rowscale_partial[i];
-  a.B = p->B; a.H = p->H; a.S = p->S; a.n_split = p->n_split; a.tiles_per_split = tps;
+  a.S = p->S;
   a.status = p->status;
-  return launch(m, 2, (unsigned)p->n_split, (unsigned)p->B, &a, stream);
+  return launch(m, 2u * (unsigned)(p->n_split > 0 ? p->B * p->n_split : p->n_clusters), 1, 1, &a, stream);
 }
 
 int ae_launch_mla_decode_paged(void* module, const AeMlaPagedParams* p, void* stream) {
   if (!module || !p || !p->q || !p->q_pe || !p->kcache || !p->block_table || !p->cache_seqlens || !p->o)
     return AE_ERR_INVALID;
   Module* m = (Module*)module;
-  if (m->cfg.kind != AE_KIND_MLA_DECODE) {
-    set_error("module kind does not match the entry point");
-    return AE_ERR_UNSUPPORTED;
-  }
-  if (m->cfg.reserved[0] != 64) {
-    set_error("paged MLA decode: pages hold 64 keys, the kernel must stream 64-row tiles");
-    return AE_ERR_UNSUPPORTED;
-  }
-  if (p->B <= 0 || p->H <= 0 || p->H > 128 || p->num_pages <= 0 || p->max_pages <= 0 || p->max_seqlen <= 0 ||
-      p->max_seqlen > (int64_t)p->max_pages * 64 || p->n_split < 1 || p->n_split > 32) {
-    set_error("paged MLA decode: need 1 <= H <= 128, 1 <= max_seqlen <= max_pages * 64, 1 <= n_split <= 32");
-    return AE_ERR_INVALID;
-  }
-  if (p->n_split > 1 && !p->o_partial) {
-    set_error("MLA decode: o_partial scratch required when n_split > 1");
-    return AE_ERR_INVALID;
-  }
-  int rc = ensure_loaded(m);
-  if (rc) return rc;
   AeMlaArgs a;
   memset(&a, 0, sizeof a);
+  int rc = mla_common(m, a, p->B, p->H, p->n_split, p->n_clusters, p->o_partial, p->rowscale_partial, p->row_info, p->lse_out);
+  if (rc) return rc;
+  if (p->num_pages <= 0 || p->max_pages <= 0 || p->max_seqlen <= 0 || p->max_seqlen > (int64_t)p->max_pages * 64) {
+    set_error("paged MLA decode: need pages and 1 <= max_seqlen <= max_pages * 64");
+    return AE_ERR_INVALID;
+  }
+  rc = ensure_loaded(m);
+  if (rc) return rc;
   const int64_t pool_rows = (int64_t)p->num_pages * 64;
-  if ((rc = make_3d_map(&a.tm_q, p->q, m->cfg.dtype, 512, p->H, p->B, 128, p->q_row_stride))) return rc;
-  if ((rc = make_3d_map(&a.tm_qpe, p->q_pe, m->cfg.dtype, 64, p->H, p->B, 128, p->q_row_stride))) return rc;
+  if ((rc = make_3d_map(&a.tm_q, p->q, m->cfg.dtype, 512, p->H, p->B, 64, p->q_row_stride))) return rc;
+  if ((rc = make_3d_map(&a.tm_qpe, p->q_pe, m->cfg.dtype, 64, p->H, p->B, 64, p->q_row_stride))) return rc;
   // the pool as one batch of num_pages * 64 rows of 576 elements: latent part and rope part are column slices
   if ((rc = make_3d_map(&a.tm_kv, p->kcache, m->cfg.dtype, 512, pool_rows, 1, 64, 576))) return rc;
   if ((rc = make_3d_map(&a.tm_kpe, (const char*)p->kcache + 512 * 2, m->cfg.dtype, 64, pool_rows, 1, 64, 576))) return rc;
   a.o = p->o;
-  a.o_part = p->o_partial;
-  for (int i = 0; i < AE_MAX_FINAL; ++i) a.fr_part[i] = p->rowscale_partial[i];
-  a.B = p->B; a.H = p->H; a.S = p->max_seqlen; a.n_split = p->n_split;
+  a.S = p->max_seqlen;
   a.status = p->status;
   a.block_table = p->block_table;
   a.seqlens = p->cache_seqlens;
   a.max_pages = p->max_pages;
-  return launch(m, 2, (unsigned)p->n_split, (unsigned)p->B, &a, stream);
+  return launch(m, 2u * (unsigned)(p->n_split > 0 ? p->B * p->n_split : p->n_clusters), 1, 1, &a, stream);
+}
+
+// blocks of the merge: AE_DV / 4 threads, at least a warp, per head
+static unsigned combine_blocks(int heads, int dv) {
+  const int tph = dv / 4 > 32 ? dv / 4 : 32, hpb = 128 / tph;
+  return (unsigned)((heads + hpb - 1) / hpb);
 }
 
 int ae_launch_mla_combine(void* module, const AeMlaParams* p, void* stream) {
@@ -762,7 +774,7 @@ int ae_launch_mla_combine(void* module, const AeMlaParams* p, void* stream) {
     set_error("module kind does not match the entry point");
     return AE_ERR_UNSUPPORTED;
   }
-  if (p->n_split < 1 || p->n_split > 32) return AE_ERR_INVALID;
+  if (p->n_split < 0 || p->n_split > 32 || (p->n_split == 0 && !p->row_info) || m->cfg.head_dim_v != 512) return AE_ERR_INVALID;
   int rc = ensure_loaded(m);
   if (rc) return rc;
   AeMlaCombineArgs a;
@@ -771,8 +783,9 @@ int ae_launch_mla_combine(void* module, const AeMlaParams* p, void* stream) {
   a.o_part = p->o_partial;
   for (int i = 0; i < AE_MAX_FINAL; ++i) a.fr_part[i] = p->rowscale_partial[i];
   a.B = p->B; a.H = p->H; a.DV = 512; a.n_split = p->n_split;
+  if (p->n_split == 0) a.row_info = p->row_info;
   a.lse_out = p->lse_out;
-  return launch(m, (unsigned)((p->H + 3) / 4), (unsigned)p->B, 1, &a, stream);
+  return launch(m, combine_blocks(p->H, 512), (unsigned)p->B, 1, &a, stream);
 }
 
 int ae_launch_attn_decode(void* module, const AeDecodeParams* p, void* stream) {
@@ -901,7 +914,7 @@ int ae_launch_decode_combine(void* module, const AeDecodeParams* p, void* stream
   a.DV = m->cfg.head_dim_v;
   a.n_split = p->n_split;
   a.part_off = p->part_off;  // rows of different lengths: each row's own number of partial slots
-  return launch(m, (unsigned)((a.H + 3) / 4), (unsigned)p->B, 1, &a, stream);
+  return launch(m, combine_blocks(a.H, a.DV), (unsigned)p->B, 1, &a, stream);
 }
 
 int ae_launch_rowscale(void* module, const AeRowScaleParams* p, void* stream) {

@@ -106,18 +106,22 @@ struct AeAttnBwdArgs {
 
 // ---- MLA split-KV decode (kernels ae_mla_decode, ae_mla_combine) --------------------------
 struct AeMlaArgs {
-  AeTmaDesc tm_q;    // dims (512, H, B), box {64, 128, 1}
-  AeTmaDesc tm_qpe;  // dims (64, H, B),  box {64, 128, 1}
-  AeTmaDesc tm_kv;   // dims (512, S, B), box {64, BN, 1}
-  AeTmaDesc tm_kpe;  // dims (64, S, B),  box {64, BN, 1}
-  void* o;           // [B, H, 512] 16-bit                       (n_split == 1)
-  float* o_part;     // [B, n_split, H, 512] fp32, normalised   (n_split > 1)
-  float* fr_part[AE_MAX_FINAL];  // each [B, n_split, H]
-  int B, H, S, n_split, tiles_per_split;
+  AeTmaDesc tm_q;    // dims (512, H, B), box {64, 64, 1}
+  AeTmaDesc tm_qpe;  // dims (64, H, B),  box {64, 64, 1}
+  AeTmaDesc tm_kv;   // dims (512, S, B), box {64, 64, 1}
+  AeTmaDesc tm_kpe;  // dims (64, S, B),  box {64, 64, 1}
+  void* o;           // [B, H, 512] 16-bit: rows that are not split
+  float* o_part;     // [slots, H, 512] fp32, normalised partials
+  float* fr_part[AE_MAX_FINAL];  // each [slots, H]
+  int B, H, S;
+  int n_split;     // > 0: cluster (b, s) = share s of row b, slot b * n_split + s; 0: equal intervals of all rows' tiles
+  int n_clusters;  // n_split == 0: intervals (slots 2 c and 2 c + 1 belong to interval c)
+  int* row_info;   // n_split == 0: [B][2] first partial slot of a row, intervals it touches (1 = written directly)
+  float* lse_out;  // [B, H] or null: first final row scale of the rows that are written directly
   u32* status;
   // paged KV (null = the dense layout above): tm_kv / tm_kpe then cover the page pool as rows (page * 64 + r) of one
-  // batch, tile i of batch row b is page block_table[b * max_pages + i], and row b holds seqlens[b] keys, clamped to
-  // [0, S], that its n_split shares divide (a share past the row's last tile writes zero partials with -inf row scales).
+  // batch, the i-th 64 keys of batch row b are page block_table[b * max_pages + i], and row b holds seqlens[b] keys, clamped
+  // to [0, S].
   const int* block_table;
   const int* seqlens;
   int max_pages;
@@ -129,6 +133,7 @@ struct AeMlaCombineArgs {
   int B, H, DV, n_split;
   const int* part_off;  // [B + 1] or null: row b owns the partial slots part_off[b] .. part_off[b + 1] - 1 (at most 32);
                         // null = n_split slots per row.  A row with a single slot was written directly and is skipped.
+  const int* row_info;  // MLA decode, or null: {first slot f, count n} per row; slot k > 0 is 2 * (f / 2 + k); n == 1: skipped
   float* lse_out;       // [B, H] or null: log-sum-exp over the splits of fr_part[0]
 };
 

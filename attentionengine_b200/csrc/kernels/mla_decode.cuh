@@ -1,252 +1,346 @@
-// MLA (multi-head latent attention) split-KV decode for sm_100a.  Replaces the reference's
-// `flash_attn` / `flash_attn_split` kernels (attention_engine/core/template/tl_template/attn/
-// mla_decode_tl.py:38-177; CuTe variant cute_template_kvshared/kernels/splitkv_mla.cu:1061-1391).
+// MLA (multi-head latent attention) decode for sm_100a over CTA pairs.  Replaces the reference's `flash_attn` /
+// `flash_attn_split` kernels (attention_engine/core/template/tl_template/attn/mla_decode_tl.py:38-177; CuTe variant
+// cute_template_kvshared/kernels/splitkv_mla.cu:1061-1391) and the scheduler of the latter (get_mla_metadata.cu:8-75).
 //
-// All H = 128 query heads of one batch row share one latent KV stream: rows of the MMA are heads.
-//   S = [q | q_pe] [kv | k_pe]^T   over 512 + 64 dims (9 K blocks of 64)        TS / SS MMAs, M = 128, N = BN
-//   row threads (thread = head): fused score_mod + online recurrence, P -> TMEM
-//   O_half += P kv[:, half]          over this CTA's 256 of the 512 value dims     TS MMA, N = 256
-// A [128 x 512] fp32 accumulator would fill all 512 TMEM columns, so the value dims are split
-// over two CTAs (blockIdx.x) that each recompute S; both read the same KV tiles, the second read
-// is an L2 hit.  blockIdx.y is the kv split, blockIdx.z the batch row.  With more than one split
-// the CTA stores its normalised partial O (fp32) and its final row scales; ae_mla_combine merges.
-// The first AE_MLA_QT (= 4) 64-wide blocks of the query block live in TMEM (16-bit pairs, the A-operand layout of a
-// TS MMA), the other five in shared memory: that leaves room for two KV stages and two S regions, so the loads of
-// tile s+1, its S GEMM and the row work of tile s overlap.  The TMEM-resident blocks first land in KV stage 0.
-// TMEM columns: S0 | S1 | O half (256) | Q blocks 0-3 (128) = 512.
-// Roles: warps 0-3 row threads, warp 4 TMA producer, warp 5 MMA issuer.
-// Expects AE_BF16, AE_NFINAL, AE_O_SCALE_ONE, AE_MLA_BN (64), AE_MLA_ALIGN_SLACK, struct AeRow, ae_online_fwd(),
-// ae_epilogue_o(), ae_final_rowscales().
+// All H <= 128 query heads of one batch row share one latent KV stream: rows of the MMAs are heads.  Per 128-key tile
+//   S = [q | q_pe] [kv | k_pe]^T   over 512 + 64 dims (9 blocks of 64)
+//   row threads: fused score_mod + online recurrence, P (16 bit) -> shared memory
+//   O += P kv[:, :512]
+// A cluster of two CTAs does it with tcgen05.mma.cta_group::2, M = 128: each CTA owns 64 heads, its O [64 x 512] fp32 takes
+// 256 TMEM columns (64 rows lie on 128 lanes: row r's first half of the columns on lane r, the second on lane r + 64), and
+// each B operand is split between the two: 64 of the 128 keys for S, half of the value dims for P V.  One CTA per head
+// block with M = 128 cannot hold O and S; splitting the value dims over two CTAs instead computed S twice (2240 clk of MMAs
+// per 64 keys and pair against about 1500 per 64 keys here).
+//
+// Work: the tiles of all batch rows in one line, cut into equal intervals, one per cluster (args.n_clusters; an interval may
+// cover the end of a row, whole rows, the beginning of a row).  A row that lies in one interval is written directly,
+// others as normalised partials that ae_mla_combine merges.  One CTA pair per row and value half had 256 CTAs in two
+// waves at 128 rows.  With args.n_split > 0 (the caller's choice) cluster (b, s) takes share s of row b instead.
+//
+// Shared memory per CTA: Q 72 KB | K 72 KB (9 blocks of 64 keys) | V 64 KB (2 x 2 blocks of 64 dims, 128 keys) | P 16 KB.
+// K and V are one tile deep but released in parts (three K blocks, half of V), which are refilled while the MMAs of the
+// other parts run; an L2 prefetch two tiles ahead covers the latency of HBM.
+// TMEM columns: O dims 0-255 (128) | O dims 256-511 (128) | S0 64 | S1 64.
+// Roles per CTA: warps 0-3 row threads (two per row), warp 4 TMA producer, warp 5 of rank 0 the MMA issuer.
+// Barriers that both CTAs' loads or row warps complete live in rank 0; every tcgen05.commit arrives in both CTAs.
+// Expects the forward prelude built with AE_RSPLIT = 2, AE_XCH_ROWS = 64.
 
-// Optional phase trace of CTA (0, 0, 0): 32-bit clock stamps behind the status word (bring-up / tuning only).
-#ifdef AE_TRACE
-#define AE_TRM(cond, region, slot) \
-  if (trace_on && (cond) && (slot) < 2048) args.status[64 + (region) * 4096 + (slot)] = (u32)clock64();
-#else
-#define AE_TRM(cond, region, slot)
-#endif
-#define AE_MLA_H 128
 #define AE_MLA_DV 512
-#define AE_MLA_DPE 64
-#define AE_MLA_NBV (AE_MLA_DV / 64)
-#define AE_MLA_NBK (AE_MLA_NBV + AE_MLA_DPE / 64)
-#define AE_MLA_DVH (AE_MLA_DV / 2)
-#define AE_MLA_QT 4        // query blocks resident in TMEM
-#define AE_MLA_STAGES 2
-#if AE_MLA_BN != 64
-#error "the MLA decode kernel streams 64-row KV tiles"
+#define AE_MLA_NBK 9       // 64-wide blocks of the 576 dims
+#define AE_MLA_BN 128      // keys per tile
+#define AE_MLA_KBLK (64 * 128)           // bytes of a K or Q block: 64 rows of 128 B
+#define AE_MLA_VBLK (AE_MLA_BN * 128)    // bytes of a V block: 128 keys of 64 dims
+#define AE_MLA_SMEM_Q 0
+#define AE_MLA_SMEM_K (AE_MLA_NBK * AE_MLA_KBLK)
+#define AE_MLA_SMEM_V (AE_MLA_SMEM_K + AE_MLA_NBK * AE_MLA_KBLK)
+#define AE_MLA_SMEM_P (AE_MLA_SMEM_V + 4 * AE_MLA_VBLK)
+#define AE_MLA_SMEM_BAR (AE_MLA_SMEM_P + 2 * AE_MLA_KBLK)
+#define AE_MLA_SMEM_XCH (AE_MLA_SMEM_BAR + 512)  // [phase][half][row] of ae_row_xchg
+#ifndef AE_MLA_PREFETCH
+#define AE_MLA_PREFETCH 2  // tiles ahead that are brought into L2 (0: none)
 #endif
-
-#define AE_MLA_QS_BYTES ((AE_MLA_NBK - AE_MLA_QT) * AE_MLA_H * 128)  // query blocks kept in shared memory
-#define AE_MLA_KV_BYTES (AE_MLA_NBK * AE_MLA_BN * 128)
-#define AE_MLA_SMEM_QS 0
-#define AE_MLA_SMEM_KV (AE_MLA_QS_BYTES)
-#define AE_MLA_SMEM_BAR (AE_MLA_SMEM_KV + AE_MLA_STAGES * AE_MLA_KV_BYTES)
 
 struct AeMlaBars {
-  u64 q_full;   // the whole query block landed in shared memory
-  u64 q_tmem;   // its first blocks were copied to TMEM (KV stage 0 is free)
-  // A KV stage is two parts with their own barriers: the CTA's own half of the value dims (4 blocks, held until the
-  // tile's P V GEMM has run) and the rest (the other half and the rope block, 5 blocks, free as soon as the S GEMM has
-  // read them).  With two stages the refill of a stage used to wait for P V of the tile before; now 40 of its 72 KB
-  // are requested one S GEMM earlier, and only the value part's 32 KB sit on the chain P V -> load -> next S GEMM.
-  u64 kv_full[AE_MLA_STAGES];    // the value part landed
-  u64 kv_empty[AE_MLA_STAGES];   // ... and was read by P V
-  u64 kx_full[AE_MLA_STAGES];    // the rest landed
-  u64 kx_empty[AE_MLA_STAGES];   // ... and was read by the S GEMM
+  u64 q_full, q_empty;
+  u64 k_full[3], k_empty[3];  // three K blocks each
+  u64 v_full[2], v_empty[2];  // value dims 0-255 / 256-511
   u64 s_full[2];
-  u64 o_done;
+  u64 p_full;   // the row warps of both CTAs
+  u64 pv_done;
   AeCtaCtl ctl;
+  int row0, tile0, share, total;
+};
+static_assert(sizeof(AeMlaBars) <= 512, "barrier block");
+
+// Load with the byte count going to a barrier of the pair's rank 0 (cluster address `bar`).
+AE_DEVICE void mla_load(void* dst, const AeTmaDesc* d, u32 bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(dst)), "l"((u64)d), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+AE_DEVICE void mla_prefetch(const AeTmaDesc* d, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"((u64)d), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+AE_DEVICE void mla_expect(u32 bar, u32 bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+struct AeMlaSeg {
+  int b, t0, t1;   // tiles [t0, t1) of batch row b
+  int n_t, len;    // tiles and keys of the row
 };
 
-extern "C" __global__ void __launch_bounds__(192, 1) ae_mla_decode(const __grid_constant__ AeMlaArgs args) {
+extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) ae_mla_decode(const __grid_constant__ AeMlaArgs args) {
   extern __shared__ u8 smem_raw[];
   u8* smem = smem_align1024(smem_raw);
   AeMlaBars* bars = (AeMlaBars*)(smem + AE_MLA_SMEM_BAR);
   AeCtaCtl* ctl = &bars->ctl;
   const u32 warp = threadIdx.x >> 5;
   const u32 lane = threadIdx.x & 31;
-  const int dvh = blockIdx.x;    // which half of the value dims
-  const int split = blockIdx.y;
-  const int b = blockIdx.z;
+  const u32 rank = cluster_ctarank();
+  const int cl = (int)(blockIdx.x >> 1);
 
-#ifdef AE_TRACE
-  const bool trace_on = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (threadIdx.x & 31) == 0;
-#endif
-  // keys of this batch row; rows of different lengths are cut into n_split shares each by its own tiles
-  int S_b = args.S, tps = args.tiles_per_split;
-  if (args.seqlens) {
+  // keys of a row, clamped to the table; a row has at least one tile (an empty one is all masked)
+  auto row_len = [&](int b) {
+    if (!args.seqlens) return args.S;
     const int len = args.seqlens[b];
-    S_b = len < 0 ? 0 : (len < args.S ? len : args.S);
-    tps = ((S_b + AE_MLA_BN - 1) / AE_MLA_BN + args.n_split - 1) / args.n_split;
-  }
-  const int n_tiles = (S_b + AE_MLA_BN - 1) / AE_MLA_BN;
-  const int t_begin = split * tps;
-  int t_end = t_begin + tps;
-  if (t_end > n_tiles) t_end = n_tiles;
-  const int n_steps = t_end > t_begin ? t_end - t_begin : 0;
+    return len < 0 ? 0 : (len < args.S ? len : args.S);
+  };
+  auto tiles_of = [](int len) { return len > 0 ? (len + AE_MLA_BN - 1) / AE_MLA_BN : 1; };
 
   if (threadIdx.x == 0) {
     ctl->abort = 0;
-    mbar_init(&bars->q_full, 1);
-    mbar_init(&bars->q_tmem, 4);
-    mbar_init(&bars->o_done, 1);
+    mbar_init(&bars->q_full, 2);
+    mbar_init(&bars->q_empty, 1);
+    for (int i = 0; i < 3; ++i) {
+      mbar_init(&bars->k_full[i], 2);
+      mbar_init(&bars->k_empty[i], 1);
+    }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars->kv_full[i], 1);
-      mbar_init(&bars->kv_empty[i], 1);
-      mbar_init(&bars->kx_full[i], 1);
-      mbar_init(&bars->kx_empty[i], 1);
+      mbar_init(&bars->v_full[i], 2);
+      mbar_init(&bars->v_empty[i], 1);
       mbar_init(&bars->s_full[i], 1);
     }
+    mbar_init(&bars->p_full, 8);
+    mbar_init(&bars->pv_done, 1);
     mbar_fence_init();
   }
+  if (warp == 0 && args.n_split == 0) {
+    // this cluster's interval: total tiles, equal shares (a row spans at most 32 of them), the row and tile it begins at
+    int total = 0, longest = 0;
+    if (args.seqlens) {
+      for (int b = (int)lane; b < args.B; b += 32) {
+        const int n = tiles_of(row_len(b));
+        total += n;
+        longest = n > longest ? n : longest;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        total += __shfl_xor_sync(0xffffffffu, total, o);
+        const int l = __shfl_xor_sync(0xffffffffu, longest, o);
+        longest = l > longest ? l : longest;
+      }
+    } else {
+      longest = tiles_of(args.S);
+      total = longest * args.B;
+    }
+    int share = (total + args.n_clusters - 1) / args.n_clusters;
+    if (share < (longest + 30) / 31) share = (longest + 30) / 31;
+    const int g0 = cl * share;
+    int row0 = 0, tile0 = 0;
+    if (!args.seqlens) {
+      row0 = g0 / longest;
+      tile0 = g0 % longest;
+    } else if (g0 < total) {
+      int before = 0;
+      for (int base = 0; base < args.B; base += 32) {
+        const int b = base + (int)lane;
+        const int n = b < args.B ? tiles_of(row_len(b)) : 0;
+        int incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o);
+          if ((int)lane >= o) incl += y;
+        }
+        const u32 hit = __ballot_sync(0xffffffffu, b < args.B && before + incl > g0);
+        if (hit) {
+          const int src = __ffs(hit) - 1;
+          row0 = base + src;
+          tile0 = g0 - (before + __shfl_sync(0xffffffffu, incl - n, src));
+          break;
+        }
+        before += __shfl_sync(0xffffffffu, incl, 31);
+      }
+    }
+    if (lane == 0) {
+      bars->row0 = row0;
+      bars->tile0 = tile0;
+      bars->share = share;
+      bars->total = total;
+    }
+  }
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers exist before anything can arrive on them
   if (warp == 5) {
-    tmem_alloc(&ctl->tmem_base, 512);
-    tmem_relinquish();
+    tmem_alloc2(&ctl->tmem_base, 512);
+    tmem_relinquish2();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const u32 tmem = ctl->tmem_base;
-  const u32 TM_S = 0, TM_O = 128, TM_Q = 384;  // S buffer i at TM_S + 64 i
+  const u32 TM_O = 0, TM_S = 256;  // S region i at TM_S + 64 i
+
+  // ---- the cluster's segments, the same walk in every role ----
+  int w_row, w_tile, w_left;
+  if (args.n_split == 0) {
+    w_row = bars->row0;
+    w_tile = bars->tile0;
+    w_left = bars->total - cl * bars->share;
+    if (w_left > bars->share) w_left = bars->share;
+  } else {
+    w_row = cl / args.n_split;
+    const int n_t = tiles_of(row_len(w_row));
+    const int per = (n_t + args.n_split - 1) / args.n_split;
+    w_tile = (cl % args.n_split) * per;
+    w_left = n_t - w_tile < per ? n_t - w_tile : per;
+  }
+  auto next_seg = [&](AeMlaSeg& sg) -> bool {
+    if (w_left <= 0) return false;
+    sg.b = w_row;
+    sg.len = row_len(w_row);
+    sg.n_t = tiles_of(sg.len);
+    sg.t0 = w_tile;
+    const int n = sg.n_t - w_tile < w_left ? sg.n_t - w_tile : w_left;
+    sg.t1 = w_tile + n;
+    w_left -= n;
+    w_row++;
+    w_tile = 0;
+    return true;
+  };
+  AeMlaSeg sg;
 
   if (warp == 4) {
-    // =============================== TMA producer ===============================
-    if (lane == 0 && n_steps > 0) {
+    // =============================== TMA producer (both CTAs) ===============================
+    if (lane == 0) {
       tma_prefetch_desc(&args.tm_q);
       tma_prefetch_desc(&args.tm_qpe);
       tma_prefetch_desc(&args.tm_kv);
       tma_prefetch_desc(&args.tm_kpe);
-      mbar_arrive_expect_tx(&bars->q_full, AE_MLA_NBK * AE_MLA_H * 128);
-      // blocks 0 .. QT-1 pass through KV stage 0 on their way to TMEM, the rest stay in their own area
-      for (int blk = 0; blk < AE_MLA_QT; ++blk)
-        tma_load_3d(smem + AE_MLA_SMEM_KV + blk * (AE_MLA_H * 128), &args.tm_q, &bars->q_full, blk * 64, 0, b);
-      for (int blk = AE_MLA_QT; blk < AE_MLA_NBV; ++blk)
-        tma_load_3d(smem + AE_MLA_SMEM_QS + (blk - AE_MLA_QT) * (AE_MLA_H * 128), &args.tm_q, &bars->q_full, blk * 64, 0, b);
-      tma_load_3d(smem + AE_MLA_SMEM_QS + (AE_MLA_NBV - AE_MLA_QT) * (AE_MLA_H * 128), &args.tm_qpe, &bars->q_full, 0, 0, b);
-      for (int s = 0; s < n_steps; ++s) {
-        const int stage = s % AE_MLA_STAGES;
-        if (s == 0 && !mbar_wait(&bars->q_tmem, 0, ctl, args.status, 40)) break;
-        if (!mbar_wait(&bars->kx_empty[stage], ((s / AE_MLA_STAGES) & 1) ^ 1, ctl, args.status, 41)) break;
-        // dense: rows (tile * 64 ..) of batch b; paged: the tile's page in the pool (a page index outside the pool
-        // reads the fill value, it cannot fault)
-        int kv0 = (t_begin + s) * AE_MLA_BN, kb = b;
-        if (args.block_table) {
-          kv0 = args.block_table[(i64)b * args.max_pages + (t_begin + s)] * AE_MLA_BN;
-          kb = 0;
+      const u32 q_bar = mapa_u32(smem_u32(&bars->q_full), 0);
+      u32 k_bar[3], v_bar[2];
+      for (int g = 0; g < 3; ++g) k_bar[g] = mapa_u32(smem_u32(&bars->k_full[g]), 0);
+      for (int i = 0; i < 2; ++i) v_bar[i] = mapa_u32(smem_u32(&bars->v_full[i]), 0);
+      // row of the `half`-th 64 keys of tile t; keys that the row does not have come from outside the tensor (zeros), so
+      // that a page index is only read where the row has keys
+      auto kv_row = [&](const AeMlaSeg& s, int t, int half) -> int {
+        const int key = t * AE_MLA_BN + half * 64;
+        if (!args.block_table) return key;
+        if (key >= s.len) return 1 << 30;
+        return args.block_table[(i64)s.b * args.max_pages + 2 * t + half] * 64;
+      };
+      bool ok = true;
+      int it = 0, n_seg = 0;
+      auto load_v = [&](const AeMlaSeg& s, int t, int n) {
+        const int r0 = kv_row(s, t, 0), r1 = kv_row(s, t, 1), kb = args.block_table ? 0 : s.b;
+        for (int i = 0; i < 2 && ok; ++i) {
+          ok = mbar_wait_cl(&bars->v_empty[i], (n & 1) ^ 1, ctl, args.status, 41);
+          if (!ok) return;
+          mla_expect(v_bar[i], 2 * AE_MLA_VBLK);
+          for (int j = 0; j < 2; ++j) {
+            const int d0 = i * 256 + (int)rank * 128 + j * 64;
+            u8* dst = smem + AE_MLA_SMEM_V + (i * 2 + j) * AE_MLA_VBLK;
+            mla_load(dst, &args.tm_kv, v_bar[i], d0, r0, kb);
+            mla_load(dst + AE_MLA_KBLK, &args.tm_kv, v_bar[i], d0, r1, kb);
+          }
         }
-        u8* dst = smem + AE_MLA_SMEM_KV + stage * AE_MLA_KV_BYTES;
-        const int v_lo = dvh * (AE_MLA_NBV / 2), v_hi = v_lo + AE_MLA_NBV / 2;  // this CTA's value blocks
-        mbar_arrive_expect_tx(&bars->kx_full[stage], (AE_MLA_NBK - AE_MLA_NBV / 2) * (AE_MLA_BN * 128));
-        for (int blk = 0; blk < AE_MLA_NBV; ++blk)
-          if (blk < v_lo || blk >= v_hi)
-            tma_load_3d(dst + blk * (AE_MLA_BN * 128), &args.tm_kv, &bars->kx_full[stage], blk * 64, kv0, kb);
-        tma_load_3d(dst + AE_MLA_NBV * (AE_MLA_BN * 128), &args.tm_kpe, &bars->kx_full[stage], 0, kv0, kb);
-        if (!mbar_wait(&bars->kv_empty[stage], ((s / AE_MLA_STAGES) & 1) ^ 1, ctl, args.status, 41)) break;
-        mbar_arrive_expect_tx(&bars->kv_full[stage], (AE_MLA_NBV / 2) * (AE_MLA_BN * 128));
-        for (int blk = v_lo; blk < v_hi; ++blk)
-          tma_load_3d(dst + blk * (AE_MLA_BN * 128), &args.tm_kv, &bars->kv_full[stage], blk * 64, kv0, kb);
+      };
+      while (ok && next_seg(sg)) {
+        ok = mbar_wait_cl(&bars->q_empty, (n_seg & 1) ^ 1, ctl, args.status, 40);
+        if (!ok) break;
+        mla_expect(q_bar, AE_MLA_NBK * AE_MLA_KBLK);
+        for (int blk = 0; blk < AE_MLA_NBK; ++blk)
+          mla_load(smem + AE_MLA_SMEM_Q + blk * AE_MLA_KBLK, blk < 8 ? &args.tm_q : &args.tm_qpe, q_bar, blk < 8 ? blk * 64 : 0,
+                   (int)rank * 64, sg.b);
+        for (int t = sg.t0; t < sg.t1 && ok; ++t, ++it) {
+          const int r = kv_row(sg, t, (int)rank), kb = args.block_table ? 0 : sg.b;
+          for (int g = 0; g < 3 && ok; ++g) {
+            ok = mbar_wait_cl(&bars->k_empty[g], (it & 1) ^ 1, ctl, args.status, 42);
+            if (!ok) break;
+            mla_expect(k_bar[g], 3 * AE_MLA_KBLK);
+            for (int blk = 3 * g; blk < 3 * g + 3; ++blk)
+              mla_load(smem + AE_MLA_SMEM_K + blk * AE_MLA_KBLK, blk < 8 ? &args.tm_kv : &args.tm_kpe, k_bar[g],
+                       blk < 8 ? blk * 64 : 0, r, kb);
+          }
+          if (AE_MLA_PREFETCH > 0 && t + AE_MLA_PREFETCH < sg.t1) {
+            const int rp = kv_row(sg, t + AE_MLA_PREFETCH, (int)rank);
+            for (int blk = 0; blk < AE_MLA_NBK && rp < (1 << 30); ++blk)
+              mla_prefetch(blk < 8 ? &args.tm_kv : &args.tm_kpe, blk < 8 ? blk * 64 : 0, rp, kb);
+          }
+          // V follows the K of the tile after it, the order in which the MMAs free the slots
+          if (t > sg.t0 && ok) load_v(sg, t - 1, it - 1);
+        }
+        if (ok) load_v(sg, sg.t1 - 1, it - 1);
+        ++n_seg;
+      }
+      // the last release of every slot has arrived in this CTA before it may retire
+      if (ok && it > 0) {
+        ok = mbar_wait_cl(&bars->q_empty, (n_seg - 1) & 1, ctl, args.status, 50);
+        for (int g = 0; g < 3 && ok; ++g) ok = mbar_wait_cl(&bars->k_empty[g], (it - 1) & 1, ctl, args.status, 51);
+        for (int i = 0; i < 2 && ok; ++i) ok = mbar_wait_cl(&bars->v_empty[i], (it - 1) & 1, ctl, args.status, 52);
       }
     }
   } else if (warp == 5) {
-    // =============================== MMA issuer =================================
-    if (n_steps > 0) {  // all 32 lanes run the control flow; MMAs and commits are issued by an elected lane
-      const u32 idesc_s = umma_idesc_f16(AE_MLA_H, AE_MLA_BN, AE_BF16, 0, 0);
-      const u32 idesc_o = umma_idesc_f16(AE_MLA_H, AE_MLA_DVH, AE_BF16, 0, 1);
-      const u32 qs_addr = smem_u32(smem + AE_MLA_SMEM_QS);
-      const u32 kv_addr = smem_u32(smem + AE_MLA_SMEM_KV);
-      const u64 dq0 = umma_base_k(qs_addr), dk0 = umma_base_k(kv_addr);
-      const u64 dv0 = umma_base_mn(kv_addr + dvh * (AE_MLA_NBV / 2) * (AE_MLA_BN * 128), AE_MLA_BN);
-      auto issue_s = [&](int s, bool landed) -> bool {  // S_s into region s & 1
-        const int stage = s % AE_MLA_STAGES;
-        AE_TRM(true, 0, s * 8 + 0)
-        if (!landed) {
-          if (!mbar_wait_w(&bars->kx_full[stage], (s / AE_MLA_STAGES) & 1, ctl, args.status, 43)) return false;
-          if (!mbar_wait_w(&bars->kv_full[stage], (s / AE_MLA_STAGES) & 1, ctl, args.status, 44)) return false;
-        }
-        tc_fence_after_sync();
-        AE_TRM(true, 0, s * 8 + 1)
-        const u32 d = tmem + TM_S + (s & 1) * 64;
-        const u64 dks = dk0 + (u64)((stage * AE_MLA_KV_BYTES) >> 4);
+    // =============================== MMA issuer (rank 0) ====================================
+    if (rank == 0) {  // all 32 lanes run the control flow, one elected lane issues
+      const u32 idesc_s = umma_idesc_f16(128, AE_MLA_BN, AE_BF16, 0, 0);
+      const u32 idesc_o = umma_idesc_f16(128, 256, AE_BF16, 0, 1);
+      const u64 dq = umma_base_k(smem_u32(smem + AE_MLA_SMEM_Q));
+      const u64 dk = umma_base_k(smem_u32(smem + AE_MLA_SMEM_K));
+      const u64 dv = umma_base_mn(smem_u32(smem + AE_MLA_SMEM_V), AE_MLA_BN);
+      const u64 dp = umma_base_k(smem_u32(smem + AE_MLA_SMEM_P));
+      auto wait = [&](u64* bar, u32 parity, u32 site) -> bool {
+        return __all_sync(0xffffffffu, mbar_wait_cl(bar, parity, ctl, args.status, site));
+      };
+      auto issue_s = [&](int n) -> bool {  // S of the cluster's n-th tile into region n & 1
+        const u32 d = tmem + TM_S + (n & 1) * 64;
 #pragma unroll
-        for (int blk = 0; blk < AE_MLA_NBK; ++blk) {
+        for (int g = 0; g < 3; ++g) {
+          if (!wait(&bars->k_full[g], n & 1, 43)) return false;
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            const u64 db = dks + (u64)((blk * (AE_MLA_BN * 128) + kk * 32) >> 4);
-            if (blk < AE_MLA_QT)
-              umma_ts_w(d, tmem + TM_Q + blk * 32 + kk * 8, db, idesc_s, (blk | kk) > 0);
-            else
-              umma_ss_w(d, dq0 + (u64)(((blk - AE_MLA_QT) * (AE_MLA_H * 128) + kk * 32) >> 4), db, idesc_s, 1);
+            for (int blk = 3 * g; blk < 3 * g + 3; ++blk)
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk) {
+                const u64 off = (u64)((blk * AE_MLA_KBLK + kk * 32) >> 4);
+                umma_ss2(d, dq + off, dk + off, idesc_s, (blk | kk) > 0);
+              }
+            umma_commit2(&bars->k_empty[g]);
+            if (g == 2) umma_commit2(&bars->s_full[n & 1]);
           }
         }
-        umma_commit_w(&bars->kx_empty[stage]);  // the five blocks that only the S GEMM reads can be refilled
-        umma_commit_w(&bars->s_full[s & 1]);
-        AE_TRM(true, 0, s * 8 + 2)
         return true;
       };
-      // the blocks that stay in shared memory are read by the MMAs themselves: this warp waits for the TMA barrier
-      // too, not only for the row threads that saw it
-      bool ok = mbar_wait_w(&bars->q_full, 0, ctl, args.status, 49);
-      ok = ok && mbar_wait_w(&bars->q_tmem, 0, ctl, args.status, 42);
-      tc_fence_after_sync();
-      if (ok) ok = issue_s(0, false);
-      for (int s = 0; s < n_steps && ok; ++s) {
-        const int stage = s % AE_MLA_STAGES;
-        // The next S GEMM goes first if both parts of its KV tile have already landed (the other S region held P of tile
-        // s-1, whose P V GEMM was issued in the previous iteration); otherwise P V of this tile must not wait behind the
-        // load.
-        bool early = false;
-        if (s + 1 < n_steps) {
-          const int ns = (s + 1) % AE_MLA_STAGES;
-          const u32 np = ((s + 1) / AE_MLA_STAGES) & 1;
-          early = __all_sync(0xffffffffu, mbar_try_wait(&bars->kx_full[ns], np) && mbar_try_wait(&bars->kv_full[ns], np));
-          if (early) ok = issue_s(s + 1, true);
-        }
-        if (!ok) break;
-        AE_TRM(true, 0, s * 8 + 3)
-        // P of tile s: a named barrier (the four row warps arrive in every iteration, whatever happened; about 20 clk
-        // for this warp against 100 - 400 clk for an mbarrier wait)
-        named_bar_sync(1 + (s & 1), 128 + 32);
-        tc_fence_after_sync();
-        AE_TRM(true, 0, s * 8 + 4)
-        // V = this half's four 64-wide blocks of the same tile, read MN-major
-        const u64 dvs = dv0 + (u64)((stage * AE_MLA_KV_BYTES) >> 4);
+      bool ok = true;
+      int it = 0, n_seg = 0;
+      while (ok && next_seg(sg)) {
+        ok = wait(&bars->q_full, n_seg & 1, 44) && issue_s(it);
+        for (int t = sg.t0; t < sg.t1 && ok; ++t, ++it) {
+          // the S GEMM runs one tile ahead; the other region held S of tile it - 1, whose P has been handed over
+          if (t + 1 < sg.t1) ok = issue_s(it + 1);
+          if (!ok) break;
+          if (t + 2 >= sg.t1 && (t + 1 < sg.t1 || sg.t1 - sg.t0 == 1)) {
+            if (elect_one()) umma_commit2(&bars->q_empty);  // that was the segment's last S
+          }
+          ok = wait(&bars->p_full, it & 1, 45);
+          if (!ok) break;
+          tc_fence_after_sync();
 #pragma unroll
-        for (int kk = 0; kk < AE_MLA_BN / 16; ++kk)
-          umma_ts_w(tmem + TM_O, tmem + TM_S + (s & 1) * 64 + kk * 8, umma_step_mn(dvs, kk), idesc_o, (s > 0) | (kk > 0));
-        umma_commit_w(&bars->o_done);
-        umma_commit_w(&bars->kv_empty[stage]);
-        AE_TRM(true, 0, s * 8 + 5)
-        if (s + 1 < n_steps && !early) ok = issue_s(s + 1, false);
+          for (int i = 0; i < 2; ++i) {
+            if (!(ok = wait(&bars->v_full[i], it & 1, 46))) break;
+            if (elect_one()) {
+#pragma unroll
+              for (int kk = 0; kk < AE_MLA_BN / 16; ++kk)
+                umma_ss2(tmem + TM_O + i * 128, umma_step_k(dp, kk, 64), umma_step_mn(dv + (u64)((i * 2 * AE_MLA_VBLK) >> 4), kk), idesc_o,
+                         (t > sg.t0) | (kk > 0));
+              umma_commit2(&bars->v_empty[i]);
+              if (i == 1) umma_commit2(&bars->pv_done);
+            }
+          }
+        }
+        ++n_seg;
       }
     }
   } else {
-    // =============================== row threads (one per head) =================
-    const u32 row = threadIdx.x & 127;
+    // =============================== row threads (two per head) =============================
+    const u32 row = threadIdx.x & 63;        // head inside this CTA's block
+    const u32 half = (threadIdx.x >> 6) & 1;  // which half of the columns of every accumulator
     const u32 lane_base = ((warp & 3) * 32) << 16;
     const u32 tm_o = tmem + TM_O + lane_base;
-    const int h = (int)row;
-    bool ok = true;
-    // ---- query blocks 0 .. QT-1 of this head: shared memory (KV stage 0) -> TMEM, once -----------------
-    if (n_steps > 0) {
-      ok = mbar_wait(&bars->q_full, 0, ctl, args.status, 48);
-      const u8* src = smem + AE_MLA_SMEM_KV;
-      for (int blk = 0; blk < AE_MLA_QT; ++blk) {
-        u32 w[32];
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-          const uint4 v = *(const uint4*)(src + blk * (AE_MLA_H * 128) + swz128(row, ch));
-          w[ch * 4 + 0] = v.x;
-          w[ch * 4 + 1] = v.y;
-          w[ch * 4 + 2] = v.z;
-          w[ch * 4 + 3] = v.w;
-        }
-        tmem_st32(tmem + TM_Q + lane_base + blk * 32, w);  // column c holds elements 2c, 2c + 1 of the row
-      }
-      tc_wait_st();
-      tc_fence_before_sync();
-      mbar_arrive_warp(&bars->q_tmem);
-    }
+    const int h = (int)(rank * 64 + row);
+    const u32 p_bar = mapa_u32(smem_u32(&bars->p_full), 0);
     AeCustom cu;
 #pragma unroll
     for (int i = 0; i < AE_MAX_CUSTOM; ++i) {
@@ -255,130 +349,134 @@ extern "C" __global__ void __launch_bounds__(192, 1) ae_mla_decode(const __grid_
       for (int k = 0; k < 4; ++k) cu.st[i][k] = 0;
     }
     AeRow st;
-    st.init();
-    for (int s = 0; s < n_steps; ++s) {
-      const u32 tm_s = tmem + TM_S + (s & 1) * 64 + lane_base;
-      AE_TRM(warp == 0, 1, s * 8 + 0)
-      ok = ok && mbar_wait(&bars->s_full[s & 1], (s >> 1) & 1, ctl, args.status, 45);
-      tc_fence_after_sync();
-      AE_TRM(warp == 0, 1, s * 8 + 1)
-      float sc[AE_MLA_BN];
-      tmem_ld_f32x64(tm_s, sc);
-      const int kv0 = (t_begin + s) * AE_MLA_BN;
-      if (kv0 + AE_MLA_BN > S_b) {
+    st.xch = (volatile float*)(smem + AE_MLA_SMEM_XCH);
+    st.xme = half * 64 + row;
+    st.xother = (half ^ 1u) * 64 + row;
+    st.xbar = 1 + (warp & 1);  // warps w and w + 2 share their rows
+    st.xn = 64;
+    st.xphase = 0;
+    bool ok = true;
+    int it = 0, pos = 0;
+    for (int n_seg = 0; next_seg(sg); ++n_seg) {
+      st.init();
+      for (int t = sg.t0; t < sg.t1; ++t, ++it) {
+        const u32 tm_s = tmem + TM_S + (it & 1) * 64 + lane_base;
+        ok = mbar_wait_row(ok, &bars->s_full[it & 1], (it >> 1) & 1, ctl, args.status, 47);
+        tc_fence_after_sync();
+        float sc[64];
+        tmem_ld_f32x64(tm_s, sc);
+        const int kv0 = t * AE_MLA_BN + (int)half * 64;
+        if (t * AE_MLA_BN + AE_MLA_BN > sg.len) {
+          const int lim = sg.len - kv0;
 #pragma unroll
-        for (int c = 0; c < AE_MLA_BN; ++c)
-          sc[c] = kv0 + c < S_b ? sc[c] : -__int_as_float(0x7f800000);
-      }
-      const float o_scale = ae_online_fwd<AE_MLA_BN>(sc, st, b, h, 0, kv0, cu);
-      {
-        u32 pk[32];
-#pragma unroll
-        for (int half = 0; half < AE_MLA_BN / 64; ++half) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) pk[i] = pack2<AE_BF16>(sc[half * 64 + 2 * i], sc[half * 64 + 2 * i + 1]);
-          tmem_st32(tm_s + half * 32, pk);
+          for (int c = 0; c < 64; ++c) sc[c] = c < lim ? sc[c] : -__int_as_float(0x7f800000);
         }
-      }
+        float osc = 1.f;
+        ae_online_tile<1>(sc, st, sg.b, h, 0, kv0, cu, [&](auto K, float o_scale, float (&p)[64]) {
+          if constexpr (decltype(K)::value == -1) {
+            osc = o_scale;
+          } else {
+            // P V of the tile before has read P, and O is up to date
+            if (it > 0) ok = mbar_wait_row(ok, &bars->pv_done, (it - 1) & 1, ctl, args.status, 48);
+            u8* dst = smem + AE_MLA_SMEM_P + half * AE_MLA_KBLK;
+#pragma unroll
+            for (int ch = 0; ch < 8; ++ch) {
+              uint4 w;
+              w.x = pack2<AE_BF16>(p[ch * 8 + 0], p[ch * 8 + 1]);
+              w.y = pack2<AE_BF16>(p[ch * 8 + 2], p[ch * 8 + 3]);
+              w.z = pack2<AE_BF16>(p[ch * 8 + 4], p[ch * 8 + 5]);
+              w.w = pack2<AE_BF16>(p[ch * 8 + 6], p[ch * 8 + 7]);
+              *(uint4*)(dst + swz128(row, ch)) = w;
+            }
 #if !AE_O_SCALE_ONE
-      // O is rescaled only when some row of the warp needs it; only then must the previous P V GEMM have completed.
-      // Phase bookkeeping of the skipped waits: S_s may be issued before P V of tile s-1, so s_full(s) only implies
-      // that P V of tile s-2 has completed: o_done has then completed s-1 or s phases, and a parity wait for phase
-      // s-1 cannot alias.  The wait after the loop asks for phase n-1 and would alias if only n-2 had completed, so
-      // the last step always waits for its predecessor.
-      const bool rescale = __any_sync(0xffffffffu, o_scale != 1.0f);
-      if (s > 0 && (rescale || s + 1 == n_steps)) {
-        ok = ok && mbar_wait(&bars->o_done, (s - 1) & 1, ctl, args.status, 46);
-        tc_fence_after_sync();
-        if (rescale) {
+            if (t > sg.t0 && __any_sync(0xffffffffu, osc != 1.0f)) {
+              tc_fence_after_sync();
 #pragma unroll
-          for (int c = 0; c < AE_MLA_DVH / 32; ++c) {
-            float f[32];
-            u32 r[32];
-            tmem_ld_f32x32(tm_o + c * 32, f);
+              for (int c = 0; c < 8; ++c) {
+                float f[32];
+                u32 r[32];
+                tmem_ld_f32x32(tm_o + c * 32, f);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(f[i] * o_scale);
-            tmem_st32(tm_o + c * 32, r);
-          }
-        }
-      }
-#else
-      if (s > 0 && s + 1 == n_steps) {  // same phase bookkeeping: the wait after the loop must not find o_done two phases behind
-        ok = ok && mbar_wait(&bars->o_done, (s - 1) & 1, ctl, args.status, 46);
-        tc_fence_after_sync();
-      }
+                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(f[i] * osc);
+                tmem_st32(tm_o + c * 32, r);
+              }
+              tc_wait_st();
+            }
 #endif
-      tc_wait_st();
-      tc_fence_before_sync();
-      named_bar_arrive(1 + (s & 1), 128 + 32);
-      AE_TRM(warp == 0, 1, s * 8 + 2)
-    }
-
-    if (n_steps > 0) {
-      ok = ok && mbar_wait(&bars->o_done, (n_steps - 1) & 1, ctl, args.status, 47);
+            fence_proxy_async_smem();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(p_bar) : "memory");
+          }
+        });
+      }
+      ok = mbar_wait_row(ok, &bars->pv_done, (it - 1) & 1, ctl, args.status, 49);
       tc_fence_after_sync();
       const bool store = ok && h < args.H;
       const int hs = store ? h : 0;
-      if (args.n_split == 1) {
-        u16* orow = (u16*)args.o + ((i64)b * args.H + hs) * AE_MLA_DV + dvh * AE_MLA_DVH;
+      const bool whole = args.n_split > 0 ? args.n_split == 1 : (sg.t0 == 0 && sg.t1 == sg.n_t);
+      const i64 slot = args.n_split > 0 ? cl : 2 * cl + (n_seg > 0);
+      // this thread's dims: 128 of each half of the value dims
 #pragma unroll
-        for (int c = 0; c < AE_MLA_DVH / 32; ++c) {
-          float r[32];
-          tmem_ld_f32x32(tm_o + c * 32, r);
-          if (store) {
-            uint4* dst = (uint4*)(orow + c * 32);
+      for (int c = 0; c < 8; ++c) {
+        float r[32];
+        tmem_ld_f32x32(tm_o + c * 32, r);
+        const int d0 = (c >> 2) * 256 + (int)half * 128 + (c & 3) * 32;
+        if (store && whole) {
+          uint4* dst = (uint4*)((u16*)args.o + ((i64)sg.b * args.H + hs) * AE_MLA_DV + d0);
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              uint4 w;
-              w.x = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 0], st), ae_epilogue_o(r[v * 8 + 1], st));
-              w.y = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 2], st), ae_epilogue_o(r[v * 8 + 3], st));
-              w.z = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 4], st), ae_epilogue_o(r[v * 8 + 5], st));
-              w.w = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 6], st), ae_epilogue_o(r[v * 8 + 7], st));
-              dst[v] = w;
-            }
+          for (int v = 0; v < 4; ++v) {
+            uint4 w;
+            w.x = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 0], st), ae_epilogue_o(r[v * 8 + 1], st));
+            w.y = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 2], st), ae_epilogue_o(r[v * 8 + 3], st));
+            w.z = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 4], st), ae_epilogue_o(r[v * 8 + 5], st));
+            w.w = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 6], st), ae_epilogue_o(r[v * 8 + 7], st));
+            dst[v] = w;
           }
-        }
-      } else {
-        float* prow = args.o_part + (((i64)b * args.n_split + split) * args.H + hs) * AE_MLA_DV + dvh * AE_MLA_DVH;
+        } else if (store) {
+          float4* dst = (float4*)(args.o_part + (slot * args.H + hs) * AE_MLA_DV + d0);
 #pragma unroll
-        for (int c = 0; c < AE_MLA_DVH / 32; ++c) {
-          float r[32];
-          tmem_ld_f32x32(tm_o + c * 32, r);
-          if (store) {
-            float4* dst = (float4*)(prow + c * 32);
-#pragma unroll
-            for (int v = 0; v < 8; ++v)
-              dst[v] = make_float4(ae_epilogue_o(r[v * 4 + 0], st), ae_epilogue_o(r[v * 4 + 1], st),
-                                   ae_epilogue_o(r[v * 4 + 2], st), ae_epilogue_o(r[v * 4 + 3], st));
-          }
+          for (int v = 0; v < 8; ++v)
+            dst[v] = make_float4(ae_epilogue_o(r[v * 4 + 0], st), ae_epilogue_o(r[v * 4 + 1], st),
+                                 ae_epilogue_o(r[v * 4 + 2], st), ae_epilogue_o(r[v * 4 + 3], st));
         }
       }
+      tc_fence_before_sync();  // ordered before this warp's next arrival: the next segment's P V overwrites O
 #if AE_NFINAL > 0
-      if (store && dvh == 0) {
+      if (store && half == 0) {
         float fr[AE_NFINAL];
         ae_final_rowscales(st, fr);
+        if (whole) {
+          if (args.lse_out) args.lse_out[(i64)sg.b * args.H + h] = fr[0];
+        } else {
 #pragma unroll
-        for (int i = 0; i < AE_NFINAL; ++i)
-          if (args.fr_part[i]) args.fr_part[i][((i64)b * args.n_split + split) * args.H + h] = fr[i];
+          for (int i = 0; i < AE_NFINAL; ++i) args.fr_part[i][slot * args.H + h] = fr[i];
+        }
       }
 #endif
-    } else if (args.n_split > 1 && h < args.H) {
-      // rows of different lengths: this split starts past the row's last tile.  Its partial is zero with -inf row
-      // scales, which the combine pass weighs with exp(-inf - ...) = 0.
-      float4* dst = (float4*)(args.o_part + (((i64)b * args.n_split + split) * args.H + h) * AE_MLA_DV + dvh * AE_MLA_DVH);
-      for (int v = 0; v < AE_MLA_DVH / 4; ++v) dst[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (args.n_split == 0 && args.row_info && sg.t0 == 0 && rank == 0 && threadIdx.x == 0) {
+        // for the merge: first partial slot of the row and the number of intervals it touches (1 = written directly)
+        args.row_info[2 * sg.b] = (int)slot;
+        args.row_info[2 * sg.b + 1] = (pos + sg.n_t - 1) / bars->share + 1;
+      }
+      pos += sg.t1 - sg.t0;
+    }
+    if (args.n_split > 1 && it == 0 && h < args.H) {
+      // a share past the row's last tile: a zero partial with -inf row scales, which the merge weighs with exp(-inf - ...) = 0
+      float4* dst = (float4*)(args.o_part + ((i64)cl * args.H + h) * AE_MLA_DV + half * 256);
+      for (int v = 0; v < 64; ++v) dst[v] = make_float4(0.f, 0.f, 0.f, 0.f);
 #if AE_NFINAL > 0
-      if (dvh == 0)
-        for (int i = 0; i < AE_NFINAL; ++i)
-          if (args.fr_part[i]) args.fr_part[i][((i64)b * args.n_split + split) * args.H + h] = -__int_as_float(0x7f800000);
+      if (half == 0)
+        for (int i = 0; i < AE_NFINAL; ++i) args.fr_part[i][(i64)cl * args.H + h] = -__int_as_float(0x7f800000);
 #endif
     }
   }
 
   tc_fence_before_sync();
   __syncthreads();
+  cluster_sync_all();
   if (warp == 5) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem, 512);
+    tmem_dealloc2(tmem, 512);
   }
 }

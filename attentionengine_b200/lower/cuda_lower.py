@@ -700,7 +700,7 @@ def lower_attention(score_mod, mask_mod, online_func, custom_fwd_inputs: CustomI
     row_struct += (
         "#if AE_RSPLIT > 1\n"
         "AE_DEVICE float ae_row_xchg(AeRow& st, float x, int is_max) {\n"
-        "  volatile float* slot = st.xch + (st.xphase & 1u) * (AE_RSPLIT * 128);\n"
+        "  volatile float* slot = st.xch + (st.xphase & 1u) * (AE_RSPLIT * AE_XCH_ROWS);\n"
         "  slot[st.xme] = x;\n"
         "  named_bar_sync(st.xbar, st.xn);\n"
         "  const float y = slot[st.xother];\n"
@@ -831,7 +831,7 @@ def lower_attention(score_mod, mask_mod, online_func, custom_fwd_inputs: CustomI
         "AE_MASK_NEG_INF": int(str(mask_value).strip() in ("-inf", "-float('inf')")),
     }
     head = ("".join(f"#define {k} {v}\n" for k, v in defines.items())
-            + "#ifndef AE_RSPLIT\n#define AE_RSPLIT 1  // threads per score row in the kernel that includes this\n#endif\n"
+            + "#ifndef AE_RSPLIT\n#define AE_RSPLIT 1  // threads per score row in the kernel that includes this\n#endif\n#ifndef AE_XCH_ROWS\n#define AE_XCH_ROWS 128  // rows that exchange partial reductions\n#endif\n"
             + "struct AeCustom;\n")
     fwd = head + "".join(src)
     bwd = fwd + "".join(bsrc)

@@ -77,7 +77,7 @@ class MlaParams(C.Structure):
     _fields_ = [("q", C.c_void_p), ("q_pe", C.c_void_p), ("kv", C.c_void_p), ("k_pe", C.c_void_p), ("o", C.c_void_p),
                 ("o_partial", C.c_void_p), ("rowscale_partial", C.c_void_p * AE_MAX_FINAL),
                 ("B", C.c_int32), ("H", C.c_int32), ("S", C.c_int32), ("n_split", C.c_int32), ("status", C.c_void_p),
-                ("lse_out", C.c_void_p)]
+                ("lse_out", C.c_void_p), ("n_clusters", C.c_int32), ("row_info", C.c_void_p)]
 
 
 class DecodeParams(C.Structure):
@@ -102,7 +102,8 @@ class MlaPagedParams(C.Structure):
                 ("cache_seqlens", C.c_void_p), ("o", C.c_void_p), ("o_partial", C.c_void_p),
                 ("rowscale_partial", C.c_void_p * AE_MAX_FINAL),
                 ("B", C.c_int32), ("H", C.c_int32), ("num_pages", C.c_int32), ("max_pages", C.c_int32),
-                ("max_seqlen", C.c_int32), ("n_split", C.c_int32), ("status", C.c_void_p), ("q_row_stride", C.c_int64)]
+                ("max_seqlen", C.c_int32), ("n_split", C.c_int32), ("status", C.c_void_p), ("q_row_stride", C.c_int64),
+                ("lse_out", C.c_void_p), ("n_clusters", C.c_int32), ("row_info", C.c_void_p)]
 
 
 class LinearParams(C.Structure):

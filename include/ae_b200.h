@@ -218,7 +218,13 @@ typedef struct AeMlaParams {
   float* rowscale_partial[AE_MAX_FINAL_ROWSCALES]; /* each [B, n_split, H] fp32 scratch */
   int32_t B, H, S, n_split;
   uint32_t* status;
-  float* lse_out; /* ae_launch_mla_combine only, optional: [B, H] log-sum-exp over the splits of rowscale_partial[0] */
+  float* lse_out; /* optional: [B, H] final row scale 0 of rows written directly (decode), log-sum-exp over the splits of
+                     rowscale_partial[0] of merged rows (combine) */
+  /* n_split == 0: the 128-key tiles of all rows are cut into n_clusters equal intervals, one CTA pair each; a row inside one
+   * interval is written directly, the others leave partials.  o_partial is then [2 * n_clusters, H, 512], rowscale_partial
+   * [2 * n_clusters, H], and row_info [B][2] tells the combine launch which slots are a row's. */
+  int32_t n_clusters;
+  int32_t* row_info;
 } AeMlaParams;
 
 int ae_launch_mla_decode(void* module, const AeMlaParams* p, void* stream);
@@ -239,10 +245,14 @@ typedef struct AeMlaPagedParams {
   const int32_t* cache_seqlens; /* [B]: keys of each batch row, 1 <= len <= max_pages * 64 */
   void* o;                      /* [B, H, 512] */
   float* o_partial;             /* [B, n_split, H, 512] fp32 (n_split > 1) */
-  float* rowscale_partial[AE_MAX_FINAL_ROWSCALES]; /* each [B, n_split, H]; with n_split == 1 the final row scales */
+  float* rowscale_partial[AE_MAX_FINAL_ROWSCALES]; /* each [B, n_split, H] (n_split > 1) */
   int32_t B, H, num_pages, max_pages, max_seqlen, n_split; /* max_seqlen <= max_pages * 64: bound of the lengths */
   uint32_t* status;
   int64_t q_row_stride; /* elements between the heads of q and of q_pe (576: one [B, H, 576] tensor); 0 = contiguous */
+  /* as in AeMlaParams; with n_split == 1 the final row scales go to lse_out */
+  float* lse_out;
+  int32_t n_clusters;
+  int32_t* row_info;
 } AeMlaPagedParams;
 
 int ae_launch_mla_decode_paged(void* module, const AeMlaPagedParams* p, void* stream);
