@@ -9,13 +9,15 @@
 // A cluster of two CTAs does it with tcgen05.mma.cta_group::2, M = 128: each CTA owns 64 heads, its O [64 x 512] fp32 takes
 // 256 TMEM columns (64 rows lie on 128 lanes: row r's first half of the columns on lane r, the second on lane r + 64), and
 // each B operand is split between the two: 64 of the 128 keys for S, half of the value dims for P V.  One CTA per head
-// block with M = 128 cannot hold O and S; splitting the value dims over two CTAs instead computed S twice (2240 clk of MMAs
-// per 64 keys and pair against about 1500 per 64 keys here).
+// block with M = 128 cannot hold O and S; splitting the value dims over two CTAs instead computed S twice.  Here the MMAs of a
+// 128-key tile take about 1,400 (S) and 1,200 clk (P V) of the 4,300 to 5,400 clk between tiles; the rest is the loads, 136 KB
+// per CTA and tile (V comes a second time, by value dims, out of L2), 7 TB/s into shared memory over the chip.
 //
 // Work: the tiles of all batch rows in one line, cut into equal intervals, one per cluster (args.n_clusters; an interval may
 // cover the end of a row, whole rows, the beginning of a row).  A row that lies in one interval is written directly,
-// others as normalised partials that ae_mla_combine merges.  One CTA pair per row and value half had 256 CTAs in two
-// waves at 128 rows.  With args.n_split > 0 (the caller's choice) cluster (b, s) takes share s of row b instead.
+// others as normalised partials that ae_mla_combine merges.  One CTA per row, split and value half left 108 of 148 SMs
+// without work in the second wave of 128 rows: 549 us for 128 rows of 8192 keys against 321 (inputs in turn: 380) now,
+// 147 -> 39 us for a paged call of 8 rows up to 4096 keys, 274 -> 141 us for a batch that just missed a wave.  With args.n_split > 0 (the caller's choice) cluster (b, s) takes share s of row b instead.
 //
 // Shared memory per CTA: Q 72 KB | K 72 KB (9 blocks of 64 keys) | V 64 KB (2 x 2 blocks of 64 dims, 128 keys) | P 16 KB.
 // K and V are one tile deep but released in parts (three K blocks, half of V), which are refilled while the MMAs of the
@@ -37,7 +39,7 @@
 #define AE_MLA_SMEM_BAR (AE_MLA_SMEM_P + 2 * AE_MLA_KBLK)
 #define AE_MLA_SMEM_XCH (AE_MLA_SMEM_BAR + 512)  // [phase][half][row] of ae_row_xchg
 #ifndef AE_MLA_PREFETCH
-#define AE_MLA_PREFETCH 2  // tiles ahead that are brought into L2 (0: none)
+#define AE_MLA_PREFETCH 1  // tiles ahead that are brought into L2: 0 / 1 / 2 / 4 took 351 / 325 / 335 / 368 us for 128 rows of 8192 keys
 #endif
 
 struct AeMlaBars {
@@ -52,20 +54,26 @@ struct AeMlaBars {
 };
 static_assert(sizeof(AeMlaBars) <= 512, "barrier block");
 
-// Load with the byte count going to a barrier of the pair's rank 0 (cluster address `bar`).
+// Load with the byte count going to a barrier of the pair's rank 0 (cluster address `bar`).  Rank 0 alone arrives there and
+// expects the bytes of both CTAs: rank 1's loads may complete before that, but never for a phase whose slot is not free in
+// both.  A remote arrive.expect_tx.release.cluster per load group held the producers up for 1,200 clk each (562 us).
 AE_DEVICE void mla_load(void* dst, const AeTmaDesc* d, u32 bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(smem_u32(dst)), "l"((u64)d), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
+// Arrival at a barrier of the pair's rank 0.  Release at CTA scope, the default: what it announces (P, written and fenced
+// towards the async proxy) is read by this CTA's own tensor core, the barrier's CTA only issues the MMA.  With
+// .release.cluster an arrival took about 1,200 clk under load: 345 us with one of them per tile on the chain of the rows.
+AE_DEVICE void mla_arrive(u32 bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 AE_DEVICE void mla_prefetch(const AeTmaDesc* d, int c0, int c1, int c2) {
   asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"((u64)d), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
-AE_DEVICE void mla_expect(u32 bar, u32 bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
+
 
 struct AeMlaSeg {
   int b, t0, t1;   // tiles [t0, t1) of batch row b
@@ -92,14 +100,14 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
 
   if (threadIdx.x == 0) {
     ctl->abort = 0;
-    mbar_init(&bars->q_full, 2);
+    mbar_init(&bars->q_full, 1);
     mbar_init(&bars->q_empty, 1);
     for (int i = 0; i < 3; ++i) {
-      mbar_init(&bars->k_full[i], 2);
+      mbar_init(&bars->k_full[i], 1);
       mbar_init(&bars->k_empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars->v_full[i], 2);
+      mbar_init(&bars->v_full[i], 1);
       mbar_init(&bars->v_empty[i], 1);
       mbar_init(&bars->s_full[i], 1);
     }
@@ -228,7 +236,7 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
         for (int i = 0; i < 2 && ok; ++i) {
           ok = mbar_wait_cl(&bars->v_empty[i], (n & 1) ^ 1, ctl, args.status, 41);
           if (!ok) return;
-          mla_expect(v_bar[i], 2 * AE_MLA_VBLK);
+          if (rank == 0) mbar_arrive_expect_tx(&bars->v_full[i], 4 * AE_MLA_VBLK);
           for (int j = 0; j < 2; ++j) {
             const int d0 = i * 256 + (int)rank * 128 + j * 64;
             u8* dst = smem + AE_MLA_SMEM_V + (i * 2 + j) * AE_MLA_VBLK;
@@ -240,7 +248,7 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
       while (ok && next_seg(sg)) {
         ok = mbar_wait_cl(&bars->q_empty, (n_seg & 1) ^ 1, ctl, args.status, 40);
         if (!ok) break;
-        mla_expect(q_bar, AE_MLA_NBK * AE_MLA_KBLK);
+        if (rank == 0) mbar_arrive_expect_tx(&bars->q_full, 2 * AE_MLA_NBK * AE_MLA_KBLK);
         for (int blk = 0; blk < AE_MLA_NBK; ++blk)
           mla_load(smem + AE_MLA_SMEM_Q + blk * AE_MLA_KBLK, blk < 8 ? &args.tm_q : &args.tm_qpe, q_bar, blk < 8 ? blk * 64 : 0,
                    (int)rank * 64, sg.b);
@@ -249,7 +257,7 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
           for (int g = 0; g < 3 && ok; ++g) {
             ok = mbar_wait_cl(&bars->k_empty[g], (it & 1) ^ 1, ctl, args.status, 42);
             if (!ok) break;
-            mla_expect(k_bar[g], 3 * AE_MLA_KBLK);
+            if (rank == 0) mbar_arrive_expect_tx(&bars->k_full[g], 6 * AE_MLA_KBLK);
             for (int blk = 3 * g; blk < 3 * g + 3; ++blk)
               mla_load(smem + AE_MLA_SMEM_K + blk * AE_MLA_KBLK, blk < 8 ? &args.tm_kv : &args.tm_kpe, k_bar[g],
                        blk < 8 ? blk * 64 : 0, r, kb);
@@ -406,7 +414,7 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
             fence_proxy_async_smem();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(p_bar) : "memory");
+            if (lane == 0) mla_arrive(p_bar);
           }
         });
       }

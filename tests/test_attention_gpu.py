@@ -1047,3 +1047,38 @@ def test_mla_paged_lengths_outside_the_table_raise(lens):
     torch.cuda.synchronize()
     eng.check_status()
     assert not o.any() and torch.allclose(lse.cpu(), torch.tensor([1.0, 256.0]).log().view(2, 1).expand(2, H), atol=1e-5)
+
+
+@pytest.mark.parametrize("B,H,max_pages,lens,paged", [
+    (1, 16, 2, [100], False),             # less than a tile
+    (3, 64, 4, [193] * 3, False),         # two tiles a row, the last one key into its second half
+    (5, 128, 19, [1153] * 5, False),      # intervals that end inside rows, begin inside rows and hold whole rows
+    (79, 16, 5, [300] * 79, False),       # more rows than intervals
+    (1, 16, 300, [19137], False),         # one row in the most intervals a merge takes (32)
+    (6, 100, 7, [1, 64, 65, 128, 129, 448], True),  # pages of half a tile, an odd number of them, heads past the last one
+    (90, 16, 6, [1 + (37 * i) % 384 for i in range(90)], True),
+])
+def test_mla_decode_in_equal_intervals(B, H, max_pages, lens, paged):
+    """The tiles of all rows cut into equal intervals, one per CTA pair: rows written directly and rows merged from the
+    partials of several intervals, at the edges of tiles and intervals, against the oracle row by row."""
+    dtype, scale = torch.bfloat16, 1 / math.sqrt(192)
+    g = torch.Generator().manual_seed(B)
+    q = torch.randn(B, 1, H, 576, generator=g).to(dtype)
+    rows = torch.randn(B, max_pages * 64, 576, generator=g).to(dtype)
+    eng = helpers.mla_engine(B, H, max_pages * 64, dtype, scale)
+    if paged:
+        perm = torch.randperm(B * max_pages, generator=g)
+        pool = torch.empty(B * max_pages, 64, 1, 576, dtype=dtype)
+        pool[perm] = rows.view(B * max_pages, 64, 1, 576)
+        o, _ = eng.decode_paged(q.cuda(), pool.cuda(), perm.to(torch.int32).view(B, max_pages).cuda(),
+                                torch.tensor(lens, dtype=torch.int32).cuda())
+    else:
+        kv = rows[:, :lens[0]]
+        o = eng(q[..., :512].contiguous().cuda(), q[..., 512:].contiguous().cuda(), kv[:, :, None, :512].contiguous().cuda(),
+                kv[:, :, None, 512:].contiguous().cuda())
+    torch.cuda.synchronize()
+    eng.check_status()
+    for b, n in enumerate(lens):
+        ro = orc.mla_decode(q[b:b + 1, 0, :, :512], q[b:b + 1, 0, :, 512:], rows[b:b + 1, :n, None, :512],
+                            rows[b:b + 1, :n, None, 512:], scale=scale)
+        _check(f"row {b} o", o[b:b + 1, 0].cpu(), ro, dtype)
