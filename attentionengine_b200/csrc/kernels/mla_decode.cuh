@@ -16,12 +16,14 @@
 // Work: the tiles of all batch rows in one line, cut into equal intervals, one per cluster (args.n_clusters; an interval may
 // cover the end of a row, whole rows, the beginning of a row).  A row that lies in one interval is written directly,
 // others as normalised partials that ae_mla_combine merges.  One CTA per row, split and value half left 108 of 148 SMs
-// without work in the second wave of 128 rows: 549 us for 128 rows of 8192 keys against 321 (inputs in turn: 380) now,
-// 147 -> 39 us for a paged call of 8 rows up to 4096 keys, 274 -> 141 us for a batch that just missed a wave.  With args.n_split > 0 (the caller's choice) cluster (b, s) takes share s of row b instead.
+// without work in the second wave of 128 rows: 549 us for 128 rows of 8192 keys against 295 (353 under the power cap) now,
+// 147 -> 39 us for a paged call of 8 rows up to 4096 keys, 274 -> 141 us for a batch that just missed a wave.  With
+// args.n_split > 0 (the caller's choice) cluster (b, s) takes share s of row b instead.
 //
 // Shared memory per CTA: Q 72 KB | K 72 KB (9 blocks of 64 keys) | V 64 KB (2 x 2 blocks of 64 dims, 128 keys) | P 16 KB.
 // K and V are one tile deep but released in parts (three K blocks, half of V), which are refilled while the MMAs of the
-// other parts run; an L2 prefetch two tiles ahead covers the latency of HBM.
+// other parts run.  No L2 prefetch: 74 pairs with 136 KB slots cover the latency, and prefetches one or two tiles ahead, which
+// share the bulk-copy queue with the loads, took 322 us where none take 295 (128 rows of 8192), 125 / 111 (32 rows).
 // TMEM columns: O dims 0-255 (128) | O dims 256-511 (128) | S0 64 | S1 64.
 // Roles per CTA: warps 0-3 row threads (two per row), warp 4 TMA producer, warp 5 of rank 0 the MMA issuer.
 // Barriers that both CTAs' loads or row warps complete live in rank 0; every tcgen05.commit arrives in both CTAs.
@@ -38,9 +40,6 @@
 #define AE_MLA_SMEM_P (AE_MLA_SMEM_V + 4 * AE_MLA_VBLK)
 #define AE_MLA_SMEM_BAR (AE_MLA_SMEM_P + 2 * AE_MLA_KBLK)
 #define AE_MLA_SMEM_XCH (AE_MLA_SMEM_BAR + 512)  // [phase][half][row] of ae_row_xchg
-#ifndef AE_MLA_PREFETCH
-#define AE_MLA_PREFETCH 1  // tiles ahead that are brought into L2: 0 / 1 / 2 / 4 took 351 / 325 / 335 / 368 us for 128 rows of 8192 keys
-#endif
 
 struct AeMlaBars {
   u64 q_full, q_empty;
@@ -68,10 +67,6 @@ AE_DEVICE void mla_load(void* dst, const AeTmaDesc* d, u32 bar, int c0, int c1, 
 // .release.cluster an arrival took about 1,200 clk under load: 345 us with one of them per tile on the chain of the rows.
 AE_DEVICE void mla_arrive(u32 bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-AE_DEVICE void mla_prefetch(const AeTmaDesc* d, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"((u64)d), "r"(c0), "r"(c1), "r"(c2)
-               : "memory");
 }
 
 
@@ -261,11 +256,6 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
             for (int blk = 3 * g; blk < 3 * g + 3; ++blk)
               mla_load(smem + AE_MLA_SMEM_K + blk * AE_MLA_KBLK, blk < 8 ? &args.tm_kv : &args.tm_kpe, k_bar[g],
                        blk < 8 ? blk * 64 : 0, r, kb);
-          }
-          if (AE_MLA_PREFETCH > 0 && t + AE_MLA_PREFETCH < sg.t1) {
-            const int rp = kv_row(sg, t + AE_MLA_PREFETCH, (int)rank);
-            for (int blk = 0; blk < AE_MLA_NBK && rp < (1 << 30); ++blk)
-              mla_prefetch(blk < 8 ? &args.tm_kv : &args.tm_kpe, blk < 8 ? blk * 64 : 0, rp, kb);
           }
           // V follows the K of the tile after it, the order in which the MMAs free the slots
           if (t > sg.t0 && ok) load_v(sg, t - 1, it - 1);
