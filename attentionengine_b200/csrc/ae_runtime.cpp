@@ -38,6 +38,7 @@ struct Driver {
   CUresult (*cuFuncGetAttribute)(int*, CUfunction_attribute, CUfunction) = nullptr;
   CUresult (*cuLaunchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
                              CUstream, void**, void**) = nullptr;
+  CUresult (*cuLaunchKernelEx)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr;
   CUresult (*cuGetErrorString)(CUresult, const char**) = nullptr;
   CUresult (*cuMemsetD32Async)(CUdeviceptr, unsigned, size_t, CUstream) = nullptr;
   CUresult (*cuTensorMapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -69,6 +70,7 @@ Driver& driver() {
     AE_SYM(cuFuncSetAttribute, "cuFuncSetAttribute")
     AE_SYM(cuFuncGetAttribute, "cuFuncGetAttribute")
     AE_SYM(cuLaunchKernel, "cuLaunchKernel")
+    AE_SYM(cuLaunchKernelEx, "cuLaunchKernelEx")
     AE_SYM(cuGetErrorString, "cuGetErrorString")
     AE_SYM(cuMemsetD32Async, "cuMemsetD32Async")
     AE_SYM(cuTensorMapEncodeTiled, "cuTensorMapEncodeTiled")
@@ -202,6 +204,29 @@ int launch(Module* m, unsigned gx, unsigned gy, unsigned gz, void* args, void* s
   void* params[] = {args};
   AE_CU(d.cuLaunchKernel(g_fn, gx, gy, gz, (unsigned)m->cfg.threads, 1, 1, (unsigned)m->cfg.smem_bytes,
                          (CUstream)stream, params, nullptr));
+  return AE_OK;
+}
+
+// Launch of a kernel that may be brought up while the kernel in front of it in the stream still runs: it begins with
+// ae_grid_wait(), the kernel in front calls ae_grid_trigger() once its CTAs are up.  GQA decode of 2 rows of 1000 keys with
+// its merge brought up early: 12.3 -> 11.6 us; long rows unchanged.  The MLA merge (a block per head and row) launched so
+// cost the split kernel in front of it 2 % (391 -> 399, 39.5 -> 40.2 us) and goes the plain way.
+int launch_after(Module* m, unsigned gx, unsigned gy, unsigned gz, void* args, void* stream) {
+  Driver& d = driver();
+  void* params[] = {args};
+  CUlaunchAttribute attr;
+  memset(&attr, 0, sizeof attr);
+  attr.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+  attr.value.programmaticStreamSerializationAllowed = 1;
+  CUlaunchConfig cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDimX = gx; cfg.gridDimY = gy; cfg.gridDimZ = gz;
+  cfg.blockDimX = (unsigned)m->cfg.threads; cfg.blockDimY = 1; cfg.blockDimZ = 1;
+  cfg.sharedMemBytes = (unsigned)m->cfg.smem_bytes;
+  cfg.hStream = (CUstream)stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  AE_CU(d.cuLaunchKernelEx(&cfg, g_fn, params, nullptr));
   return AE_OK;
 }
 
@@ -914,7 +939,7 @@ int ae_launch_decode_combine(void* module, const AeDecodeParams* p, void* stream
   a.DV = m->cfg.head_dim_v;
   a.n_split = p->n_split;
   a.part_off = p->part_off;  // rows of different lengths: each row's own number of partial slots
-  return launch(m, combine_blocks(a.H, a.DV), (unsigned)p->B, 1, &a, stream);
+  return launch_after(m, combine_blocks(a.H, a.DV), (unsigned)p->B, 1, &a, stream);
 }
 
 int ae_launch_rowscale(void* module, const AeRowScaleParams* p, void* stream) {

@@ -69,6 +69,12 @@ AE_DEVICE void mbar_arrive_expect_tx(u64* bar, u32 bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
+// Programmatic dependent launch: the trigger lets the next kernel of the stream be brought up once every CTA of this one has
+// called it or left (nothing happens if that kernel was launched without the attribute); the wait returns when the kernels
+// in front have completed and their writes are visible.
+AE_DEVICE void ae_grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+AE_DEVICE void ae_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // One poll of an mbarrier phase.  AE_WAIT_MODE selects the instruction:
 //   0  mbarrier.try_wait with a suspend-time hint (the thread may be parked by the hardware; fewest issue slots)
 //   1  mbarrier.try_wait without a hint

@@ -296,6 +296,9 @@ ae_attn_fwd(const __grid_constant__ AeAttnFwdArgs args) {
   __syncthreads();
   tc_fence_after_sync();
   const u32 tmem = ctl->tmem_base;
+#if AE_DECODE
+  ae_grid_trigger();
+#endif
 #if AE_MASK_MODE == 2
   n_steps = bars->n_steps;
 #endif

@@ -28,6 +28,7 @@ extern "C" __global__ void __launch_bounds__(128) ae_mla_combine(const AeMlaComb
   const int h = blockIdx.x * AE_CMB_HPB + threadIdx.x / AE_CMB_TPH;
   const int b = blockIdx.y;
   if (h >= args.H) return;  // warp-uniform
+  ae_grid_wait();  // GQA decode brings it up under the split kernel; everything read below is in place from here on
   int n_split = args.n_split;
   i64 slot0 = (i64)b * n_split, slot1 = slot0 + 1, step = 1;  // slots slot0, slot1, slot1 + step, ...
   if (args.part_off) {

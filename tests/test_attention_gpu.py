@@ -1082,3 +1082,23 @@ def test_mla_decode_in_equal_intervals(B, H, max_pages, lens, paged):
         ro = orc.mla_decode(q[b:b + 1, 0, :, :512], q[b:b + 1, 0, :, 512:], rows[b:b + 1, :n, None, :512],
                             rows[b:b + 1, :n, None, 512:], scale=scale)
         _check(f"row {b} o", o[b:b + 1, 0].cpu(), ro, dtype)
+
+
+def test_split_decode_with_its_merge_in_a_graph():
+    """The merge is launched to come up under the split kernel; captured and replayed on new inputs it still follows it."""
+    B, Hq, Hkv, Skv, D, dtype = 2, 32, 8, 1000, 128, torch.float16
+    eng = helpers.decode_engine(B, Hq, Hkv, 1, Skv, D, dtype)
+    g = torch.Generator().manual_seed(3)
+    q, k, v = (torch.randn(B, n, h, D, generator=g).to(dtype).cuda() for n, h in ((1, Hq), (Skv, Hkv), (Skv, Hkv)))
+    eng(q, k, v)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        o = eng(q, k, v)
+    for _ in range(3):
+        for t in (q, k, v):
+            t.copy_(torch.randn(t.shape, generator=g).to(dtype))
+        graph.replay()
+        torch.cuda.synchronize()
+        eng.check_status()
+        assert torch.equal(o, eng(q, k, v))
