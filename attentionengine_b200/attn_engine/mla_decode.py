@@ -66,6 +66,8 @@ class MlaDecode:
                     raise rt.AeError(f"{name} must be a CUDA tensor: this back end has no CPU path")
                 if t.dtype != self.dtype:
                     raise TypeError(f"{name} has dtype {t.dtype}, engine was built for {self.dtype}")
+            if q.dim() == kv.dim() == 4 and 0 in (q.shape[0], q.shape[2], kv.shape[1]):
+                raise rt.AeError(f"MLA decode of an empty problem: q {tuple(q.shape)}, kv {tuple(kv.shape)}")
             raise ValueError("expected q [B,1,H,512], q_pe [B,1,H,64], kv [B,S,1,512], k_pe [B,S,1,64]")
         o, self.last_num_split = res
         return o

@@ -411,6 +411,7 @@ py::object mla(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, const Tens
   const int64_t B = q.size(0), H = q.size(2), S = kv.size(1);
   if (!same(q, {B, 1, H, 512}) || !same(q_pe, {B, 1, H, 64}) || !same(kv, {B, S, 1, 512}) || !same(k_pe, {B, S, 1, 64}))
     return py::none();
+  if (B == 0 || H == 0 || S == 0) return py::none();  // the cut into intervals below divides by the tiles of a row
   py::gil_scoped_release nogil;
   c10::cuda::CUDAGuard guard(q.device());
   at::AutoGradMode no_grad(false);
