@@ -149,6 +149,26 @@ class _AttnKernels:
         return self._bwd_fused
 
 
+class _AttentionFn(torch.autograd.Function):
+    """The call as a Python autograd function, for what the native node cannot stand for: forward mode (refused by
+    PyTorch) and torch.jit.trace (recorded by it)."""
+
+    @staticmethod
+    def forward(ctx, eng, block_mask, q, k, v, *custom):
+        o, finals, ctx.lists = eng._launch_fwd(q, k, v, custom, block_mask, return_lists=True)
+        ctx.eng, ctx.n_final = eng, len(finals)
+        ctx.save_for_backward(q, k, v, o, *finals, *custom)
+        return o
+
+    @staticmethod
+    def backward(ctx, d_o):
+        q, k, v, o, *rest = ctx.saved_tensors
+        finals, custom = rest[:ctx.n_final], rest[ctx.n_final:]
+        with torch.cuda.device(q.device):
+            dq, dk, dv = ctx.eng._launch_bwd(q, k, v, o, d_o, finals, custom, ctx.lists)
+        return (None, None, dq, dk, dv) + (None,) * len(custom)
+
+
 def custom_slots(specs) -> list:
     """What the native host path needs of the custom inputs: (slot, 16-bit tile?, index slot of every dim)."""
     return [(sp.slot, bool(sp.is_16bit), [int(d) for d in sp.dim_slots]) for sp in specs]
@@ -392,25 +412,30 @@ class AttentionEngine:
         return self._ensure_lists(q.device, block_mask if block_mask is not None else (
             self.block_mask if self.extern_block_mask else None), B, Hq, Sq, Skv)
 
-    def _refuse(self, q, k, v, custom):
-        """The native path did not take these tensors: raise what is wrong with them."""
+    def _check_call(self, q, k, v, custom):
+        """Raise what is wrong with the tensors of a call."""
         _, Sq, _, Skv, _ = self._check_qkv(q, k, v)
         for t in custom:
             if not t.is_cuda:
                 raise rt.AeError("custom inputs must be CUDA tensors: this back end has no CPU path")
         self._custom_args(custom, Sq, Skv)
-        raise ValueError("tensors do not fit this engine")
 
-    def _launch_fwd(self, q, k, v, custom, block_mask=None):
+    def _launch_fwd(self, q, k, v, custom, block_mask=None, return_lists=False):
         """Forward without autograd: (o, [final row scales])."""
         lists = self._tile_lists(q, k, v, block_mask)
         res = rt.host().attn(self._native_plan(), self, q, k, v, custom, lists, True)
-        return res if res is not None else self._refuse(q, k, v, custom)
+        if res is None:
+            self._check_call(q, k, v, custom)
+            raise ValueError("tensors do not fit this engine")
+        return (*res, lists) if return_lists else res
 
     def _apply(self, q, k, v, custom, block_mask):
         lists = self._tile_lists(q, k, v, block_mask) if self.mask_mode == 2 else None
         o = rt.host().attn(self._plan or self._native_plan(), self, q, k, v, custom, lists, False)
-        return o if o is not None else self._refuse(q, k, v, custom)
+        if o is None:
+            self._check_call(q, k, v, custom)
+            o = _AttentionFn.apply(self, block_mask, q, k, v, *custom)
+        return o
 
     def decode_paged(self, q, kcache, block_table, cache_seqlens, num_split=None):
         """kv_shared engines: decode over a paged KV pool with one length per batch row, returns (out, lse)."""

@@ -49,6 +49,24 @@ def _align(t: torch.Tensor, names: tuple, ndim: int) -> torch.Tensor:
     return t.reshape(shape)
 
 
+class _Scan(torch.autograd.Function):
+    """The scan on the mod-ed tensors as a Python autograd function, for what the native node cannot stand for: forward mode
+    (refused by PyTorch) and torch.jit.trace (recorded by it)."""
+
+    @staticmethod
+    def forward(ctx, eng, q, k, v, a):
+        q, k, v, a = q.contiguous(), k.contiguous(), v.contiguous(), a.float().contiguous()
+        ctx.eng = eng
+        hs = eng._new_states(v) if (any(ctx.needs_input_grad) and v.shape[3] == 64) else None
+        ctx.save_for_backward(q, k, v, a, hs)
+        return eng._launch(q, k, v, a, h_out=hs)
+
+    @staticmethod
+    def backward(ctx, d_o):
+        q, k, v, a, hs = ctx.saved_tensors
+        return (None, *ctx.eng._launch_bwd(q, k, v, a, d_o.contiguous(), hs=hs))
+
+
 class _RowScale(torch.autograd.Function):
     """y = x * s[..., None] for x [B, H, T, D] 16-bit and s [B, H, T]: the `v * dt` shape of mod, as one streaming
     kernel each way (csrc/kernels/rowscale.cuh) instead of PyTorch's broadcast multiply and 64-wide reduction."""
@@ -502,7 +520,8 @@ class LinearAttentionEngine:
     def _native_scan(self, q, k, v, a):
         """The scan on the mod-ed tensors as one autograd node; gradients flow on into the eager mods through torch autograd
         (the reference chains the traced mod derivatives by hand, linear_tl.py:1203-1214)."""
-        return rt.host().scan(self._native_plan(), self._fwd_kernel(v.shape[3])[0].handle.value, self, q, k, v, a)
+        o = rt.host().scan(self._native_plan(), self._fwd_kernel(v.shape[3])[0].handle.value, self, q, k, v, a)
+        return o if o is not None else _Scan.apply(self, q, k, v, a)
 
     def _scan(self, q, k, v, a):
         """The scan on heads of any supported size, from kernels that take 128 key dims and 64 / 128 value dims.

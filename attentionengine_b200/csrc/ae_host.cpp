@@ -16,6 +16,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pybind.h>
 #include <ATen/ATen.h>
 
@@ -115,6 +116,16 @@ bool wants_grad(std::initializer_list<const Tensor*> ts) {
   if (!at::GradMode::is_enabled()) return false;
   for (const Tensor* t : ts)
     if (t->defined() && t->requires_grad()) return true;
+  return false;
+}
+
+// Calls that a native node cannot stand for: it has no forward-mode rule (the result would lose the tangent in silence), and
+// torch.jit.trace would record the result's allocation and not the kernel.  The front end takes them through
+// torch.autograd.Function, which PyTorch knows to refuse and to record.
+bool needs_function(std::initializer_list<const Tensor*> ts) {
+  if (torch::jit::tracer::isTracing()) return true;
+  for (const Tensor* t : ts)
+    if (torch::autograd::isFwGradDefined(*t)) return true;
   return false;
 }
 
@@ -249,12 +260,18 @@ struct AttnNode : Node {
   std::string name() const override { return "AttentionEngineBackward"; }
 };
 
-// o = engine(q, k, v, *custom); None when the tensors do not fit.  `with_finals`: (o, [final row scales]) without autograd.
+// o = engine(q, k, v, *custom); None when the tensors do not fit or the call needs an autograd function.  `with_finals`:
+// (o, [final row scales]) without autograd.
 py::object attn(const std::shared_ptr<AttnPlan>& plan, py::handle eng, const Tensor& q, const Tensor& k, const Tensor& v,
                 py::handle custom, py::handle lists, bool with_finals) {
   Dims d;
   if (!attn_dims(*plan, q, k, v, d)) return py::none();
   std::vector<Tensor> C = tensors_of(custom), L = tensors_of(lists), F(plan->n_final);
+  if (!with_finals) {
+    bool function = needs_function({&q, &k, &v});
+    for (const Tensor& c : C) function = function || needs_function({&c});
+    if (function) return py::none();
+  }
   Tensor o, status;
   {
     py::gil_scoped_release nogil;
@@ -718,13 +735,16 @@ Tensor scan_run(const std::shared_ptr<ScanPlan>& plan, void* kernel, py::handle 
   return y;
 }
 
+// None when the call needs an autograd function.
 py::object scan(const std::shared_ptr<ScanPlan>& plan, uint64_t kernel, py::handle eng, const Tensor& q, const Tensor& k,
                 const Tensor& v, const Tensor& a) {
+  if (needs_function({&q, &k, &v, &a})) return py::none();
   return py::cast(scan_run(plan, handle(kernel), eng, q, k, v, a, Tensor(), Tensor(), Tensor()));
 }
 
 // The Mamba2 block: x * s[b, h, t] into the scan, + x * d[head] after it, decay * asc[head] (None: decay as passed).  None
-// when the operands are not of that form at run time (the caller then takes the mods one by one).
+// when the operands are not of that form at run time or the call needs an autograd function (the caller then takes the mods
+// one by one).
 py::object scan_block(const std::shared_ptr<ScanPlan>& plan, py::handle eng, const Tensor& q, const Tensor& k, const Tensor& x,
                       const Tensor& decay, const Tensor& s, const Tensor& d, const std::optional<Tensor>& asc) {
   for (const Tensor* t : {&q, &k, &x})
@@ -736,6 +756,7 @@ py::object scan_block(const std::shared_ptr<ScanPlan>& plan, py::handle eng, con
   if (d.numel() != H || d.scalar_type() != at::kFloat) return py::none();
   if (decay.dim() != 3 || !same(decay, {B, H, T}) || q.size(0) != B || k.size(0) != B || q.size(2) != T || k.size(2) != T)
     return py::none();
+  if (needs_function({&q, &k, &x, &decay, &s, &d}) || (asc && needs_function({&*asc}))) return py::none();
   if (asc && (!asc->is_cuda() || asc->numel() != H || asc->scalar_type() != at::kFloat)) return py::none();
   if (!plan->fwd_mods) eng.attr("_load_block_kernel")();
   return py::cast(scan_run(plan, plan->fwd_mods, eng, q, k, x, decay, s, d, asc ? *asc : Tensor()));

@@ -3,9 +3,10 @@ import math
 
 import pytest
 import torch
+import torch.autograd.forward_ad as fwAD
 
 import helpers
-from attentionengine_b200 import runtime as rt
+from attentionengine_b200 import AttentionEngine, CustomIO, runtime as rt
 
 pytestmark = pytest.mark.gpu
 
@@ -21,3 +22,68 @@ def test_mla_of_an_empty_problem_raises(B, H, S):
     args = [torch.zeros(s, dtype=torch.float16, device="cuda") for s in ((B, 1, H, 512), (B, 1, H, 64), (B, S, 1, 512), (B, S, 1, 64))]
     with pytest.raises(rt.AeError, match="empty"):
         eng(*args)
+
+
+# ---------------------------------------------------------------------------------------------------- nodes
+def _attention(mask="causal", S=300, D=64, dtype=torch.float16):
+    """An attention call: (engine, q, k, v, d_o) with GQA heads."""
+    B, Hq, Hkv = 2, 4, 2
+    if mask == "window":
+        eng = AttentionEngine(helpers.metas(B, Hq, Hkv, S, D, D, dtype), CustomIO({}), score_mod=lambda s, c, b, h, q, kv: s * D ** -0.5,
+                              mask_mod=lambda b, h, q, kv: torch.logical_and(q >= kv, q - kv <= 130), online_func=helpers.OnlineSoftmax())
+        assert eng.mask_mode == 2
+    else:
+        eng = helpers.softmax_engine(B, Hq, Hkv, S, D, D, dtype, True)
+    return (eng, *helpers.seeded_qkv(B, Hq, Hkv, S, D, D, dtype, seed=1, device="cuda"))
+
+
+def _block(T=200, H=4, dtype=torch.bfloat16, seed=2):
+    """A Mamba2 block call: (engine, [C, B, x, step, A, step16, skip], d_o)."""
+    x, step, A, Bm, Cm = (t.cuda() for t in helpers.mamba2_inputs(2, H, T, 128, 64, dtype, seed=seed))
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    eng = helpers.mamba2_engine(2, H, T, 128, 64, dtype, d_skip=True)
+    return eng, [Cm, Bm, x, step, A.view(1, H), step.to(dtype), torch.randn(1, H, generator=g, device="cuda")], torch.randn(x.shape, generator=g, device="cuda", dtype=dtype)
+
+
+def test_forward_mode_is_refused():
+    """Neither kernel has a forward-mode rule: a dual tensor among the inputs raises, it does not lose its tangent."""
+    eng, q, k, v, _ = _attention()
+    scan, args, _ = _block()
+    with fwAD.dual_level():
+        for i in range(3):
+            a = [q, k, v]
+            a[i] = fwAD.make_dual(a[i], torch.ones_like(a[i]))
+            with pytest.raises(NotImplementedError, match="jvp"):
+                eng(*a)
+        for i in range(len(args)):
+            a = list(args)
+            a[i] = fwAD.make_dual(a[i], torch.ones_like(a[i]))
+            with pytest.raises(NotImplementedError, match="jvp"):
+                scan(*a)
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("mask", ["causal", "window"])
+def test_traced_attention_runs_its_kernel(mask):
+    """torch.jit.trace records the call: on other inputs the traced function computes, with gradients."""
+    eng, q, k, v, d_o = _attention(mask)
+    f = torch.jit.trace(lambda a, b, c: eng(a, b, c) * 2, (q, k, v), check_trace=False)
+    q2, k2, v2 = (torch.randn_like(t).requires_grad_() for t in (q, k, v))
+    o = f(q2, k2, v2)
+    got = (o, *torch.autograd.grad(o, (q2, k2, v2), d_o))
+    o = eng(q2, k2, v2) * 2
+    want = (o, *torch.autograd.grad(o, (q2, k2, v2), d_o))
+    assert torch.equal(got[0], want[0])
+    for x, y in zip(got[1:], want[1:]):  # dQ: fp32 additions in any order, rounded to fp16
+        torch.testing.assert_close(x, y, rtol=2 ** -9, atol=2 ** -9)
+
+
+@pytest.mark.filterwarnings("ignore")
+def test_traced_scan_runs_its_kernel():
+    """The same for the Mamba2 block, whose mods then run one by one: their results are rounded to bf16 in between."""
+    eng, args, _ = _block()
+    f = torch.jit.trace(lambda *a: eng(*a), tuple(args), check_trace=False)
+    other = _block(seed=3)[1]
+    o = eng(*other)
+    err = (f(*other).float() - o.float()).norm() / o.float().norm()
+    assert err < 4 * 2 ** -8  # v * step and the output before the skip, each rounded once more
