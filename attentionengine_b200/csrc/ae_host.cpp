@@ -192,7 +192,7 @@ struct AttnNode : Node {
 
   variable_list apply(variable_list&& grads) override {
     variable_list out(3 + custom.size());
-    if (!grads[0].defined()) return out;
+    if (!grads[0].defined()) grads[0] = input_metadata(0).zeros_like();  // as torch.autograd.Function does
     Tensor Q, K, V, O;
     std::vector<Tensor> F, C, lists;
     {
@@ -575,7 +575,7 @@ struct ScanNode : Node {
 
   variable_list apply(variable_list&& grads) override {
     variable_list out(mods ? 7 : 4);
-    if (!grads[0].defined()) return out;
+    if (!grads[0].defined()) grads[0] = input_metadata(0).zeros_like();  // as torch.autograd.Function does
     Tensor q, k, v, a, x, s, d, asc, hs;
     {
       std::lock_guard<std::mutex> lock(mutex_);

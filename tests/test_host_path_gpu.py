@@ -87,3 +87,23 @@ def test_traced_scan_runs_its_kernel():
     o = eng(*other)
     err = (f(*other).float() - o.float()).norm() / o.float().norm()
     assert err < 4 * 2 ** -8  # v * step and the output before the skip, each rounded once more
+
+
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+def test_undefined_gradient_counts_as_zero():
+    eng, q, k, v, _ = _attention()
+    scan, args, _ = _block()
+    for f, leaves in ((eng, [q, k, v]), (scan, args)):
+        for t in leaves:
+            t.requires_grad_()
+        _NoGradient.apply(f(*leaves)).sum().backward()
+        assert all(t.grad is not None and not t.grad.any() for t in leaves)
