@@ -100,6 +100,8 @@ class MlaDecode:
         B, one, H, D = q.shape
         if one != 1 or D != 576 or H > 128:
             raise ValueError("expected q [B, 1, H <= 128, 576]")
+        if B == 0 or H == 0:
+            raise rt.AeError(f"MLA decode of an empty problem: q {tuple(q.shape)}")
         if kcache.dim() == 4:
             if kcache.shape[2] != 1:
                 raise ValueError("expected kcache [num_pages, 64, 1, 576]")

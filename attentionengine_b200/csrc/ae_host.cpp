@@ -8,6 +8,7 @@
 // Convention: a call whose tensors do not fit its engine returns None without launching anything; the Python front end
 // then runs its own checks, which raise the error that names the reason.
 #include <Python.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -460,21 +461,56 @@ py::object mla(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, const Tens
   return py::make_tuple(o, n_split ? (double)n_split : std::max(merge ? 1.0 + 1.0 / B : 1.0, (double)p.n_clusters / B));
 }
 
-// Pinned landing place of the row lengths and the event behind their copy, one per thread and device.
+// Pinned landing place of the row lengths and the event behind their copy, one per thread.
 struct Lengths {
   int32_t* host = nullptr;
   int64_t room = 0;
   int device = -1;
   cudaEvent_t copied = nullptr;
-  ~Lengths() {
+  void release() {
     if (host) cudaFreeHost(host);
     if (copied) cudaEventDestroy(copied);
+    host = nullptr;
+    copied = nullptr;
+    room = 0;
+    device = -1;
+  }
+  void make(int dev, int64_t n) {  // nothing is left behind that a failed allocation would make look usable
+    if (device == dev && room >= n) return;
+    release();
+    C10_CUDA_CHECK(cudaHostAlloc((void**)&host, (size_t)n * 4, cudaHostAllocDefault));
+    C10_CUDA_CHECK(cudaEventCreateWithFlags(&copied, cudaEventDisableTiming));
+    room = n;
+    device = dev;
+  }
+  ~Lengths() { release(); }
+};
+
+// A copy into the landing place: waited for on every way out, so that the thread's next call finds no older one in flight.
+struct Landing {
+  Lengths& land;
+  cudaStream_t st;
+  bool recorded = false, waiting = true;
+  Landing(Lengths& l, const Tensor& lens, cudaStream_t s) : land(l), st(s) {
+    C10_CUDA_CHECK(cudaMemcpyAsync(l.host, lens.data_ptr(), (size_t)lens.numel() * 4, cudaMemcpyDeviceToHost, s));
+  }
+  void record() {
+    C10_CUDA_CHECK(cudaEventRecord(land.copied, st));
+    recorded = true;
+  }
+  cudaError_t wait() {
+    waiting = false;
+    return recorded ? cudaEventSynchronize(land.copied) : cudaStreamSynchronize(st);
+  }
+  ~Landing() {
+    if (waiting) (void)wait();
   }
 };
 
-// (o, lse, shares per row) over a paged cache; n_split 0: equal intervals of all rows' tiles.  The row lengths are checked on the host, as before, but behind the launches: their copy is
-// queued in front of the kernels, which clamp every length to the block table themselves, so the stream never drains for
-// the check.  Returns None when the tensors do not fit, or an empty tuple for lengths outside their range.
+// (o, lse, shares per row) over a paged cache; n_split 0: equal intervals of all rows' tiles.  The row lengths are checked on
+// the host behind the launches: their copy is queued in front of the kernels, which clamp every length to the block table
+// themselves, so the stream never drains for the check.  Returns None when the tensors do not fit, or an empty tuple for
+// lengths outside their range.
 py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, const Tensor& pool, const Tensor& table_in,
                      const Tensor& lens_in, int n_split) {
   const MlaPlan& P = *plan;
@@ -483,6 +519,7 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
   const bool d4 = pool.dim() == 4;
   if ((!d4 && pool.dim() != 3) || pool.size(1) != 64 || pool.size(-1) != 576 || (d4 && pool.size(2) != 1)) return py::none();
   const int64_t B = q.size(0), H = q.size(2);
+  if (B == 0 || H == 0) return py::none();
   if (table_in.dim() != 2 || table_in.size(0) != B || lens_in.dim() != 1 || lens_in.size(0) != B) return py::none();
   py::gil_scoped_release nogil;
   c10::cuda::CUDAGuard guard(q.device());
@@ -490,20 +527,17 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
   const auto ints = q.options().dtype(at::kInt);
   const Tensor table = table_in.to(ints).contiguous(), lens = lens_in.to(ints).contiguous();
   const int64_t max_pages = table.size(1);
+  if (max_pages == 0) {
+    py::gil_scoped_acquire gil;
+    return py::tuple();
+  }
+  TORCH_CHECK(c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None,
+              "paged MLA decode reads the row lengths on the host: it cannot be captured into a CUDA graph");
   static thread_local Lengths land;
   cudaStream_t st = (cudaStream_t)stream_of(q);
-  if (land.device != q.device().index() || land.room < B) {
-    if (land.host) cudaFreeHost(land.host);
-    if (land.copied) cudaEventDestroy(land.copied);
-    land.host = nullptr;
-    land.copied = nullptr;
-    C10_CUDA_CHECK(cudaHostAlloc((void**)&land.host, (size_t)B * 4, cudaHostAllocDefault));
-    land.room = B;
-    C10_CUDA_CHECK(cudaEventCreateWithFlags(&land.copied, cudaEventDisableTiming));
-    land.device = q.device().index();
-  }
-  C10_CUDA_CHECK(cudaMemcpyAsync(land.host, lens.data_ptr(), (size_t)B * 4, cudaMemcpyDeviceToHost, st));
-  C10_CUDA_CHECK(cudaEventRecord(land.copied, st));
+  land.make(q.device().index(), B);
+  Landing landing(land, lens, st);
+  landing.record();
 
   const Tensor Q = q.contiguous();
   Tensor o = at::empty({B, 1, H, 512}, q.options());
@@ -538,7 +572,7 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
     m.lse_out = p.lse_out;
     check(ae_launch_mla_combine(P.combine, &m, st), "ae_launch_mla_combine");
   }
-  C10_CUDA_CHECK(cudaEventSynchronize(land.copied));
+  C10_CUDA_CHECK(landing.wait());
   bool in_range = true;
   for (int64_t b = 0; b < B; ++b) in_range = in_range && land.host[b] >= 1 && land.host[b] <= max_pages * 64;
   py::gil_scoped_acquire gil;

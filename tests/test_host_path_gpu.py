@@ -107,3 +107,46 @@ def test_undefined_gradient_counts_as_zero():
             t.requires_grad_()
         _NoGradient.apply(f(*leaves)).sum().backward()
         assert all(t.grad is not None and not t.grad.any() for t in leaves)
+
+
+# ---------------------------------------------------------------------------------------------------- paged MLA
+def _paged(B=2, H=16, pages=4):
+    g = torch.Generator(device="cuda").manual_seed(7)
+    q = torch.randn(B, 1, H, 576, generator=g, device="cuda", dtype=torch.float16)
+    pool = torch.randn(B * pages, 64, 1, 576, generator=g, device="cuda", dtype=torch.float16)
+    return _mla(B, H, pages * 64), q, pool, torch.arange(B * pages, dtype=torch.int32, device="cuda").view(B, pages), \
+        torch.tensor([100, pages * 64], dtype=torch.int32, device="cuda")
+
+
+def test_paged_mla_waits_for_its_lengths_when_a_launch_fails():
+    """The copy of the lengths into the thread's landing place is queued in front of the launches: a call that fails there
+    returns behind the copy, so that the next one, on any stream, has the place to itself."""
+    eng, q, pool, table, lens = _paged()
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)  # ten milliseconds or so in front of the copy
+        before = side.record_event()
+        with pytest.raises(rt.AeError):
+            eng.decode_paged(q, pool[:0], table, lens)
+        assert before.query()
+    with pytest.raises(ValueError, match="cache_seqlens"):
+        eng.decode_paged(q, pool, table[:, :0], lens)
+    with pytest.raises(rt.AeError, match="empty"):
+        eng.decode_paged(q[:0], pool, table[:0], lens[:0])
+    o, _ = eng.decode_paged(q, pool, table, lens)
+    torch.cuda.synchronize()
+    assert torch.isfinite(o).all()
+
+
+def test_paged_mla_is_refused_under_capture():
+    eng, q, pool, table, lens = _paged()
+    want = eng.decode_paged(q, pool, table, lens)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        with pytest.raises(RuntimeError, match="captured"):
+            eng.decode_paged(q, pool, table, lens)
+        q.add_(0)
+    got = eng.decode_paged(q, pool, table, lens)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
