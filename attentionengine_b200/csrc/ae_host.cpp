@@ -514,13 +514,16 @@ struct Landing {
 py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, const Tensor& pool, const Tensor& table_in,
                      const Tensor& lens_in, int n_split) {
   const MlaPlan& P = *plan;
-  if (!good4(q, P.dtype) || q.size(1) != 1 || q.size(3) != 576 || q.size(2) > 128) return py::none();
+  if (!q.is_cuda() || q.scalar_type() != P.dtype || q.dim() != 4 || q.size(1) != 1 || q.size(3) != 576 || q.size(2) > 128)
+    return py::none();
   if (!pool.is_cuda() || pool.scalar_type() != P.dtype || !pool.is_contiguous()) return py::none();
   const bool d4 = pool.dim() == 4;
   if ((!d4 && pool.dim() != 3) || pool.size(1) != 64 || pool.size(-1) != 576 || (d4 && pool.size(2) != 1)) return py::none();
   const int64_t B = q.size(0), H = q.size(2);
   if (B == 0 || H == 0) return py::none();
-  if (table_in.dim() != 2 || table_in.size(0) != B || lens_in.dim() != 1 || lens_in.size(0) != B) return py::none();
+  if (table_in.dim() < 2 || table_in.size(0) != B || table_in.numel() != B * table_in.size(1) || lens_in.dim() != 1 ||
+      lens_in.size(0) != B)
+    return py::none();
   py::gil_scoped_release nogil;
   c10::cuda::CUDAGuard guard(q.device());
   at::AutoGradMode no_grad(false);
@@ -539,7 +542,8 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
   Landing landing(land, lens, st);
   landing.record();
 
-  const Tensor Q = q.contiguous();
+  Tensor Q = q.contiguous();
+  if (reinterpret_cast<uintptr_t>(Q.data_ptr()) % 16) Q = Q.clone();  // TMA reads from 16-byte boundaries
   Tensor o = at::empty({B, 1, H, 512}, q.options());
   const auto f32 = q.options().dtype(at::kFloat);
   Tensor lse = at::empty({B, H}, f32);

@@ -150,3 +150,15 @@ def test_paged_mla_is_refused_under_capture():
         q.add_(0)
     got = eng.decode_paged(q, pool, table, lens)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+def test_paged_mla_takes_any_layout_of_q():
+    """q with another stride order, or on a base that TMA cannot read, is copied; a block table may have trailing ones."""
+    eng, q, pool, table, lens = _paged()
+    want = eng.decode_paged(q, pool, table, lens)
+    odd = torch.empty(q.numel() + 1, dtype=q.dtype, device="cuda")[1:].view(q.shape).copy_(q)
+    turned = q.transpose(2, 3).contiguous().transpose(2, 3)
+    assert odd.data_ptr() % 16 and turned.stride(3) != 1
+    for got in (eng.decode_paged(odd, pool, table, lens), eng.decode_paged(turned, pool, table, lens),
+                eng.decode_paged(q, pool, table[..., None], lens)):
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
