@@ -164,7 +164,7 @@ class AttnDecode:
 
     def _run(self, q, k, v, custom, meta, block_table):
         if meta is None:
-            n_split = self.num_split or self.pick_splits(q.shape[0], k.shape[1])
+            n_split = self.num_split or (self.pick_splits(q.shape[0], k.shape[1]) if q.dim() == k.dim() == 4 else 1)
             m = None
         else:
             n_split = 1
@@ -210,4 +210,8 @@ class AttnDecode:
                 raise NotImplementedError("tile-shaped custom inputs are not wired into the decode kernel")
             if not t.is_cuda:
                 raise rt.AeError("custom inputs must be CUDA tensors: this back end has no CPU path")
+            if any(slot >= 0 for slot in sp.dim_slots[t.dim():]):
+                raise ValueError(f"custom input {sp.name}: expected {len(sp.shape)} dims, got {tuple(t.shape)}")
+        if block_table is not None and not block_table.is_cuda:
+            raise rt.AeError("block_table must be a CUDA tensor: this back end has no CPU path")
         raise ValueError("tensors do not fit this engine")

@@ -137,14 +137,17 @@ std::vector<Tensor> tensors_of(const py::handle& seq) {
   return out;
 }
 
-// Pointers and strides of the custom inputs, by the slots the generated functors read; false when one does not fit.
+// Pointers and strides of the custom inputs, by the slots the generated functors read; false when one does not fit.  A decode
+// call takes no tile-shaped input, and of the others whatever has the dims it indexes; the rest need the dims of their spec.
 bool custom_args(const std::vector<Custom>& specs, std::vector<Tensor>& ts, at::ScalarType dtype, int64_t Sq, int64_t Skv,
-                 bool allow16, const void* (&ptr)[AE_MAX_CUSTOM_INPUTS], int64_t (&st)[AE_MAX_CUSTOM_INPUTS][4]) {
+                 bool decode, const void* (&ptr)[AE_MAX_CUSTOM_INPUTS], int64_t (&st)[AE_MAX_CUSTOM_INPUTS][4]) {
   if (specs.size() != ts.size()) return false;
   for (size_t i = 0; i < specs.size(); ++i) {
     const Custom& sp = specs[i];
-    if (!ts[i].is_cuda() || (size_t)ts[i].dim() != sp.dim_slots.size()) return false;
-    if (sp.is16 && (!allow16 || Sq % 128 || Skv % 128)) return false;
+    if (!ts[i].is_cuda() || (!decode && (size_t)ts[i].dim() != sp.dim_slots.size())) return false;
+    if (sp.is16 && (decode || Sq % 128 || Skv % 128)) return false;
+    for (size_t d = ts[i].dim(); d < sp.dim_slots.size(); ++d)
+      if (sp.dim_slots[d] >= 0) return false;
     const at::ScalarType want = sp.is16 ? dtype : at::kFloat;
     if (ts[i].scalar_type() != want) ts[i] = ts[i].to(want);
     ptr[sp.slot] = ts[i].data_ptr();
@@ -230,7 +233,7 @@ struct AttnNode : Node {
     strides3(Q, p.q_stride); strides3(K, p.k_stride); strides3(V, p.v_stride); strides3(O, p.o_stride);
     strides3(dO, p.do_stride); strides3(dq, p.dq_stride); strides3(dk, p.dk_stride); strides3(dv, p.dv_stride);
     for (size_t i = 0; i < F.size(); ++i) p.final_rowscales[i] = (const float*)F[i].data_ptr();
-    custom_args(plan->custom, C, plan->dtype, d.Sq, d.Skv, true, p.custom, p.custom_stride);
+    custom_args(plan->custom, C, plan->dtype, d.Sq, d.Skv, false, p.custom, p.custom_stride);
     if (!lists.empty()) {
       p.block_count = (const int32_t*)lists[0].data_ptr(); p.block_index = (const int32_t*)lists[1].data_ptr();
       p.block_count_t = (const int32_t*)lists[2].data_ptr(); p.block_index_t = (const int32_t*)lists[3].data_ptr();
@@ -281,7 +284,7 @@ py::object attn(const std::shared_ptr<AttnPlan>& plan, py::handle eng, const Ten
     AeAttnParams p;
     memset(&p, 0, sizeof p);
     std::vector<Tensor> c = C;
-    if (!custom_args(plan->custom, c, plan->dtype, d.Sq, d.Skv, true, p.custom, p.custom_stride)) {
+    if (!custom_args(plan->custom, c, plan->dtype, d.Sq, d.Skv, false, p.custom, p.custom_stride)) {
       o = Tensor();
     } else {
       o = at::empty({d.B, d.Sq, d.Hq, plan->DV}, q.options());
@@ -376,7 +379,7 @@ py::object decode(const std::shared_ptr<DecodePlan>& plan, const Tensor& q, cons
   c10::cuda::CUDAGuard guard(q.device());
   at::AutoGradMode no_grad(false);
   Tensor o;
-  if (custom_args(P.custom, C, P.dtype, P.Sq, p.Skv, false, p.custom, p.custom_stride)) {
+  if (custom_args(P.custom, C, P.dtype, P.Sq, p.Skv, true, p.custom, p.custom_stride)) {
     o = at::empty({B, P.Sq, P.Hq, P.DV}, q.options());
     p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr(); p.o = o.data_ptr();
     strides3(q, p.q_stride); strides3(k, p.k_stride); strides3(v, p.v_stride);

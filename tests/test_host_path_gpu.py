@@ -6,7 +6,7 @@ import torch
 import torch.autograd.forward_ad as fwAD
 
 import helpers
-from attentionengine_b200 import AttentionEngine, CustomIO, runtime as rt
+from attentionengine_b200 import AttentionEngine, CustomIO, meta_tensor, runtime as rt
 
 pytestmark = pytest.mark.gpu
 
@@ -162,3 +162,20 @@ def test_paged_mla_takes_any_layout_of_q():
     for got in (eng.decode_paged(odd, pool, table, lens), eng.decode_paged(turned, pool, table, lens),
                 eng.decode_paged(q, pool, table[..., None], lens)):
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+def test_decode_takes_custom_inputs_by_the_dims_it_indexes():
+    """A decode call reads a custom input by its named dims: it may lack dims that are not indexed and have more at the end."""
+    B, H, S, D, dtype = 2, 4, 300, 64, torch.float16
+    eng = AttentionEngine(tuple(meta_tensor(B, H, n, D, dtype=dtype) for n in (1, S, S)), CustomIO({"scale": (1,), "slope": (1, "heads")}),
+                          score_mod=lambda s, c, b, h, q, kv: s * c.input_tensors["scale"] + c.input_tensors["slope"] * s, mask_mod=None,
+                          online_func=helpers.OnlineSoftmaxSplit())
+    g = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = (torch.randn(B, n, H, D, generator=g, device="cuda", dtype=dtype) for n in (1, S, S))
+    scale, slope = torch.tensor([0.1], device="cuda"), torch.rand(1, H, generator=g, device="cuda")
+    want = eng(q, k, v, scale, slope)
+    assert torch.equal(eng(q, k, v, scale[0], slope[..., None]), want)
+    with pytest.raises(ValueError, match="slope"):
+        eng(q, k, v, scale, slope[0])
+    with pytest.raises(ValueError, match="contiguous last dimension"):
+        eng(q, k[0, 0], v, scale, slope)
