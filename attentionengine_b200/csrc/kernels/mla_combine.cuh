@@ -48,7 +48,8 @@ extern "C" __global__ void __launch_bounds__(128) ae_mla_combine(const AeMlaComb
   for (int i = 0; i < AE_NFINAL; ++i) fr[i] = lane < n_split ? args.fr_part[i][my_slot * args.H + h] : -__int_as_float(0x7f800000);
 #if AE_NFINAL > 0
   if (args.lse_out) {
-    const float m = ae_warp_max(fr[0]);
+    float m = ae_warp_max(fr[0]);
+    if (fabsf(m) == __int_as_float(0x7f800000)) m = 0.f;  // all -inf stays -inf, an inf stays inf
     const float sum = ae_warp_sum(lane < n_split ? expf(fr[0] - m) : 0.f);
     if (threadIdx.x % AE_CMB_TPH == 0) args.lse_out[(i64)b * args.H + h] = m + logf(sum);
   }

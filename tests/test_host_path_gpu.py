@@ -7,6 +7,8 @@ import torch.autograd.forward_ad as fwAD
 
 import helpers
 from attentionengine_b200 import AttentionEngine, CustomIO, meta_tensor, runtime as rt
+from attentionengine_b200.attn_engine import OnlineFunc
+from attentionengine_b200.core import SymbolScalar, Var
 
 pytestmark = pytest.mark.gpu
 
@@ -179,3 +181,31 @@ def test_decode_takes_custom_inputs_by_the_dims_it_indexes():
         eng(q, k, v, scale, slope[0])
     with pytest.raises(ValueError, match="contiguous last dimension"):
         eng(q, k[0, 0], v, scale, slope)
+
+
+class _PlainExp(helpers.OnlineSoftmaxSplit):
+    """Softmax without the running maximum: its sums under- and overflow."""
+
+    def __init__(self):
+        OnlineFunc.__init__(self, {"r": SymbolScalar("r", Var("0.0"))}, {"lse": SymbolScalar("lse", Var("0.0"))}, CustomIO())
+
+    @staticmethod
+    def online_fwd(scores, online_rowscales, b, h, q_idx):
+        scores = scores.exp()
+        return scores, {"r": online_rowscales["r"] + scores.get_reduce("sum")}, SymbolScalar("o_scale", Var("1"))
+
+    @staticmethod
+    def online_fwd_epilogue(o, online_rowscales, b, h, q_idx):
+        return o, {"lse": online_rowscales["r"].log()}
+
+
+@pytest.mark.parametrize("shift", [-1000.0, 1000.0])
+def test_paged_mla_infinite_log_sum_exp(shift):
+    """Rows whose sums are all 0 or infinite have the log-sum-exp -inf or inf, merged (second row) or not (first row)."""
+    B, H, S, dtype = 2, 16, 2048, torch.float16
+    metas = (meta_tensor(B, H, 1, 576, dtype=dtype), meta_tensor(B, 1, S, 576, dtype=dtype), meta_tensor(B, 1, S, 512, dtype=dtype))
+    eng = AttentionEngine(metas, CustomIO({}), score_mod=lambda s, c, b, h, q, kv: s * 0.01 + shift, mask_mod=None, online_func=_PlainExp(),
+                          kv_shared=True)
+    _, q, pool, table, _ = _paged(B, H, S // 64)
+    _, lse = eng.decode_paged(q, pool, table, torch.tensor([100, S], dtype=torch.int32, device="cuda"))
+    assert (lse == math.copysign(math.inf, shift)).all()
