@@ -88,8 +88,9 @@ class AttnDecode:
         if self.combine is None:
             return 1
         n_tiles = -(-Skv // 128)
-        if (B, n_tiles) in self._splits:
-            return self._splits[B, n_tiles]
+        known = self._splits.get((B, n_tiles))  # one look: another thread may clear the table
+        if known is not None:
+            return known
         units = B * (self.Hkv if self.Hq > self.Hkv else self.Hq)
         best, best_cost = 1, None
         for n in range(1, min(32, n_tiles) + 1):

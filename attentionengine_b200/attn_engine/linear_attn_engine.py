@@ -181,11 +181,12 @@ class LinearAttentionEngine:
         if not (plan.bwd_mods if mods else plan.bwd):
             states, bwd = self._bwd_kernels(mods)
             plan.states = states.handle.value
+            plan.head_sum = self._head_sum_kernel(128).handle.value
+            # last: another thread that finds it set launches all of them
             if mods:
                 plan.bwd_mods = bwd.handle.value
             else:
                 plan.bwd = bwd.handle.value
-            plan.head_sum = self._head_sum_kernel(128).handle.value
         return 1
 
     def _bwd_from_saved(self, q, k, v, a, g, hs, x, s, d, asc):
