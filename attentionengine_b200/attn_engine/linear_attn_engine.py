@@ -179,8 +179,7 @@ class LinearAttentionEngine:
             return 0
         plan = self._plan
         if not (plan.bwd_mods if mods else plan.bwd):
-            states, bwd = self._bwd_kernels(mods)
-            plan.states = states.handle.value
+            bwd = self._bwd_kernels(mods)[1]
             plan.head_sum = self._head_sum_kernel(128).handle.value
             # last: another thread that finds it set launches all of them
             if mods:
@@ -490,33 +489,8 @@ class LinearAttentionEngine:
     def _launch(self, q, k, v, a, vscale=None, dskip=None, v_out=None, h_out=None, ascale=None):
         """The scan kernel.  With ``vscale`` [B, H, T] / ``dskip`` [H] fp32 the build with the mods inside runs: scan of
         v * vscale plus v * dskip[h]; ``v_out`` receives the scaled v."""
-        B, HQ, T, DK = q.shape
-        H, DV = v.shape[1], v.shape[3]
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        a = a.float().contiguous()
-        o = torch.empty(B, H, T, DV, dtype=self.dtype, device=q.device)
-        p = rt.LinearParams()
-        p.q, p.k, p.v, p.a, p.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), o.data_ptr()
-        mods = vscale is not None or dskip is not None
-        if mods:
-            if vscale is not None:
-                p.vscale, p.vscale_16bit = vscale.data_ptr(), int(vscale.dtype != torch.float32)
-            if dskip is not None:
-                p.dskip = dskip.data_ptr()
-            if v_out is not None:
-                p.v_out = v_out.data_ptr()
-        if h_out is not None:
-            p.h_states_out = h_out.data_ptr()
-        if ascale is not None:  # [H] fp32: the scan runs on a * ascale[h]
-            p.ascale = ascale.data_ptr()
-        p.B, p.H, p.HQ, p.HK, p.T = B, H, HQ, k.shape[1], T
-        if self._status is None or self._status.device != q.device:
-            self._status = torch.zeros(1, dtype=torch.int32, device=q.device)
-        p.status = self._status.data_ptr()
-        stream = C.c_void_p(torch.cuda.current_stream(q.device).cuda_stream)
-        rt.check(rt.lib().ae_launch_linear_fwd(self._fwd_kernel(DV, mods)[0].handle, C.byref(p), stream),
-                 "ae_launch_linear_fwd")
-        return o
+        kernel = self._fwd_kernel(v.shape[3], vscale is not None or dskip is not None)[0].handle.value
+        return rt.host().scan_forward(self._native_plan(), kernel, q, k, v, a, vscale, dskip, ascale, v_out, h_out)
 
     def _native_scan(self, q, k, v, a):
         """The scan on the mod-ed tensors as one autograd node; gradients flow on into the eager mods through torch autograd

@@ -589,9 +589,8 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
 
 // ---------------------------------------------------------------------------------------------------- scan
 struct ScanPlan : Plan {
-  void *fwd = nullptr;       // blocks of 128 key dims and this plan's value dims
-  void *fwd_mods = nullptr;  // the build with the Mamba2 block's mods inside (64 value dims)
-  void *states = nullptr, *bwd = nullptr, *bwd_mods = nullptr, *head_sum = nullptr;  // set when first needed
+  void *fwd_mods = nullptr;  // the forward built with the Mamba2 block's mods inside (64 value dims)
+  void *bwd = nullptr, *bwd_mods = nullptr, *head_sum = nullptr;  // set when first needed
 };
 
 // the tensors of one scan; s / d / asc undefined without the block's mods
@@ -609,7 +608,7 @@ struct ScanNode : Node {
   std::shared_ptr<ScanPlan> plan;
   std::shared_ptr<PyObject> eng;
   ScanSaved saved;
-  bool mods = false, has_asc = false, has_hs = false;
+  bool mods = false, has_asc = false;
   Tensor status;
   std::vector<int64_t> d_shape, asc_shape;
   at::ScalarType d_dtype = at::kFloat, asc_dtype = at::kFloat;
@@ -623,7 +622,7 @@ struct ScanNode : Node {
       q = saved.q.unpack(), k = saved.k.unpack(), v = saved.v.unpack(), a = saved.a.unpack();
       if (mods) x = saved.x.unpack(), s = saved.s.unpack(), d = saved.d.unpack();
       if (has_asc) asc = saved.asc.unpack();
-      if (has_hs) hs = saved.hs.unpack();
+      hs = saved.hs.unpack();
     }
     at::AutoGradMode no_grad(false);
     c10::cuda::CUDAGuard guard(q.device());
@@ -636,7 +635,7 @@ struct ScanNode : Node {
       return with_python([&] {
         py::handle e(eng.get());
         auto opt = [](const Tensor& t) -> py::object { return t.defined() ? py::cast(t) : py::none(); };
-        py::tuple r = e.attr("_bwd_from_saved")(q, k, v, a, g, opt(hs), opt(x), opt(s), opt(d), opt(asc));
+        py::tuple r = e.attr("_bwd_from_saved")(q, k, v, a, g, hs, opt(x), opt(s), opt(d), opt(asc));
         for (size_t i = 0; i < out.size(); ++i)
           if (!r[i].is_none()) out[i] = r[i].cast<Tensor>();
         if (mods) {
@@ -650,8 +649,6 @@ struct ScanNode : Node {
     AeLinearBwdParams p;
     memset(&p, 0, sizeof p);
     void* st = stream_of(q);
-    const bool recompute = !hs.defined();
-    if (recompute) hs = at::empty({B, H, (T + 127) / 128, 128, 64}, o16);
     Tensor dq_h = at::empty({B, H, T, 128}, o16), dk_h = at::empty({B, H, T, 128}, o16), dv = at::empty({B, H, T, 64}, o16);
     Tensor da = at::empty({B, H, T}, f32), gs, gd, gasc;
     p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr(); p.a = (const float*)a.data_ptr(); p.d_o = g.data_ptr();
@@ -671,7 +668,6 @@ struct ScanNode : Node {
       p.ascale = (const float*)asc.data_ptr();
       p.gasc = (float*)gasc.data_ptr();
     }
-    if (recompute) check(ae_launch_linear_states(plan->states, &p, st), "ae_launch_linear_states");
     check(ae_launch_linear_bwd(mods ? plan->bwd_mods : plan->bwd, &p, st), "ae_launch_linear_bwd");
     auto head_sum = [&](const Tensor& in, int heads) {
       if (heads == H) return in;
@@ -701,6 +697,27 @@ struct ScanNode : Node {
   std::string name() const override { return mods ? "ScaleScanSkipBackward" : "LinearScanBackward"; }
 };
 
+// One launch of the scan kernel on contiguous tensors; those after `a` may be undefined: the row scale, skip weight and decay
+// scale of the Mamba2 block (a kernel built with the mods inside), and what receives the scaled v and the chunk start-states.
+Tensor scan_launch(ScanPlan& plan, void* kernel, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& s,
+                   const Tensor& d, const Tensor& asc, const Tensor& v_out, const Tensor& hs) {
+  AeLinearParams p;
+  memset(&p, 0, sizeof p);
+  Tensor y = at::empty({q.size(0), v.size(1), q.size(2), v.size(3)}, q.options());
+  auto ptr = [](const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; };
+  p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr(); p.a = (const float*)a.data_ptr(); p.o = y.data_ptr();
+  p.vscale = ptr(s);
+  p.vscale_16bit = s.defined() && s.scalar_type() != at::kFloat;
+  p.dskip = (const float*)ptr(d);
+  p.ascale = (const float*)ptr(asc);
+  p.v_out = ptr(v_out);
+  p.h_states_out = ptr(hs);
+  p.B = (int)q.size(0); p.H = (int)v.size(1); p.HQ = (int)q.size(1); p.HK = (int)k.size(1); p.T = (int)q.size(2);
+  p.status = word(plan.status_for(q));
+  check(ae_launch_linear_fwd(kernel, &p, stream_of(q)), "ae_launch_linear_fwd");
+  return y;
+}
+
 // y = scan(q, k, v, a), or with s, d (and asc): y = scan(q, k, v * s[..., None], a * asc[head]) + v * d[head] as one node.
 // q / k have 128 dims; v has 64 dims with mods, 64 or 128 (no gradient) without.
 Tensor scan_run(const std::shared_ptr<ScanPlan>& plan, void* kernel, py::handle eng, const Tensor& q_, const Tensor& k_,
@@ -715,32 +732,18 @@ Tensor scan_run(const std::shared_ptr<ScanPlan>& plan, void* kernel, py::handle 
     q = q_.contiguous(); k = k_.contiguous(); v = v_.contiguous();
     a = a_.to(at::kFloat).contiguous();
     const int64_t B = q.size(0), T = q.size(2), H = v.size(1), DV = v.size(3);
-    AeLinearParams p;
-    memset(&p, 0, sizeof p);
-    y = at::empty({B, H, T, DV}, q.options());
-    p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr(); p.a = (const float*)a.data_ptr(); p.o = y.data_ptr();
     if (mods) {
       s = s_.contiguous();
       d = d_.to(at::kFloat).reshape({-1}).contiguous();
-      p.vscale = s.data_ptr(); p.vscale_16bit = s.scalar_type() != at::kFloat;
-      p.dskip = (const float*)d.data_ptr();
-      if (asc_.defined()) {
-        asc = asc_.to(at::kFloat).reshape({-1}).contiguous();
-        p.ascale = (const float*)asc.data_ptr();
-      }
-      if (need) {
-        v_out = at::empty_like(v);
-        p.v_out = v_out.data_ptr();
-      }
+      if (asc_.defined()) asc = asc_.to(at::kFloat).reshape({-1}).contiguous();
+      if (need) v_out = at::empty_like(v);
     }
-    if (need && DV == 64) {  // the reverse pass reads the chunk start-states the forward has at hand
+    if (need) {  // the reverse pass reads the chunk start-states the forward has at hand
+      TORCH_CHECK(DV == 64, "the scan has gradients in value blocks of 64 dims");
       hs = at::empty({B, H, (T + 127) / 128, 128, DV}, q.options());
-      p.h_states_out = hs.data_ptr();
     }
-    p.B = (int)B; p.H = (int)H; p.HQ = (int)q.size(1); p.HK = (int)k.size(1); p.T = (int)T;
+    y = scan_launch(*plan, kernel, q, k, v, a, s, d, asc, v_out, hs);
     status = plan->status_for(q);
-      p.status = word(status);
-    check(ae_launch_linear_fwd(kernel, &p, stream_of(q)), "ae_launch_linear_fwd");
   }
   if (need) {
     auto node = std::shared_ptr<ScanNode>(new ScanNode(), torch::autograd::deleteNode);
@@ -770,10 +773,22 @@ Tensor scan_run(const std::shared_ptr<ScanPlan>& plan, void* kernel, py::handle 
         node->asc_dtype = asc_.scalar_type();
       }
     }
-    if ((node->has_hs = hs.defined())) sv.hs = SavedVariable(hs, false);
+    sv.hs = SavedVariable(hs, false);
     torch::autograd::set_history(y, node);
   }
   return y;
+}
+
+// The launch alone, for the front end's autograd function and for direct use.
+Tensor scan_forward(const std::shared_ptr<ScanPlan>& plan, uint64_t kernel, const Tensor& q, const Tensor& k, const Tensor& v,
+                    const Tensor& a, const std::optional<Tensor>& s, const std::optional<Tensor>& d, const std::optional<Tensor>& asc,
+                    const std::optional<Tensor>& v_out, const std::optional<Tensor>& hs) {
+  py::gil_scoped_release nogil;
+  c10::cuda::CUDAGuard guard(q.device());
+  at::AutoGradMode no_grad(false);
+  auto opt = [](const std::optional<Tensor>& t) { return t ? *t : Tensor(); };
+  return scan_launch(*plan, handle(kernel), q.contiguous(), k.contiguous(), v.contiguous(), a.to(at::kFloat).contiguous(), opt(s),
+                     opt(d), opt(asc), opt(v_out), opt(hs));
 }
 
 // None when the call needs an autograd function.
@@ -846,12 +861,13 @@ PYBIND11_MODULE(_ae_host, m) {
         auto p = std::make_shared<ScanPlan>();
         p->dtype = bf16 ? at::kBFloat16 : at::kHalf;
         return p;
-      })) AE_HANDLE(ScanPlan, fwd_mods) AE_HANDLE(ScanPlan, states) AE_HANDLE(ScanPlan, bwd) AE_HANDLE(ScanPlan, bwd_mods)
+      })) AE_HANDLE(ScanPlan, fwd_mods) AE_HANDLE(ScanPlan, bwd) AE_HANDLE(ScanPlan, bwd_mods)
           AE_HANDLE(ScanPlan, head_sum) AE_STATUS(ScanPlan);
   m.def("attn", torch::wrap_pybind_function(&attn));
   m.def("decode", torch::wrap_pybind_function(&decode));
   m.def("mla", torch::wrap_pybind_function(&mla));
   m.def("mla_paged", torch::wrap_pybind_function(&mla_paged));
+  m.def("scan_forward", torch::wrap_pybind_function(&scan_forward));
   m.def("scan", torch::wrap_pybind_function(&scan));
   m.def("scan_block", torch::wrap_pybind_function(&scan_block));
 }

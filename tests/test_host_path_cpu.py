@@ -21,7 +21,7 @@ def test_scan_backward_kernels_are_complete_when_they_are_found(mods):
     eng = helpers.mamba2_engine(1, 2, 128, 128, 64, torch.bfloat16, d_skip=True)
     eng._plan = Plan()
     assert eng._native_bwd(1, 2, False, mods, 0) == 1
-    assert sorted(eng._plan.order) == sorted(["states", "head_sum", "bwd_mods" if mods else "bwd"])
+    assert sorted(eng._plan.order) == sorted(["head_sum", "bwd_mods" if mods else "bwd"])
     assert eng._plan.order[-1] == ("bwd_mods" if mods else "bwd")
 
 
