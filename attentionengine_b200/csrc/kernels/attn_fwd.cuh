@@ -41,6 +41,9 @@
 #ifndef AE_P_PIECES
 #define AE_P_PIECES (AE_PINGPONG ? 1 : 2)
 #endif
+#if AE_P_PIECES != 1 && AE_P_PIECES != 2
+#error "P is handed over in one or two blocks: the MMA warp takes no more, and a block is stored 64 columns at a time"
+#endif
 #define AE_ROW_WARPS (4 * AE_NQ)
 // One thread per row holds a tile's 128 scores, the P it makes of them and the packed block on its way to TMEM: the row
 // warpgroups take registers from the TMA / MMA warpgroup (launched with 168 per thread; 208 + 208 + 88 = 3 x 168; with 72

@@ -740,6 +740,7 @@ def lower_attention(score_mod, mask_mod, online_func, custom_fwd_inputs: CustomI
                "// made; what only the row states need (the row sum of a softmax) follows the last block.\n"
                "template <int PIECES, int N, class Sink>\nAE_DEVICE void ae_online_tile(float (&s)[N], AeRow& st, int b, int h, int q_idx, "
                "int kv0, const AeCustom& cu, Sink&& sink) {\n"
+               "  static_assert(PIECES == 1 || PIECES == 2, \"P in one or two blocks\");\n"
                "  static_assert(N % (8 * PIECES) == 0, \"tile loops take eight columns at a time\");\n"
                + pre + f"  const float o_scale_ = {o_expr};\n  float p_[N];\n"
                + "".join(f"  float {n}[N];\n" for n, _ in tiles)
@@ -748,7 +749,6 @@ def lower_attention(score_mod, mask_mod, online_func, custom_fwd_inputs: CustomI
                "    #pragma unroll\n    for (int c = c0; c < c0 + N / PIECES; ++c) {\n" + element + "    }\n    sink(K, o_scale_, p_);\n  };\n"
                "  block(AeInt<0>{});\n"
                "  if constexpr (PIECES > 1) block(AeInt<1>{});\n"
-               "  if constexpr (PIECES > 2) { block(AeInt<2>{}); block(AeInt<3>{}); }\n"
                + post + "".join(f"  const float n_{k} = {e};\n" for k, e in new_exprs.items())
                + "".join(f"  st.st_{k} = n_{k};\n" for k in new_exprs) + "}\n"
                "// The same with P left in s[]; returns o_scale.\n"

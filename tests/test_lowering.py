@@ -185,3 +185,13 @@ def test_block_mask_of_the_wrong_shape_is_refused_on_the_host():
     assert win._ensure_lists("cpu", None, B, H, 1024, 1024)[0].shape == (B, H, 8)
     with pytest.raises(ValueError, match="inferred for"):
         win._ensure_lists("cpu", None, B, H, 2048, 2048)
+
+
+def test_forward_refuses_a_hand_over_of_p_that_it_does_not_implement():
+    """Four blocks of P would compile, store nothing and drop half of P V: the kernel says no when it is built."""
+    from attentionengine_b200 import runtime as rt
+    from attentionengine_b200 import examples
+    k = examples.softmax_engine(1, 2, 2, 256, 64, 64, torch.float16, True).kernels
+    cfg = rt.KernelConfig(kind=rt.KIND_ATTN_FWD, dtype=rt.DTYPE_F16, head_dim=64, head_dim_v=64, threads=384, smem_bytes=0, stages=2, mask_mode=1)
+    with pytest.raises(rt.AeError, match="one or two blocks"):
+        rt.compile_module(rt.kernel_source("attn_fwd.cuh", prelude=k.low.prelude_fwd, defines={"AE_P_PIECES": 4}), "ae_attn_fwd", cfg)
