@@ -179,7 +179,10 @@ AE_DEVICE void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: 
 AE_DEVICE void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Non-blocking arrival on a named barrier (the waiting side calls named_bar_sync with the same id and count).
 // A named barrier costs the waiting warp about 20 clk, an mbarrier wait 100 - 400 clk; it has no time-out, so it is
-// only used where the arriving side is guaranteed to arrive (row threads arrive in every iteration, aborted or not).
+// only used where the arriving side is guaranteed to arrive.  Two contracts give that guarantee.  The backward's row threads
+// arrive in every iteration, aborted or not.  The forward's arrive once more for the step in which their wait gave up, then
+// leave: there the waiting warp has to read ctl->abort before the first named_bar_sync of every step (attn_fwd.cuh, behind
+// its wait for K and V), and finds it set, because the abort word was written before that last arrival.
 AE_DEVICE void named_bar_arrive(u32 id, u32 nthreads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }

@@ -63,12 +63,13 @@ AE_DEVICE void mla_load(void* dst, const AeTmaDesc* d, u32 bar, int c0, int c1, 
       : "memory");
 }
 // Arrival at a barrier of the pair's rank 0.  Release at CTA scope, the default: what it announces (P, written and fenced
-// towards the async proxy) is read by this CTA's own tensor core, the barrier's CTA only issues the MMA.  With
-// .release.cluster an arrival took about 1,200 clk under load: 345 us with one of them per tile on the chain of the rows.
+// towards the async proxy) is read by this CTA's own tensor core, the barrier's CTA only issues the MMA.  That is a reliance
+// on the hardware: the PTX memory model orders rank 1's writes before rank 0's MMA only with a release at cluster scope.  With
+// .release.cluster in rank 1 alone an arrival takes about 1,200 clk under load, on the chain of the rows: 128 rows of 8192
+// keys 291 -> 340 us, 32 rows 99 -> 127, 8 rows of 4096 35.5 -> 39.1.
 AE_DEVICE void mla_arrive(u32 bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-
 
 struct AeMlaSeg {
   int b, t0, t1;   // tiles [t0, t1) of batch row b
