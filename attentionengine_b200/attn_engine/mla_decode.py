@@ -45,7 +45,7 @@ class MlaDecode:
         from .attn_engine import OnlineFunc
         overridden = getattr(type(online_func), "combine", None) is not OnlineFunc.combine
         self._auto_split = 0 if overridden or not self.low.final_names else 1  # row state without a combine: rows stay whole
-        self.last_num_split = None
+        self.last_num_split = None  # of the last call: the most shares that a row was cut into
         self._plan = None  # the native side, made at the first call
 
     def _native_plan(self):

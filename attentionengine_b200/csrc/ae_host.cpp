@@ -421,6 +421,23 @@ struct MlaScratch {
   }
 };
 
+// The most intervals that a row touches, cut as the kernel cuts them (ae_mla_decode): `keys(b)` of every row.
+template <class Keys>
+int most_shares(int64_t B, int64_t clusters, Keys&& keys) {
+  auto tiles = [&](int64_t b) { return std::max<int64_t>(1, (keys(b) + 127) / 128); };
+  int64_t total = 0, longest = 0, before = 0, most = 1;
+  for (int64_t b = 0; b < B; ++b) {
+    total += tiles(b);
+    longest = std::max(longest, tiles(b));
+  }
+  const int64_t share = std::max((total + clusters - 1) / clusters, (longest + 30) / 31);
+  for (int64_t b = 0; b < B; ++b) {
+    most = std::max(most, (before % share + tiles(b) - 1) / share + 1);
+    before += tiles(b);
+  }
+  return (int)most;
+}
+
 bool same(const Tensor& t, std::initializer_list<int64_t> shape) { return t.sizes() == at::IntArrayRef(shape.begin(), shape.size()); }
 
 py::object mla(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, const Tensor& q_pe, const Tensor& kv, const Tensor& k_pe,
@@ -460,8 +477,9 @@ py::object mla(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, const Tens
   void* st = stream_of(q);
   check(ae_launch_mla_decode(P.kernel, &p, st), "ae_launch_mla_decode");
   if (merge) check(ae_launch_mla_combine(P.combine, &p, st), "ae_launch_mla_combine");
+  const int shares = n_split ? n_split : most_shares(B, p.n_clusters, [&](int64_t) { return S; });
   py::gil_scoped_acquire gil;
-  return py::make_tuple(o, n_split ? (double)n_split : std::max(merge ? 1.0 + 1.0 / B : 1.0, (double)p.n_clusters / B));
+  return py::make_tuple(o, shares);
 }
 
 // Pinned landing place of the row lengths and the event behind their copy, one per thread.
@@ -510,7 +528,7 @@ struct Landing {
   }
 };
 
-// (o, lse, shares per row) over a paged cache; n_split 0: equal intervals of all rows' tiles.  The row lengths are checked on
+// (o, lse, most shares of a row) over a paged cache; n_split 0: equal intervals of all rows' tiles.  The row lengths are checked on
 // the host behind the launches: their copy is queued in front of the kernels, which clamp every length to the block table
 // themselves, so the stream never drains for the check.  Returns None when the tensors do not fit, or an empty tuple for
 // lengths outside their range.
@@ -582,9 +600,10 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
   C10_CUDA_CHECK(landing.wait());
   bool in_range = true;
   for (int64_t b = 0; b < B; ++b) in_range = in_range && land.host[b] >= 1 && land.host[b] <= max_pages * 64;
+  const int shares = n_split || !in_range ? n_split : most_shares(B, p.n_clusters, [&](int64_t b) { return (int64_t)land.host[b]; });
   py::gil_scoped_acquire gil;
   if (!in_range) return py::tuple();
-  return py::make_tuple(o, lse, n_split ? (double)n_split : (double)p.n_clusters / B);
+  return py::make_tuple(o, lse, shares);
 }
 
 // ---------------------------------------------------------------------------------------------------- scan

@@ -1054,7 +1054,8 @@ def test_mla_paged_lengths_outside_the_table_raise(lens):
     (3, 64, 4, [193] * 3, False),         # two tiles a row, the last one key into its second half
     (5, 128, 19, [1153] * 5, False),      # intervals that end inside rows, begin inside rows and hold whole rows
     (79, 16, 5, [300] * 79, False),       # more rows than intervals
-    (1, 16, 300, [19137], False),         # one row in the most intervals a merge takes (32)
+    (1, 16, 300, [19137], False),         # one row in many intervals (30)
+    (2, 16, 310, [128, 19840], True),     # a row that begins inside an interval and touches the most a merge takes (32)
     (6, 100, 7, [1, 64, 65, 128, 129, 448], True),  # pages of half a tile, an odd number of them, heads past the last one
     (90, 16, 6, [1 + (37 * i) % 384 for i in range(90)], True),
 ])

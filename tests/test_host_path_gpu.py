@@ -209,3 +209,20 @@ def test_paged_mla_infinite_log_sum_exp(shift):
     _, q, pool, table, _ = _paged(B, H, S // 64)
     _, lse = eng.decode_paged(q, pool, table, torch.tensor([100, S], dtype=torch.int32, device="cuda"))
     assert (lse == math.copysign(math.inf, shift)).all()
+
+
+@pytest.mark.parametrize("H,pages,lens,most", [
+    (16, 310, [128, 19840], 32),       # 156 tiles: intervals of 5, so that no row touches more than 32; the second begins inside one
+    (16, 4, [100, 256], 2),            # 3 tiles in two intervals of 2
+    (16, 2, [128, 128, 128], 1),       # whole rows
+    (16, 64, [1, 4096, 300], 17),      # 1 + 32 + 3 tiles in intervals of 2
+])
+def test_last_num_split_counts_the_shares_of_a_row(H, pages, lens, most):
+    B = len(lens)
+    eng, q, pool, table, _ = _paged(B, H, pages)
+    eng.decode_paged(q, pool, table, torch.tensor(lens, dtype=torch.int32, device="cuda"))
+    assert eng._mla.last_num_split == most
+    if len(set(lens)) == 1:
+        kv = pool.view(B, pages * 64, 1, 576)[:, :lens[0]]
+        eng(q[..., :512], q[..., 512:], kv[..., :512], kv[..., 512:])
+        assert eng._mla.last_num_split == most
