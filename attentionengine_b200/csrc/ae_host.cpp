@@ -847,6 +847,7 @@ py::object scan_block(const std::shared_ptr<ScanPlan>& plan, py::handle eng, con
                 [](cls& p, std::optional<Tensor> t) { p.status = t ? *t : Tensor(); })
 
 PYBIND11_MODULE(_ae_host, m) {
+  m.attr("built_for") = AE_HOST_BUILT_FOR;  // the build step looks for this text in the file
   py::class_<AttnPlan, std::shared_ptr<AttnPlan>>(m, "AttnPlan")
       .def(py::init([](uint64_t fwd, bool bf16, int D, int DV, int n_final, bool uses_doosum, py::list custom) {
         auto p = std::make_shared<AttnPlan>();

@@ -36,3 +36,13 @@ def test_split_counts_survive_a_cleared_table():
     want = dec.pick_splits(2, 1000)
     dec._splits = Cleared(dec._splits)
     assert dec.pick_splits(2, 1000) == want
+
+
+def test_extension_for_another_torch_is_rebuilt(tmp_path):
+    import __graft_entry__ as entry
+    out, dep = tmp_path / "x.so", tmp_path / "x.cpp"
+    dep.write_text("")
+    assert entry.host_is_stale(str(out), [str(dep)], "built for A")
+    out.write_bytes(b"\0..built for A\0")
+    assert not entry.host_is_stale(str(out), [str(dep)], "built for A")
+    assert entry.host_is_stale(str(out), [str(dep)], "built for B")
