@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import os
 import ctypes as C
+import warnings
 from typing import Optional
 
 import torch
@@ -108,6 +109,9 @@ class _AttnKernels:
         self.low = low
         self.D, self.DV, self.dtype_tag, self.mask_mode, self.stages = D, DV, dtype_tag, mask_mode, stages
         self.tuned = tuned or {}  # tile choices of the backward kernels (attentionengine_b200/tune.py)
+        if tuple(self.tuned.get("fwd_form", (1, 0))) != (1, 0):
+            warnings.warn(f"tuned entry: fwd_form {self.tuned['fwd_form']} is ignored, the forward has one thread per score row "
+                          "and no turn-taking")
         smem = 2 * 128 * D * 2 + stages * 128 * (D + DV) * 2 + 512 + 1024
         if mask_mode == 2:
             smem += 4 * MAX_LIST_KV_TILES  # the CTA's merged tile walk

@@ -2,6 +2,7 @@
 needs one and is exercised on a B200 by ``python -m attentionengine_b200.tune``)."""
 import json
 
+import pytest
 import torch
 
 from attentionengine_b200 import tune
@@ -64,3 +65,8 @@ def test_batch_ranges_of_the_backward_launches():
     # the scan's reverse pass: one CTA per (batch row, head), 80 heads
     assert ab.batch_ranges(8, 80, 148, 2) == 2 and ab.batch_ranges(8, 80, 148, 4) == 4
     assert ab.batch_ranges(2, 80, 148, 4) == 1                         # a single row would leave SMs empty
+
+
+def test_tuned_entry_of_a_forward_form_that_is_gone_warns():
+    with pytest.warns(UserWarning, match="fwd_form"):
+        helpers.softmax_engine(1, 2, 2, 256, 64, 64, torch.float16, True, tuned_config={"fwd_form": [2, 1]})
