@@ -1,9 +1,11 @@
 """The native host path (csrc/ae_host.cpp): what it refuses, and what its autograd nodes owe to the rest of PyTorch."""
 import math
+from concurrent.futures import ThreadPoolExecutor
 
 import pytest
 import torch
 import torch.autograd.forward_ad as fwAD
+import torch.utils.checkpoint
 
 import helpers
 from attentionengine_b200 import AttentionEngine, CustomIO, meta_tensor, runtime as rt
@@ -226,3 +228,89 @@ def test_last_num_split_counts_the_shares_of_a_row(H, pages, lens, most):
         kv = pool.view(B, pages * 64, 1, 576)[:, :lens[0]]
         eng(q[..., :512], q[..., 512:], kv[..., :512], kv[..., 512:])
         assert eng._mla.last_num_split == most
+
+
+# ---------------------------------------------------------------------------------------------------- what nodes owe autograd
+@pytest.fixture(params=["attention", "block", "scan"])
+def call(request):
+    """(f, leaves, output gradient) of an attention call, of the Mamba2 block and of the plain scan."""
+    if request.param == "attention":
+        eng, q, k, v, d_o = _attention()
+        return eng, [t.requires_grad_() for t in (q, k, v)], d_o
+    eng, args, d_o = _block()
+    if request.param == "scan":
+        eng = helpers.mamba2_engine(2, 4, 200, 128, 64, torch.bfloat16)
+        args = args[:-1]
+    return eng, [t.requires_grad_() for t in args], d_o
+
+
+def _same(got, want):
+    """The outputs bit for bit; gradients up to the order of dQ's fp32 additions and a rounding to 16 bits."""
+    assert torch.equal(got[0], want[0])
+    for x, y in zip(got[1:], want[1:]):
+        assert (x.float() - y.float()).norm() <= 2 ** -8 * y.float().norm()
+
+
+def _once(f, leaves, d_o):
+    o = f(*leaves)
+    return (o, *torch.autograd.grad(o, leaves, d_o))
+
+
+def test_saved_tensors_go_through_hooks(call):
+    f, leaves, d_o = call
+    want = _once(*call)
+    packed, unpacked = [], []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(t), t.detach().cpu())[1],
+                                                  lambda t: (unpacked.append(t), t.cuda())[1]):
+        o = f(*leaves)
+    _same((o, *torch.autograd.grad(o, leaves, d_o)), want)
+    assert len(packed) == len(unpacked) >= len(leaves)
+
+
+def test_checkpointed_call(call):
+    f, leaves, d_o = call
+    o = torch.utils.checkpoint.checkpoint(f, *leaves, use_reentrant=False)
+    _same((o, *torch.autograd.grad(o, leaves, d_o)), _once(*call))
+
+
+def test_backward_from_another_thread_and_a_second_one(call):
+    f, leaves, d_o = call
+    want = _once(*call)
+    o = f(*leaves)
+    with ThreadPoolExecutor(1) as pool:
+        _same((o, *pool.submit(torch.autograd.grad, o, leaves, d_o, True).result()), want)
+    _same((o, *torch.autograd.grad(o, leaves, d_o)), want)  # the graph was kept once, and is released now
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(o, leaves, d_o)
+
+
+def test_call_on_a_side_stream(call):
+    """The call and its backward run on the stream that is current, behind what is queued there."""
+    f, leaves, d_o = call
+    want = _once(*call)
+    late = [torch.zeros_like(t) for t in leaves]
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)
+        for t, u in zip(late, leaves):
+            t.copy_(u.detach())
+        got = _once(f, [t.requires_grad_() for t in late], d_o)
+    side.synchronize()
+    _same(got, want)
+
+
+def test_modified_input_is_noticed(call):
+    f, leaves, d_o = call
+    mid = [t * 1 for t in leaves]
+    o = f(*mid)
+    with torch.no_grad():
+        mid[0].add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        o.backward(d_o)
+
+
+def test_empty_inputs_raise(call):
+    f, leaves, _ = call
+    with pytest.raises((rt.AeError, ValueError)):
+        f(*(t[:0] if t.shape[0] > 1 else t for t in leaves))
