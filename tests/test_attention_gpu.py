@@ -1085,6 +1085,26 @@ def test_mla_decode_in_equal_intervals(B, H, max_pages, lens, paged):
         _check(f"row {b} o", o[b:b + 1, 0].cpu(), ro, dtype)
 
 
+def test_mla_decode_repeats_bit_for_bit_under_load():
+    """The pair's hand-over of P relies on the hardware for its order (mla_arrive): a lost write would show as a result that
+    differs from run to run, so the same call is repeated while copies on another stream load the memory system."""
+    B, H, S, dtype = 40, 128, 1900, torch.bfloat16
+    eng = helpers.mla_engine(B, H, S, dtype, 1 / math.sqrt(192))
+    g = torch.Generator(device="cuda").manual_seed(4)
+    args = [torch.randn(s, generator=g, device="cuda", dtype=dtype) for s in ((B, 1, H, 512), (B, 1, H, 64), (B, S, 1, 512), (B, S, 1, 64))]
+    want = eng(*args)
+    side, src = torch.cuda.Stream(), torch.zeros(1 << 27, dtype=torch.int32, device="cuda")
+    dst = torch.empty_like(src)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        for _ in range(60):
+            dst.copy_(src)
+    outs = [eng(*args) for _ in range(100)]
+    torch.cuda.synchronize()
+    eng.check_status()
+    assert all(torch.equal(o, want) for o in outs)
+
+
 def test_split_decode_with_its_merge_in_a_graph():
     """The merge is launched to come up under the split kernel; captured and replayed on new inputs it still follows it."""
     B, Hq, Hkv, Skv, D, dtype = 2, 32, 8, 1000, 128, torch.float16
