@@ -87,12 +87,21 @@ struct Custom {
 
 struct Plan {
   at::ScalarType dtype = at::kHalf;
-  Tensor status;  // one word per engine; reallocated when the engine moves to another device
+  Tensor status;  // one word per engine; reallocated when the engine moves to another device, under `mu`
   Tensor status_for(const Tensor& like) {
     std::lock_guard<std::mutex> lk(mu);
     if (!status.defined() || status.device() != like.device())
       status = at::zeros({1}, like.options().dtype(at::kInt));
     return status;
+  }
+  // the front end's side, which holds the interpreter's lock: calls in other threads do not
+  Tensor status_now() {
+    std::lock_guard<std::mutex> lk(mu);
+    return status;
+  }
+  void set_status(Tensor t) {
+    std::lock_guard<std::mutex> lk(mu);
+    status = std::move(t);
   }
   std::mutex mu;
 };
@@ -843,8 +852,11 @@ py::object scan_block(const std::shared_ptr<ScanPlan>& plan, py::handle eng, con
   .def_property(#name, [](const cls& p) { return (uint64_t)(uintptr_t)p.name; }, \
                 [](cls& p, uint64_t h) { p.name = handle(h); })
 #define AE_STATUS(cls)                                                                                     \
-  .def_property("status", [](const cls& p) -> py::object { return p.status.defined() ? py::cast(p.status) : py::none(); }, \
-                [](cls& p, std::optional<Tensor> t) { p.status = t ? *t : Tensor(); })
+  .def_property("status", [](cls& p) -> py::object {                                                        \
+                  Tensor t = p.status_now();                                                                 \
+                  return t.defined() ? py::cast(t) : py::none();                                             \
+                },                                                                                           \
+                [](cls& p, std::optional<Tensor> t) { p.set_status(t ? *t : Tensor()); })
 
 PYBIND11_MODULE(_ae_host, m) {
   m.attr("built_for") = AE_HOST_BUILT_FOR;  // the build step looks for this text in the file

@@ -314,3 +314,25 @@ def test_empty_inputs_raise(call):
     f, leaves, _ = call
     with pytest.raises((rt.AeError, ValueError)):
         f(*(t[:0] if t.shape[0] > 1 else t for t in leaves))
+
+
+def test_calls_in_threads():
+    """One new engine, several threads with a stream each, and its status word looked at while their first calls make it."""
+    eng, q, k, v, _ = _attention()
+    want = eng(q, k, v)
+    torch.cuda.synchronize()
+    eng, *_ = _attention()
+
+    def work(_):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            outs = [eng(q, k, v) for _ in range(20)]
+            torch.cuda.current_stream().synchronize()
+            return all(torch.equal(o, want) for o in outs)
+
+    with ThreadPoolExecutor(4) as pool:
+        jobs = [pool.submit(work, i) for i in range(8)]
+        seen = [eng._status for _ in range(1000)]
+        assert all(j.result() for j in jobs)
+    torch.cuda.synchronize()
+    eng.check_status()
+    assert all(s is None or s.is_cuda for s in seen)
