@@ -144,6 +144,7 @@ class LinearAttentionEngine:
         self._bwd_mods = None
         self._streams = {}
         self._fwd_by_dv = {}
+        self._cut_kernels = {}
         self._rowscale_mods = {}
         # The kernels work on blocks of 128 key dims x 64 or 128 value dims.  Larger heads (simple_gla / retention_linear
         # of the reference use D = 256, DV = 512) are sums over key blocks of independent value blocks, see _scan().
@@ -158,6 +159,28 @@ class LinearAttentionEngine:
         if self._plan is None:
             self._plan = rt.host().ScanPlan(self._bf16)
         return self._plan
+
+    def _load_segment_kernels(self, dv: int, mods: bool, reverse: bool):
+        """Called by the native path before the first scan over a sequence cut into segments."""
+        plan = self._plan
+        # setdefault: what a thread has handed to the plan is not replaced by another thread's build
+        parts = self._cut_kernels.get(dv) or self._cut_kernels.setdefault(dv, self._build_segments(dv))
+        setattr(plan, f"seg{dv}", parts.handle.value)
+        key = (dv, mods, reverse)
+        scan = self._cut_kernels.get(key) or self._cut_kernels.setdefault(
+            key, self._build_bwd(mods, cut=True) if reverse else self._fwd_kernel(dv, mods, cut=True)[0])
+        # last: another thread that finds it set launches all of them
+        name = "bwd" if reverse else "fwd"
+        setattr(plan, f"{name}_mods_cut" if mods else "bwd_cut" if reverse else f"fwd_cut{dv}", scan.handle.value)
+
+    def _build_segments(self, dv: int):
+        """What the segments of a sequence add to the state, for scans of too few walks to fill the GPU."""
+        stages = 2 if dv == 64 else 1
+        pre = f"#define AE_BF16 {int(self._bf16)}\n#define AE_LIN_DV {dv}\n#define AE_LIN_STAGES {stages}\n"
+        smem = stages * (128 * 128 * 2 + 128 * dv * 2) + 256 + 1024  # two CTAs per SM
+        cfg = rt.KernelConfig(kind=rt.KIND_LINEAR_SEGMENTS, dtype=rt.DTYPE_BF16 if self._bf16 else rt.DTYPE_F16, head_dim=128,
+                              head_dim_v=dv, threads=192, smem_bytes=smem, stages=stages, mask_mode=0)
+        return rt.compile_module(rt.kernel_source("linear_segments.cuh", prelude=pre), "ae_linear_segments", cfg)
 
     @property
     def _status(self):
@@ -205,21 +228,22 @@ class LinearAttentionEngine:
                        n_heads=x.shape[1])
         return dq, dk, gx, da, gs, rows.sum(dim=2), res[4] if asc is not None else None
 
-    def _fwd_kernel(self, dv: int, mods: bool = False):
+    def _fwd_kernel(self, dv: int, mods: bool = False, cut: bool = False):
         """The forward kernel for value blocks of ``dv``; ``mods``: the build with the row scale of v and the skip
-        connection inside."""
-        key = (dv, mods)
+        connection inside; ``cut``: the one for a sequence in segments."""
+        key = (dv, mods, cut)
         if key not in self._fwd_by_dv:
             stages = 2 if dv == 64 else 1
             nwg = int(os.environ.get("AE_B200_LIN_FWD_NWG", LIN_FWD_NWG))
             prelude = (f"#define AE_BF16 {int(self._bf16)}\n#define AE_LIN_DV {dv}\n#define AE_LIN_STAGES {stages}\n"
-                       f"#define AE_LIN_MODS {int(mods)}\n#define AE_LIN_NWG {nwg}\n")
+                       f"#define AE_LIN_MODS {int(mods)}\n#define AE_LIN_NWG {nwg}\n"
+                       + ("#define AE_LIN_CUT 1\n" if cut else ""))
             # K/V ring, rescaled V, state copy, cumulative decays, barriers, output staging tile, alignment slack
             smem = stages * (2 * 128 * 128 * 2 + 128 * dv * 2) + 3 * 128 * dv * 2 + 1024 + 2048 + 1024
             cfg = rt.KernelConfig(kind=rt.KIND_LINEAR_FWD, dtype=rt.DTYPE_BF16 if self._bf16 else rt.DTYPE_F16,
                                   head_dim=128, head_dim_v=dv, threads=nwg * 128 + 64, smem_bytes=smem, stages=stages,
                                   mask_mode=0)
-            cfg.reserved[0] = int(mods)
+            cfg.reserved[0], cfg.reserved[1] = int(mods), int(cut)
             src = rt.kernel_source("linear_fwd.cuh", prelude=prelude)
             self._fwd_by_dv[key] = (rt.compile_module(src, "ae_linear_fwd", cfg), src)
         return self._fwd_by_dv[key]
@@ -243,18 +267,18 @@ class LinearAttentionEngine:
             self._bwd = (states, self._build_bwd(False))
         return self._bwd
 
-    def _build_bwd(self, mods: bool):
+    def _build_bwd(self, mods: bool, cut: bool = False):
         DV = 64
         tag = rt.DTYPE_BF16 if self._bf16 else rt.DTYPE_F16
         # row warpgroups of the reverse pass (2: the second one takes half of the P / dS pass and of the output phase)
         nwg = int(os.environ.get("AE_B200_LIN_BWD_NWG", LIN_BWD_NWG))
         pre = (f"#define AE_BF16 {int(self._bf16)}\n#define AE_LIN_DV {DV}\n#define AE_LIN_STAGES 2\n"
-               f"#define AE_LB_NWG {nwg}\n#define AE_LB_MODS {int(mods)}\n")
+               f"#define AE_LB_NWG {nwg}\n#define AE_LB_MODS {int(mods)}\n" + ("#define AE_LIN_CUT 1\n" if cut else ""))
         smem_b = (2 * 128 * 128 * 2 + 2 * 128 * DV * 2 + 128 * DV * 2 + 2 * 128 * 128 * 2
                   + 128 * DV * 2 + 128 * DV * 2 + int(mods) * 128 * DV * 2 + 1024 + 256 + 512 + 1024)
         cfg = rt.KernelConfig(kind=rt.KIND_LINEAR_BWD, dtype=tag, head_dim=128, head_dim_v=DV,
                               threads=nwg * 128 + 64, smem_bytes=smem_b, stages=1, mask_mode=0)
-        cfg.reserved[0] = int(mods)
+        cfg.reserved[0], cfg.reserved[1] = int(mods), int(cut)
         return rt.compile_module(rt.kernel_source("linear_bwd.cuh", prelude=pre), "ae_linear_bwd", cfg)
 
     def _new_states(self, v):

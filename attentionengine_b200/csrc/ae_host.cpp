@@ -619,6 +619,67 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
 struct ScanPlan : Plan {
   void *fwd_mods = nullptr;  // the forward built with the Mamba2 block's mods inside (64 value dims)
   void *bwd = nullptr, *bwd_mods = nullptr, *head_sum = nullptr;  // set when first needed
+  // what a sequence cut into segments takes, set when first needed: the contributions by value dims, and the scan kernels'
+  // builds that start from them
+  void *seg64 = nullptr, *seg128 = nullptr;
+  void *fwd_cut64 = nullptr, *fwd_cut128 = nullptr, *fwd_mods_cut = nullptr, *bwd_cut = nullptr, *bwd_mods_cut = nullptr;
+  int segments = 0;  // segments a sequence is cut into; 0: as many as seg_chunks() finds
+};
+
+// Chunks per segment of a scan of `walks` (batch, head) walks over n chunks.  A walk is a chain, and a launch lasts as long as
+// the walks on the fullest SM; segments shorten the chain and fill idle SMs, at the price of a launch that computes what
+// every segment but one adds to the state (two CTAs per SM) and of summing those in front of a segment.  Microseconds as
+// measured on a B200 over 1 to 16 segments: a CTA of the scan 5 + chunk_us per chunk + 0.25 per segment, one of the
+// contributions 3 + 1.3 per chunk, 3 for the second launch.  Forward (chunk_us 2.95), one cut against the best one:
+// 8 walks of 64 chunks 195 -> 30 (16 segments), 48 of 56 173 -> 93 (3), 320 of 24 (more walks than SMs) 227 uncut, 231 in two.
+int seg_chunks(const ScanPlan& plan, int64_t walks, int64_t n, int device, double chunk_us) {
+  if (plan.segments) return (int)((n + plan.segments - 1) / plan.segments);
+  int sms = 0;
+  C10_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  auto rounds = [](int64_t ctas, int64_t room) { return (double)((ctas + room - 1) / room); };
+  int64_t best = n;
+  double least = rounds(walks, sms) * (n * chunk_us + 5);
+  for (int64_t p = 2; p <= std::min<int64_t>(n, 16); ++p) {
+    const int64_t len = (n + p - 1) / p, cut = (n + len - 1) / len;
+    const double t = rounds(walks * cut, sms) * (len * chunk_us + 5 + 0.25 * cut) + rounds(walks * (cut - 1), 2 * sms) * (len * 1.3 + 3) + 3;
+    if (t < least) least = t, best = len;
+  }
+  return (int)best;
+}
+
+// Scratch of a cut and the launch that fills it; nothing with one segment.  `scan` is the plan's kernel for the other case.
+struct Segments {
+  Tensor buf;
+  int chunks = 0, count = 1;
+  float *state = nullptr, *decay = nullptr;
+  void* scan = nullptr;
+  Segments(const ScanPlan& plan, py::handle eng, bool mods, const Tensor& rows, const Tensor& values, const Tensor& a, const Tensor& asc, const Tensor& vscale,
+           bool reverse, double chunk_us, uint32_t* status) {
+    const int64_t B = values.size(0), H = values.size(1), T = values.size(2), DV = values.size(3), n = (T + 127) / 128;
+    if (n < 2) return;
+    chunks = seg_chunks(plan, B * H, n, values.device().index(), chunk_us);
+    count = (int)((n + chunks - 1) / chunks);
+    if (count == 1) return;
+    void* const& kernel = DV == 64 ? plan.seg64 : plan.seg128;
+    void* const& cut = reverse ? (mods ? plan.bwd_mods_cut : plan.bwd_cut)
+                               : (mods ? plan.fwd_mods_cut : DV == 64 ? plan.fwd_cut64 : plan.fwd_cut128);
+    if (!cut) with_python([&] { eng.attr("_load_segment_kernels")((int)DV, mods, reverse); });
+    scan = cut;
+    const int64_t slots = B * H * (count - 1);
+    buf = at::empty({slots * (128 * DV + 1)}, a.options());
+    state = (float*)buf.data_ptr();
+    decay = state + slots * 128 * DV;
+    AeLinearSegParams p;
+    memset(&p, 0, sizeof p);
+    p.rows = rows.data_ptr(); p.values = values.data_ptr(); p.a = (const float*)a.data_ptr();
+    p.ascale = asc.defined() ? (const float*)asc.data_ptr() : nullptr;
+    p.vscale = vscale.defined() ? vscale.data_ptr() : nullptr;
+    p.vscale_16bit = vscale.defined() && vscale.scalar_type() != at::kFloat;
+    p.B = (int)B; p.H = (int)H; p.HR = (int)rows.size(1); p.T = (int)T;
+    p.seg_chunks = chunks; p.reverse = reverse; p.seg_state = state; p.seg_decay = decay;
+    p.status = status;
+    check(ae_launch_linear_segments(kernel, &p, stream_of(values)), "ae_launch_linear_segments");
+  }
 };
 
 // the tensors of one scan; s / d / asc undefined without the block's mods
@@ -628,7 +689,7 @@ struct ScanSaved {
 };
 
 Tensor sum_over_batch(const Tensor& t, const std::vector<int64_t>& shape, at::ScalarType dtype) {
-  // [B, H] -> the operand's shape; one batch row needs no sum
+  // [B, H] (times segments) -> the operand's shape; a single row needs no sum
   return (t.size(0) == 1 ? t : t.sum(0)).reshape(shape).to(dtype);
 }
 
@@ -684,19 +745,21 @@ struct ScanNode : Node {
     p.da = (float*)da.data_ptr();
     p.B = B; p.H = H; p.HQ = HQ; p.HK = HK; p.T = T;
     p.status = word(status);
+    const Segments seg(*plan, eng.get(), mods, q, g, a, asc, Tensor(), true, 5.6, p.status);
+    p.seg_chunks = seg.chunks; p.seg_state = seg.state; p.seg_decay = seg.decay;
     if (mods) {
       gs = at::empty_like(s);
-      gd = at::empty({B, H}, f32);
+      gd = at::empty({B * seg.count, H}, f32);
       p.x = x.data_ptr(); p.vscale = s.data_ptr(); p.dskip = (const float*)d.data_ptr();
       p.gs = gs.data_ptr(); p.gd = (float*)gd.data_ptr();
       p.vscale_16bit = s.scalar_type() != at::kFloat;
     }
     if (asc.defined()) {
-      gasc = at::empty({B, H}, f32);
+      gasc = at::empty({B * seg.count, H}, f32);
       p.ascale = (const float*)asc.data_ptr();
       p.gasc = (float*)gasc.data_ptr();
     }
-    check(ae_launch_linear_bwd(mods ? plan->bwd_mods : plan->bwd, &p, st), "ae_launch_linear_bwd");
+    check(ae_launch_linear_bwd(seg.scan ? seg.scan : mods ? plan->bwd_mods : plan->bwd, &p, st), "ae_launch_linear_bwd");
     auto head_sum = [&](const Tensor& in, int heads) {
       if (heads == H) return in;
       Tensor y = at::empty({B, heads, T, 128}, o16);
@@ -725,10 +788,10 @@ struct ScanNode : Node {
   std::string name() const override { return mods ? "ScaleScanSkipBackward" : "LinearScanBackward"; }
 };
 
-// One launch of the scan kernel on contiguous tensors; those after `a` may be undefined: the row scale, skip weight and decay
+// The scan kernel on contiguous tensors, in segments where that is faster (with `eng`, whose builds it then takes); those after `a` may be undefined: the row scale, skip weight and decay
 // scale of the Mamba2 block (a kernel built with the mods inside), and what receives the scaled v and the chunk start-states.
 Tensor scan_launch(ScanPlan& plan, void* kernel, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& s,
-                   const Tensor& d, const Tensor& asc, const Tensor& v_out, const Tensor& hs) {
+                   const Tensor& d, const Tensor& asc, const Tensor& v_out, const Tensor& hs, py::handle eng = {}) {
   AeLinearParams p;
   memset(&p, 0, sizeof p);
   Tensor y = at::empty({q.size(0), v.size(1), q.size(2), v.size(3)}, q.options());
@@ -742,6 +805,12 @@ Tensor scan_launch(ScanPlan& plan, void* kernel, const Tensor& q, const Tensor& 
   p.h_states_out = ptr(hs);
   p.B = (int)q.size(0); p.H = (int)v.size(1); p.HQ = (int)q.size(1); p.HK = (int)k.size(1); p.T = (int)q.size(2);
   p.status = word(plan.status_for(q));
+  std::optional<Segments> seg;
+  if (eng) {
+    seg.emplace(plan, eng, s.defined(), k, v, a, asc, s, false, 2.95, p.status);
+    p.seg_chunks = seg->chunks; p.seg_state = seg->state; p.seg_decay = seg->decay;
+    if (seg->scan) kernel = seg->scan;
+  }
   check(ae_launch_linear_fwd(kernel, &p, stream_of(q)), "ae_launch_linear_fwd");
   return y;
 }
@@ -770,7 +839,7 @@ Tensor scan_run(const std::shared_ptr<ScanPlan>& plan, void* kernel, py::handle 
       TORCH_CHECK(DV == 64, "the scan has gradients in value blocks of 64 dims");
       hs = at::empty({B, H, (T + 127) / 128, 128, DV}, q.options());
     }
-    y = scan_launch(*plan, kernel, q, k, v, a, s, d, asc, v_out, hs);
+    y = scan_launch(*plan, kernel, q, k, v, a, s, d, asc, v_out, hs, eng);
     status = plan->status_for(q);
   }
   if (need) {
@@ -807,7 +876,7 @@ Tensor scan_run(const std::shared_ptr<ScanPlan>& plan, void* kernel, py::handle 
   return y;
 }
 
-// The launch alone, for the front end's autograd function and for direct use.
+// One launch of the scan kernel, for the front end's autograd function and for direct use: bit-equal states to ae_linear_states.
 Tensor scan_forward(const std::shared_ptr<ScanPlan>& plan, uint64_t kernel, const Tensor& q, const Tensor& k, const Tensor& v,
                     const Tensor& a, const std::optional<Tensor>& s, const std::optional<Tensor>& d, const std::optional<Tensor>& asc,
                     const std::optional<Tensor>& v_out, const std::optional<Tensor>& hs) {
@@ -894,7 +963,10 @@ PYBIND11_MODULE(_ae_host, m) {
         p->dtype = bf16 ? at::kBFloat16 : at::kHalf;
         return p;
       })) AE_HANDLE(ScanPlan, fwd_mods) AE_HANDLE(ScanPlan, bwd) AE_HANDLE(ScanPlan, bwd_mods)
-          AE_HANDLE(ScanPlan, head_sum) AE_STATUS(ScanPlan);
+          AE_HANDLE(ScanPlan, head_sum) AE_HANDLE(ScanPlan, seg64) AE_HANDLE(ScanPlan, seg128)
+          AE_HANDLE(ScanPlan, fwd_cut64) AE_HANDLE(ScanPlan, fwd_cut128) AE_HANDLE(ScanPlan, fwd_mods_cut)
+          AE_HANDLE(ScanPlan, bwd_cut) AE_HANDLE(ScanPlan, bwd_mods_cut)
+      .def_readwrite("segments", &ScanPlan::segments) AE_STATUS(ScanPlan);
   m.def("attn", torch::wrap_pybind_function(&attn));
   m.def("decode", torch::wrap_pybind_function(&decode));
   m.def("mla", torch::wrap_pybind_function(&mla));

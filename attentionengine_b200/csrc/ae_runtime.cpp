@@ -1029,6 +1029,56 @@ static int make_bhtd_map(AeTmaDesc* out, const void* base, int dtype, int64_t B,
   return AE_OK;
 }
 
+// Segments of a scan over T steps (1 without a cut), or 0 when the operands of a cut are not complete.
+static int scan_segments(const Module* m, int T, int seg_chunks, const float* state, const float* decay, int* chunks) {
+  const int n = (T + 127) / 128;
+  *chunks = n;
+  if (seg_chunks <= 0 || seg_chunks >= n) return 1;
+  if (m->cfg.kind != AE_KIND_LINEAR_SEGMENTS && m->cfg.reserved[1] != 1) {
+    set_error("linear attention in segments: needs a module built for a cut sequence (reserved[1] = 1)");
+    return 0;
+  }
+  if (!state || !decay || (reinterpret_cast<uintptr_t>(state) & 15) || (reinterpret_cast<uintptr_t>(decay) & 3)) {
+    set_error("linear attention in segments: seg_state (16-byte aligned) and seg_decay are required");
+    return 0;
+  }
+  *chunks = seg_chunks;
+  return (n + seg_chunks - 1) / seg_chunks;
+}
+
+int ae_launch_linear_segments(void* module, const AeLinearSegParams* p, void* stream) {
+  if (!module || !p || !p->rows || !p->values || !p->a) return AE_ERR_INVALID;
+  Module* m = (Module*)module;
+  if (m->cfg.kind != AE_KIND_LINEAR_SEGMENTS) {
+    set_error("module kind does not match the entry point");
+    return AE_ERR_UNSUPPORTED;
+  }
+  const int DV = m->cfg.head_dim_v;
+  if (p->B <= 0 || p->H <= 0 || p->HR <= 0 || p->T <= 0 || p->H % p->HR || m->cfg.head_dim != 128 || (DV != 64 && DV != 128)) {
+    set_error("linear attention: need H % HQ == 0, H % HK == 0, DK = 128, DV in {64, 128}");
+    return AE_ERR_INVALID;
+  }
+  AeLinearSegArgs a;
+  memset(&a, 0, sizeof a);
+  const int n_seg = scan_segments(m, p->T, p->seg_chunks, p->seg_state, p->seg_decay, &a.seg_chunks);
+  if (n_seg == 0) return AE_ERR_INVALID;
+  if (n_seg == 1) return AE_OK;  // nothing in front of the first segment
+  if (p->vscale && (reinterpret_cast<uintptr_t>(p->vscale) & (p->vscale_16bit ? 1 : 3))) {
+    set_error("linear attention: vscale must be aligned to its element size");
+    return AE_ERR_INVALID;
+  }
+  int rc = ensure_loaded(m);
+  if (rc) return rc;
+  if ((rc = make_bhtd_map(&a.tm_k, p->rows, m->cfg.dtype, p->B, p->HR, p->T, 128, 128))) return rc;
+  if ((rc = make_bhtd_map(&a.tm_v, p->values, m->cfg.dtype, p->B, p->H, p->T, DV, 128))) return rc;
+  a.a = p->a; a.ascale = p->ascale; a.vscale = p->vscale; a.vscale_16 = p->vscale_16bit;
+  a.B = p->B; a.H = p->H; a.HK = p->HR; a.T = p->T;
+  a.reverse = p->reverse;
+  a.seg_state = p->seg_state; a.seg_decay = p->seg_decay;
+  a.status = p->status;
+  return launch(m, (unsigned)p->H, (unsigned)p->B, (unsigned)(n_seg - 1), &a, stream);
+}
+
 int ae_launch_linear_fwd(void* module, const AeLinearParams* p, void* stream) {
   if (!module || !p || !p->q || !p->k || !p->v || !p->a || !p->o) return AE_ERR_INVALID;
   Module* m = (Module*)module;
@@ -1085,7 +1135,12 @@ int ae_launch_linear_fwd(void* module, const AeLinearParams* p, void* stream) {
     set_error("linear attention: vscale / dskip / v_out need a module built with the mods inside (reserved[0] = 1)");
     return AE_ERR_INVALID;
   }
-  return launch(m, (unsigned)p->H, (unsigned)p->B, 1, &a, stream);
+  const int n_seg = scan_segments(m, p->T, p->seg_chunks, p->seg_state, p->seg_decay, &a.seg_chunks);
+  if (n_seg == 0) return AE_ERR_INVALID;
+  if (n_seg == 1) return launch(m, (unsigned)p->H, (unsigned)p->B, 1, &a, stream);
+  a.seg_state = p->seg_state;
+  a.seg_decay = p->seg_decay;
+  return launch_after(m, (unsigned)p->H, (unsigned)p->B, (unsigned)n_seg, &a, stream);
 }
 
 static int fill_linear_bwd(Module* m, const AeLinearBwdParams* p, AeLinearBwdArgs* a, int kind) {
@@ -1164,7 +1219,12 @@ int ae_launch_linear_bwd(void* module, const AeLinearBwdParams* p, void* stream)
   AeLinearBwdArgs a;
   int rc = fill_linear_bwd(m, p, &a, AE_KIND_LINEAR_BWD);
   if (rc) return rc;
-  return launch(m, (unsigned)p->H, (unsigned)p->B, 1, &a, stream);
+  const int n_seg = scan_segments(m, p->T, p->seg_chunks, p->seg_state, p->seg_decay, &a.seg_chunks);
+  if (n_seg == 0) return AE_ERR_INVALID;
+  if (n_seg == 1) return launch(m, (unsigned)p->H, (unsigned)p->B, 1, &a, stream);
+  a.seg_state = p->seg_state;
+  a.seg_decay = p->seg_decay;
+  return launch_after(m, (unsigned)p->H, (unsigned)p->B, (unsigned)n_seg, &a, stream);
 }
 
 }  // extern "C"

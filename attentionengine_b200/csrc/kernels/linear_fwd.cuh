@@ -24,6 +24,13 @@
 // is x, the scan runs on v = x * vscale[b, h, t] (the row thread that rescales its row of the V tile for the state
 // update anyway also scales it in place for P v and writes v out for the backward), and the output row gets
 // + x * dskip[h] from a copy of the raw row kept in shared memory.  Two streaming passes over x and one over o less.
+//
+// A sequence may be cut into segments of args.seg_chunks chunks, one CTA each (grid z): a CTA behind the first starts from
+// S = sum over the segments j in front of it of exp(decay of the segments between) L_j, with L_j from linear_segments.cuh.
+// That is a build of its own (AE_LIN_CUT): carrying it in the plain one cost a walk of eight chunks 28.0 -> 30.3 us.
+#ifndef AE_LIN_CUT
+#define AE_LIN_CUT 0
+#endif
 #ifndef AE_LIN_MODS
 #define AE_LIN_MODS 0
 #endif
@@ -86,7 +93,15 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
   const int b = blockIdx.y;
   const int hq = h / (args.H / args.HQ);
   const int hk = h / (args.H / args.HK);
-  const int n_chunks = (args.T + AE_LIN_C - 1) / AE_LIN_C;
+  const int n_total = (args.T + AE_LIN_C - 1) / AE_LIN_C;
+#if AE_LIN_CUT
+  const int c_begin = (int)blockIdx.z * args.seg_chunks;  // chunks are counted from the start of the segment below
+  const int n_chunks = min(args.seg_chunks, n_total - c_begin);
+  const bool carried = blockIdx.z > 0;  // the segment starts from a state
+#else
+  const int c_begin = 0, n_chunks = n_total;
+  constexpr bool carried = false;
+#endif
 
   if (threadIdx.x == 0) {
     ctl->abort = 0;
@@ -137,18 +152,18 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
           const int cs = c - 1;  // its row threads have written and fenced the state copy and the scaled V tile
           ok = mbar_wait(&bars->prep_done, cs & 1, ctl, args.status, 60);
           if (!ok) break;
-          if (st_h && cs >= 1) {
+          if (st_h && (cs >= 1 || carried)) {
             for (int dh = 0; dh < AE_LIN_DV / 64; ++dh)
               tma_store_3d(&args.tm_hout, smem + AE_LIN_SMEM_H + dh * (AE_LIN_DK * 128), dh * 64, 0,
-                           (b * args.H + h) * n_chunks + cs);
+                           (b * args.H + h) * n_total + c_begin + cs);
           }
           if (st_v) {
             const u8* vt = smem + AE_LIN_SMEM_STAGE + (cs % AE_LIN_STAGES) * AE_LIN_STAGE_BYTES + 2 * AE_LIN_Q_BYTES;
             for (int dh = 0; dh < AE_LIN_DV / 64; ++dh)
-              tma_store_4d(&args.tm_vout, vt + dh * (AE_LIN_C * 128), dh * 64, cs * AE_LIN_C, h, b);
+              tma_store_4d(&args.tm_vout, vt + dh * (AE_LIN_C * 128), dh * 64, (c_begin + cs) * AE_LIN_C, h, b);
           }
           tma_store_commit();
-          if (st_h && cs >= 1) {
+          if (st_h && (cs >= 1 || carried)) {
             tma_store_wait_read();  // the state copy is rewritten by the row threads of the next chunk
             mbar_arrive(&bars->hb_free);
           }
@@ -161,13 +176,13 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
           u8* st = smem + AE_LIN_SMEM_STAGE + stage * AE_LIN_STAGE_BYTES;
           mbar_arrive_expect_tx(&bars->full[stage], AE_LIN_STAGE_BYTES);
           for (int dh = 0; dh < AE_LIN_DK / 64; ++dh) {
-            tma_load_4d(st + dh * (AE_LIN_C * 128), &args.tm_q, &bars->full[stage], dh * 64, c * AE_LIN_C, hq, b);
+            tma_load_4d(st + dh * (AE_LIN_C * 128), &args.tm_q, &bars->full[stage], dh * 64, (c_begin + c) * AE_LIN_C, hq, b);
             tma_load_4d(st + AE_LIN_Q_BYTES + dh * (AE_LIN_C * 128), &args.tm_k, &bars->full[stage], dh * 64,
-                        c * AE_LIN_C, hk, b);
+                        (c_begin + c) * AE_LIN_C, hk, b);
           }
           for (int dh = 0; dh < AE_LIN_DV / 64; ++dh)
             tma_load_4d(st + 2 * AE_LIN_Q_BYTES + dh * (AE_LIN_C * 128), &args.tm_v, &bars->full[stage], dh * 64,
-                        c * AE_LIN_C, h, b);
+                        (c_begin + c) * AE_LIN_C, h, b);
         }
         if (c >= 1) {
           // the output tile of chunk c - 1 (complete at the end of that chunk; the loads of chunk c are already out)
@@ -175,7 +190,7 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
           ok = mbar_wait(&bars->y_full, cy & 1, ctl, args.status, 62);
           if (!ok) break;
           for (int dh = 0; dh < AE_LIN_DV / 64; ++dh)
-            tma_store_4d(&args.tm_o, smem + AE_LIN_SMEM_Y + dh * (AE_LIN_C * 128), dh * 64, cy * AE_LIN_C, h, b);
+            tma_store_4d(&args.tm_o, smem + AE_LIN_SMEM_Y + dh * (AE_LIN_C * 128), dh * 64, (c_begin + cy) * AE_LIN_C, h, b);
           tma_store_commit();
           tma_store_wait_read();  // the rows of the next chunk write the tile again
           mbar_arrive(&bars->y_free);
@@ -214,7 +229,7 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
         ok = mbar_wait_w(&bars->prep_done, c & 1, ctl, args.status, 53);
         if (!ok) break;
         tc_fence_after_sync();
-        if (c > 0) {
+        if (c > 0 || carried) {
           // Oi = q h   (h: [DK rows][DV contiguous], MN-major B)
 #pragma unroll
           for (int kk = 0; kk < AE_LIN_DK / 16; ++kk)
@@ -224,7 +239,7 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
         // H (+)= k^T v'   (k tile read MN-major as A: [chunk rows][DK contiguous]; v' likewise as B)
 #pragma unroll
         for (int kk = 0; kk < AE_LIN_C / 16; ++kk)
-          umma_ss_w(tmem + TM_H, umma_step_mn(bk_mn + so, kk), umma_step_mn(bv2_mn, kk), idesc_h, (c > 0) | (kk > 0));
+          umma_ss_w(tmem + TM_H, umma_step_mn(bk_mn + so, kk), umma_step_mn(bv2_mn, kk), idesc_h, carried | (c > 0) | (kk > 0));
         umma_commit_w(&bars->h_done);
         ok = mbar_wait_w(&bars->p_full, c & 1, ctl, args.status, 54);
         if (!ok) break;
@@ -232,7 +247,7 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
 #pragma unroll
         for (int kk = 0; kk < AE_LIN_C / 16; ++kk)
           umma_ts_w(tmem + TM_O, tmem + TM_S + kk * 8 + ((AE_LIN_NWG > 1 && kk >= AE_LIN_C / 32) ? 64 : 0),
-                    umma_step_mn(bv_mn + so, kk), idesc_oi, (c > 0) | (kk > 0));
+                    umma_step_mn(bv_mn + so, kk), idesc_oi, carried | (c > 0) | (kk > 0));
         umma_commit_w(&bars->o_done);
         umma_commit_w(&bars->empty[stage]);
         if (c + 1 < n_chunks) ok = issue_s(c + 1);
@@ -256,7 +271,8 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
     // ahead: a global load at the top of every chunk would sit on the chain of dependent phases.
     auto load_a = [&](int tt) { return tt < args.T ? a_row[tt] : 0.f; };
     const u32 wg = warp >> 2;  // 0: the group that also runs the cumulative sum
-    float a_next = load_a((int)r);
+    const int t_begin = c_begin * AE_LIN_C;
+    float a_next = load_a(t_begin + (int)r);
     // a decay mod of the form decay * custom[heads]; applied where the prefetched value is used, not where it is loaded
     const float asc = args.ascale ? args.ascale[h] : 1.f;
 #if AE_LIN_MODS
@@ -267,7 +283,7 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
       const i64 si = ((i64)b * args.H + h) * args.T + tt;
       return vs16 ? (u32)((const u16*)args.vscale)[si] : ((const u32*)args.vscale)[si];
     };
-    u32 vs_next = load_vs((int)r);
+    u32 vs_next = load_vs(t_begin + (int)r);
 #endif
     // Inclusive cumulative sum of the log-decay over a chunk and the column factors of its decay matrix (first group
     // only).  It runs one chunk ahead, while the P v MMAs of the chunk at hand are under way: at the top of the chunk
@@ -293,11 +309,29 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
     float g_nxt = 0.f;
     if (wg == 0) {
       g_nxt = cum_sum(a_next * asc, gs, cf_all);
-      a_next = load_a(AE_LIN_C + (int)r);
+      a_next = load_a(t_begin + AE_LIN_C + (int)r);
     }
+#if AE_LIN_CUT
+    if (carried) {  // the state the segment starts from: this thread's row and columns, into TMEM
+      ae_grid_wait();
+      const i64 slot = ((i64)b * args.H + h) * (gridDim.z - 1);
+#pragma unroll
+      for (int c2 = 0; c2 < AE_LIN_DV / 32 / AE_LIN_NWG; ++c2) {
+        const int cc = (int)wg * (AE_LIN_DV / 32 / AE_LIN_NWG) + c2;
+        float acc[32];
+        scan_segment_sum(acc, args.seg_state, args.seg_decay, slot, 0, (int)blockIdx.z, AE_LIN_DK * AE_LIN_DV, cc, r);
+        u32 w[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(acc[i]);
+        tmem_st32(tmem + TM_H + lane_base + cc * 32, w);
+      }
+      tc_wait_st();
+    }
+#endif
     for (int c = 0; c < n_chunks; ++c) {
       const int stage = c % AE_LIN_STAGES;
-      const int t = c * AE_LIN_C + (int)r;
+      const int t = t_begin + c * AE_LIN_C + (int)r;
+      const bool live = c > 0 || carried;  // the chunk starts from a state
       AE_TRL(warp == 0, 1, c * 16 + 0)
       // ---- A: the chunk's cumulative log-decays were summed during the chunk before (cum_sum) -----
       float* gc = gs + (c & 1) * 128;
@@ -319,15 +353,17 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
 #endif
       AE_TRL(warp == 0, 1, c * 16 + 1)
       // ---- B: incoming state -> bf16 copy for q h, and decay it in place --------------------
-      if (c == 0 && args.h_out && wg == 0) {  // the first chunk starts from zero; the later ones leave through the producer's bulk stores
-        u16* hrow = (u16*)args.h_out + (((i64)b * args.H + h) * n_chunks * AE_LIN_DK + r) * AE_LIN_DV;
+      if (!live && args.h_out && wg == 0) {  // the first chunk starts from zero; the later ones leave through the producer's bulk stores
+        u16* hrow = (u16*)args.h_out + (((i64)b * args.H + h) * n_total * AE_LIN_DK + r) * AE_LIN_DV;
 #pragma unroll
         for (int i = 0; i < AE_LIN_DV / 8; ++i) *(uint4*)(hrow + i * 8) = make_uint4(0, 0, 0, 0);
       }
-      if (c > 0) {
-        // the bulk store of the previous chunk's copy has read it (long ago: it was issued a chunk earlier)
-        if (args.h_out && c >= 2) ok = ok && mbar_wait(&bars->hb_free, (c - 2) & 1, ctl, args.status, 61);
-        ok = ok && mbar_wait(&bars->h_done, (c - 1) & 1, ctl, args.status, 55);
+      if (live) {
+        // the bulk store of the previous chunk's copy has read it (long ago: it was issued a chunk earlier); the first
+        // chunk that has a copy is chunk 0 of a segment behind the first, else chunk 1
+        const int copies = carried ? c : c - 1;
+        if (args.h_out && copies >= 1) ok = ok && mbar_wait(&bars->hb_free, (copies - 1) & 1, ctl, args.status, 61);
+        if (c > 0) ok = ok && mbar_wait(&bars->h_done, (c - 1) & 1, ctl, args.status, 55);
         tc_fence_after_sync();
         const float dec = ae_exp(g_last);
         u8* hb = smem + AE_LIN_SMEM_H;
@@ -454,7 +490,7 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
       ok = ok && mbar_wait(&bars->oi_full, c & 1, ctl, args.status, 58);
       AE_TRL(warp == 0, 1, c * 16 + 7)
       tc_fence_after_sync();
-      if (c > 0) {
+      if (live) {
         const float eg = ae_exp(g);
 #pragma unroll
         for (int c2 = 0; c2 < AE_LIN_DV / 32 / AE_LIN_NWG; ++c2) {
@@ -518,6 +554,9 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
       // and each warp arrives there only after this point
       AE_TRL(warp == 0, 1, c * 16 + 10)
     }
+#if AE_LIN_CUT
+    if (!carried) ae_grid_wait();  // a kernel ends after the one it was brought up under
+#endif
   }
 
   tc_fence_before_sync();

@@ -1,0 +1,184 @@
+// State contributions of the segments of a linear-attention / SSD scan, for sm_100a.
+//
+// The scan kernels walk a head's chunks one after the other, so a problem with fewer (batch, head) walks than SMs leaves the
+// rest idle for the whole walk.  Such a problem is cut into segments of whole chunks along the sequence: this kernel
+// computes what every segment adds to the state on its own, all segments at once, and the scan kernels (one CTA per
+// batch, head and segment) start from the decayed sum over the segments in front of theirs (behind it, for the reverse pass).
+//
+//     forward   L = sum_t exp(sum of a over the segment's steps behind t) k_t^T v_t
+//     reverse   L = sum_t exp(sum of a over the segment's steps up to and with t) q_t^T dO_t
+//
+// Both are one accumulation without a recurrence: walked from the far end (forward: last chunk first; reverse: first
+// chunk first) the weight of a step is exp of a running sum <= 0, and the accumulator in TMEM is read once, at the end.  A chunk
+// is a load of two tiles, one pass over the V (dO) tile and eight MMAs, with nothing that waits for the chunk before;
+// what bounds it is the pass over the tile and the loads, so two CTAs share an SM.
+// The weighted values are rounded to 16 bits as in the scan kernels; sums, decays and results are fp32.
+// Roles: warps 0-3 row threads (thread r = step r of the chunk, then state row r), warp 4 TMA producer, warp 5 MMA issuer.
+// Expects AE_BF16, AE_LIN_DV (64 or 128), AE_LIN_STAGES.
+
+#define AE_LG_C 128
+#define AE_LG_DK 128
+#define AE_LG_K_BYTES (AE_LG_C * AE_LG_DK * 2)
+#define AE_LG_V_BYTES (AE_LG_C * AE_LIN_DV * 2)
+#define AE_LG_STAGE_BYTES (AE_LG_K_BYTES + AE_LG_V_BYTES)
+#define AE_LG_SMEM_BAR (AE_LIN_STAGES * AE_LG_STAGE_BYTES)
+
+struct AeLgBars {
+  u64 full[AE_LIN_STAGES];
+  u64 prep[AE_LIN_STAGES];   // the stage's V tile carries the weights
+  u64 empty[AE_LIN_STAGES];  // the MMAs have read the stage
+  u64 done;
+  float tot[2][4];  // warp totals of the chunk's log-decays, by chunk parity
+  AeCtaCtl ctl;
+};
+
+extern "C" __global__ void __launch_bounds__(192, 2) ae_linear_segments(const __grid_constant__ AeLinearSegArgs args) {
+  extern __shared__ u8 smem_raw[];
+  u8* smem = smem_align1024(smem_raw);
+  AeLgBars* bars = (AeLgBars*)(smem + AE_LG_SMEM_BAR);
+  AeCtaCtl* ctl = &bars->ctl;
+  const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int hk = h / (args.H / args.HK);
+  const bool rev = args.reverse != 0;
+  const int n_total = (args.T + AE_LG_C - 1) / AE_LG_C;
+  const int c_begin = ((int)blockIdx.z + (rev ? 1 : 0)) * args.seg_chunks;  // the first (reverse: last) segment has no reader
+  const int n_chunks = min(args.seg_chunks, n_total - c_begin);
+  auto chunk_at = [&](int i) { return rev ? c_begin + i : c_begin + n_chunks - 1 - i; };
+
+  ae_grid_trigger();  // the scan kernel may be brought up
+  if (threadIdx.x == 0) {
+    ctl->abort = 0;
+    for (int i = 0; i < AE_LIN_STAGES; ++i) {
+      mbar_init(&bars->full[i], 1);
+      mbar_init(&bars->prep[i], 4);
+      mbar_init(&bars->empty[i], 1);
+    }
+    mbar_init(&bars->done, 1);
+    mbar_fence_init();
+  }
+  if (warp == 5) {
+    tmem_alloc(&ctl->tmem_base, 128);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const u32 tmem = ctl->tmem_base;
+
+  if (warp == 4) {
+    if (lane == 0) {
+      tma_prefetch_desc(&args.tm_k);
+      tma_prefetch_desc(&args.tm_v);
+      for (int i = 0; i < n_chunks; ++i) {
+        const int stage = i % AE_LIN_STAGES, c = chunk_at(i);
+        if (!mbar_wait(&bars->empty[stage], ((i / AE_LIN_STAGES) & 1) ^ 1, ctl, args.status, 91)) break;
+        u8* st = smem + stage * AE_LG_STAGE_BYTES;
+        mbar_arrive_expect_tx(&bars->full[stage], AE_LG_STAGE_BYTES);
+        for (int dh = 0; dh < AE_LIN_DV / 64; ++dh)
+          tma_load_4d(st + AE_LG_K_BYTES + dh * (AE_LG_C * 128), &args.tm_v, &bars->full[stage], dh * 64, c * AE_LG_C, h, b);
+        for (int dh = 0; dh < AE_LG_DK / 64; ++dh)
+          tma_load_4d(st + dh * (AE_LG_C * 128), &args.tm_k, &bars->full[stage], dh * 64, c * AE_LG_C, hk, b);
+      }
+    }
+  } else if (warp == 5) {
+    const u32 idesc = umma_idesc_f16(AE_LG_DK, AE_LIN_DV, AE_BF16, 1, 1);
+    const u64 bk_mn = umma_base_mn(smem_u32(smem), AE_LG_C);
+    const u64 bv_mn = umma_base_mn(smem_u32(smem + AE_LG_K_BYTES), AE_LG_C);
+    bool ok = true;
+    for (int i = 0; i < n_chunks && ok; ++i) {
+      const int stage = i % AE_LIN_STAGES;
+      const u64 so = (u64)((stage * AE_LG_STAGE_BYTES) >> 4);
+      ok = mbar_wait_w(&bars->full[stage], (i / AE_LIN_STAGES) & 1, ctl, args.status, 92) &&
+           mbar_wait_w(&bars->prep[stage], (i / AE_LIN_STAGES) & 1, ctl, args.status, 93);
+      if (!ok) break;
+      tc_fence_after_sync();
+#pragma unroll
+      for (int kk = 0; kk < AE_LG_C / 16; ++kk)
+        umma_ss_w(tmem, umma_step_mn(bk_mn + so, kk), umma_step_mn(bv_mn + so, kk), idesc, (i > 0) | (kk > 0));
+      umma_commit_w(&bars->empty[stage]);
+      if (i == n_chunks - 1) umma_commit_w(&bars->done);
+    }
+    // no commit may still be on its way into the shared memory of a CTA that has retired: the last ones of the ring
+    for (int i = max(0, n_chunks - AE_LIN_STAGES); i < n_chunks && ok; ++i)
+      ok = mbar_wait_w(&bars->empty[i % AE_LIN_STAGES], (i / AE_LIN_STAGES) & 1, ctl, args.status, 94);
+  } else {
+    const u32 r = threadIdx.x;
+    const u32 lane_base = (warp * 32) << 16;
+    const i64 bh = (i64)b * args.H + h;
+    const float* a_row = args.a + bh * args.T;
+    const float asc = args.ascale ? args.ascale[h] : 1.f;
+    const bool vs16 = args.vscale_16 != 0;
+    auto step_of = [&](int i) { return chunk_at(i) * AE_LG_C + (int)r; };
+    auto load_a = [&](int i) { return i < n_chunks && step_of(i) < args.T ? a_row[step_of(i)] : 0.f; };
+    auto load_vs = [&](int i) -> u32 {  // raw bits: converting at once would wait for the load
+      if (!args.vscale || i >= n_chunks || step_of(i) >= args.T) return vs16 ? (AE_BF16 ? 0x3f80u : 0x3c00u) : 0x3f800000u;
+      const i64 si = bh * args.T + step_of(i);
+      return vs16 ? (u32)((const u16*)args.vscale)[si] : ((const u32*)args.vscale)[si];
+    };
+    float a_next = load_a(0), carry = 0.f;
+    u32 vs_next = load_vs(0);
+    bool ok = true;
+    for (int i = 0; i < n_chunks; ++i) {
+      const int stage = i % AE_LIN_STAGES;
+      float g = a_next * asc;
+      const float vsc = vs16 ? unpack_lo<AE_BF16>(vs_next) : __uint_as_float(vs_next);
+      a_next = load_a(i + 1);
+      vs_next = load_vs(i + 1);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float n = __shfl_up_sync(0xffffffffu, g, o);
+        if (lane >= (u32)o) g += n;
+      }
+      float* tot = bars->tot[i & 1];
+      if (lane == 31) tot[warp] = g;
+      named_bar_sync(1, 128);
+      float all = 0.f;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        if ((u32)w < warp) g += tot[w];
+        all += tot[w];
+      }
+      const float wgt = ae_exp(carry + (rev ? g : all - g));
+      carry += all;
+      ok = ok && mbar_wait(&bars->full[stage], (i / AE_LIN_STAGES) & 1, ctl, args.status, 95);
+      u8* vt = smem + stage * AE_LG_STAGE_BYTES + AE_LG_K_BYTES;  // row r of the tile is this thread's alone
+#pragma unroll
+      for (int ch = 0; ch < AE_LIN_DV / 8; ++ch) {
+        const u32 off = tile_off(r, ch * 8, AE_LG_C);
+        uint4 x = *(const uint4*)(vt + off);
+        u32* xw = (u32*)&x;
+        if (args.vscale) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            xw[e] = pack2<AE_BF16>(unpack_lo<AE_BF16>(xw[e]) * vsc, unpack_hi<AE_BF16>(xw[e]) * vsc);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          xw[e] = pack2<AE_BF16>(unpack_lo<AE_BF16>(xw[e]) * wgt, unpack_hi<AE_BF16>(xw[e]) * wgt);
+        *(uint4*)(vt + off) = x;
+      }
+      fence_proxy_async_smem();
+      mbar_arrive_warp(&bars->prep[stage]);
+    }
+    ok = ok && mbar_wait(&bars->done, 0, ctl, args.status, 96);
+    tc_fence_after_sync();
+    const i64 slot = bh * gridDim.z + blockIdx.z;
+    float4* out = (float4*)args.seg_state + slot * (AE_LG_DK * AE_LIN_DV / 4);  // [DV / 4][DK] of float4: lanes side by side
+#pragma unroll
+    for (int cc = 0; cc < AE_LIN_DV / 32; ++cc) {
+      float f[32];
+      tmem_ld_f32x32(tmem + lane_base + cc * 32, f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        out[(cc * 8 + e) * AE_LG_DK + r] = make_float4(f[e * 4], f[e * 4 + 1], f[e * 4 + 2], f[e * 4 + 3]);
+    }
+    if (r == 0) args.seg_decay[slot] = carry;
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 5) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, 128);
+  }
+}

@@ -26,6 +26,7 @@ KIND_ATTN_DECODE = 10
 KIND_ROWSCALE = 11
 KIND_ATTN_BWD_FUSED, KIND_ATTN_BWD_CAST = 12, 13
 KIND_ATTN_FWD_PAIR = 14
+KIND_LINEAR_SEGMENTS = 15
 DTYPE_F16, DTYPE_BF16 = 0, 1
 
 
@@ -110,7 +111,15 @@ class LinearParams(C.Structure):
     _fields_ = [("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p), ("a", C.c_void_p), ("o", C.c_void_p),
                 ("B", C.c_int32), ("H", C.c_int32), ("HQ", C.c_int32), ("HK", C.c_int32), ("T", C.c_int32),
                 ("status", C.c_void_p), ("vscale", C.c_void_p), ("dskip", C.c_void_p), ("v_out", C.c_void_p),
-                ("vscale_16bit", C.c_int32), ("h_states_out", C.c_void_p), ("ascale", C.c_void_p)]
+                ("vscale_16bit", C.c_int32), ("h_states_out", C.c_void_p), ("ascale", C.c_void_p),
+                ("seg_chunks", C.c_int32), ("seg_state", C.c_void_p), ("seg_decay", C.c_void_p)]
+
+
+class LinearSegParams(C.Structure):
+    _fields_ = [("rows", C.c_void_p), ("values", C.c_void_p), ("a", C.c_void_p), ("ascale", C.c_void_p),
+                ("vscale", C.c_void_p), ("vscale_16bit", C.c_int32), ("B", C.c_int32), ("H", C.c_int32), ("HR", C.c_int32),
+                ("T", C.c_int32), ("seg_chunks", C.c_int32), ("reverse", C.c_int32), ("seg_state", C.c_void_p),
+                ("seg_decay", C.c_void_p), ("status", C.c_void_p)]
 
 
 class LinearBwdParams(C.Structure):
@@ -119,7 +128,7 @@ class LinearBwdParams(C.Structure):
                 ("B", C.c_int32), ("H", C.c_int32), ("HQ", C.c_int32), ("HK", C.c_int32), ("T", C.c_int32),
                 ("status", C.c_void_p), ("x", C.c_void_p), ("vscale", C.c_void_p), ("dskip", C.c_void_p),
                 ("gs", C.c_void_p), ("gd", C.c_void_p), ("vscale_16bit", C.c_int32), ("ascale", C.c_void_p),
-                ("gasc", C.c_void_p)]
+                ("gasc", C.c_void_p), ("seg_chunks", C.c_int32), ("seg_state", C.c_void_p), ("seg_decay", C.c_void_p)]
 
 
 _lib = None
@@ -127,7 +136,8 @@ _lib_lock = threading.Lock()
 
 EXPORTS = ["ae_compile", "ae_module_from_cubin", "ae_module_cubin", "ae_query", "ae_release", "ae_strerror",
            "ae_last_error", "ae_launch_attn_fwd", "ae_launch_attn_bwd_prep", "ae_launch_attn_bwd_dq",
-           "ae_launch_attn_bwd_dkv", "ae_launch_attn_bwd_fused", "ae_launch_attn_bwd_dq_cast", "ae_launch_probe", "ae_launch_attn_bwd_static_scratch", "ae_launch_mla_decode", "ae_launch_mla_combine", "ae_launch_mla_decode_paged", "ae_launch_attn_decode", "ae_launch_decode_combine", "ae_launch_rowscale", "ae_launch_linear_fwd", "ae_launch_linear_states", "ae_launch_linear_bwd"]
+           "ae_launch_attn_bwd_dkv", "ae_launch_attn_bwd_fused", "ae_launch_attn_bwd_dq_cast", "ae_launch_probe", "ae_launch_attn_bwd_static_scratch", "ae_launch_mla_decode", "ae_launch_mla_combine", "ae_launch_mla_decode_paged", "ae_launch_attn_decode", "ae_launch_decode_combine", "ae_launch_rowscale", "ae_launch_linear_fwd", "ae_launch_linear_states", "ae_launch_linear_bwd",
+           "ae_launch_linear_segments"]
 
 
 def lib() -> C.CDLL:
@@ -161,6 +171,7 @@ def lib() -> C.CDLL:
             L.ae_launch_decode_combine.argtypes = [C.c_void_p, C.POINTER(DecodeParams), C.c_void_p]
             L.ae_launch_rowscale.argtypes = [C.c_void_p, C.POINTER(RowScaleParams), C.c_void_p]
             L.ae_launch_linear_fwd.argtypes = [C.c_void_p, C.POINTER(LinearParams), C.c_void_p]
+            L.ae_launch_linear_segments.argtypes = [C.c_void_p, C.POINTER(LinearSegParams), C.c_void_p]
             L.ae_launch_linear_states.argtypes = [C.c_void_p, C.POINTER(LinearBwdParams), C.c_void_p]
             L.ae_launch_linear_bwd.argtypes = [C.c_void_p, C.POINTER(LinearBwdParams), C.c_void_p]
             L.ae_launch_probe.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int,

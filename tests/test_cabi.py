@@ -31,9 +31,10 @@ def test_struct_sizes_match_header():
     import subprocess
     import tempfile
     names = ["AeKernelConfig", "AeKernelInfo", "AeAttnParams", "AeAttnBwdParams", "AeDecodeParams", "AeRowScaleParams",
-             "AeMlaParams", "AeMlaPagedParams", "AeLinearParams", "AeLinearBwdParams", "AeDecodeWorkItem"]
+             "AeMlaParams", "AeMlaPagedParams", "AeLinearParams", "AeLinearBwdParams", "AeDecodeWorkItem",
+             "AeLinearSegParams"]
     mirrors = [rt.KernelConfig, rt.KernelInfo, rt.AttnParams, rt.AttnBwdParams, rt.DecodeParams, rt.RowScaleParams,
-               rt.MlaParams, rt.MlaPagedParams, rt.LinearParams, rt.LinearBwdParams, C.c_int32 * 4]
+               rt.MlaParams, rt.MlaPagedParams, rt.LinearParams, rt.LinearBwdParams, C.c_int32 * 4, rt.LinearSegParams]
     src = '#include <stdio.h>\n#include "ae_b200.h"\nint main(){' + \
           "".join(f'printf("%zu\\n", sizeof({n}));' for n in names) + "return 0;}\n"
     with tempfile.TemporaryDirectory() as d:
