@@ -783,6 +783,8 @@ int ae_launch_mla_decode_paged(void* module, const AeMlaPagedParams* p, void* st
   a.block_table = p->block_table;
   a.seqlens = p->cache_seqlens;
   a.max_pages = p->max_pages;
+  a.lens_host = p->lens_host;
+  a.lens_call = p->lens_call;
   return launch(m, 2u * (unsigned)(p->n_split > 0 ? p->B * p->n_split : p->n_clusters), 1, 1, &a, stream);
 }
 
@@ -810,7 +812,9 @@ int ae_launch_mla_combine(void* module, const AeMlaParams* p, void* stream) {
   a.B = p->B; a.H = p->H; a.DV = 512; a.n_split = p->n_split;
   if (p->n_split == 0) a.row_info = p->row_info;
   a.lse_out = p->lse_out;
-  return launch(m, combine_blocks(p->H, 512), (unsigned)p->B, 1, &a, stream);
+  // more blocks than an SM holds at a time on every SM: four heads by a thread
+  a.heads_per_thread = p->B * p->H > 148 * 16 ? 4 : 1;
+  return launch_after(m, combine_blocks((p->H + a.heads_per_thread - 1) / a.heads_per_thread, 512), (unsigned)p->B, 1, &a, stream);
 }
 
 int ae_launch_attn_decode(void* module, const AeDecodeParams* p, void* stream) {

@@ -125,6 +125,8 @@ struct AeMlaArgs {
   const int* block_table;
   const int* seqlens;
   int max_pages;
+  int* lens_host;  // or null: pinned host memory, receives seqlens at [1 ...] and then lens_call at [0]
+  int lens_call;
 };
 struct AeMlaCombineArgs {
   void* o;
@@ -135,6 +137,7 @@ struct AeMlaCombineArgs {
                         // null = n_split slots per row.  A row with a single slot was written directly and is skipped.
   const int* row_info;  // MLA decode, or null: {first slot f, count n} per row; slot k > 0 is 2 * (f / 2 + k); n == 1: skipped
   float* lse_out;       // [B, H] or null: log-sum-exp over the splits of fr_part[0]
+  int heads_per_thread; // 1 or 4 (512 value dims only)
 };
 
 // ---- chunked linear attention / SSD scan forward (kernel ae_linear_fwd) -------------------

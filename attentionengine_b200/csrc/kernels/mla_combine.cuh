@@ -2,7 +2,7 @@
 // cute_template_kvshared/kernels/mla_combine.cu:14-152).  Lane k of every warp holds the final row scales of split k
 // (n_split <= 32; absent splits hold -inf), the traced OnlineFunc.combine runs with its reductions over the split dimension
 // as warp-shuffle reductions and leaves each lane with the weight of its split.  A thread sums four value dims over the
-// splits, AE_DV / 4 threads (at least a warp) per (batch row, head): latency-bound, so the loads of four splits are in flight
+// splits, AE_DV / 4 threads (at least a warp) per (batch row, head): latency-bound, so the loads of several splits are in flight
 // (one warp per head, one split after the other, took 11.6 us for 8 x 128 heads of 512 dims and 10 splits).
 // Expects AE_BF16, AE_NFINAL, AE_DV and ae_combine(const float* fr_of_this_lane) -> weight of this lane's split.
 
@@ -23,12 +23,81 @@ AE_DEVICE float ae_warp_sum(float x) {
 #define AE_CMB_HPB (128 / AE_CMB_TPH)                 // heads per block
 static_assert(AE_DV % 4 == 0 && AE_DV <= 512, "value head dim");
 
-extern "C" __global__ void __launch_bounds__(128) ae_mla_combine(const AeMlaCombineArgs args) {
+// HPT heads of a row by one thread: four where the blocks would otherwise come in several rounds, each a chain of four dependent
+// loads (128 rows of 128 heads, most of them in two splits).
+template <int HPT>
+AE_DEVICE void ae_combine_heads(const AeMlaCombineArgs& args, int n_split, i64 slot0, i64 slot1, i64 step) {
+  constexpr int FLY = HPT == 1 ? 8 : 4;  // splits in flight
   const int lane = threadIdx.x & 31;
-  const int h = blockIdx.x * AE_CMB_HPB + threadIdx.x / AE_CMB_TPH;
   const int b = blockIdx.y;
-  if (h >= args.H) return;  // warp-uniform
-  ae_grid_wait();  // GQA decode brings it up under the split kernel; everything read below is in place from here on
+  const int h0 = (blockIdx.x * AE_CMB_HPB + threadIdx.x / AE_CMB_TPH) * HPT;
+  if (h0 >= args.H) return;  // warp-uniform
+  const i64 my_slot = lane == 0 ? slot0 : slot1 + (lane - 1) * step;
+  float fr[HPT][AE_NFINAL > 0 ? AE_NFINAL : 1], w[HPT];
+#pragma unroll
+  for (int e = 0; e < HPT; ++e) {
+    const int h = h0 + e < args.H ? h0 + e : args.H - 1;
+#pragma unroll
+    for (int i = 0; i < AE_NFINAL; ++i) fr[e][i] = lane < n_split ? args.fr_part[i][my_slot * args.H + h] : -__int_as_float(0x7f800000);
+  }
+#pragma unroll
+  for (int e = 0; e < HPT; ++e) {
+#if AE_NFINAL > 0
+    if (args.lse_out) {
+      float m = ae_warp_max(fr[e][0]);
+      if (fabsf(m) == __int_as_float(0x7f800000)) m = 0.f;  // all -inf stays -inf, an inf stays inf
+      const float sum = ae_warp_sum(lane < n_split ? expf(fr[e][0] - m) : 0.f);
+      if (threadIdx.x % AE_CMB_TPH == 0 && h0 + e < args.H) args.lse_out[(i64)b * args.H + h0 + e] = m + logf(sum);
+    }
+#endif
+    w[e] = ae_combine(fr[e]);
+    if (lane >= n_split) w[e] = 0.f;
+  }
+  const int d0 = (threadIdx.x % AE_CMB_TPH) * 4;
+  const bool active = d0 < AE_DV;
+  const float* src = args.o_part + (i64)h0 * AE_DV + (active ? d0 : 0);
+  const i64 row = (i64)args.H * AE_DV;
+  float4 acc[HPT];
+#pragma unroll
+  for (int e = 0; e < HPT; ++e) acc[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k0 = 0; k0 < n_split; k0 += FLY) {
+    float4 v[HPT][FLY];
+#pragma unroll
+    for (int j = 0; j < FLY; ++j) {
+      const int k = k0 + j;
+      const float* from = src + (k == 0 ? slot0 : slot1 + (k - 1) * step) * row;
+#pragma unroll
+      for (int e = 0; e < HPT; ++e) {
+        v[e][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (k < n_split && h0 + e < args.H) v[e][j] = *(const float4*)(from + e * AE_DV);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < FLY; ++j) {
+#pragma unroll
+      for (int e = 0; e < HPT; ++e) {
+        const float wk = __shfl_sync(0xffffffffu, w[e], (k0 + j) & 31);
+        if (k0 + j >= n_split) continue;
+        acc[e].x += wk * v[e][j].x;
+        acc[e].y += wk * v[e][j].y;
+        acc[e].z += wk * v[e][j].z;
+        acc[e].w += wk * v[e][j].w;
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < HPT; ++e) {
+    if (!active || h0 + e >= args.H) continue;
+    uint2 o2;
+    o2.x = pack2<AE_BF16>(acc[e].x, acc[e].y);
+    o2.y = pack2<AE_BF16>(acc[e].z, acc[e].w);
+    *(uint2*)((u16*)args.o + ((i64)b * args.H + h0 + e) * AE_DV + d0) = o2;
+  }
+}
+
+extern "C" __global__ void __launch_bounds__(128) ae_mla_combine(const AeMlaCombineArgs args) {
+  const int b = blockIdx.y;
+  ae_grid_wait();  // brought up under the split kernel; everything read below is in place from here on
   int n_split = args.n_split;
   i64 slot0 = (i64)b * n_split, slot1 = slot0 + 1, step = 1;  // slots slot0, slot1, slot1 + step, ...
   if (args.part_off) {
@@ -42,48 +111,8 @@ extern "C" __global__ void __launch_bounds__(128) ae_mla_combine(const AeMlaComb
     step = 2;
   }
   if ((args.part_off || args.row_info) && n_split <= 1) return;  // written directly by the split kernel
-  float fr[AE_NFINAL > 0 ? AE_NFINAL : 1];
-  const i64 my_slot = lane == 0 ? slot0 : slot1 + (lane - 1) * step;
-#pragma unroll
-  for (int i = 0; i < AE_NFINAL; ++i) fr[i] = lane < n_split ? args.fr_part[i][my_slot * args.H + h] : -__int_as_float(0x7f800000);
-#if AE_NFINAL > 0
-  if (args.lse_out) {
-    float m = ae_warp_max(fr[0]);
-    if (fabsf(m) == __int_as_float(0x7f800000)) m = 0.f;  // all -inf stays -inf, an inf stays inf
-    const float sum = ae_warp_sum(lane < n_split ? expf(fr[0] - m) : 0.f);
-    if (threadIdx.x % AE_CMB_TPH == 0) args.lse_out[(i64)b * args.H + h] = m + logf(sum);
-  }
+#if AE_DV == 512
+  if (args.heads_per_thread == 4) return ae_combine_heads<4>(args, n_split, slot0, slot1, step);
 #endif
-  float w = ae_combine(fr);
-  if (lane >= n_split) w = 0.f;
-  const int d0 = (threadIdx.x % AE_CMB_TPH) * 4;
-  const bool active = d0 < AE_DV;
-  const float* src = args.o_part + (i64)h * AE_DV + (active ? d0 : 0);
-  const i64 row = (i64)args.H * AE_DV;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int k0 = 0; k0 < n_split; k0 += 4) {
-    float4 v[4];
-    float wk[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int k = k0 + j;
-      wk[j] = __shfl_sync(0xffffffffu, w, k & 31);
-      v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (k < n_split) v[j] = *(const float4*)(src + (k == 0 ? slot0 : slot1 + (k - 1) * step) * row);
-      else wk[j] = 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      acc.x += wk[j] * v[j].x;
-      acc.y += wk[j] * v[j].y;
-      acc.z += wk[j] * v[j].z;
-      acc.w += wk[j] * v[j].w;
-    }
-  }
-  if (active) {
-    uint2 o2;
-    o2.x = pack2<AE_BF16>(acc.x, acc.y);
-    o2.y = pack2<AE_BF16>(acc.z, acc.w);
-    *(uint2*)((u16*)args.o + ((i64)b * args.H + h) * AE_DV + d0) = o2;
-  }
+  ae_combine_heads<1>(args, n_split, slot0, slot1, step);
 }

@@ -114,9 +114,10 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
   if (warp == 0 && args.n_split == 0) {
     // this cluster's interval: total tiles, equal shares (a row spans at most 32 of them), the row and tile it begins at
     int total = 0, longest = 0;
+    const int n_mine = args.seqlens && (int)lane < args.B ? tiles_of(row_len((int)lane)) : 0;  // the first 32 rows are read once
     if (args.seqlens) {
       for (int b = (int)lane; b < args.B; b += 32) {
-        const int n = tiles_of(row_len(b));
+        const int n = b < 32 ? n_mine : tiles_of(row_len(b));
         total += n;
         longest = n > longest ? n : longest;
       }
@@ -141,7 +142,7 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
       int before = 0;
       for (int base = 0; base < args.B; base += 32) {
         const int b = base + (int)lane;
-        const int n = b < args.B ? tiles_of(row_len(b)) : 0;
+        const int n = base == 0 ? n_mine : b < args.B ? tiles_of(row_len(b)) : 0;
         int incl = n;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -175,6 +176,14 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
   __syncthreads();
   tc_fence_after_sync();
   const u32 tmem = ctl->tmem_base;
+  if (args.lens_host && blockIdx.x == 1 && warp == 5) {
+    // The row lengths for the caller, who checks them on the host: written to its pinned memory by a warp that has no other
+    // work, then the call's number, which the caller waits for.  A copy in front of the kernel held it up for 6 us.
+    for (int b = (int)lane; b < args.B; b += 32) ((volatile int*)args.lens_host)[1 + b] = args.seqlens[b];
+    __threadfence_system();
+    __syncwarp();
+    if (lane == 0) ((volatile int*)args.lens_host)[0] = args.lens_call;
+  }
   const u32 TM_O = 0, TM_S = 256;  // S region i at TM_S + 64 i
 
   // ---- the cluster's segments, the same walk in every role ----
@@ -356,6 +365,8 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
     st.xphase = 0;
     bool ok = true;
     int it = 0, pos = 0;
+    // 32 columns of this warp's rows on their way out: 4 KB of the P tile, free once P V of a segment's last tile has read it
+    u8* const stg = smem + AE_MLA_SMEM_P + warp * 4096;
     for (int n_seg = 0; next_seg(sg); ++n_seg) {
       st.init();
       for (int t = sg.t0; t < sg.t1; ++t, ++it) {
@@ -409,20 +420,24 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
           }
         });
       }
+      if (w_left <= 0) ae_grid_trigger();  // the merge may be brought up; earlier its blocks cost this kernel 2 %
       ok = mbar_wait_row(ok, &bars->pv_done, (it - 1) & 1, ctl, args.status, 49);
       tc_fence_after_sync();
       const bool store = ok && h < args.H;
-      const int hs = store ? h : 0;
       const bool whole = args.n_split > 0 ? args.n_split == 1 : (sg.t0 == 0 && sg.t1 == sg.n_t);
       const i64 slot = args.n_split > 0 ? cl : 2 * cl + (n_seg > 0);
-      // this thread's dims: 128 of each half of the value dims
+      // This thread's dims: 128 of each half of the value dims, 32 at a time.  A thread that stored its own row wrote 16 bytes
+      // of 32 lines with each instruction (8,192 L2 requests a segment, about 4 us); through the staging tile a warp writes
+      // whole lines of a few rows.
+      const bool all_ok = __all_sync(0xffffffffu, ok);
+      const int h_first = (int)(rank * 64 + (warp & 1) * 32);  // head of this warp's first row
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         float r[32];
         tmem_ld_f32x32(tm_o + c * 32, r);
         const int d0 = (c >> 2) * 256 + (int)half * 128 + (c & 3) * 32;
-        if (store && whole) {
-          uint4* dst = (uint4*)((u16*)args.o + ((i64)sg.b * args.H + hs) * AE_MLA_DV + d0);
+        __syncwarp();  // the chunk before has been read
+        if (whole) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             uint4 w;
@@ -430,16 +445,33 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
             w.y = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 2], st), ae_epilogue_o(r[v * 8 + 3], st));
             w.z = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 4], st), ae_epilogue_o(r[v * 8 + 5], st));
             w.w = pack2<AE_BF16>(ae_epilogue_o(r[v * 8 + 6], st), ae_epilogue_o(r[v * 8 + 7], st));
-            dst[v] = w;
+            *(uint4*)(stg + lane * 64 + ((v ^ ((lane >> 1) & 3)) * 16)) = w;
           }
-        } else if (store) {
-          float4* dst = (float4*)(args.o_part + (slot * args.H + hs) * AE_MLA_DV + d0);
+          __syncwarp();
+          u16* dst = (u16*)args.o + (i64)sg.b * args.H * AE_MLA_DV + d0 + (lane & 3) * 8;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {  // eight rows of 64 bytes
+            const u32 rr = i * 8 + (lane >> 2);
+            if (all_ok && h_first + (int)rr < args.H)
+              *(uint4*)(dst + (i64)(h_first + (int)rr) * AE_MLA_DV) = *(const uint4*)(stg + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) * 16));
+          }
+        } else {
 #pragma unroll
           for (int v = 0; v < 8; ++v)
-            dst[v] = make_float4(ae_epilogue_o(r[v * 4 + 0], st), ae_epilogue_o(r[v * 4 + 1], st),
-                                 ae_epilogue_o(r[v * 4 + 2], st), ae_epilogue_o(r[v * 4 + 3], st));
+            *(float4*)(stg + lane * 128 + ((v ^ (lane & 7)) * 16)) =
+                make_float4(ae_epilogue_o(r[v * 4 + 0], st), ae_epilogue_o(r[v * 4 + 1], st),
+                            ae_epilogue_o(r[v * 4 + 2], st), ae_epilogue_o(r[v * 4 + 3], st));
+          __syncwarp();
+          float* dst = args.o_part + slot * args.H * AE_MLA_DV + d0 + (lane & 7) * 4;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {  // four rows of 128 bytes
+            const u32 rr = i * 4 + (lane >> 3);
+            if (all_ok && h_first + (int)rr < args.H)
+              *(float4*)(dst + (i64)(h_first + (int)rr) * AE_MLA_DV) = *(const float4*)(stg + rr * 128 + (((lane & 7) ^ (rr & 7)) * 16));
+          }
         }
       }
+      __syncwarp();  // the next segment writes P here
       tc_fence_before_sync();  // ordered before this warp's next arrival: the next segment's P V overwrites O
 #if AE_NFINAL > 0
       if (store && half == 0) {

@@ -104,7 +104,8 @@ class MlaPagedParams(C.Structure):
                 ("rowscale_partial", C.c_void_p * AE_MAX_FINAL),
                 ("B", C.c_int32), ("H", C.c_int32), ("num_pages", C.c_int32), ("max_pages", C.c_int32),
                 ("max_seqlen", C.c_int32), ("n_split", C.c_int32), ("status", C.c_void_p), ("q_row_stride", C.c_int64),
-                ("lse_out", C.c_void_p), ("n_clusters", C.c_int32), ("row_info", C.c_void_p)]
+                ("lse_out", C.c_void_p), ("n_clusters", C.c_int32), ("row_info", C.c_void_p), ("lens_host", C.c_void_p),
+                ("lens_call", C.c_int32)]
 
 
 class LinearParams(C.Structure):

@@ -254,6 +254,10 @@ typedef struct AeMlaPagedParams {
   float* lse_out;
   int32_t n_clusters;
   int32_t* row_info;
+  /* optional: B + 1 words of pinned host memory that the device can write.  The kernel stores cache_seqlens at [1 ...] and
+   * then lens_call at [0]: the lengths as the kernel saw them, without a copy in front of it. */
+  int32_t* lens_host;
+  int32_t lens_call;
 } AeMlaPagedParams;
 
 int ae_launch_mla_decode_paged(void* module, const AeMlaPagedParams* p, void* stream);
