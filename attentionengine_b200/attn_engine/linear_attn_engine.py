@@ -160,18 +160,15 @@ class LinearAttentionEngine:
             self._plan = rt.host().ScanPlan(self._bf16)
         return self._plan
 
-    def _load_segment_kernels(self, dv: int, mods: bool, reverse: bool):
+    def _load_segment_kernels(self, dv: int, mods: bool):
         """Called by the native path before the first scan over a sequence cut into segments."""
         plan = self._plan
         # setdefault: what a thread has handed to the plan is not replaced by another thread's build
         parts = self._cut_kernels.get(dv) or self._cut_kernels.setdefault(dv, self._build_segments(dv))
         setattr(plan, f"seg{dv}", parts.handle.value)
-        key = (dv, mods, reverse)
-        scan = self._cut_kernels.get(key) or self._cut_kernels.setdefault(
-            key, self._build_bwd(mods, cut=True) if reverse else self._fwd_kernel(dv, mods, cut=True)[0])
+        scan = self._cut_kernels.get((dv, mods)) or self._cut_kernels.setdefault((dv, mods), self._fwd_kernel(dv, mods, cut=True)[0])
         # last: another thread that finds it set launches all of them
-        name = "bwd" if reverse else "fwd"
-        setattr(plan, f"{name}_mods_cut" if mods else "bwd_cut" if reverse else f"fwd_cut{dv}", scan.handle.value)
+        setattr(plan, "fwd_mods_cut" if mods else f"fwd_cut{dv}", scan.handle.value)
 
     def _build_segments(self, dv: int):
         """What the segments of a sequence add to the state, for scans of too few walks to fill the GPU."""
@@ -267,18 +264,18 @@ class LinearAttentionEngine:
             self._bwd = (states, self._build_bwd(False))
         return self._bwd
 
-    def _build_bwd(self, mods: bool, cut: bool = False):
+    def _build_bwd(self, mods: bool):
         DV = 64
         tag = rt.DTYPE_BF16 if self._bf16 else rt.DTYPE_F16
         # row warpgroups of the reverse pass (2: the second one takes half of the P / dS pass and of the output phase)
         nwg = int(os.environ.get("AE_B200_LIN_BWD_NWG", LIN_BWD_NWG))
         pre = (f"#define AE_BF16 {int(self._bf16)}\n#define AE_LIN_DV {DV}\n#define AE_LIN_STAGES 2\n"
-               f"#define AE_LB_NWG {nwg}\n#define AE_LB_MODS {int(mods)}\n" + ("#define AE_LIN_CUT 1\n" if cut else ""))
+               f"#define AE_LB_NWG {nwg}\n#define AE_LB_MODS {int(mods)}\n")
         smem_b = (2 * 128 * 128 * 2 + 2 * 128 * DV * 2 + 128 * DV * 2 + 2 * 128 * 128 * 2
                   + 128 * DV * 2 + 128 * DV * 2 + int(mods) * 128 * DV * 2 + 1024 + 256 + 512 + 1024)
         cfg = rt.KernelConfig(kind=rt.KIND_LINEAR_BWD, dtype=tag, head_dim=128, head_dim_v=DV,
                               threads=nwg * 128 + 64, smem_bytes=smem_b, stages=1, mask_mode=0)
-        cfg.reserved[0], cfg.reserved[1] = int(mods), int(cut)
+        cfg.reserved[0] = int(mods)
         return rt.compile_module(rt.kernel_source("linear_bwd.cuh", prelude=pre), "ae_linear_bwd", cfg)
 
     def _new_states(self, v):

@@ -624,24 +624,27 @@ py::object mla_paged(const std::shared_ptr<MlaPlan>& plan, const Tensor& q, cons
 struct ScanPlan : Plan {
   void *fwd_mods = nullptr;  // the forward built with the Mamba2 block's mods inside (64 value dims)
   void *bwd = nullptr, *bwd_mods = nullptr, *head_sum = nullptr;  // set when first needed
-  // what a sequence cut into segments takes, set when first needed: the contributions by value dims, and the scan kernels'
+  // what a sequence cut into segments takes, set when first needed: the contributions by value dims, and the scan kernel's
   // builds that start from them
   void *seg64 = nullptr, *seg128 = nullptr;
-  void *fwd_cut64 = nullptr, *fwd_cut128 = nullptr, *fwd_mods_cut = nullptr, *bwd_cut = nullptr, *bwd_mods_cut = nullptr;
+  void *fwd_cut64 = nullptr, *fwd_cut128 = nullptr, *fwd_mods_cut = nullptr;
   int segments = 0;  // segments a sequence is cut into; 0: as many as seg_chunks() finds
 };
 
 // Chunks per segment of a scan of `walks` (batch, head) walks over n chunks.  A walk is a chain, and a launch lasts as long as
 // the walks on the fullest SM; segments shorten the chain and fill idle SMs, at the price of a launch that computes what
 // every segment but one adds to the state (two CTAs per SM) and of summing those in front of a segment.  Microseconds as
-// measured on a B200 over 1 to 16 segments: a CTA of the scan 5 + chunk_us per chunk + 0.25 per segment, one of the
-// contributions 3 + 1.3 per chunk, 3 for the second launch.  Forward (chunk_us 2.95), one cut against the best one:
+// measured on a B200 over 1 to 16 segments: a CTA of the scan 5 + 2.95 per chunk + 0.25 per segment, one of the
+// contributions 3 + 1.3 per chunk, 3 for the second launch.  One walk against the best cut:
 // 8 walks of 64 chunks 195 -> 30 (16 segments), 48 of 56 173 -> 93 (3), 320 of 24 (more walks than SMs) 227 uncut, 231 in two.
-int seg_chunks(const ScanPlan& plan, int64_t walks, int64_t n, int device, double chunk_us) {
+// Only without gradients: a segment's start is a sum of fp32 states in another order than the walk's, and a training step's results
+// do not depend on how many heads and rows run beside, bit for bit.
+int seg_chunks(const ScanPlan& plan, int64_t walks, int64_t n, int device) {
   if (plan.segments) return (int)((n + plan.segments - 1) / plan.segments);
   int sms = 0;
   C10_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   auto rounds = [](int64_t ctas, int64_t room) { return (double)((ctas + room - 1) / room); };
+  const double chunk_us = 2.95;
   int64_t best = n;
   double least = rounds(walks, sms) * (n * chunk_us + 5);
   for (int64_t p = 2; p <= std::min<int64_t>(n, 16); ++p) {
@@ -658,17 +661,15 @@ struct Segments {
   int chunks = 0, count = 1;
   float *state = nullptr, *decay = nullptr;
   void* scan = nullptr;
-  Segments(const ScanPlan& plan, py::handle eng, bool mods, const Tensor& rows, const Tensor& values, const Tensor& a, const Tensor& asc, const Tensor& vscale,
-           bool reverse, double chunk_us, uint32_t* status) {
-    const int64_t B = values.size(0), H = values.size(1), T = values.size(2), DV = values.size(3), n = (T + 127) / 128;
+  Segments(const ScanPlan& plan, py::handle eng, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& asc, const Tensor& vscale, uint32_t* status) {
+    const int64_t B = v.size(0), H = v.size(1), T = v.size(2), DV = v.size(3), n = (T + 127) / 128;
     if (n < 2) return;
-    chunks = seg_chunks(plan, B * H, n, values.device().index(), chunk_us);
+    chunks = seg_chunks(plan, B * H, n, v.device().index());
     count = (int)((n + chunks - 1) / chunks);
     if (count == 1) return;
     void* const& kernel = DV == 64 ? plan.seg64 : plan.seg128;
-    void* const& cut = reverse ? (mods ? plan.bwd_mods_cut : plan.bwd_cut)
-                               : (mods ? plan.fwd_mods_cut : DV == 64 ? plan.fwd_cut64 : plan.fwd_cut128);
-    if (!cut) with_python([&] { eng.attr("_load_segment_kernels")((int)DV, mods, reverse); });
+    void* const& cut = vscale.defined() ? plan.fwd_mods_cut : DV == 64 ? plan.fwd_cut64 : plan.fwd_cut128;
+    if (!cut) with_python([&] { eng.attr("_load_segment_kernels")((int)DV, vscale.defined()); });
     scan = cut;
     const int64_t slots = B * H * (count - 1);
     buf = at::empty({slots * (128 * DV + 1)}, a.options());
@@ -676,14 +677,14 @@ struct Segments {
     decay = state + slots * 128 * DV;
     AeLinearSegParams p;
     memset(&p, 0, sizeof p);
-    p.rows = rows.data_ptr(); p.values = values.data_ptr(); p.a = (const float*)a.data_ptr();
+    p.k = k.data_ptr(); p.v = v.data_ptr(); p.a = (const float*)a.data_ptr();
     p.ascale = asc.defined() ? (const float*)asc.data_ptr() : nullptr;
     p.vscale = vscale.defined() ? vscale.data_ptr() : nullptr;
     p.vscale_16bit = vscale.defined() && vscale.scalar_type() != at::kFloat;
-    p.B = (int)B; p.H = (int)H; p.HR = (int)rows.size(1); p.T = (int)T;
-    p.seg_chunks = chunks; p.reverse = reverse; p.seg_state = state; p.seg_decay = decay;
+    p.B = (int)B; p.H = (int)H; p.HK = (int)k.size(1); p.T = (int)T;
+    p.seg_chunks = chunks; p.seg_state = state; p.seg_decay = decay;
     p.status = status;
-    check(ae_launch_linear_segments(kernel, &p, stream_of(values)), "ae_launch_linear_segments");
+    check(ae_launch_linear_segments(kernel, &p, stream_of(v)), "ae_launch_linear_segments");
   }
 };
 
@@ -694,7 +695,7 @@ struct ScanSaved {
 };
 
 Tensor sum_over_batch(const Tensor& t, const std::vector<int64_t>& shape, at::ScalarType dtype) {
-  // [B, H] (times segments) -> the operand's shape; a single row needs no sum
+  // [B, H] -> the operand's shape; one batch row needs no sum
   return (t.size(0) == 1 ? t : t.sum(0)).reshape(shape).to(dtype);
 }
 
@@ -750,21 +751,19 @@ struct ScanNode : Node {
     p.da = (float*)da.data_ptr();
     p.B = B; p.H = H; p.HQ = HQ; p.HK = HK; p.T = T;
     p.status = word(status);
-    const Segments seg(*plan, eng.get(), mods, q, g, a, asc, Tensor(), true, 5.6, p.status);
-    p.seg_chunks = seg.chunks; p.seg_state = seg.state; p.seg_decay = seg.decay;
     if (mods) {
       gs = at::empty_like(s);
-      gd = at::empty({B * seg.count, H}, f32);
+      gd = at::empty({B, H}, f32);
       p.x = x.data_ptr(); p.vscale = s.data_ptr(); p.dskip = (const float*)d.data_ptr();
       p.gs = gs.data_ptr(); p.gd = (float*)gd.data_ptr();
       p.vscale_16bit = s.scalar_type() != at::kFloat;
     }
     if (asc.defined()) {
-      gasc = at::empty({B * seg.count, H}, f32);
+      gasc = at::empty({B, H}, f32);
       p.ascale = (const float*)asc.data_ptr();
       p.gasc = (float*)gasc.data_ptr();
     }
-    check(ae_launch_linear_bwd(seg.scan ? seg.scan : mods ? plan->bwd_mods : plan->bwd, &p, st), "ae_launch_linear_bwd");
+    check(ae_launch_linear_bwd(mods ? plan->bwd_mods : plan->bwd, &p, st), "ae_launch_linear_bwd");
     auto head_sum = [&](const Tensor& in, int heads) {
       if (heads == H) return in;
       Tensor y = at::empty({B, heads, T, 128}, o16);
@@ -812,7 +811,7 @@ Tensor scan_launch(ScanPlan& plan, void* kernel, const Tensor& q, const Tensor& 
   p.status = word(plan.status_for(q));
   std::optional<Segments> seg;
   if (eng) {
-    seg.emplace(plan, eng, s.defined(), k, v, a, asc, s, false, 2.95, p.status);
+    seg.emplace(plan, eng, k, v, a, asc, s, p.status);
     p.seg_chunks = seg->chunks; p.seg_state = seg->state; p.seg_decay = seg->decay;
     if (seg->scan) kernel = seg->scan;
   }
@@ -844,7 +843,7 @@ Tensor scan_run(const std::shared_ptr<ScanPlan>& plan, void* kernel, py::handle 
       TORCH_CHECK(DV == 64, "the scan has gradients in value blocks of 64 dims");
       hs = at::empty({B, H, (T + 127) / 128, 128, DV}, q.options());
     }
-    y = scan_launch(*plan, kernel, q, k, v, a, s, d, asc, v_out, hs, eng);
+    y = scan_launch(*plan, kernel, q, k, v, a, s, d, asc, v_out, hs, need ? py::handle() : eng);
     status = plan->status_for(q);
   }
   if (need) {
@@ -970,7 +969,6 @@ PYBIND11_MODULE(_ae_host, m) {
       })) AE_HANDLE(ScanPlan, fwd_mods) AE_HANDLE(ScanPlan, bwd) AE_HANDLE(ScanPlan, bwd_mods)
           AE_HANDLE(ScanPlan, head_sum) AE_HANDLE(ScanPlan, seg64) AE_HANDLE(ScanPlan, seg128)
           AE_HANDLE(ScanPlan, fwd_cut64) AE_HANDLE(ScanPlan, fwd_cut128) AE_HANDLE(ScanPlan, fwd_mods_cut)
-          AE_HANDLE(ScanPlan, bwd_cut) AE_HANDLE(ScanPlan, bwd_mods_cut)
       .def_readwrite("segments", &ScanPlan::segments) AE_STATUS(ScanPlan);
   m.def("attn", torch::wrap_pybind_function(&attn));
   m.def("decode", torch::wrap_pybind_function(&decode));

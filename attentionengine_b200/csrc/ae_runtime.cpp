@@ -1051,14 +1051,14 @@ static int scan_segments(const Module* m, int T, int seg_chunks, const float* st
 }
 
 int ae_launch_linear_segments(void* module, const AeLinearSegParams* p, void* stream) {
-  if (!module || !p || !p->rows || !p->values || !p->a) return AE_ERR_INVALID;
+  if (!module || !p || !p->k || !p->v || !p->a) return AE_ERR_INVALID;
   Module* m = (Module*)module;
   if (m->cfg.kind != AE_KIND_LINEAR_SEGMENTS) {
     set_error("module kind does not match the entry point");
     return AE_ERR_UNSUPPORTED;
   }
   const int DV = m->cfg.head_dim_v;
-  if (p->B <= 0 || p->H <= 0 || p->HR <= 0 || p->T <= 0 || p->H % p->HR || m->cfg.head_dim != 128 || (DV != 64 && DV != 128)) {
+  if (p->B <= 0 || p->H <= 0 || p->HK <= 0 || p->T <= 0 || p->H % p->HK || m->cfg.head_dim != 128 || (DV != 64 && DV != 128)) {
     set_error("linear attention: need H % HQ == 0, H % HK == 0, DK = 128, DV in {64, 128}");
     return AE_ERR_INVALID;
   }
@@ -1073,11 +1073,10 @@ int ae_launch_linear_segments(void* module, const AeLinearSegParams* p, void* st
   }
   int rc = ensure_loaded(m);
   if (rc) return rc;
-  if ((rc = make_bhtd_map(&a.tm_k, p->rows, m->cfg.dtype, p->B, p->HR, p->T, 128, 128))) return rc;
-  if ((rc = make_bhtd_map(&a.tm_v, p->values, m->cfg.dtype, p->B, p->H, p->T, DV, 128))) return rc;
+  if ((rc = make_bhtd_map(&a.tm_k, p->k, m->cfg.dtype, p->B, p->HK, p->T, 128, 128))) return rc;
+  if ((rc = make_bhtd_map(&a.tm_v, p->v, m->cfg.dtype, p->B, p->H, p->T, DV, 128))) return rc;
   a.a = p->a; a.ascale = p->ascale; a.vscale = p->vscale; a.vscale_16 = p->vscale_16bit;
-  a.B = p->B; a.H = p->H; a.HK = p->HR; a.T = p->T;
-  a.reverse = p->reverse;
+  a.B = p->B; a.H = p->H; a.HK = p->HK; a.T = p->T;
   a.seg_state = p->seg_state; a.seg_decay = p->seg_decay;
   a.status = p->status;
   return launch(m, (unsigned)p->H, (unsigned)p->B, (unsigned)(n_seg - 1), &a, stream);
@@ -1223,12 +1222,7 @@ int ae_launch_linear_bwd(void* module, const AeLinearBwdParams* p, void* stream)
   AeLinearBwdArgs a;
   int rc = fill_linear_bwd(m, p, &a, AE_KIND_LINEAR_BWD);
   if (rc) return rc;
-  const int n_seg = scan_segments(m, p->T, p->seg_chunks, p->seg_state, p->seg_decay, &a.seg_chunks);
-  if (n_seg == 0) return AE_ERR_INVALID;
-  if (n_seg == 1) return launch(m, (unsigned)p->H, (unsigned)p->B, 1, &a, stream);
-  a.seg_state = p->seg_state;
-  a.seg_decay = p->seg_decay;
-  return launch_after(m, (unsigned)p->H, (unsigned)p->B, (unsigned)n_seg, &a, stream);
+  return launch(m, (unsigned)p->H, (unsigned)p->B, 1, &a, stream);
 }
 
 }  // extern "C"

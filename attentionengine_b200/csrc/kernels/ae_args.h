@@ -171,15 +171,14 @@ struct AeLinearArgs {
 
 // ---- state contributions of the segments of a scan (kernel ae_linear_segments) -------------
 struct AeLinearSegArgs {
-  AeTmaDesc tm_k;  // [B, HK, T, DK]: k, or q for the reverse pass
-  AeTmaDesc tm_v;  // [B, H, T, DV]: v, or dO for the reverse pass
+  AeTmaDesc tm_k;  // [B, HK, T, DK]
+  AeTmaDesc tm_v;  // [B, H, T, DV]
   const float* a;       // [B, H, T]
   const float* ascale;  // [H] or null
   const void* vscale;   // [B, H, T] or null: the values are tm_v's times this
   int vscale_16;
   int B, H, HK, T;
   int seg_chunks;
-  int reverse;
   float* seg_state;  // [B * H, grid z][DV / 4][128][4]
   float* seg_decay;  // [B * H, grid z]: sum of the log-decays over the segment
   u32* status;
@@ -214,10 +213,6 @@ struct AeLinearBwdArgs {
   // then the gradient of a as passed (times ascale[h]) and gasc [B, H] receives sum_t (gradient of the scaled decay) * a.
   const float* ascale;  // [H] or null
   float* gasc;          // [B, H] (required with ascale)
-  // ae_linear_bwd over segments as in AeLinearArgs (slots of the segments behind the first); gd and gasc are then [B, P, H].
-  const float* seg_state;
-  const float* seg_decay;
-  int seg_chunks;
 };
 
 // ---- row-scale mod and its backward (kernels ae_rowscale_fwd, ae_rowscale_bwd) ---------------

@@ -644,15 +644,13 @@ AE_DEVICE u64 umma_step_mn(u64 d0, int kk) { return d0 + (u64)(kk * 128); }
 // byte offset of the 16-byte chunk `ch` of row `r` inside a [rows][128 B] swizzled block
 AE_DEVICE u32 swz128(u32 r, u32 ch) { return r * 128 + ((ch ^ (r & 7)) << 4); }
 // byte offset of element column `col` (multiple of 8) of row `r` in a tile of 64-wide blocks of `rows` rows
-// Columns cc * 32 ... of row r of the state that the segments in [first, last) leave behind them, in walk order (first > last: from
-// first down to last + 1): fp32 slots [DV / 4][128] of float4, each decayed by the segments walked after it.
-AE_DEVICE void scan_segment_sum(float (&acc)[32], const float* state, const float* decay, i64 slot, int first, int last, int slot_floats,
-                                int cc, u32 r) {
+// Columns cc * 32 ... of row r of the state that the first n segments leave behind them: fp32 slots [DV / 4][128] of float4, each
+// decayed by the segments after it.
+AE_DEVICE void scan_segment_sum(float (&acc)[32], const float* state, const float* decay, i64 slot, int n, int slot_floats, int cc, u32 r) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-  const int step = first <= last ? 1 : -1;
 #pragma unroll 2
-  for (int j = first; j != last; j += step) {
+  for (int j = 0; j < n; ++j) {
     const float4* src = (const float4*)(state + (slot + j) * slot_floats) + cc * 8 * 128 + r;
     const float dec = ae_exp(decay[slot + j]);
 #pragma unroll

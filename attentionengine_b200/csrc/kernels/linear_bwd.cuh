@@ -29,13 +29,7 @@
 // the row threads keep their piece of the dO row from phase C in registers (the dO tile is refilled before the output
 // phase) and write gx = dv * s + dO * d[h] where dv went, the row sums gs = <dv, x> (dv rounded to 16 bits first, as
 // the separate kernel saw it) per step, and one sum of <dO, x> per (batch, head) for the gradient of d.
-// A sequence may be cut into segments of args.seg_chunks chunks, one CTA each (grid z), as in the forward: a CTA in front of
-// the last segment starts from the dH that the segments behind it leave, from linear_segments.cuh.  A build of its own
-// (AE_LIN_CUT).
 // Expects AE_BF16, AE_LIN_DV (64).
-#ifndef AE_LIN_CUT
-#define AE_LIN_CUT 0
-#endif
 
 #ifdef AE_TRACE  // clock stamps of CTA (0, 0)'s row warp 0 and MMA warp into the status buffer (experiments)
 #define AE_TRL(cond, region, slot) \
@@ -109,16 +103,7 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
   const int h = blockIdx.x, b = blockIdx.y;
   const int hq = h / (args.H / args.HQ);
   const int hk = h / (args.H / args.HK);
-  const int n_total = (args.T + AE_LB_C - 1) / AE_LB_C;
-#if AE_LIN_CUT
-  const int c_begin = (int)blockIdx.z * args.seg_chunks;
-  const int n_chunks = min(args.seg_chunks, n_total - c_begin);  // of this segment, walked from its last to c_begin
-  const int c_last = c_begin + n_chunks - 1;
-  const bool carried = blockIdx.z + 1 < gridDim.z;  // the walk starts from the dH of the segments behind
-#else
-  const int n_chunks = n_total, c_last = n_total - 1;
-  constexpr bool carried = false;
-#endif
+  const int n_chunks = (args.T + AE_LB_C - 1) / AE_LB_C;
 
   if (threadIdx.x == 0) {
     ctl->abort = 0;
@@ -169,7 +154,7 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
       // dO (the two that come from HBM and are not read by the row threads' output phase) at the chunk's last MMA, the
       // rest when the row threads hand the tiles back.  The output tiles of the chunk before go out in between.
       for (int it = 0; it <= n_chunks && ok; ++it) {
-        const int c = c_last - it;
+        const int c = n_chunks - 1 - it;
         if (it >= 1) {
           ok = mbar_wait(&bars->out_full, (it - 1) & 1, ctl, args.status, 82);
           if (!ok) break;
@@ -193,7 +178,7 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
         }
         if (it >= 1) {
           // the output tiles of the chunk before: ready a little before its last tiles are handed back
-          const int co = c_last + 1 - it;
+          const int co = n_chunks - it;
           ok = mbar_wait(&bars->o_ready, (it - 1) & 1, ctl, args.status, 80);
           if (!ok) break;
           // dv now (a small group of its own: its tile is rewritten early in the next chunk); dq and dk go out after
@@ -207,7 +192,7 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
           mbar_arrive_expect_tx(&bars->full_h, AE_LB_H_BYTES + AE_LB_MODS * AE_LB_V_BYTES);
           for (int dh = 0; dh < AE_LIN_DV / 64; ++dh)
             tma_load_3d(smem + AE_LB_SMEM_HC + dh * (AE_LB_DK * 128), &args.tm_h, &bars->full_h, dh * 64, 0,
-                        (b * args.H + h) * n_total + c);
+                        (b * args.H + h) * n_chunks + c);
 #if AE_LB_MODS
           // x is first read by the output phase, at the far end of the chunk: it travels with the start state, behind
           // q and k, which the chunk's first MMA waits for
@@ -216,7 +201,7 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
 #endif
         }
         if (it >= 1) {
-          const int co = c_last + 1 - it;
+          const int co = n_chunks - it;
           for (int dh = 0; dh < AE_LB_DK / 64; ++dh) {
             tma_store_4d(&args.tm_dq, smem + AE_LB_SMEM_P + dh * (AE_LB_C * 128), dh * 64, co * AE_LB_C, h, b);
             tma_store_4d(&args.tm_dk, smem + AE_LB_SMEM_DS + dh * (AE_LB_C * 128), dh * 64, co * AE_LB_C, h, b);
@@ -275,7 +260,7 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
         // dH (+)= q^T (dO o exp(g))
 #pragma unroll
         for (int kk = 0; kk < AE_LB_C / 16; ++kk)
-          umma_ss_w(tmem + TM_DH, umma_step_mn(mQ, kk), umma_step_mn(mDO2, kk), id_mnmn_dv, carried | (it > 0) | (kk > 0));
+          umma_ss_w(tmem + TM_DH, umma_step_mn(mQ, kk), umma_step_mn(mDO2, kk), id_mnmn_dv, (it > 0) | (kk > 0));
         ok = mbar_wait_w(&bars->pds_full, par, ctl, args.status, 74) && mbar_wait_w(&bars->full_h, par, ctl, args.status, 84);
         if (!ok) break;
         tc_fence_after_sync();
@@ -312,7 +297,7 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
     bool ok = true;
     // this thread's log-decay of the chunk at hand, requested one chunk ahead (the load would otherwise sit at the top
     // of every chunk's chain)
-    float a_next = (c_last * AE_LB_C + (int)r) < args.T ? a_row[c_last * AE_LB_C + (int)r] : 0.f;
+    float a_next = ((n_chunks - 1) * AE_LB_C + (int)r) < args.T ? a_row[(n_chunks - 1) * AE_LB_C + (int)r] : 0.f;
     // a decay mod of the form decay * custom[heads] (applied where the prefetched value is used): da leaves as the
     // gradient of the decay as passed, and sum_t (gradient of the scaled decay) * decay is the gradient of the scale
     const float asc = args.ascale ? args.ascale[h] : 1.f;
@@ -325,7 +310,7 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
       if (tt < 0 || tt >= args.T) return 0u;
       return vs16 ? (u32)((const u16*)args.vscale)[bh * args.T + tt] : ((const u32*)args.vscale)[bh * args.T + tt];
     };
-    u32 vs_next = load_vs(c_last * AE_LB_C + (int)r);
+    u32 vs_next = load_vs((n_chunks - 1) * AE_LB_C + (int)r);
     const float dsk = args.dskip[h];
     float acc_o = 0.f;  // this thread's share of <dO, x> over all chunks
 #endif
@@ -379,41 +364,10 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
     if (wg == 0) {
       g_nxt = cum_sum(a_next * asc, gs);
       araw_nxt = a_next;
-      a_next = n_chunks >= 2 ? a_row[(c_last - 1) * AE_LB_C + (int)r] : 0.f;  // chunks before the last one are full
+      a_next = n_chunks >= 2 ? a_row[(n_chunks - 2) * AE_LB_C + (int)r] : 0.f;  // chunks before the last one are full
     }
-#if AE_LIN_CUT
-    if (carried) {  // the dH the walk starts from: this thread's row and columns, into TMEM; its product with the state there
-      ae_grid_wait();
-      const i64 slot = bh * (gridDim.z - 1) - 1;  // the slots begin at segment 1
-      const u16* h_next = (const u16*)args.h_states + ((bh * n_total + c_last + 1) * AE_LB_DK + r) * AE_LIN_DV;
-      float hd = 0.f;
-#pragma unroll
-      for (int c2 = 0; c2 < AE_LIN_DV / 32 / AE_LB_NWG; ++c2) {
-        const int cc = (int)wg * (AE_LIN_DV / 32 / AE_LB_NWG) + c2;
-        float acc[32];
-        scan_segment_sum(acc, args.seg_state, args.seg_decay, slot, (int)gridDim.z - 1, (int)blockIdx.z, AE_LB_DK * AE_LIN_DV, cc, r);
-        u32 w[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(acc[i]);
-        tmem_st32(tmem + TM_DH + lane_base + cc * 32, w);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint4 x = *(const uint4*)(h_next + cc * 32 + i * 8);
-          const u32 xw[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-          for (int e2 = 0; e2 < 4; ++e2)
-            hd += unpack_lo<AE_BF16>(xw[e2]) * acc[i * 8 + e2 * 2] + unpack_hi<AE_BF16>(xw[e2]) * acc[i * 8 + e2 * 2 + 1];
-        }
-      }
-      tc_wait_st();
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) hd += __shfl_xor_sync(0xffffffffu, hd, o);
-      if (lane == 0) misc[16 + warp] = hd;  // the slots of odd chunks: first written again by chunk 1
-    }
-#endif
     for (int it = 0; it < n_chunks; ++it) {
-      const int c = c_last - it;
-      const bool more = it + 1 < n_chunks;
+      const int c = n_chunks - 1 - it;
       const u32 par = it & 1;
       const int t = c * AE_LB_C + (int)r;
       const bool row_ok = t < args.T;
@@ -433,10 +387,6 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
 #else
       named_bar_sync(1, 128);
 #endif
-      if (it == 0 && carried && wg == 0) {
-#pragma unroll
-        for (int w = 0; w < AE_LB_ROWW; ++w) carry += misc[16 + w];
-      }
       const float g_last = gc[AE_LB_C - 1];
       eg = ae_exp(g);
       wj = ae_exp(g_last - g);
@@ -444,7 +394,7 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
       // ---- B: dH' -> 16-bit copy, then decay dH in place ------------------------------------------
       {
         u8* dhb = smem + AE_LB_SMEM_DHB;
-        if (it > 0 || carried) {
+        if (it > 0) {
           const float dec = ae_exp(g_last);
 #pragma unroll
           for (int c2 = 0; c2 < AE_LIN_DV / 32 / AE_LB_NWG; ++c2) {
@@ -565,10 +515,10 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
       AE_TRL(warp == 0, 1, it * 16 + 8)
       if (wg == 0) {  // under the chunk's last MMAs
         if (it > 0) finish_da((it - 1) & 1);
-        if (more) {
+        if (c > 0) {
           g_nxt = cum_sum(a_next * asc, gs + (par ^ 1) * 128);
           araw_nxt = a_next;
-          a_next = it + 2 < n_chunks ? a_row[t - 2 * AE_LB_C] : 0.f;
+          a_next = c >= 2 ? a_row[t - 2 * AE_LB_C] : 0.f;
         }
       }
       AE_TRL(warp == 0, 1, it * 16 + 13)
@@ -714,7 +664,7 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
         for (int o = 16; o > 0; o >>= 1) acc_a += __shfl_xor_sync(0xffffffffu, acc_a, o);
         if (lane == 0) misc[warp & 3] = acc_a;
         named_bar_sync(1, 128);
-        if (threadIdx.x == 0) args.gasc[AE_LIN_CUT ? ((i64)b * gridDim.z + blockIdx.z) * args.H + h : bh] = misc[0] + misc[1] + misc[2] + misc[3];
+        if (threadIdx.x == 0) args.gasc[bh] = misc[0] + misc[1] + misc[2] + misc[3];
       }
     }
 #if AE_LB_MODS
@@ -727,11 +677,8 @@ extern "C" __global__ void __launch_bounds__(AE_LB_ROWW * 32 + 64, 1) ae_linear_
       float tot = 0.f;
 #pragma unroll
       for (int w = 0; w < AE_LB_ROWW; ++w) tot += misc[24 + w];
-      args.gd[AE_LIN_CUT ? ((i64)b * gridDim.z + blockIdx.z) * args.H + h : bh] = tot;
+      args.gd[bh] = tot;
     }
-#endif
-#if AE_LIN_CUT
-    if (!carried) ae_grid_wait();  // a kernel ends after the one it was brought up under
 #endif
   }
   tc_fence_before_sync();

@@ -319,7 +319,7 @@ extern "C" __global__ void __launch_bounds__(AE_LIN_ROWW * 32 + 64, 1) ae_linear
       for (int c2 = 0; c2 < AE_LIN_DV / 32 / AE_LIN_NWG; ++c2) {
         const int cc = (int)wg * (AE_LIN_DV / 32 / AE_LIN_NWG) + c2;
         float acc[32];
-        scan_segment_sum(acc, args.seg_state, args.seg_decay, slot, 0, (int)blockIdx.z, AE_LIN_DK * AE_LIN_DV, cc, r);
+        scan_segment_sum(acc, args.seg_state, args.seg_decay, slot, (int)blockIdx.z, AE_LIN_DK * AE_LIN_DV, cc, r);
         u32 w[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(acc[i]);

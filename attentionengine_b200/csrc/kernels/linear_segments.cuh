@@ -2,16 +2,15 @@
 //
 // The scan kernels walk a head's chunks one after the other, so a problem with fewer (batch, head) walks than SMs leaves the
 // rest idle for the whole walk.  Such a problem is cut into segments of whole chunks along the sequence: this kernel
-// computes what every segment adds to the state on its own, all segments at once, and the scan kernels (one CTA per
-// batch, head and segment) start from the decayed sum over the segments in front of theirs (behind it, for the reverse pass).
+// computes what every segment adds to the state on its own, all segments at once, and the scan kernel (one CTA per
+// batch, head and segment) starts from the decayed sum over the segments in front of its own.
 //
-//     forward   L = sum_t exp(sum of a over the segment's steps behind t) k_t^T v_t
-//     reverse   L = sum_t exp(sum of a over the segment's steps up to and with t) q_t^T dO_t
+//     L = sum_t exp(sum of a over the segment's steps behind t) k_t^T v_t
 //
-// Both are one accumulation without a recurrence: walked from the far end (forward: last chunk first; reverse: first
-// chunk first) the weight of a step is exp of a running sum <= 0, and the accumulator in TMEM is read once, at the end.  A chunk
-// is a load of two tiles, one pass over the V (dO) tile and eight MMAs, with nothing that waits for the chunk before;
-// what bounds it is the pass over the tile and the loads, so two CTAs share an SM.
+// is one accumulation without a recurrence: walked from the last chunk to the first the weight of a step is exp of a running
+// sum <= 0, and the accumulator in TMEM is read once, at the end.  A chunk is a load of two tiles, one pass over the V tile and
+// eight MMAs, with nothing that waits for the chunk before; what bounds it is the pass over the tile and the loads, so two CTAs
+// share an SM (1.3 us a chunk, the scan 2.95).
 // The weighted values are rounded to 16 bits as in the scan kernels; sums, decays and results are fp32.
 // Roles: warps 0-3 row threads (thread r = step r of the chunk, then state row r), warp 4 TMA producer, warp 5 MMA issuer.
 // Expects AE_BF16, AE_LIN_DV (64 or 128), AE_LIN_STAGES.
@@ -40,11 +39,10 @@ extern "C" __global__ void __launch_bounds__(192, 2) ae_linear_segments(const __
   const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.x, b = blockIdx.y;
   const int hk = h / (args.H / args.HK);
-  const bool rev = args.reverse != 0;
   const int n_total = (args.T + AE_LG_C - 1) / AE_LG_C;
-  const int c_begin = ((int)blockIdx.z + (rev ? 1 : 0)) * args.seg_chunks;  // the first (reverse: last) segment has no reader
+  const int c_begin = (int)blockIdx.z * args.seg_chunks;  // the last segment has no reader
   const int n_chunks = min(args.seg_chunks, n_total - c_begin);
-  auto chunk_at = [&](int i) { return rev ? c_begin + i : c_begin + n_chunks - 1 - i; };
+  auto chunk_at = [&](int i) { return c_begin + n_chunks - 1 - i; };
 
   ae_grid_trigger();  // the scan kernel may be brought up
   if (threadIdx.x == 0) {
@@ -139,7 +137,7 @@ extern "C" __global__ void __launch_bounds__(192, 2) ae_linear_segments(const __
         if ((u32)w < warp) g += tot[w];
         all += tot[w];
       }
-      const float wgt = ae_exp(carry + (rev ? g : all - g));
+      const float wgt = ae_exp(carry + (all - g));
       carry += all;
       ok = ok && mbar_wait(&bars->full[stage], (i / AE_LIN_STAGES) & 1, ctl, args.status, 95);
       u8* vt = smem + stage * AE_LG_STAGE_BYTES + AE_LG_K_BYTES;  // row r of the tile is this thread's alone

@@ -117,9 +117,9 @@ class LinearParams(C.Structure):
 
 
 class LinearSegParams(C.Structure):
-    _fields_ = [("rows", C.c_void_p), ("values", C.c_void_p), ("a", C.c_void_p), ("ascale", C.c_void_p),
-                ("vscale", C.c_void_p), ("vscale_16bit", C.c_int32), ("B", C.c_int32), ("H", C.c_int32), ("HR", C.c_int32),
-                ("T", C.c_int32), ("seg_chunks", C.c_int32), ("reverse", C.c_int32), ("seg_state", C.c_void_p),
+    _fields_ = [("k", C.c_void_p), ("v", C.c_void_p), ("a", C.c_void_p), ("ascale", C.c_void_p),
+                ("vscale", C.c_void_p), ("vscale_16bit", C.c_int32), ("B", C.c_int32), ("H", C.c_int32), ("HK", C.c_int32),
+                ("T", C.c_int32), ("seg_chunks", C.c_int32), ("seg_state", C.c_void_p),
                 ("seg_decay", C.c_void_p), ("status", C.c_void_p)]
 
 
@@ -129,7 +129,7 @@ class LinearBwdParams(C.Structure):
                 ("B", C.c_int32), ("H", C.c_int32), ("HQ", C.c_int32), ("HK", C.c_int32), ("T", C.c_int32),
                 ("status", C.c_void_p), ("x", C.c_void_p), ("vscale", C.c_void_p), ("dskip", C.c_void_p),
                 ("gs", C.c_void_p), ("gd", C.c_void_p), ("vscale_16bit", C.c_int32), ("ascale", C.c_void_p),
-                ("gasc", C.c_void_p), ("seg_chunks", C.c_int32), ("seg_state", C.c_void_p), ("seg_decay", C.c_void_p)]
+                ("gasc", C.c_void_p)]
 
 
 _lib = None

@@ -338,8 +338,8 @@ typedef struct AeLinearParams {
   /* Any module, optional: a decay mod of the form `decay * custom[heads]` (Mamba2's `decay_mod = dt * A`,
    * attn_script/mamba2_ngroup1.py:26-29) inside the kernel - the scan runs on a * ascale[h]. */
   const float* ascale; /* [H] */
-  /* Modules compiled with AE_LIN_CUT (config reserved[1] = 1) only: the sequence in P = ceil(ceil(T/128) / seg_chunks) > 1 segments of seg_chunks 128-step chunks, one CTA each.
-   * seg_state / seg_decay are then what `ae_launch_linear_segments` has written for the same a, ascale and seg_chunks, in
+  /* Modules compiled with AE_LIN_CUT (config reserved[1] = 1) only: the sequence in P = ceil(ceil(T/128) / seg_chunks) > 1 segments
+   * of seg_chunks 128-step chunks, one CTA each.  seg_state / seg_decay are then what `ae_launch_linear_segments` has written for the same a, ascale and seg_chunks, in
    * the launch right in front of this one on the same stream.  0: one walk over the sequence. */
   int32_t seg_chunks;
   const float* seg_state; /* fp32 [B, H, P - 1, DK * DV] */
@@ -349,18 +349,16 @@ typedef struct AeLinearParams {
 int ae_launch_linear_fwd(void* module, const AeLinearParams* p, void* stream);
 
 /* What every segment of a sequence adds to the state of the scan (module kind AE_KIND_LINEAR_SEGMENTS, kernel
- * "ae_linear_segments"), for scans with too few (batch, head) walks to fill the GPU.  reverse == 0: rows = k, values = v (times
- * vscale when given), for ae_launch_linear_fwd; reverse == 1: rows = q, values = d_o, for ae_launch_linear_bwd. */
+ * "ae_linear_segments"), for scans with too few (batch, head) walks to fill the GPU. */
 typedef struct AeLinearSegParams {
-  const void* rows;   /* [B, HR, T, DK] */
-  const void* values; /* [B, H, T, DV]  */
-  const float* a;     /* [B, H, T]      */
-  const float* ascale; /* [H] or null   */
-  const void* vscale;  /* [B, H, T] or null */
+  const void* k;   /* [B, HK, T, DK] */
+  const void* v;   /* [B, H, T, DV]  */
+  const float* a;  /* [B, H, T]      */
+  const float* ascale; /* [H] or null */
+  const void* vscale;  /* [B, H, T] or null: the scan runs on v times this */
   int32_t vscale_16bit;
-  int32_t B, H, HR, T;
+  int32_t B, H, HK, T;
   int32_t seg_chunks;
-  int32_t reverse;
   float* seg_state; /* out */
   float* seg_decay; /* out */
   uint32_t* status;
@@ -438,10 +436,6 @@ typedef struct AeLinearBwdParams {
    * (gradient of a * ascale[h]) * a - sum them over B for the gradient of ascale. */
   const float* ascale; /* [H] */
   float* gasc;         /* out [B, H] */
-  /* Segments as in AeLinearParams (ae_launch_linear_bwd only); gd and gasc are then [B, P, H]. */
-  int32_t seg_chunks;
-  const float* seg_state;
-  const float* seg_decay;
 } AeLinearBwdParams;
 
 int ae_launch_linear_states(void* module, const AeLinearBwdParams* p, void* stream);
