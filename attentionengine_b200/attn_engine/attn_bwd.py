@@ -253,6 +253,7 @@ def launch_bwd(eng, q, k, v, o, d_o, finals, custom, lists=None):
                 p.final_rowscales[j] = f[sl].data_ptr()
             if delta is not None:
                 p.delta = delta[sl].data_ptr()
+                p.dq_cleared = 1
             p.B = nb
             sp = C.c_void_p(st.cuda_stream)
             if delta is not None:
@@ -263,11 +264,13 @@ def launch_bwd(eng, q, k, v, o, d_o, finals, custom, lists=None):
                 done[i - 1].record(st)
                 main.wait_event(done[i - 1])
         return dq, dk, dv
+    if mode == "fused":  # dQ accumulator, cleared by the pre-pass, or by the launcher on the stream without one
+        acc = torch.empty(B, Sq, Hq, eng.D, dtype=torch.float32, device=dev)
+        p.dq_accum = acc.data_ptr()
+        p.dq_cleared = int(delta is not None)
     if delta is not None:
         rt.check(L.ae_launch_attn_bwd_prep(kern.prep.handle, C.byref(p), stream), "ae_launch_attn_bwd_prep")
     if mode == "fused":
-        acc = torch.empty(B, Sq, Hq, eng.D, dtype=torch.float32, device=dev)  # cleared by the launcher on the stream
-        p.dq_accum = acc.data_ptr()
         rt.check(L.ae_launch_attn_bwd_fused(kern.fused.handle, C.byref(p), stream), "ae_launch_attn_bwd_fused")
         rt.check(L.ae_launch_attn_bwd_dq_cast(kern.cast.handle, C.byref(p), stream), "ae_launch_attn_bwd_dq_cast")
     else:

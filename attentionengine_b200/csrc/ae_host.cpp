@@ -256,6 +256,7 @@ struct AttnNode : Node {
     void* st = stream_of(Q);
     if (plan->uses_doosum) {
       p.delta = p.dq_accum + acc;
+      p.dq_cleared = 1;
       check(ae_launch_attn_bwd_prep(plan->prep, &p, st), "ae_launch_attn_bwd_prep");
     }
     check(ae_launch_attn_bwd_fused(plan->fused, &p, st), "ae_launch_attn_bwd_fused");

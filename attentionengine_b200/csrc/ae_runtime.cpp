@@ -569,6 +569,14 @@ int ae_launch_attn_bwd_prep(void* module, const AeAttnBwdParams* p, void* stream
     return AE_ERR_INVALID;
   }
   a.B = p->B; a.Hq = p->Hq; a.Sq = p->Sq; a.DV = m->cfg.head_dim_v;
+  a.D = m->cfg.head_dim;
+  if (p->dq_cleared) {
+    if (!p->dq_accum || (reinterpret_cast<uintptr_t>(p->dq_accum) & 15)) {
+      set_error("dq_cleared: the pre-pass needs the 16-byte aligned dq_accum to clear");
+      return AE_ERR_INVALID;
+    }
+    a.dq_acc = p->dq_accum;
+  }
   // 16 bytes per lane, four rows per lane group and iteration; the CTAs stride over the rest
   const int64_t rows = (int64_t)p->B * p->Sq * p->Hq;
   const int64_t rows_per_cta = 8 * (32 / (m->cfg.head_dim_v / 8)) * 4;
@@ -652,6 +660,12 @@ int ae_launch_attn_bwd_fused(void* module, const AeAttnBwdParams* p, void* strea
                                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
   }
+  if (p->dq_cleared) {
+    // Brought up under the pre-pass, CTAs land where that has left room first; a grid that does not fill the GPU then shares
+    // TPCs while others stay idle (56 CTAs behind 110 blocks: a step of 152 us took 173), so it is launched behind it.
+    const bool fills = (int64_t)a.n_kt * p->Hkv * p->B >= 148;
+    return (fills ? launch_after : launch)(m, (unsigned)a.n_kt, (unsigned)p->Hkv, (unsigned)p->B, &a, stream);
+  }
   const size_t words = (size_t)p->B * p->Sq * p->Hq * m->cfg.head_dim;
   AE_CU(driver().cuMemsetD32Async((CUdeviceptr)(uintptr_t)p->dq_accum, 0u, words, (CUstream)stream));
   return launch(m, (unsigned)a.n_kt, (unsigned)p->Hkv, (unsigned)p->B, &a, stream);
@@ -678,7 +692,7 @@ int ae_launch_attn_bwd_dq_cast(void* module, const AeAttnBwdParams* p, void* str
   const int64_t vecs = (int64_t)p->B * p->Sq * p->Hq * (m->cfg.head_dim / 8);
   int64_t blocks = (vecs + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  return launch(m, (unsigned)blocks, 1, 1, &a, stream);
+  return launch_after(m, (unsigned)blocks, 1, 1, &a, stream);
 }
 
 static int make_3d_map(AeTmaDesc* out, const void* base, int dtype, int64_t cols, int64_t rows, int64_t batch,

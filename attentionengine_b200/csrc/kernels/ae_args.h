@@ -73,6 +73,8 @@ struct AeAttnBwdPrepArgs {
   i64 o_sb, o_ss, o_sh;
   i64 do_sb, do_ss, do_sh;
   int B, Hq, Sq, DV;
+  float* dq_acc;  // or null: [B, Sq, Hq, D] to clear
+  int D;
 };
 
 // dQ pass (kernel ae_attn_bwd_dq): one CTA per 128-row q tile, streams K/V tiles.

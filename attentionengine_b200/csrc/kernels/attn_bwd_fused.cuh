@@ -201,6 +201,7 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  ae_grid_wait();  // brought up under the pre-pass: delta and the cleared dQ buffer are in place from here on
   const u32 tmem = ctl->tmem_base;
   const u32 TM_DK = 0, TM_DV = AE_D, TM_S = AE_D + AE_DV, TM_DP = TM_S + AE_FU_BN;  // dQ_s aliases TM_DP
 
@@ -629,6 +630,7 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
 
     // ---- epilogue: dK / dV rows ----------------------------------------------------------
     if (s > 0) {
+      ae_grid_trigger();  // the cast may be brought up: its blocks would hold SMs from other ranges' CTAs if they came earlier
       ok = ok && mbar_wait(&bars->acc_done, 0, ctl, args.status, 37);
       tc_fence_after_sync();
     }
@@ -676,6 +678,7 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
 // dq[b, s, h, :] (16-bit, any strides) = dq_acc[b, s, h, :] (fp32, contiguous [B, Sq, Hq, D]): the conversion pass after
 // ae_attn_bwd_fused, the `flash_bwd_post` of the reference (attn_tl.py:436-455).  Eight elements per thread.
 extern "C" __global__ void __launch_bounds__(256) ae_attn_bwd_dq_cast(const __grid_constant__ AeAttnBwdArgs args) {
+  ae_grid_wait();  // brought up as the main kernel's CTAs end
   const i64 n_vec = (i64)args.B * args.Sq * args.Hq * (AE_D / 8);
   for (i64 i = (i64)blockIdx.x * 256 + threadIdx.x; i < n_vec; i += (i64)gridDim.x * 256) {
     const int dv = (int)(i % (AE_D / 8));

@@ -3,6 +3,9 @@
 // HBM-bound.  A row is shared by AE_DV / 8 lanes (16 bytes per lane and tensor); rows are taken in (batch, position,
 // head) order, the order they lie in memory, four row groups per warp and iteration so that eight 16-byte loads per lane
 // are in flight; the CTAs stride over the rows.
+// With args.dq_acc the kernel also clears the one-pass backward's fp32 dQ buffer, whose rows lie in the same order: a memset of its
+// own between this kernel and the main one cost its launch and two gaps (2 x 16 heads of 4000 positions: 15.7 us here, 11.9 us there
+// and 4 us of gaps; 21.4 us together).
 // Expects AE_DV (a multiple of 64, at most 256) and AE_BF16.
 
 #define AE_PREP_TPR (AE_DV / 8)         // lanes per row
@@ -13,6 +16,7 @@
 #endif
 
 extern "C" __global__ void __launch_bounds__(256) ae_attn_bwd_prep(const AeAttnBwdPrepArgs args) {
+  ae_grid_trigger();  // the main kernel may be brought up
   const int lane = threadIdx.x & 31;
   const i64 warp0 = ((i64)blockIdx.x * 256 + threadIdx.x) >> 5;
   const i64 n_warps = ((i64)gridDim.x * 256) >> 5;
@@ -34,6 +38,10 @@ extern "C" __global__ void __launch_bounds__(256) ae_attn_bwd_prep(const AeAttnB
         ov[u] = *(const uint4*)((const u16*)args.o + (i64)b * args.o_sb + (i64)s * args.o_ss + (i64)h * args.o_sh + col);
         dv[u] = *(const uint4*)((const u16*)args.d_o + (i64)b * args.do_sb + (i64)s * args.do_ss + (i64)h * args.do_sh + col);
         dst[u] = ((i64)b * args.Hq + h) * args.Sq + s;
+        if (args.dq_acc) {
+          float4* z = (float4*)(args.dq_acc + row * args.D);
+          for (int i = lane % AE_PREP_TPR; i < args.D / 4; i += AE_PREP_TPR) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
       }
     }
 #pragma unroll

@@ -71,7 +71,7 @@ class AttnBwdParams(C.Structure):
                 ("block_count", C.c_void_p), ("block_index", C.c_void_p),
                 ("block_count_t", C.c_void_p), ("block_index_t", C.c_void_p),
                 ("B", C.c_int32), ("Hq", C.c_int32), ("Hkv", C.c_int32), ("Sq", C.c_int32), ("Skv", C.c_int32),
-                ("status", C.c_void_p), ("dq_accum", C.c_void_p)]
+                ("status", C.c_void_p), ("dq_accum", C.c_void_p), ("dq_cleared", C.c_int32)]
 
 
 class MlaParams(C.Structure):

@@ -164,6 +164,9 @@ typedef struct AeAttnBwdParams {
   int32_t B, Hq, Hkv, Sq, Skv;
   uint32_t* status;
   float* dq_accum; /* [B, Sq, Hq, D] fp32 contiguous scratch (one-pass form only; 16-byte aligned) */
+  /* Nonzero in both calls: ae_launch_attn_bwd_prep clears dq_accum on its way, and ae_launch_attn_bwd_fused, the next launch on
+   * the stream, does not.  0: the fused launch clears it. */
+  int32_t dq_cleared;
 } AeAttnBwdParams;
 
 int ae_launch_attn_bwd_prep(void* module, const AeAttnBwdParams* p, void* stream);
