@@ -496,6 +496,34 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
       for (int j = 0; j < AE_NCS; ++j) fr[j] = e == 0 ? cv[j].x : (e == 1 ? cv[j].y : (e == 2 ? cv[j].z : cv[j].w));
     };
 
+    // Masked tiles (one or two of a walk's) run the code of all others and a pass that clears what the mask leaves out.  A second,
+    // masked instantiation of the phases was some 15 KB of instructions that each such tile had to fetch anew, 4.7 us more than an
+    // unmasked tile: window of 1024 over 4000 positions 291 us, 215 with as many unmasked steps; the whole step 428 -> 393 us.
+    u32 keep[NCH];  // bit i: this thread's element i of chunk ci is kept; set in phase A of a masked step, used in both phases
+    auto keep_bits = [&](const AeFuStep& st, int c) -> u32 {
+      // the ends of the sequences by whole words: a CTA with the last kv rows masks every step of its walk
+      const int lim = args.Sq - (st.q0 + c * 32);
+      u32 bits = !row_valid || lim <= 0 ? 0u : lim < 32 ? (1u << lim) - 1u : 0xffffffffu;
+#if AE_MASK_MODE != 0
+      if (st.partial) {
+        u32 in = 0;
+        constexpr int kUnroll = AE_MASK_MODE == 3 ? 32 : 8;  // a short loop where few tiles are masked, mode 3 masks every one
+#pragma unroll kUnroll
+        for (int i = 0; i < 32; ++i) in |= (u32)ae_mask(b, st.hq, st.q0 + c * 32 + i, kv_idx) << i;
+        bits &= in;
+      }
+#endif
+      return bits;
+    };
+    auto clear_pairs = [&](u32 (&x)[16], u32 bits) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (!(bits & (1u << (2 * i)))) x[i] &= 0xffff0000u;
+        if (!(bits & (2u << (2 * i)))) x[i] &= 0x0000ffffu;
+      }
+    };
+    auto drops = [](u32 bits) { return __any_sync(0xffffffffu, bits != 0xffffffffu); };  // some row of the warp loses an element
+
     // ---- phase A of step s: P^T from S^T, kept in registers and written over S^T as 16-bit pairs ----------
     auto phase_a_step = [&](const AeFuStep& st, int s) {
       const float* csb = cs + (s & 1) * (AE_FU_BN * AE_NCS);
@@ -506,8 +534,7 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
       ok = ok && mbar_wait(&bars->s_full, s & 1, ctl, args.status, 36);
       tc_fence_after_sync();
       AE_TRF((warp & 3) == 0, 1 + wg, s * 8 + 1)
-      auto body = [&](auto masked_tag) {
-        constexpr bool kMasked = decltype(masked_tag)::value;
+      {
 #pragma unroll
         for (int ci = 0; ci < NCH; ++ci) {
           const int c = wg + AE_FU_NWG * ci;
@@ -519,33 +546,30 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
             float4 cv[AE_NCS];
 #pragma unroll
             for (int j = 0; j < AE_NCS; ++j) cv[j] = *(const float4*)(csb + j * AE_FU_BN + c * 32 + i);
-            float p4[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const int q_idx = st.q0 + c * 32 + i + e;
               float fr[AE_NCS];
               col_scales(e, fr, cv);
-              float p = ae_bwd_p(sv[i + e], fr, b, st.hq, q_idx, kv_idx, cu, i + e);
-              if (kMasked) {
-                bool keep = row_valid & (q_idx < args.Sq);  // bitwise and selects: short-circuit forms became one branch per element
-#if AE_MASK_MODE != 0
-                keep = keep & (!st.partial | ae_mask(b, st.hq, q_idx, kv_idx));
-#endif
-                p = keep ? p : 0.f;
-              }
-              p4[e] = p;
-              pkeep[ci][i + e] = p;
+              pkeep[ci][i + e] = ae_bwd_p(sv[i + e], fr, b, st.hq, q_idx, kv_idx, cu, i + e);
 #if AE_DS_USES_S
               skeep[ci][i + e] = sv[i + e];
 #endif
             }
-            pk[(i >> 1) + 0] = pack2<AE_BF16>(p4[0], p4[1]);
-            pk[(i >> 1) + 1] = pack2<AE_BF16>(p4[2], p4[3]);
+            pk[(i >> 1) + 0] = pack2<AE_BF16>(pkeep[ci][i], pkeep[ci][i + 1]);
+            pk[(i >> 1) + 1] = pack2<AE_BF16>(pkeep[ci][i + 2], pkeep[ci][i + 3]);
+          }
+          if (masked) {
+            keep[ci] = keep_bits(st, c);
+            if (drops(keep[ci])) {
+              clear_pairs(pk, keep[ci]);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) pkeep[ci][i] = keep[ci] & (1u << i) ? pkeep[ci][i] : 0.f;
+            }
           }
           tmem_st16(tm_s + c * 32, pk);  // pairs go over this chunk's own first 16 columns
         }
-      };
-      if (masked) body(AeTrue{}); else body(AeFalse{});
+      }
       tc_wait_st();
       tc_fence_before_sync();
       named_bar_arrive(1, AE_FU_NROW + 32);
@@ -560,8 +584,7 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
       ok = ok && mbar_wait(&bars->dp_full, s & 1, ctl, args.status, 40);
       tc_fence_after_sync();
       AE_TRF((warp & 3) == 0, 1 + wg, s * 8 + 3)
-      auto body = [&](auto masked_tag) {
-        constexpr bool kMasked = decltype(masked_tag)::value;
+      {
 #pragma unroll
         for (int ci = 0; ci < NCH; ++ci) {
           const int c = wg + AE_FU_NWG * ci;
@@ -584,21 +607,12 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
 #else
               const float sraw = 0.f;
 #endif
-              bool keep = true;
-              if (kMasked) {
-                keep = row_valid & (q_idx < args.Sq);
-#if AE_MASK_MODE != 0
-                keep = keep & (!st.partial | ae_mask(b, st.hq, q_idx, kv_idx));
-#endif
-              }
-              float dsv = ae_bwd_ds(sraw, keep ? dp[i + e] : 0.f, pkeep[ci][i + e], fr, fr[AE_NFINAL], b, st.hq, q_idx,
-                                    kv_idx, cu);
-              if (kMasked) dsv = keep ? dsv : 0.f;
-              ds4[e] = dsv;
+              ds4[e] = ae_bwd_ds(sraw, dp[i + e], pkeep[ci][i + e], fr, fr[AE_NFINAL], b, st.hq, q_idx, kv_idx, cu);
             }
             dk[(i >> 1) + 0] = pack2<AE_BF16>(ds4[0], ds4[1]);
             dk[(i >> 1) + 1] = pack2<AE_BF16>(ds4[2], ds4[3]);
           }
+          if (masked && drops(keep[ci])) clear_pairs(dk, keep[ci]);
           // row `row` of the [kv][q] tile, q columns c * 32 .. c * 32 + 31: four 16-byte pieces of one 64-column block
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -606,8 +620,7 @@ ae_attn_bwd_fused(const __grid_constant__ AeAttnBwdArgs args) {
             *(uint4*)(ds_tile + tile_off(row, col, AE_FU_BM)) = make_uint4(dk[i * 4 + 0], dk[i * 4 + 1], dk[i * 4 + 2], dk[i * 4 + 3]);
           }
         }
-      };
-      if (masked) body(AeTrue{}); else body(AeFalse{});
+      }
       fence_proxy_async_smem();  // the tile is read by tcgen05.mma (async proxy)
       tc_fence_before_sync();
       named_bar_arrive(2, AE_FU_NROW + 32);
