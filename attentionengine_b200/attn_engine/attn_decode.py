@@ -21,6 +21,8 @@ positions.
 """
 from __future__ import annotations
 
+import threading
+
 import torch
 
 from .. import runtime as rt
@@ -28,6 +30,7 @@ from ..lower.cuda_lower import lower_attention, lower_combine
 
 N_SM = 148
 MAX_ROWS = 256  # two 128-row tiles per CTA
+_CUT_LOCK = threading.Lock()
 
 
 class AttnDecode:
@@ -60,6 +63,8 @@ class AttnDecode:
         self.kernel = rt.compile_module(self.src, "ae_attn_fwd", cfg)
         self.combine = None
         self.combine_src = None
+        self._cut_parts = None  # prelude, traced combine and configuration of the kernel for intervals and clusters
+        self._cut_kernel = None
         from .attn_engine import OnlineFunc
         overridden = getattr(type(online_func), "combine", None) is not OnlineFunc.combine
         # OnlineFunc.combine left at its default gives every split the weight 1: right for online functions without
@@ -67,6 +72,9 @@ class AttnDecode:
         if overridden or not self.low.final_names:
             functor = lower_combine(online_func)
             if functor is not None:
+                if nq == 1:
+                    cut_cfg = rt.KernelConfig.from_buffer_copy(bytes(cfg))
+                    self._cut_parts = (prelude, functor, cut_cfg)
                 comb = (rt.KERNEL_DIR / "mla_combine.cuh").read_text().replace("//%%AE_COMBINE_FUNCTOR%%", functor)
                 head = (rt.KERNEL_DIR / "ae_sm100.cuh").read_text().replace("#pragma once\n", "") + \
                     (rt.KERNEL_DIR / "ae_args.h").read_text()
@@ -78,32 +86,56 @@ class AttnDecode:
         self.num_split = None  # None = choose per call
         self.last_num_split = None
         self._plan = None  # the native side, made at the first call
-        self._splits = {}  # (batch rows, kv tiles) -> split count
+        self._splits = {}  # (batch rows, kv tiles) -> (split count, whether the splits merge in a cluster)
+
+    @property
+    def units(self):
+        return self.Hkv if self.Hq > self.Hkv else self.Hq
 
     def pick_splits(self, B: int, Skv: int) -> int:
-        """Split count that minimises waves x (kv tiles per split + 3): a CTA occupies an SM alone, so the CTAs run in
-        waves of 148, and each CTA pays about three tile periods to fill its pipeline and write its partials (measured
-        at B = 16: 2 splits 0.131 ms, 8 splits 0.139 ms).  No empty split; one split when the online function has row
-        state but no combine of its own."""
+        """How many splits a call of one length takes, see ``_pick``.  One when the online function has row state but no combine of
+        its own."""
+        return self._pick(B, Skv)[0]
+
+    def _pick(self, B: int, Skv: int):
+        """(splits, whether they merge in a cluster), by tile periods: a CTA occupies an SM alone, so the CTAs run in waves of 148,
+        and each pays about three periods to fill its pipeline and write its partials (measured at B = 16: 2 splits 0.131 ms,
+        8 splits 0.139 ms).  Two to four short splits, at most one wave, are a cluster and merge in it where that is at most a
+        tile period and a half behind the split that the launch of a merge follows (clusters of eight CTAs with a whole SM's
+        shared memory each do not all fit at once: 16 of them took two rounds, 17 -> 29 us).  No empty split."""
         if self.combine is None:
-            return 1
+            return 1, False
         n_tiles = -(-Skv // 128)
         known = self._splits.get((B, n_tiles))  # one look: another thread may clear the table
         if known is not None:
             return known
-        units = B * (self.Hkv if self.Hq > self.Hkv else self.Hq)
-        best, best_cost = 1, None
+        units = B * self.units
+        best, cost = (1, False), None
         for n in range(1, min(32, n_tiles) + 1):
             tps = -(-n_tiles // n)
             if (n - 1) * tps >= n_tiles:
                 continue
-            cost = -(-units * n // N_SM) * (tps + 3)
-            if best_cost is None or cost < best_cost:
-                best, best_cost = n, cost
+            c = -(-units * n // N_SM) * (tps + 3)
+            if cost is None or c < cost:
+                best, cost = (n, False), c
+        if best[0] > 1 and self._cut_parts is not None:
+            for n in range(2, min(4, n_tiles) + 1):
+                tps = -(-n_tiles // n)
+                if (n - 1) * tps < n_tiles and tps <= 8 and units * n <= 128 and tps + 3 - 1.5 < cost:
+                    best, cost = (n, True), tps + 3 - 1.5
         if len(self._splits) >= 4096:  # a serving loop over many batch sizes and lengths must not grow without bound
             self._splits.clear()
         self._splits[B, n_tiles] = best
         return best
+
+    def _load_cut_kernel(self):
+        if self._cut_kernel is None:
+            prelude, functor, cfg = self._cut_parts
+            src = rt.kernel_source("attn_decode.cuh", prelude=prelude).replace("//%%AE_COMBINE_FUNCTOR%%", functor)
+            with _CUT_LOCK:  # what a thread has handed to the plan is not replaced by another thread's build
+                if self._cut_kernel is None:
+                    self._cut_kernel = rt.compile_module(src, "ae_attn_decode", cfg)
+        self._native_plan().cut = self._cut_kernel.handle.value
 
     # ------------------------------------------------------------------------------------------------------
     # rows of different lengths
@@ -118,7 +150,7 @@ class AttnDecode:
         if lens.dim() != 1 or int(lens.min()) < 1:
             raise ValueError("cache_seqlens must be a 1-D tensor of positive lengths")
         B = lens.numel()
-        units = self.Hkv if self.Hq > self.Hkv else self.Hq
+        units = self.units
         tiles = (lens + 127) // 128
         if self.combine is None:
             g = int(tiles.max())  # no combine: one share per row
@@ -135,11 +167,16 @@ class AttnDecode:
             for sidx in range(n):
                 items.append((b, sidx, sidx * per, min(per, nt - sidx * per)))
             part_off.append(part_off[-1] + n)
+        # Long rows: the kernel cuts all rows into equal intervals itself (by its own reading of the lengths; the work list is then
+        # not used).  Every row it begins costs a CTA about two tile periods, which the shares above pay side by side: 64 rows up to
+        # 700 keys 33 us in shares, 39 in intervals; up to 8192 keys 210 and 199.
+        intervals = N_SM // units if self._cut_parts is not None and B > 1 and int(tiles.sum()) >= 16 * B else 0
         dev = device if device is not None else (cache_seqlens.device if isinstance(cache_seqlens, torch.Tensor)
                                                  and cache_seqlens.is_cuda else torch.device("cuda"))
         return {"work": torch.tensor(items, dtype=torch.int32).to(dev), "n_items": len(items),
                 "part_off": torch.tensor(part_off, dtype=torch.int32).to(dev), "n_slots": part_off[-1],
-                "seqlens": lens.to(torch.int32).to(dev), "max_seqlen": int(lens.max()), "tiles_per_share": g, "B": B}
+                "seqlens": lens.to(torch.int32).to(dev), "max_seqlen": int(lens.max()), "tiles_per_share": g, "B": B,
+                "intervals": intervals}
 
     def decode_varlen(self, q, k, v, cache_seqlens, *custom, block_table=None, metadata=None):
         """``q`` [B, q_len, Hq, D]; dense ``k`` / ``v`` [B, S_max, Hkv, D] of which row b uses its first
@@ -165,12 +202,16 @@ class AttnDecode:
 
     def _run(self, q, k, v, custom, meta, block_table):
         if meta is None:
-            n_split = self.num_split or (self.pick_splits(q.shape[0], k.shape[1]) if q.dim() == k.dim() == 4 else 1)
+            cut, n_split, in_cluster = 0, self.num_split, False
+            if not n_split:
+                n_split, in_cluster = self._pick(q.shape[0], k.shape[1]) if q.dim() == k.dim() == 4 else (1, False)
             m = None
         else:
-            n_split = 1
+            n_split, cut, in_cluster = 1, meta.get("intervals", 0), False
             m = (meta["work"], meta["n_items"], meta["seqlens"], meta["part_off"], meta["n_slots"], meta["max_seqlen"], meta["B"])
-        o = rt.host().decode(self._plan or self._native_plan(), q, k, v, custom, n_split, m, block_table)
+        if (cut or in_cluster) and (self._plan is None or not self._plan.cut):
+            self._load_cut_kernel()
+        o = rt.host().decode(self._plan or self._native_plan(), q, k, v, custom, n_split, m, block_table, cut, in_cluster)
         if o is None:
             self._refuse(q, k, v, custom, meta, block_table, n_split)
         self.last_num_split = n_split if meta is None else meta["n_slots"] / q.shape[0]

@@ -339,13 +339,14 @@ py::object attn(const std::shared_ptr<AttnPlan>& plan, py::handle eng, const Ten
 // ---------------------------------------------------------------------------------------------------- split-KV decode
 struct DecodePlan : Plan {
   void *kernel = nullptr, *combine = nullptr;
+  void* cut = nullptr;  // intervals and merges in a cluster, set when first needed
   int Hq = 0, Hkv = 0, Sq = 0, D = 0, DV = 0, n_final = 0;
   std::vector<Custom> custom;
 };
 
 // `meta`: None, or (work, n_items, seqlens, part_off, n_slots, max_seqlen, B) of a schedule; `table`: None or the block table.
 py::object decode(const std::shared_ptr<DecodePlan>& plan, const Tensor& q, const Tensor& k, const Tensor& v, py::handle custom,
-                  int n_split, py::handle meta, const std::optional<Tensor>& table) {
+                  int n_split, py::handle meta, const std::optional<Tensor>& table, int intervals, bool in_cluster) {
   const DecodePlan& P = *plan;
   if (!good4(q, P.dtype) || !good4(k, P.dtype) || !good4(v, P.dtype)) return py::none();
   const int B = (int)q.size(0), Skv = (int)k.size(1);
@@ -368,7 +369,7 @@ py::object decode(const std::shared_ptr<DecodePlan>& plan, const Tensor& q, cons
     p.seqlens = (const int32_t*)keep[1].data_ptr();
     p.part_off = (const int32_t*)keep[2].data_ptr();
     n_slots = m[4].cast<int64_t>();
-    merge = n_slots > B;
+    merge = n_slots > B || intervals;
     p.Skv = max_seqlen;
     n_split = 1;
   }
@@ -383,7 +384,19 @@ py::object decode(const std::shared_ptr<DecodePlan>& plan, const Tensor& q, cons
   } else if (k.size(0) != B) {
     return py::none();
   }
+  const int64_t units = P.Hq > P.Hkv ? P.Hkv : P.Hq, rows = P.Hq > P.Hkv ? P.Hq / P.Hkv : P.Sq;
+  if ((intervals || in_cluster) && !P.cut) return py::none();
+  if (intervals) {
+    p.n_intervals = (int)std::min<int64_t>(intervals, (int64_t)B * ((p.Skv + 127) / 128));
+    if (p.n_intervals < 1) return py::none();
+    n_slots = 2 * units * p.n_intervals;
+  }
   if (merge && !P.combine) return py::none();
+  if (in_cluster) {  // the kernel merges
+    merge = false;
+    n_slots = 0;
+    p.in_cluster = 1;
+  }
   std::vector<Tensor> C = tensors_of(custom);
   py::gil_scoped_release nogil;
   c10::cuda::CUDAGuard guard(q.device());
@@ -393,16 +406,17 @@ py::object decode(const std::shared_ptr<DecodePlan>& plan, const Tensor& q, cons
     o = at::empty({B, P.Sq, P.Hq, P.DV}, q.options());
     p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr(); p.o = o.data_ptr();
     strides3(q, p.q_stride); strides3(k, p.k_stride); strides3(v, p.v_stride);
-    if (n_slots) {  // the partial outputs and their row scales in one allocation
-      const int64_t rows = n_slots * P.Sq * P.Hq;
-      keep.push_back(at::empty({rows * (P.DV + P.n_final)}, q.options().dtype(at::kFloat)));
+    if (n_slots) {  // the partial outputs, their row scales and the table of the units' rows in one allocation
+      const int64_t n = n_slots * (intervals ? rows : P.Sq * P.Hq);
+      keep.push_back(at::empty({n * (P.DV + P.n_final) + (intervals ? 2 * B * units : 0)}, q.options().dtype(at::kFloat)));
       p.o_partial = (float*)keep.back().data_ptr();
-      for (int i = 0; i < P.n_final; ++i) p.rowscale_partial[i] = p.o_partial + rows * P.DV + rows * i;
+      for (int i = 0; i < P.n_final; ++i) p.rowscale_partial[i] = p.o_partial + n * P.DV + n * i;
+      if (intervals) p.row_info = (int32_t*)(p.o_partial + n * (P.DV + P.n_final));
     }
     p.B = B; p.Hq = P.Hq; p.Hkv = P.Hkv; p.Sq = P.Sq; p.n_split = n_split;
     p.status = word(plan->status_for(q));
     void* st = stream_of(q);
-    check(ae_launch_attn_decode(P.kernel, &p, st), "ae_launch_attn_decode");
+    check(ae_launch_attn_decode(intervals || in_cluster ? P.cut : P.kernel, &p, st), "ae_launch_attn_decode");
     if (merge) check(ae_launch_decode_combine(P.combine, &p, st), "ae_launch_decode_combine");
   }
   py::gil_scoped_acquire gil;
@@ -952,7 +966,7 @@ PYBIND11_MODULE(_ae_host, m) {
         p->Hq = Hq; p->Hkv = Hkv; p->Sq = Sq; p->D = D; p->DV = DV; p->n_final = n_final;
         p->custom = customs_from(custom);
         return p;
-      })) AE_STATUS(DecodePlan);
+      })) AE_HANDLE(DecodePlan, cut) AE_STATUS(DecodePlan);
   py::class_<MlaPlan, std::shared_ptr<MlaPlan>>(m, "MlaPlan")
       .def(py::init([](uint64_t kernel, uint64_t combine, bool bf16, int n_final, int pairs) {
         auto p = std::make_shared<MlaPlan>();

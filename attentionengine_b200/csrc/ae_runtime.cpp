@@ -230,6 +230,28 @@ int launch_after(Module* m, unsigned gx, unsigned gy, unsigned gz, void* args, v
   return AE_OK;
 }
 
+// Launch in clusters of cx CTAs along x.
+int launch_cluster(Module* m, unsigned gx, unsigned gy, unsigned gz, unsigned cx, void* args, void* stream) {
+  Driver& d = driver();
+  void* params[] = {args};
+  CUlaunchAttribute attr;
+  memset(&attr, 0, sizeof attr);
+  attr.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+  attr.value.clusterDim.x = cx;
+  attr.value.clusterDim.y = 1;
+  attr.value.clusterDim.z = 1;
+  CUlaunchConfig cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDimX = gx; cfg.gridDimY = gy; cfg.gridDimZ = gz;
+  cfg.blockDimX = (unsigned)m->cfg.threads; cfg.blockDimY = 1; cfg.blockDimZ = 1;
+  cfg.sharedMemBytes = (unsigned)m->cfg.smem_bytes;
+  cfg.hStream = (CUstream)stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  AE_CU(d.cuLaunchKernelEx(&cfg, g_fn, params, nullptr));
+  return AE_OK;
+}
+
 // Tensor map over a [B, S, H, D] tensor (element strides sb, ss, sh; d contiguous) seen as
 // (d, h, s, b) with a box of {64, 1, rows, 1} and 128-byte swizzle: one box is a `rows` x 128 B
 // tile in the K-major (for Q/K) or MN-major (for V) layout the UMMA descriptors expect.
@@ -661,8 +683,8 @@ int ae_launch_attn_bwd_fused(void* module, const AeAttnBwdParams* p, void* strea
                                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
   }
   if (p->dq_cleared) {
-    // Brought up under the pre-pass, CTAs land where that has left room first; a grid that does not fill the GPU then shares
-    // TPCs while others stay idle (56 CTAs behind 110 blocks: a step of 152 us took 173), so it is launched behind it.
+    // Brought up under the pre-pass, CTAs land where that has left room first: a grid that does not fill the GPU would crowd there
+    // while other SMs stay idle, so it is launched behind it.
     const bool fills = (int64_t)a.n_kt * p->Hkv * p->B >= 148;
     return (fills ? launch_after : launch)(m, (unsigned)a.n_kt, (unsigned)p->Hkv, (unsigned)p->B, &a, stream);
   }
@@ -848,9 +870,22 @@ int ae_launch_attn_decode(void* module, const AeDecodeParams* p, void* stream) {
     return AE_ERR_UNSUPPORTED;
   }
   if (m->cfg.mask_mode != 0 && m->cfg.mask_mode != 3) return AE_ERR_UNSUPPORTED;
-  const bool varlen = p->work != nullptr;
+  const bool varlen = p->work != nullptr, cut = p->n_intervals > 0;
+  if ((cut || p->in_cluster) != (m->kernel == "ae_attn_decode") || (cut && p->in_cluster) || ((cut || p->in_cluster) && rows > 128)) {
+    set_error("intervals and merges in a cluster are the module kernel ae_attn_decode's, with at most 128 rows per unit");
+    return AE_ERR_INVALID;
+  }
   int tps = 0;
-  if (varlen) {
+  if (cut) {
+    if (p->n_intervals > 4096 || !p->o_partial || !p->row_info) {
+      set_error("intervals need the partial buffers and row_info");
+      return AE_ERR_INVALID;
+    }
+  } else if (varlen) {
+    if (p->in_cluster) {
+      set_error("a merge in a cluster takes rows of one length");
+      return AE_ERR_INVALID;
+    }
     if (!p->seqlens || !p->part_off || p->n_items <= 0 || !p->o_partial) {
       set_error("a work list needs seqlens, part_off, n_items > 0 and the partial buffers");
       return AE_ERR_INVALID;
@@ -862,9 +897,13 @@ int ae_launch_attn_decode(void* module, const AeDecodeParams* p, void* stream) {
       set_error("n_split leaves a split without kv tiles");
       return AE_ERR_INVALID;
     }
-    if (p->n_split > 1 && !p->o_partial) return AE_ERR_INVALID;
+    if (p->n_split > 1 && !p->o_partial && !p->in_cluster) return AE_ERR_INVALID;
+    if (p->in_cluster && (p->n_split < 2 || p->n_split > 8)) {
+      set_error("a merge in a cluster takes 2 to 8 splits");
+      return AE_ERR_INVALID;
+    }
   }
-  if (varlen || p->n_split > 1)
+  if (cut || varlen || (p->n_split > 1 && !p->in_cluster))
     for (int i = 0; i < m->cfg.reserved[1] && i < AE_MAX_FINAL; ++i)
       if (!p->rowscale_partial[i]) return AE_ERR_INVALID;
   if (p->block_table && (p->max_pages <= 0 || p->num_pages <= 0)) {
@@ -933,7 +972,15 @@ int ae_launch_attn_decode(void* module, const AeDecodeParams* p, void* stream) {
   args.block_table = p->block_table;
   args.max_pages = p->max_pages;
   const unsigned units = (unsigned)(gq > 1 ? p->Hkv : p->Hq);
+  args.units = (int)units;
+  args.n_intervals = p->n_intervals;
+  args.row_info = p->row_info;
+  if (cut) return launch(m, units, (unsigned)p->n_intervals, 1, &args, stream);
   if (varlen) return launch(m, (unsigned)p->n_items, units, 1, &args, stream);
+  if (p->in_cluster) {
+    args.in_cluster = 1;
+    return launch_cluster(m, (unsigned)p->n_split, units, (unsigned)p->B, (unsigned)p->n_split, &args, stream);
+  }
   return launch(m, (unsigned)p->n_split, units, (unsigned)p->B, &args, stream);
 }
 
@@ -944,7 +991,8 @@ int ae_launch_decode_combine(void* module, const AeDecodeParams* p, void* stream
     set_error("module kind does not match the entry point");
     return AE_ERR_UNSUPPORTED;
   }
-  if ((!p->part_off && (p->n_split < 2 || p->n_split > 32)) || m->cfg.head_dim_v % 4) return AE_ERR_INVALID;
+  if (p->n_intervals > 0 ? !p->row_info : !p->part_off && (p->n_split < 2 || p->n_split > 32)) return AE_ERR_INVALID;
+  if (m->cfg.head_dim_v % 4) return AE_ERR_INVALID;
   int rc = ensure_loaded(m);
   if (rc) return rc;
   AeMlaCombineArgs a;
@@ -956,7 +1004,15 @@ int ae_launch_decode_combine(void* module, const AeDecodeParams* p, void* stream
   a.H = p->Sq * p->Hq;  // one output row per (query position, head)
   a.DV = m->cfg.head_dim_v;
   a.n_split = p->n_split;
-  a.part_off = p->part_off;  // rows of different lengths: each row's own number of partial slots
+  if (p->n_intervals > 0) {
+    const bool grouped = p->Hq > p->Hkv;
+    a.row_info = p->row_info;
+    a.gq = grouped ? p->Hq / p->Hkv : 1;
+    a.units = grouped ? p->Hkv : p->Hq;
+    a.unit_rows = grouped ? a.gq : p->Sq;
+  } else {
+    a.part_off = p->part_off;  // rows of different lengths: each row's own number of partial slots
+  }
   return launch_after(m, combine_blocks(a.H, a.DV), (unsigned)p->B, 1, &a, stream);
 }
 

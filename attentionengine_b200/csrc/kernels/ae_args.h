@@ -62,6 +62,12 @@ struct AeAttnFwdArgs {
   const int* part_off;     // [B + 1] first partial-result slot of each row (its splits are consecutive slots)
   const int* block_table;  // [B, max_pages] page of each 128-key tile of a row; K / V are then pools [pages * 128, Hkv, D]
   int max_pages;
+  // ae_attn_decode (attn_decode.cuh) only: head units of a row; the tiles of all rows in equal intervals for each unit (> 0), with
+  // partials [units, 2 * n_intervals, rows, DV], fr_part [units, 2 * n_intervals, rows] and row_info [B * units][2] for the merge
+  int units;
+  int n_intervals;
+  int* row_info;
+  int in_cluster;  // the n_split (2 ... 8) CTAs of a unit are a cluster and merge their partials in it
 };
 
 // ---- attention backward ------------------------------------------------------------
@@ -137,7 +143,10 @@ struct AeMlaCombineArgs {
   int B, H, DV, n_split;
   const int* part_off;  // [B + 1] or null: row b owns the partial slots part_off[b] .. part_off[b + 1] - 1 (at most 32);
                         // null = n_split slots per row.  A row with a single slot was written directly and is skipped.
-  const int* row_info;  // MLA decode, or null: {first slot f, count n} per row; slot k > 0 is 2 * (f / 2 + k); n == 1: skipped
+  const int* row_info;  // intervals, or null: {first slot f, count n} per row (and unit); slot k > 0 is 2 * (f / 2 + k); n == 1: skipped
+  int units, unit_rows; // GQA decode in intervals: output row x of a batch row is row x / units of unit x % units (one row per
+                        // head and position), or with gq > 1 row x % gq of unit x / gq; 0 units: row_info is per batch row
+  int gq;
   float* lse_out;       // [B, H] or null: log-sum-exp over the splits of fr_part[0]
   int heads_per_thread; // 1 or 4 (512 value dims only)
 };

@@ -26,19 +26,17 @@ static_assert(AE_DV % 4 == 0 && AE_DV <= 512, "value head dim");
 // HPT heads of a row by one thread: four where the blocks would otherwise come in several rounds, each a chain of four dependent
 // loads (128 rows of 128 heads, most of them in two splits).
 template <int HPT>
-AE_DEVICE void ae_combine_heads(const AeMlaCombineArgs& args, int n_split, i64 slot0, i64 slot1, i64 step) {
+AE_DEVICE void ae_combine_heads(const AeMlaCombineArgs& args, int h0, int n_split, i64 slot0, i64 slot1, i64 step, int in_slot, int per_slot) {
   constexpr int FLY = HPT == 1 ? 8 : 4;  // splits in flight
   const int lane = threadIdx.x & 31;
   const int b = blockIdx.y;
-  const int h0 = (blockIdx.x * AE_CMB_HPB + threadIdx.x / AE_CMB_TPH) * HPT;
-  if (h0 >= args.H) return;  // warp-uniform
   const i64 my_slot = lane == 0 ? slot0 : slot1 + (lane - 1) * step;
   float fr[HPT][AE_NFINAL > 0 ? AE_NFINAL : 1], w[HPT];
 #pragma unroll
   for (int e = 0; e < HPT; ++e) {
-    const int h = h0 + e < args.H ? h0 + e : args.H - 1;
+    const int x = h0 + e < args.H ? in_slot + e : in_slot;
 #pragma unroll
-    for (int i = 0; i < AE_NFINAL; ++i) fr[e][i] = lane < n_split ? args.fr_part[i][my_slot * args.H + h] : -__int_as_float(0x7f800000);
+    for (int i = 0; i < AE_NFINAL; ++i) fr[e][i] = lane < n_split ? args.fr_part[i][my_slot * per_slot + x] : -__int_as_float(0x7f800000);
   }
 #pragma unroll
   for (int e = 0; e < HPT; ++e) {
@@ -55,8 +53,8 @@ AE_DEVICE void ae_combine_heads(const AeMlaCombineArgs& args, int n_split, i64 s
   }
   const int d0 = (threadIdx.x % AE_CMB_TPH) * 4;
   const bool active = d0 < AE_DV;
-  const float* src = args.o_part + (i64)h0 * AE_DV + (active ? d0 : 0);
-  const i64 row = (i64)args.H * AE_DV;
+  const float* src = args.o_part + (i64)in_slot * AE_DV + (active ? d0 : 0);
+  const i64 row = (i64)per_slot * AE_DV;
   float4 acc[HPT];
 #pragma unroll
   for (int e = 0; e < HPT; ++e) acc[e] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -77,7 +75,7 @@ AE_DEVICE void ae_combine_heads(const AeMlaCombineArgs& args, int n_split, i64 s
 #pragma unroll
       for (int e = 0; e < HPT; ++e) {
         const float wk = __shfl_sync(0xffffffffu, w[e], (k0 + j) & 31);
-        if (k0 + j >= n_split) continue;
+        if (k0 + j >= n_split || wk == 0.f) continue;  // a split without a kept key weighs nothing, whatever it holds
         acc[e].x += wk * v[e][j].x;
         acc[e].y += wk * v[e][j].y;
         acc[e].z += wk * v[e][j].z;
@@ -97,22 +95,36 @@ AE_DEVICE void ae_combine_heads(const AeMlaCombineArgs& args, int n_split, i64 s
 
 extern "C" __global__ void __launch_bounds__(128) ae_mla_combine(const AeMlaCombineArgs args) {
   const int b = blockIdx.y;
+#if AE_DV == 512
+  const int hpt = args.heads_per_thread;
+#else
+  const int hpt = 1;
+#endif
+  const int h0 = (int)(blockIdx.x * AE_CMB_HPB + threadIdx.x / AE_CMB_TPH) * hpt;
   ae_grid_wait();  // brought up under the split kernel; everything read below is in place from here on
-  int n_split = args.n_split;
+  if (h0 >= args.H) return;  // warp-uniform
+  int n_split = args.n_split, in_slot = h0, per_slot = args.H;
   i64 slot0 = (i64)b * n_split, slot1 = slot0 + 1, step = 1;  // slots slot0, slot1, slot1 + step, ...
   if (args.part_off) {
     slot0 = args.part_off[b];
     slot1 = slot0 + 1;
     n_split = args.part_off[b + 1] - args.part_off[b];
   } else if (args.row_info) {
-    slot0 = args.row_info[2 * b];
-    n_split = args.row_info[2 * b + 1];
+    i64 at = b;
+    if (args.units) {
+      const int unit = args.gq > 1 ? h0 / args.gq : h0 % args.units;
+      in_slot = args.gq > 1 ? h0 % args.gq : h0 / args.units;
+      per_slot = args.unit_rows;
+      at = (i64)b * args.units + unit;
+    }
+    slot0 = args.row_info[2 * at];
+    n_split = args.row_info[2 * at + 1];
     slot1 = 2 * (slot0 / 2 + 1);
     step = 2;
   }
   if ((args.part_off || args.row_info) && n_split <= 1) return;  // written directly by the split kernel
 #if AE_DV == 512
-  if (args.heads_per_thread == 4) return ae_combine_heads<4>(args, n_split, slot0, slot1, step);
+  if (hpt == 4) return ae_combine_heads<4>(args, h0, n_split, slot0, slot1, step, in_slot, per_slot);
 #endif
-  ae_combine_heads<1>(args, n_split, slot0, slot1, step);
+  ae_combine_heads<1>(args, h0, n_split, slot0, slot1, step, in_slot, per_slot);
 }

@@ -89,7 +89,8 @@ class DecodeParams(C.Structure):
                 ("B", C.c_int32), ("Hq", C.c_int32), ("Hkv", C.c_int32), ("Sq", C.c_int32), ("Skv", C.c_int32),
                 ("n_split", C.c_int32), ("status", C.c_void_p),
                 ("work", C.c_void_p), ("n_items", C.c_int32), ("seqlens", C.c_void_p), ("part_off", C.c_void_p),
-                ("block_table", C.c_void_p), ("max_pages", C.c_int32), ("num_pages", C.c_int32)]
+                ("block_table", C.c_void_p), ("max_pages", C.c_int32), ("num_pages", C.c_int32), ("n_intervals", C.c_int32),
+                ("row_info", C.c_void_p), ("in_cluster", C.c_int32)]
 
 
 class RowScaleParams(C.Structure):

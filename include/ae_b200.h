@@ -307,6 +307,16 @@ typedef struct AeDecodeParams {
   const int32_t* part_off;    /* [B + 1]; o_partial / rowscale_partial then hold part_off[B] slots */
   const int32_t* block_table; /* [B, max_pages] */
   int32_t max_pages, num_pages;
+  /* n_intervals > 0 (module kernel "ae_attn_decode" of attn_decode.cuh, at most 128 rows per unit; the work list is not read): for
+   * every head unit the 128-key tiles of all rows in one line, cut into n_intervals equal intervals, one CTA each.  The kernel cuts
+   * by `seqlens` (or Skv) itself.  With U head units of R rows, o_partial is [U, 2 * n_intervals, R, DV], rowscale_partial
+   * [U, 2 * n_intervals, R], and row_info [B * U][2] tells the combine launch which slots are a unit's row (a row inside one
+   * interval is written directly). */
+  int32_t n_intervals;
+  int32_t* row_info;
+  /* Nonzero (the same module, rows of one length, 2 <= n_split <= 8): the splits of a unit run as one cluster and merge in it;
+   * no partial buffers and no combine launch. */
+  int32_t in_cluster;
 } AeDecodeParams;
 
 int ae_launch_attn_decode(void* module, const AeDecodeParams* p, void* stream);
