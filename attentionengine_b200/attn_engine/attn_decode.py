@@ -167,8 +167,8 @@ class AttnDecode:
             for sidx in range(n):
                 items.append((b, sidx, sidx * per, min(per, nt - sidx * per)))
             part_off.append(part_off[-1] + n)
-        # Long rows: the kernel cuts all rows into equal intervals itself (by its own reading of the lengths; the work list is then
-        # not used).  Every row it begins costs a CTA about two tile periods, which the shares above pay side by side: 64 rows up to
+        # Long rows: the kernel cuts all rows into equal intervals itself, by its own reading of the lengths; the work list then serves
+        # another engine that the schedule is handed to (see _run).  Every row it begins costs a CTA about two tile periods, which the shares above pay side by side: 64 rows up to
         # 700 keys 33 us in shares, 39 in intervals; up to 8192 keys 210 and 199.
         intervals = N_SM // units if self._cut_parts is not None and B > 1 and int(tiles.sum()) >= 16 * B else 0
         dev = device if device is not None else (cache_seqlens.device if isinstance(cache_seqlens, torch.Tensor)
@@ -176,7 +176,7 @@ class AttnDecode:
         return {"work": torch.tensor(items, dtype=torch.int32).to(dev), "n_items": len(items),
                 "part_off": torch.tensor(part_off, dtype=torch.int32).to(dev), "n_slots": part_off[-1],
                 "seqlens": lens.to(torch.int32).to(dev), "max_seqlen": int(lens.max()), "tiles_per_share": g, "B": B,
-                "intervals": intervals}
+                "intervals": intervals, "units": units}
 
     def decode_varlen(self, q, k, v, cache_seqlens, *custom, block_table=None, metadata=None):
         """``q`` [B, q_len, Hq, D]; dense ``k`` / ``v`` [B, S_max, Hkv, D] of which row b uses its first
@@ -207,7 +207,9 @@ class AttnDecode:
                 n_split, in_cluster = self._pick(q.shape[0], k.shape[1]) if q.dim() == k.dim() == 4 else (1, False)
             m = None
         else:
-            n_split, cut, in_cluster = 1, meta.get("intervals", 0), False
+            # the work list serves any engine, intervals only one with the head units they were counted for and the kernel for them
+            cut = meta.get("intervals", 0) if self._cut_parts is not None and meta.get("units") == self.units else 0
+            n_split, in_cluster = 1, False
             m = (meta["work"], meta["n_items"], meta["seqlens"], meta["part_off"], meta["n_slots"], meta["max_seqlen"], meta["B"])
         if (cut or in_cluster) and (self._plan is None or not self._plan.cut):
             self._load_cut_kernel()
