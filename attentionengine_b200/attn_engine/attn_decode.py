@@ -14,7 +14,8 @@ GPU once.
 Rows of different lengths and paged K / V (the serving call of the reference's kv-shared path,
 core/template/cute_template_kvshared/flash_mla_interface.py:73-113 with its scheduler
 kernels/get_mla_metadata.cu:8-75) are ``decode_varlen``: ``schedule(cache_seqlens)`` cuts every row into shares of
-about equal size, one CTA each, and the result is reused by every layer of a decode step.
+about equal size, one CTA each, or for each head unit the line of all rows' tiles into equal intervals (attn_decode.cuh), and the
+result is reused by every layer of a decode step.
 A ``mask_mod`` is applied element by element (mask mode 3), the dense mask input of the reference's TL decode
 (core/lower/lower_decode_gqa.py:390-396); the query position it sees is the row's index among the engine's q_len
 positions.
@@ -143,7 +144,8 @@ class AttnDecode:
     def schedule(self, cache_seqlens, device=None, waves: int = 1):
         """Work list for a batch whose rows hold ``cache_seqlens[b]`` keys: every row is cut into shares of at most
         ``g`` 128-key tiles, ``g`` chosen so that the shares of all rows and head units fill the GPU ``waves`` times
-        (at least 2 tiles per share, at most 32 shares per row).  Returns a dict of device tensors that
+        (at least 2 tiles per share, at most 32 shares per row); or, for long rows, the number of equal intervals that all
+        rows' tiles are cut into for each head unit (``_pick_intervals``).  Returns a dict of device tensors that
         ``decode_varlen`` takes; compute it once per decode step and reuse it for every layer (the reference's
         ``get_mla_metadata`` is used the same way).  Reads the lengths on the host (one small copy)."""
         lens = torch.as_tensor(cache_seqlens).to("cpu", torch.int64)
@@ -167,16 +169,34 @@ class AttnDecode:
             for sidx in range(n):
                 items.append((b, sidx, sidx * per, min(per, nt - sidx * per)))
             part_off.append(part_off[-1] + n)
-        # Long rows: the kernel cuts all rows into equal intervals itself, by its own reading of the lengths; the work list then serves
-        # another engine that the schedule is handed to (see _run).  Every row it begins costs a CTA about two tile periods, which the shares above pay side by side: 64 rows up to
-        # 700 keys 33 us in shares, 39 in intervals; up to 8192 keys 210 and 199.
-        intervals = N_SM // units if self._cut_parts is not None and B > 1 and int(tiles.sum()) >= 16 * B else 0
+        # Waves asked for by the caller are shares' alone.  The work list is made in any case: an engine with other head units that is
+        # handed the schedule takes it (see _run).
+        intervals = self._pick_intervals(B, tiles, items) if waves == 1 else 0
         dev = device if device is not None else (cache_seqlens.device if isinstance(cache_seqlens, torch.Tensor)
                                                  and cache_seqlens.is_cuda else torch.device("cuda"))
         return {"work": torch.tensor(items, dtype=torch.int32).to(dev), "n_items": len(items),
                 "part_off": torch.tensor(part_off, dtype=torch.int32).to(dev), "n_slots": part_off[-1],
                 "seqlens": lens.to(torch.int32).to(dev), "max_seqlen": int(lens.max()), "tiles_per_share": g, "B": B,
                 "intervals": intervals, "units": units}
+
+    def _pick_intervals(self, B, tiles, items) -> int:
+        """Intervals per head unit for long rows (the kernel cuts all rows' tiles into them by its own reading of the lengths), or 0
+        where the shares ``items`` are expected to be faster.  Microseconds, as measured over 1 to 128 units, 2 to 64 rows, even,
+        uniform and skewed lengths, dense and paged: a tile takes a CTA 1.3 (in shares 1.15 at 64 dims) and all CTAs together 0.0101 of
+        HBM; a share costs three tiles more than it holds, an interval 2 us for every row that it begins.  Intervals are one
+        wave of N_SM // units CTAs a unit, so they leave SMs idle where the units do not divide N_SM.  In shares / in intervals:
+        64 rows up to 8192 keys over 8 units (144 CTAs) 216 / 189; 16 rows of 4096 over 80 units (80 CTAs) 436 / 659; 64 of 4096 over 32
+        units (128 CTAs) 670 / 704; 4 rows up to 8192 over 1 unit 17 / 21; 6 rows of 16384 over 48 units of 64 dims 277 / 329."""
+        n, total, units = N_SM // self.units, int(tiles.sum()), self.units
+        if self._cut_parts is None or n == 0 or B == 1 or total < 16 * B:
+            return 0
+        size = (self.D + self.DV) / 256
+        together = 0.0101 * size * total * units
+        longest = max(x[3] for x in items) + 3
+        in_turn = min(-(-units * len(items) // N_SM) * longest, units * (total + 3 * len(items)) / N_SM + 0.7 * longest)
+        shares = 10 + max(together, (1 + 0.3 * size) * in_turn)
+        per_cta = max(-(-total // n), -(-int(tiles.max()) // 31))
+        return n if 16 + max(together, 1.3 * per_cta + 2 * (1 - (-B // n))) < shares else 0
 
     def decode_varlen(self, q, k, v, cache_seqlens, *custom, block_table=None, metadata=None):
         """``q`` [B, q_len, Hq, D]; dense ``k`` / ``v`` [B, S_max, Hkv, D] of which row b uses its first
@@ -216,7 +236,10 @@ class AttnDecode:
         o = rt.host().decode(self._plan or self._native_plan(), q, k, v, custom, n_split, m, block_table, cut, in_cluster)
         if o is None:
             self._refuse(q, k, v, custom, meta, block_table, n_split)
-        self.last_num_split = n_split if meta is None else meta["n_slots"] / q.shape[0]
+        if meta is None:
+            self.last_num_split = n_split
+        else:  # pieces of a row on average; every end of an interval but the last counted as a cut
+            self.last_num_split = (meta["B"] + cut - 1 if cut else meta["n_slots"]) / meta["B"]
         return o
 
     def _refuse(self, q, k, v, custom, meta, block_table, n_split):

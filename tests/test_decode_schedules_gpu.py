@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
     (1, 8, 2),
 ])
 def test_schedule_of_another_engine(Sq, Hq, Hkv):
-    lens, D, dtype = [4000, 130, 2500, 3000], 128, torch.float16
+    lens, D, dtype = [8192, 130, 5000, 7000], 128, torch.float16
     B, S = len(lens), max(lens)
     meta = helpers.decode_engine(B, 32, 8, 1, S, D, dtype).decode_schedule(torch.tensor(lens), device="cuda")
     assert meta["intervals"] > 0
@@ -32,3 +32,17 @@ def test_schedule_of_another_engine(Sq, Hq, Hkv):
     keep = torch.arange(S, device="cuda")[None, :] < lengths[:, None]
     ref = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s.masked_fill(~keep[:, None, None], float("-inf")), -1), vf)
     parity.check("o", o, ref, dtype, stages=2)  # P and the stored O
+
+
+def test_waves_are_honoured_and_the_count_is_of_the_path_taken():
+    lens, D, dtype = [8192, 130, 5000, 7000], 128, torch.float16
+    B, S = len(lens), max(lens)
+    eng = helpers.decode_engine(B, 32, 8, 1, S, D, dtype)
+    q, k, v = (torch.randn(B, n, h, D, device="cuda", dtype=dtype) for n, h in ((1, 32), (S, 8), (S, 8)))
+    lengths = torch.tensor(lens, device="cuda")
+    cut, twice = eng.decode_schedule(lengths), eng._decode.schedule(lengths, waves=2)
+    assert cut["intervals"] == 18 and twice["intervals"] == 0 and twice["n_slots"] > cut["n_slots"]
+    eng.decode_varlen(q, k, v, lengths, metadata=cut)
+    assert eng._decode.last_num_split == (B + 17) / B
+    eng.decode_varlen(q, k, v, lengths, metadata=twice)
+    assert eng._decode.last_num_split == twice["n_slots"] / B
