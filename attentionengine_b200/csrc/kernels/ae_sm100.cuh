@@ -664,3 +664,14 @@ AE_DEVICE void scan_segment_sum(float (&acc)[32], const float* state, const floa
   }
 }
 AE_DEVICE u32 tile_off(u32 r, u32 col, u32 rows) { return (col >> 6) * (rows * 128) + swz128(r, (col & 63) >> 3); }
+// Merges of split-KV results, lane k holding split k's weight and final row scales: the splits without a kept key, one bit each.  Their
+// weight is 0 and a row scale (a log-sum-exp, a row maximum) is -inf; their partial is 0 / 0 and left out.  The weight alone
+// does not tell: a split far below the others has the weight 0 as well, and an infinity among its values belongs in the result
+// as it would in one pass over all keys (0 * inf).
+template <int N>
+AE_DEVICE u32 ae_empty_splits(const float (&fr)[N], float w) {
+  bool no_key = false;
+#pragma unroll
+  for (int i = 0; i < N; ++i) no_key |= fr[i] == -__int_as_float(0x7f800000);
+  return __ballot_sync(0xffffffffu, no_key && w == 0.f);
+}

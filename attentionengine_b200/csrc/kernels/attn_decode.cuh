@@ -462,11 +462,12 @@ extern "C" __global__ void __launch_bounds__(AE_NTHREADS, 1) ae_attn_decode(cons
         for (int k = 0; k < 8; ++k) v[k] = k < n ? ld_cluster_f32(mapa_u32(part + 4 * (x * AE_DV + d), k)) : 0.f;
         float w = ae_combine(fr);
         if ((int)lane >= n) w = 0.f;
+        const u32 empty = AE_NFINAL > 0 ? ae_empty_splits(fr, w) : 0u;
         float acc = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const float wk = __shfl_sync(0xffffffffu, w, k);
-          if (k < n && wk != 0.f) acc += wk * v[k];  // a split without a kept key weighs nothing, whatever it holds
+          if (k < n && !(empty >> k & 1u)) acc += wk * v[k];
         }
         const int h = args.gq > 1 ? unit * args.gq + x : unit, q = args.gq > 1 ? 0 : x;
         ((u16*)args.o)[(i64)b * args.o_sb + (i64)q * args.o_ss + (i64)h * args.o_sh + d] = (u16)(pack2<AE_BF16>(acc, 0.f) & 0xffffu);

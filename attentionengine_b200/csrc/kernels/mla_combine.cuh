@@ -32,6 +32,7 @@ AE_DEVICE void ae_combine_heads(const AeMlaCombineArgs& args, int h0, int n_spli
   const int b = blockIdx.y;
   const i64 my_slot = lane == 0 ? slot0 : slot1 + (lane - 1) * step;
   float fr[HPT][AE_NFINAL > 0 ? AE_NFINAL : 1], w[HPT];
+  u32 empty[HPT];  // splits without a kept key
 #pragma unroll
   for (int e = 0; e < HPT; ++e) {
     const int x = h0 + e < args.H ? in_slot + e : in_slot;
@@ -50,6 +51,7 @@ AE_DEVICE void ae_combine_heads(const AeMlaCombineArgs& args, int h0, int n_spli
 #endif
     w[e] = ae_combine(fr[e]);
     if (lane >= n_split) w[e] = 0.f;
+    empty[e] = AE_NFINAL > 0 ? ae_empty_splits(fr[e], w[e]) : 0u;
   }
   const int d0 = (threadIdx.x % AE_CMB_TPH) * 4;
   const bool active = d0 < AE_DV;
@@ -75,7 +77,7 @@ AE_DEVICE void ae_combine_heads(const AeMlaCombineArgs& args, int h0, int n_spli
 #pragma unroll
       for (int e = 0; e < HPT; ++e) {
         const float wk = __shfl_sync(0xffffffffu, w[e], (k0 + j) & 31);
-        if (k0 + j >= n_split || wk == 0.f) continue;  // a split without a kept key weighs nothing, whatever it holds
+        if (k0 + j >= n_split || (empty[e] >> ((k0 + j) & 31) & 1u)) continue;
         acc[e].x += wk * v[e][j].x;
         acc[e].y += wk * v[e][j].y;
         acc[e].z += wk * v[e][j].z;
