@@ -172,9 +172,9 @@ class LinearAttentionEngine:
 
     def _build_segments(self, dv: int):
         """What the segments of a sequence add to the state, for scans of too few walks to fill the GPU."""
-        stages = 2 if dv == 64 else 1
+        stages = 2
         pre = f"#define AE_BF16 {int(self._bf16)}\n#define AE_LIN_DV {dv}\n#define AE_LIN_STAGES {stages}\n"
-        smem = stages * (128 * 128 * 2 + 128 * dv * 2) + 256 + 1024  # two CTAs per SM
+        smem = stages * (128 * 128 * 2 + 128 * 64 * 2) + 256 + 1024  # 64 value dims a CTA, two CTAs per SM
         cfg = rt.KernelConfig(kind=rt.KIND_LINEAR_SEGMENTS, dtype=rt.DTYPE_BF16 if self._bf16 else rt.DTYPE_F16, head_dim=128,
                               head_dim_v=dv, threads=192, smem_bytes=smem, stages=stages, mask_mode=0)
         return rt.compile_module(rt.kernel_source("linear_segments.cuh", prelude=pre), "ae_linear_segments", cfg)

@@ -654,7 +654,7 @@ struct ScanPlan : Plan {
 // 8 walks of 64 chunks 195 -> 30 (16 segments), 48 of 56 173 -> 93 (3), 320 of 24 (more walks than SMs) 227 uncut, 231 in two.
 // Only without gradients: a segment's start is a sum of fp32 states in another order than the walk's, and a training step's results
 // do not depend on how many heads and rows run beside, bit for bit.
-int seg_chunks(const ScanPlan& plan, int64_t walks, int64_t n, int device) {
+int seg_chunks(const ScanPlan& plan, int64_t walks, int64_t n, int64_t dv, int device) {
   if (plan.segments) return (int)((n + plan.segments - 1) / plan.segments);
   int sms = 0;
   C10_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
@@ -664,7 +664,7 @@ int seg_chunks(const ScanPlan& plan, int64_t walks, int64_t n, int device) {
   double least = rounds(walks, sms) * (n * chunk_us + 5);
   for (int64_t p = 2; p <= std::min<int64_t>(n, 16); ++p) {
     const int64_t len = (n + p - 1) / p, cut = (n + len - 1) / len;
-    const double t = rounds(walks * cut, sms) * (len * chunk_us + 5 + 0.25 * cut) + rounds(walks * (cut - 1), 2 * sms) * (len * 1.3 + 3) + 3;
+    const double t = rounds(walks * cut, sms) * (len * chunk_us + 5 + 0.25 * cut) + rounds(walks * (dv / 64) * (cut - 1), 2 * sms) * (len * 1.3 + 3) + 3;
     if (t < least) least = t, best = len;
   }
   return (int)best;
@@ -679,7 +679,7 @@ struct Segments {
   Segments(const ScanPlan& plan, py::handle eng, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& asc, const Tensor& vscale, uint32_t* status) {
     const int64_t B = v.size(0), H = v.size(1), T = v.size(2), DV = v.size(3), n = (T + 127) / 128;
     if (n < 2) return;
-    chunks = seg_chunks(plan, B * H, n, v.device().index());
+    chunks = seg_chunks(plan, B * H, n, DV, v.device().index());
     count = (int)((n + chunks - 1) / chunks);
     if (count == 1) return;
     void* const& kernel = DV == 64 ? plan.seg64 : plan.seg128;

@@ -1150,7 +1150,7 @@ int ae_launch_linear_segments(void* module, const AeLinearSegParams* p, void* st
   a.B = p->B; a.H = p->H; a.HK = p->HK; a.T = p->T;
   a.seg_state = p->seg_state; a.seg_decay = p->seg_decay;
   a.status = p->status;
-  return launch(m, (unsigned)p->H, (unsigned)p->B, (unsigned)(n_seg - 1), &a, stream);
+  return launch(m, (unsigned)(p->H * (DV / 64)), (unsigned)p->B, (unsigned)(n_seg - 1), &a, stream);  // 64 value dims each
 }
 
 int ae_launch_linear_fwd(void* module, const AeLinearParams* p, void* stream) {

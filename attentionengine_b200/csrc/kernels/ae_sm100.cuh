@@ -652,7 +652,7 @@ AE_DEVICE void scan_segment_sum(float (&acc)[32], const float* state, const floa
 #pragma unroll 2
   for (int j = 0; j < n; ++j) {
     const float4* src = (const float4*)(state + (slot + j) * slot_floats) + cc * 8 * 128 + r;
-    const float dec = ae_exp(decay[slot + j]);
+    const float dec = j > 0 ? ae_exp(decay[slot + j]) : 0.f;  // nothing in front of the first segment
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const float4 l = src[e * 128];
