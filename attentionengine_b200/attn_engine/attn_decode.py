@@ -22,8 +22,6 @@ positions.
 """
 from __future__ import annotations
 
-import threading
-
 import torch
 
 from .. import runtime as rt
@@ -31,7 +29,6 @@ from ..lower.cuda_lower import lower_attention, lower_combine
 
 N_SM = 148
 MAX_ROWS = 256  # two 128-row tiles per CTA
-_CUT_LOCK = threading.Lock()
 
 
 class AttnDecode:
@@ -64,8 +61,7 @@ class AttnDecode:
         self.kernel = rt.compile_module(self.src, "ae_attn_fwd", cfg)
         self.combine = None
         self.combine_src = None
-        self._cut_parts = None  # prelude, traced combine and configuration of the kernel for intervals and clusters
-        self._cut_kernel = None
+        self.cut_kernel = None  # for intervals and clusters
         from .attn_engine import OnlineFunc
         overridden = getattr(type(online_func), "combine", None) is not OnlineFunc.combine
         # OnlineFunc.combine left at its default gives every split the weight 1: right for online functions without
@@ -73,9 +69,9 @@ class AttnDecode:
         if overridden or not self.low.final_names:
             functor = lower_combine(online_func)
             if functor is not None:
-                if nq == 1:
-                    cut_cfg = rt.KernelConfig.from_buffer_copy(bytes(cfg))
-                    self._cut_parts = (prelude, functor, cut_cfg)
+                if nq == 1:  # built here like the others: lengths decide at run time, and a serving call should not wait for a compiler
+                    cut_src = rt.kernel_source("attn_decode.cuh", prelude=prelude).replace("//%%AE_COMBINE_FUNCTOR%%", functor)
+                    self.cut_kernel = rt.compile_module(cut_src, "ae_attn_decode", rt.KernelConfig.from_buffer_copy(bytes(cfg)))
                 comb = (rt.KERNEL_DIR / "mla_combine.cuh").read_text().replace("//%%AE_COMBINE_FUNCTOR%%", functor)
                 head = (rt.KERNEL_DIR / "ae_sm100.cuh").read_text().replace("#pragma once\n", "") + \
                     (rt.KERNEL_DIR / "ae_args.h").read_text()
@@ -119,7 +115,7 @@ class AttnDecode:
             c = -(-units * n // N_SM) * (tps + 3)
             if cost is None or c < cost:
                 best, cost = (n, False), c
-        if best[0] > 1 and self._cut_parts is not None:
+        if best[0] > 1 and self.cut_kernel is not None:
             for n in range(2, min(4, n_tiles) + 1):
                 tps = -(-n_tiles // n)
                 if (n - 1) * tps < n_tiles and tps <= 8 and units * n <= 128 and tps + 3 - 1.5 < cost:
@@ -128,15 +124,6 @@ class AttnDecode:
             self._splits.clear()
         self._splits[B, n_tiles] = best
         return best
-
-    def _load_cut_kernel(self):
-        if self._cut_kernel is None:
-            prelude, functor, cfg = self._cut_parts
-            src = rt.kernel_source("attn_decode.cuh", prelude=prelude).replace("//%%AE_COMBINE_FUNCTOR%%", functor)
-            with _CUT_LOCK:  # what a thread has handed to the plan is not replaced by another thread's build
-                if self._cut_kernel is None:
-                    self._cut_kernel = rt.compile_module(src, "ae_attn_decode", cfg)
-        self._native_plan().cut = self._cut_kernel.handle.value
 
     # ------------------------------------------------------------------------------------------------------
     # rows of different lengths
@@ -188,7 +175,7 @@ class AttnDecode:
         64 rows up to 8192 keys over 8 units (144 CTAs) 216 / 189; 16 rows of 4096 over 80 units (80 CTAs) 436 / 659; 64 of 4096 over 32
         units (128 CTAs) 670 / 704; 4 rows up to 8192 over 1 unit 17 / 21; 6 rows of 16384 over 48 units of 64 dims 277 / 329."""
         n, total, units = N_SM // self.units, int(tiles.sum()), self.units
-        if self._cut_parts is None or n == 0 or B == 1 or total < 16 * B:
+        if self.cut_kernel is None or n == 0 or B == 1 or total < 16 * B:
             return 0
         size = (self.D + self.DV) / 256
         together = 0.0101 * size * total * units
@@ -213,7 +200,8 @@ class AttnDecode:
             from .attn_engine import custom_slots
             self._plan = rt.host().DecodePlan(self.kernel.handle.value, self.combine.handle.value if self.combine else 0,
                                               self.dtype == torch.bfloat16, self.Hq, self.Hkv, self.Sq, self.D, self.DV,
-                                              len(self.low.final_names), custom_slots(self.low.custom))
+                                              len(self.low.final_names), custom_slots(self.low.custom),
+                                              self.cut_kernel.handle.value if self.cut_kernel else 0)
         return self._plan
 
     @property
@@ -228,11 +216,9 @@ class AttnDecode:
             m = None
         else:
             # the work list serves any engine, intervals only one with the head units they were counted for and the kernel for them
-            cut = meta.get("intervals", 0) if self._cut_parts is not None and meta.get("units") == self.units else 0
+            cut = meta.get("intervals", 0) if self.cut_kernel is not None and meta.get("units") == self.units else 0
             n_split, in_cluster = 1, False
             m = (meta["work"], meta["n_items"], meta["seqlens"], meta["part_off"], meta["n_slots"], meta["max_seqlen"], meta["B"])
-        if (cut or in_cluster) and (self._plan is None or not self._plan.cut):
-            self._load_cut_kernel()
         o = rt.host().decode(self._plan or self._native_plan(), q, k, v, custom, n_split, m, block_table, cut, in_cluster)
         if o is None:
             self._refuse(q, k, v, custom, meta, block_table, n_split)

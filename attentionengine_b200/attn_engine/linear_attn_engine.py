@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 
 import torch
 
@@ -34,6 +35,7 @@ LIN_DECAY_SCALE = 1  # a decay mod `decay * c[heads]` inside the scan kernels of
 LIN_BWD_MODS = 1  # the row scale of v and the skip term inside the reverse pass (0: a streaming kernel after it)
 LIN_BWD_NWG = 2  # row warpgroups of the reverse pass of the scan (measured: 4.05 against 4.33 ms at cfg4)
 
+_BUILD_LOCK = threading.Lock()
 _DIM_POS = {"batch": 0, "heads": 1, "seq_len": 2}
 
 
@@ -151,6 +153,11 @@ class LinearAttentionEngine:
         self._dv_block = self.DV if self.DV in (64, 128) else (128 if self.DV % 128 == 0 else 64)
         self.fwd, self.tl_code = self._fwd_kernel(self._dv_block)
         self._block = self._block_operands()
+        # What a scan of this size without gradients takes is built here, not in the first call; other lengths and batches than
+        # the engine was made for build theirs when they first need them.
+        walks, n = self.B * self.H * (self.DV // self._dv_block), -(-self.T // 128)
+        if rt.host().best_seg_chunks(walks, n, self._dv_block, 148) < n:
+            self._segment_kernels(self._dv_block, self._block is not None)
         self._decay_factor = None
         if "decay" in self._traced:
             self._decay_factor = self._factor(self._traced["decay"][1], self._traced["decay"][0], ("heads",))
@@ -162,13 +169,17 @@ class LinearAttentionEngine:
 
     def _load_segment_kernels(self, dv: int, mods: bool):
         """Called by the native path before the first scan over a sequence cut into segments."""
+        parts, scan = self._segment_kernels(dv, mods)
         plan = self._plan
-        # setdefault: what a thread has handed to the plan is not replaced by another thread's build
-        parts = self._cut_kernels.get(dv) or self._cut_kernels.setdefault(dv, self._build_segments(dv))
         setattr(plan, f"seg{dv}", parts.handle.value)
-        scan = self._cut_kernels.get((dv, mods)) or self._cut_kernels.setdefault((dv, mods), self._fwd_kernel(dv, mods, cut=True)[0])
         # last: another thread that finds it set launches all of them
         setattr(plan, "fwd_mods_cut" if mods else f"fwd_cut{dv}", scan.handle.value)
+
+    def _segment_kernels(self, dv: int, mods: bool):
+        with _BUILD_LOCK:  # what a thread has handed to the plan is not replaced by another thread's build
+            if dv not in self._cut_kernels:
+                self._cut_kernels[dv] = self._build_segments(dv)
+            return self._cut_kernels[dv], self._fwd_kernel(dv, mods, cut=True)[0]
 
     def _build_segments(self, dv: int):
         """What the segments of a sequence add to the state, for scans of too few walks to fill the GPU."""

@@ -339,7 +339,7 @@ py::object attn(const std::shared_ptr<AttnPlan>& plan, py::handle eng, const Ten
 // ---------------------------------------------------------------------------------------------------- split-KV decode
 struct DecodePlan : Plan {
   void *kernel = nullptr, *combine = nullptr;
-  void* cut = nullptr;  // intervals and merges in a cluster, set when first needed
+  void* cut = nullptr;  // intervals and merges in a cluster
   int Hq = 0, Hkv = 0, Sq = 0, D = 0, DV = 0, n_final = 0;
   std::vector<Custom> custom;
 };
@@ -654,10 +654,7 @@ struct ScanPlan : Plan {
 // 8 walks of 64 chunks 195 -> 30 (16 segments), 48 of 56 173 -> 93 (3), 320 of 24 (more walks than SMs) 227 uncut, 231 in two.
 // Only without gradients: a segment's start is a sum of fp32 states in another order than the walk's, and a training step's results
 // do not depend on how many heads and rows run beside, bit for bit.
-int seg_chunks(const ScanPlan& plan, int64_t walks, int64_t n, int64_t dv, int device) {
-  if (plan.segments) return (int)((n + plan.segments - 1) / plan.segments);
-  int sms = 0;
-  C10_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+int best_seg_chunks(int64_t walks, int64_t n, int64_t dv, int sms) {
   auto rounds = [](int64_t ctas, int64_t room) { return (double)((ctas + room - 1) / room); };
   const double chunk_us = 2.95;
   int64_t best = n;
@@ -668,6 +665,13 @@ int seg_chunks(const ScanPlan& plan, int64_t walks, int64_t n, int64_t dv, int d
     if (t < least) least = t, best = len;
   }
   return (int)best;
+}
+
+int seg_chunks(const ScanPlan& plan, int64_t walks, int64_t n, int64_t dv, int device) {
+  if (plan.segments) return (int)((n + plan.segments - 1) / plan.segments);
+  int sms = 0;
+  C10_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  return best_seg_chunks(walks, n, dv, sms);
 }
 
 // Scratch of a cut and the launch that fills it; nothing with one segment.  `scan` is the plan's kernel for the other case.
@@ -959,14 +963,14 @@ PYBIND11_MODULE(_ae_host, m) {
       })) AE_HANDLE(AttnPlan, prep) AE_HANDLE(AttnPlan, fused) AE_HANDLE(AttnPlan, cast) AE_STATUS(AttnPlan);
   py::class_<DecodePlan, std::shared_ptr<DecodePlan>>(m, "DecodePlan")
       .def(py::init([](uint64_t kernel, uint64_t combine, bool bf16, int Hq, int Hkv, int Sq, int D, int DV, int n_final,
-                       py::list custom) {
+                       py::list custom, uint64_t cut) {
         auto p = std::make_shared<DecodePlan>();
-        p->kernel = handle(kernel); p->combine = handle(combine);
+        p->kernel = handle(kernel); p->combine = handle(combine); p->cut = handle(cut);
         p->dtype = bf16 ? at::kBFloat16 : at::kHalf;
         p->Hq = Hq; p->Hkv = Hkv; p->Sq = Sq; p->D = D; p->DV = DV; p->n_final = n_final;
         p->custom = customs_from(custom);
         return p;
-      })) AE_HANDLE(DecodePlan, cut) AE_STATUS(DecodePlan);
+      })) AE_STATUS(DecodePlan);
   py::class_<MlaPlan, std::shared_ptr<MlaPlan>>(m, "MlaPlan")
       .def(py::init([](uint64_t kernel, uint64_t combine, bool bf16, int n_final, int pairs) {
         auto p = std::make_shared<MlaPlan>();
@@ -992,4 +996,5 @@ PYBIND11_MODULE(_ae_host, m) {
   m.def("scan_forward", torch::wrap_pybind_function(&scan_forward));
   m.def("scan", torch::wrap_pybind_function(&scan));
   m.def("scan_block", torch::wrap_pybind_function(&scan_block));
+  m.def("best_seg_chunks", &best_seg_chunks);
 }
