@@ -234,8 +234,8 @@ def launch_bwd(eng, q, k, v, o, d_o, finals, custom, lists=None):
     batch_free = all(p.custom_stride[i][0] == 0 for i in range(rt.AE_MAX_CUSTOM))
     n_parts = _batch_parts(B, Hq, Sq, dev) if (mode == "fused" and lists is None and batch_free) else 1
     if n_parts > 1:
-        # Batch ranges on streams of their own: the HBM-bound kernels around the main one (clearing the fp32 dQ buffer,
-        # delta = rowsum(O dO), the cast of dQ) of one range run next to the tensor-bound main kernel of another
+        # Batch ranges on streams of their own: the HBM-bound kernels around the main one (the pre-pass, delta = rowsum(O dO) and
+        # the clear of the fp32 dQ buffer, and the cast of dQ) of one range run next to the tensor-bound main kernel of another
         # instead of in front of and behind the whole pass.
         acc = torch.empty(B, Sq, Hq, eng.D, dtype=torch.float32, device=dev)
         main = torch.cuda.current_stream(dev)

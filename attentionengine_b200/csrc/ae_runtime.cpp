@@ -208,9 +208,10 @@ int launch(Module* m, unsigned gx, unsigned gy, unsigned gz, void* args, void* s
 }
 
 // Launch of a kernel that may be brought up while the kernel in front of it in the stream still runs: it begins with
-// ae_grid_wait(), the kernel in front calls ae_grid_trigger() once its CTAs are up.  GQA decode of 2 rows of 1000 keys with
-// its merge brought up early: 12.3 -> 11.6 us; long rows unchanged.  The MLA merge (a block per head and row) launched so
-// cost the split kernel in front of it 2 % (391 -> 399, 39.5 -> 40.2 us) and goes the plain way.
+// ae_grid_wait(), the kernel in front calls ae_grid_trigger().  Where that call stands is measured per pair.  At the beginning, where the
+// later kernel's blocks fit beside and only wait (GQA decode of 2 rows of 1000 keys under its merge 12.3 -> 11.6 us; segments and
+// scan; pre-pass and main kernel of the backward); near the end, where they would take SMs or bandwidth from CTAs still to come
+// (the MLA merge brought up at once cost its decode kernel 2 %; the cast behind the backward's main kernel).
 int launch_after(Module* m, unsigned gx, unsigned gy, unsigned gz, void* args, void* stream) {
   Driver& d = driver();
   void* params[] = {args};

@@ -643,7 +643,6 @@ AE_DEVICE u64 umma_step_k(u64 d0, int kk, int rows) {
 AE_DEVICE u64 umma_step_mn(u64 d0, int kk) { return d0 + (u64)(kk * 128); }
 // byte offset of the 16-byte chunk `ch` of row `r` inside a [rows][128 B] swizzled block
 AE_DEVICE u32 swz128(u32 r, u32 ch) { return r * 128 + ((ch ^ (r & 7)) << 4); }
-// byte offset of element column `col` (multiple of 8) of row `r` in a tile of 64-wide blocks of `rows` rows
 // Columns cc * 32 ... of row r of the state that the first n segments leave behind them: fp32 slots [DV / 4][128] of float4, each
 // decayed by the segments after it.
 AE_DEVICE void scan_segment_sum(float (&acc)[32], const float* state, const float* decay, i64 slot, int n, int slot_floats, int cc, u32 r) {
@@ -663,6 +662,7 @@ AE_DEVICE void scan_segment_sum(float (&acc)[32], const float* state, const floa
     }
   }
 }
+// byte offset of element column `col` (multiple of 8) of row `r` in a tile of 64-wide blocks of `rows` rows
 AE_DEVICE u32 tile_off(u32 r, u32 col, u32 rows) { return (col >> 6) * (rows * 128) + swz128(r, (col & 63) >> 3); }
 // Merges of split-KV results, lane k holding split k's weight and final row scales: the splits without a kept key, one bit each.  Their
 // weight is 0 and a row scale (a log-sum-exp, a row maximum) is -inf; their partial is 0 / 0 and left out.  The weight alone

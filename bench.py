@@ -550,12 +550,13 @@ def main():
         p.B, p.Hq, p.Hkv, p.Sq, p.Skv = B, Hq, Hkv, S, S
         p.status = eng._get_status(dev).data_ptr()
         st = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-        kernels["ae_attn_bwd_prep"] = {"ms": time_call(lambda: rt.check(L.ae_launch_attn_bwd_prep(kern.prep.handle, C.byref(p), st))),
-                                       "flops": 0.0, "bytes": 2.0 * B * S * Hq * D * 2 + B * Hq * S * 4}
-        if mode == "fused":
+        if mode == "fused":  # as the operator launches them: the pre-pass clears the fp32 accumulator, inside its time
             acc = torch.empty(B, S, Hq, D, dtype=torch.float32, device=dev)
-            p.dq_accum = acc.data_ptr()
-            # the launcher clears the fp32 accumulator on the stream before the kernel: that clear is inside this time
+            p.dq_accum, p.dq_cleared = acc.data_ptr(), 1
+        kernels["ae_attn_bwd_prep"] = {"ms": time_call(lambda: rt.check(L.ae_launch_attn_bwd_prep(kern.prep.handle, C.byref(p), st))),
+                                       "flops": 0.0,
+                                       "bytes": 2.0 * B * S * Hq * D * 2 + B * Hq * S * 4 + (B * S * Hq * D * 4 if mode == "fused" else 0)}
+        if mode == "fused":
             kernels["ae_attn_bwd_fused"] = {"ms": time_call(lambda: rt.check(L.ae_launch_attn_bwd_fused(kern.fused.handle, C.byref(p), st))),
                                             "flops": 5 * gemm, "executed_flops": 5 * gemm}
             kernels["ae_attn_bwd_dq_cast"] = {"ms": time_call(lambda: rt.check(L.ae_launch_attn_bwd_dq_cast(kern.cast.handle, C.byref(p), st))),
