@@ -97,9 +97,14 @@ class AttnDecode:
     def _pick(self, B: int, Skv: int):
         """(splits, whether they merge in a cluster), by tile periods: a CTA occupies an SM alone, so the CTAs run in waves of 148,
         and each pays about three periods to fill its pipeline and write its partials (measured at B = 16: 2 splits 0.131 ms,
-        8 splits 0.139 ms).  Two to four short splits, at most one wave, are a cluster and merge in it where that is at most a
-        tile period and a half behind the split that the launch of a merge follows (clusters of eight CTAs with a whole SM's
-        shared memory each do not all fit at once: 16 of them took two rounds, 17 -> 29 us).  No empty split."""
+        8 splits 0.139 ms).  No empty split.
+
+        Up to eight short splits of few rows are a cluster and merge in it: one launch, 6.6 us of the host's time instead of
+        9.8.  The GPU takes 0.3 to 0.5 us longer than with the launch that merges, 8 to 12 us a call of up to two tiles a split, less than
+        the host needs for what surrounds it; longer splits are the GPU's time alone, and captured calls take the launch (same
+        bits, see attn_decode.cuh).  At most 16 rows a unit (64 rows: 10.3 -> 11.7 us).  All clusters at once, a whole SM's shared memory a
+        CTA: 112 CTAs in clusters of seven and eight (16 clusters of eight took two rounds, 9.8 -> 16.4 us), and up to 96 of the
+        smaller ones (32 clusters of four 12.8 -> 13.8); seven or eight splits that are more are four, of two tiles."""
         if self.combine is None:
             return 1, False
         n_tiles = -(-Skv // 128)
@@ -107,23 +112,23 @@ class AttnDecode:
         if known is not None:
             return known
         units = B * self.units
-        best, cost = (1, False), None
+        best, cost = 1, None
         for n in range(1, min(32, n_tiles) + 1):
             tps = -(-n_tiles // n)
             if (n - 1) * tps >= n_tiles:
                 continue
             c = -(-units * n // N_SM) * (tps + 3)
             if cost is None or c < cost:
-                best, cost = (n, False), c
-        if best[0] > 1 and self.cut_kernel is not None:
-            for n in range(2, min(4, n_tiles) + 1):
-                tps = -(-n_tiles // n)
-                if (n - 1) * tps < n_tiles and tps <= 8 and units * n <= 128 and tps + 3 - 1.5 < cost:
-                    best, cost = (n, True), tps + 3 - 1.5
+                best, cost = n, c
+        pick = best, False
+        n = 4 if 6 < best <= 8 and units * best > 112 else best
+        if 1 < n <= 8 and self.cut_kernel is not None and self.rows <= 16 and -(-n_tiles // n) <= 2 and \
+                units * n <= (112 if n > 6 else 96):
+            pick = n, True
         if len(self._splits) >= 4096:  # a serving loop over many batch sizes and lengths must not grow without bound
             self._splits.clear()
-        self._splits[B, n_tiles] = best
-        return best
+        self._splits[B, n_tiles] = pick
+        return pick
 
     # ------------------------------------------------------------------------------------------------------
     # rows of different lengths

@@ -121,6 +121,12 @@ bool good4(const Tensor& t, at::ScalarType dtype) {
 }
 
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+bool capturing(void* stream) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing((cudaStream_t)stream, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();  // the default stream while another one captures: the launch will say so
+  return false;
+}
 
 bool wants_grad(std::initializer_list<const Tensor*> ts) {
   if (!at::GradMode::is_enabled()) return false;
@@ -384,6 +390,7 @@ py::object decode(const std::shared_ptr<DecodePlan>& plan, const Tensor& q, cons
   } else if (k.size(0) != B) {
     return py::none();
   }
+  if (in_cluster && capturing(stream_of(q))) in_cluster = false;  // bit for bit the same, see attn_decode.cuh
   const int64_t units = P.Hq > P.Hkv ? P.Hkv : P.Hq, rows = P.Hq > P.Hkv ? P.Hq / P.Hkv : P.Sq;
   if ((intervals || in_cluster) && !P.cut) return py::none();
   if (intervals) {

@@ -10,8 +10,10 @@
 //     keys at the same time, side by side as the heads of a key lie in memory: with the units of a row one after the other the 64
 //     rows took 217.  Rows of one length are as even in plain splits and read faster there (16 rows of 8192 keys 96 us, 102 in
 //     intervals).
-//   args.in_cluster: short calls.  The splits of a unit (grid: split, unit, batch row) are the CTAs of one cluster, which leave their
-//     partials in shared memory and merge them there, without a second launch: 2 rows of 1000 keys 12.3 -> 11.3 us.
+//   args.in_cluster: short calls made one by one.  The splits of a unit (grid: split, unit, batch row) are the CTAs of one cluster,
+//     which leave their partials in shared memory and merge them there: one launch for the host instead of two (6.6 us a call instead of
+//     9.8).  The GPU itself is 0.3 to 0.5 us quicker with the launch that merges, brought up under its split kernel (2 rows of 1000 keys
+//     in four splits 10.2 us, in clusters 10.5), so captured calls take that.
 // A segment is a stretch of tiles of one row; a row inside one interval is written directly, others leave normalised fp32 partials
 // for ae_mla_combine.
 //
@@ -36,6 +38,15 @@ AE_DEVICE float ld_cluster_f32(u32 addr) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
+AE_DEVICE void ld_cluster(float (&v)[2], u32 addr) {
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "r"(addr) : "memory");
+}
+AE_DEVICE void ld_cluster(float (&v)[4], u32 addr) {
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+               : "r"(addr)
+               : "memory");
+}
 
 #define AE_BM 128
 #define AE_BN 128
@@ -53,7 +64,8 @@ AE_DEVICE float ld_cluster_f32(u32 addr) {
 #define AE_SMEM_K AE_Q_BYTES
 #define AE_SMEM_V (AE_SMEM_K + AE_STAGES * AE_K_BYTES)
 #define AE_SMEM_BAR (AE_SMEM_V + AE_STAGES * AE_V_BYTES)
-static_assert(128 * (AE_DV + AE_NFINAL) * 4 <= AE_STAGES * (AE_K_BYTES + AE_V_BYTES), "a cluster's partials lie in the K / V ring");
+#define AE_PART_LD (AE_DV + 4)  // floats from row to row of a cluster's partials: the threads of a warp, a row each, in different banks
+static_assert(128 * (AE_PART_LD + AE_NFINAL) * 4 <= AE_STAGES * (AE_K_BYTES + AE_V_BYTES), "a cluster's partials lie in the K / V ring");
 
 struct AeDecBars {
   u64 q_full, q_free;  // Q of a segment has landed; its last S GEMM has read it
@@ -391,7 +403,7 @@ extern "C" __global__ void __launch_bounds__(AE_NTHREADS, 1) ae_attn_decode(cons
       const int slot = 2 * (unit * args.n_intervals + (int)blockIdx.y) + (n_seg > 0);
       const i64 part_row = (i64)slot * args.rows + row;
       u16* orow = (u16*)args.o + (i64)b * args.o_sb + (i64)(store ? q_idx : 0) * args.o_ss + (i64)h_row * args.o_sh;
-      float* prow = args.in_cluster ? (float*)(smem + AE_SMEM_K) + (row_valid ? row : 0) * AE_DV : args.o_part + part_row * AE_DV;
+      float* prow = args.in_cluster ? (float*)(smem + AE_SMEM_K) + (row_valid ? row : 0) * AE_PART_LD : args.o_part + part_row * AE_DV;
       // tcgen05.ld is warp-collective: every lane of the warp runs it; only the stores are per-row.
       if ((int)(warp * 32) < args.rows) {
 #pragma unroll
@@ -426,7 +438,7 @@ extern "C" __global__ void __launch_bounds__(AE_NTHREADS, 1) ae_attn_decode(cons
 #pragma unroll
         for (int i = 0; i < AE_NFINAL; ++i) {
           if (args.in_cluster)
-            ((float*)(smem + AE_SMEM_K))[args.rows * (AE_DV + i) + (int)row] = fr[i];
+            ((float*)(smem + AE_SMEM_K))[args.rows * (AE_PART_LD + i) + (int)row] = fr[i];
           else
             args.fr_part[i][part_row] = fr[i];
         }
@@ -443,34 +455,45 @@ extern "C" __global__ void __launch_bounds__(AE_NTHREADS, 1) ae_attn_decode(cons
   }
 
   if (args.in_cluster) {
-    // ---- the unit's splits meet: lane k holds what split k left (see mla_combine.cuh), 32 value dims of a row per warp ----
+    // ---- the unit's splits meet: lane k holds what split k left (see mla_combine.cuh), a row per warp, all
+    // its dims at once: with 32 of them per step, a unit of 8 rows in two splits was four steps of two trips to other SMs each, and
+    // with the threads' rows 512 bytes apart their stores met in one bank (8 rows of 256 keys 9.98 -> 7.6 us, 8 units of 1000 keys
+    // 10.24 -> 10.16).  Bit for bit what the launch that merges gives for the same splits. ----
     __syncthreads();  // the producer's and the issuer's warps whole again
     cluster_sync_all();
     if (warp < 4) {
+      constexpr int VEC = AE_DV / 32;  // dims of a lane
       const int n = args.n_split, b = (int)blockIdx.z;
       const u32 part = smem_u32(smem + AE_SMEM_K);
-      for (int item = (int)(cluster_ctarank() * 4 + warp); item < args.rows * (AE_DV / 32); item += n * 4) {
-        const int x = item / (AE_DV / 32), d = item % (AE_DV / 32) * 32 + (int)lane;
+      for (int x = (int)(cluster_ctarank() * 4 + warp); x < args.rows; x += n * 4) {
         float fr[AE_NFINAL > 0 ? AE_NFINAL : 1];
 #pragma unroll
         for (int i = 0; i < AE_NFINAL; ++i) {
-          const float far = ld_cluster_f32(mapa_u32(part + 4 * (args.rows * (AE_DV + i) + x), (int)lane < n ? lane : 0));
+          const float far = ld_cluster_f32(mapa_u32(part + 4 * (args.rows * (AE_PART_LD + i) + x), (int)lane < n ? lane : 0));
           fr[i] = (int)lane < n ? far : -__int_as_float(0x7f800000);
         }
-        float v[8];
+        float v[8][VEC];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = k < n ? ld_cluster_f32(mapa_u32(part + 4 * (x * AE_DV + d), k)) : 0.f;
+        for (int k = 0; k < 8; ++k)
+          if (k < n) ld_cluster(v[k], mapa_u32(part + 4 * (x * AE_PART_LD + (int)lane * VEC), k));
         float w = ae_combine(fr);
         if ((int)lane >= n) w = 0.f;
         const u32 empty = AE_NFINAL > 0 ? ae_empty_splits(fr, w) : 0u;
-        float acc = 0.f;
+        float acc[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const float wk = __shfl_sync(0xffffffffu, w, k);
-          if (k < n && !(empty >> k & 1u)) acc += wk * v[k];
+          if (k < n && !(empty >> k & 1u)) {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[e] += wk * v[k][e];
+          }
         }
         const int h = args.gq > 1 ? unit * args.gq + x : unit, q = args.gq > 1 ? 0 : x;
-        ((u16*)args.o)[(i64)b * args.o_sb + (i64)q * args.o_ss + (i64)h * args.o_sh + d] = (u16)(pack2<AE_BF16>(acc, 0.f) & 0xffffu);
+        u32* dst = (u32*)((u16*)args.o + (i64)b * args.o_sb + (i64)q * args.o_ss + (i64)h * args.o_sh + lane * VEC);
+#pragma unroll
+        for (int e = 0; e < VEC; e += 2) dst[e / 2] = pack2<AE_BF16>(acc[e], acc[e + 1]);
       }
     }
     cluster_sync_all();  // no CTA leaves while another reads its shared memory
