@@ -657,8 +657,9 @@ struct ScanPlan : Plan {
 // the walks on the fullest SM; segments shorten the chain and fill idle SMs, at the price of a launch that computes what
 // every segment but one adds to the state (two CTAs per SM) and of summing those in front of a segment.  Microseconds as
 // measured on a B200 over 1 to 16 segments: a CTA of the scan 5 + 2.95 per chunk + 0.25 per segment, one of the
-// contributions 3 + 1.3 per chunk, 3 for the second launch.  One walk against the best cut:
-// 8 walks of 64 chunks 195 -> 30 (16 segments), 48 of 56 173 -> 93 (3), 320 of 24 (more walks than SMs) 227 uncut, 231 in two.
+// contributions (64 value dims) 3 + 1.3 per chunk, 3 for the second launch.  One walk against the cut, microseconds a call among
+// others: 8 walks of 64 chunks 154 -> 30 (16 segments), 48 of 56 140 -> 90 (6), 32 of 64 with 128 value dims 224 -> 93 (4), 320 of 24
+// (more walks than SMs) 227 uncut, 231 in two.
 // Only without gradients: a segment's start is a sum of fp32 states in another order than the walk's, and a training step's results
 // do not depend on how many heads and rows run beside, bit for bit.
 int best_seg_chunks(int64_t walks, int64_t n, int64_t dv, int sms) {
