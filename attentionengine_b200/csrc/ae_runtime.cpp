@@ -849,9 +849,10 @@ int ae_launch_mla_combine(void* module, const AeMlaParams* p, void* stream) {
   a.B = p->B; a.H = p->H; a.DV = 512; a.n_split = p->n_split;
   if (p->n_split == 0) a.row_info = p->row_info;
   a.lse_out = p->lse_out;
-  // more blocks than fit at a time (64 registers a thread: 8 an SM): four heads by a thread (114 rows of 16 heads: 103.0 -> 100.2 us
-  // of the call)
-  a.heads_per_thread = p->B * p->H > 148 * 8 ? 4 : 1;
+  // Two rounds of blocks (64 registers a thread: 8 an SM) or more: four heads by a thread.  Fewer are faster with one, which has eight
+  // splits in flight instead of four: 10 rows of 6000 keys and 128 heads 31.6 us, 34.4 with four heads; 114 x 3418 with 16 heads 97.5,
+  // 98.5; 36 x 4000 with 64 heads (2304 blocks) 47.6, 47.1.
+  a.heads_per_thread = p->B * p->H > 148 * 16 ? 4 : 1;
   return launch_after(m, combine_blocks((p->H + a.heads_per_thread - 1) / a.heads_per_thread, 512), (unsigned)p->B, 1, &a, stream);
 }
 

@@ -432,7 +432,7 @@ extern "C" __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) a
       const bool all_ok = __all_sync(0xffffffffu, ok);
       const int h_first = (int)(rank * 64 + (warp & 1) * 32);  // head of this warp's first row
       // One chunk's code for all eight: unrolled, they were instructions fetched anew for every segment (microseconds, unrolled ->
-      // not: 40 rows of 2000 keys and 128 heads 45.4 -> 42.9, 16 heads 37.1 -> 33.7, 114 x 3418 and 16 heads 103.2 -> 100.2).
+      // not: 40 rows of 2000 keys and 128 heads 45.4 -> 42.9, 16 heads 37.1 -> 33.7).
       const int n_out = h_first < args.H ? 8 : 0;  // a warp without a head of the call has nothing to write
 #pragma unroll 1
       for (int c = 0; c < n_out; ++c) {
